@@ -100,8 +100,8 @@ int dst_create(int device, dst_handle** out) {
 int dst_destroy(dst_handle* h) {
     if (!h) return DST_OK;
     DeviceGuard g(h->device);
-    cudaFree(h->nodes); cudaFree(h->quads); cudaFree(h->leaf_gid); cudaFree(h->leaf_parent); cudaFree(h->arrive);
-    cudaFree(h->node_parent); cudaFree(h->node_first); cudaFree(h->node_count); cudaFree(h->child_cost);
+    cudaFree(h->nodes); cudaFree(h->quads); cudaFree(h->leaf_parent); cudaFree(h->arrive);
+    cudaFree(h->node_parent);
     cudaFree(h->keys); cudaFree(h->keys_alt); cudaFree(h->vals); cudaFree(h->vals_alt); cudaFree(h->block_hist);
     cudaFree(h->header); cudaFree(h->status); cudaFree(h->cache); cudaFree(h->arena); cudaFree(h->cam_dev);
     if (h->log_needed_host) cudaFreeHost(h->log_needed_host);
@@ -210,7 +210,7 @@ int dst_bvh_info(const dst_handle* h, int64_t* surfels, int64_t* nodes, int64_t*
     if (!h) return DST_E_ARG;
     if (surfels) *surfels = h->built ? h->P : 0;
     if (nodes) *nodes = h->built ? (h->P > 1 ? h->P - 1 : 1) : 0;
-    if (device_bytes) *device_bytes = h->cap * (64 + 48 + 4 + 4 + 4 + 16 + 8 + 20) + h->hist_cap * 1024 + h->cache_cap * 64 + h->arena_cap * 4 * DST_ARENA_FLOATS +
+    if (device_bytes) *device_bytes = h->cap * (64 + 64 + 4 + 4 + 4 + 24) + h->hist_cap * 1024 + h->cache_cap * 64 + h->arena_cap * 4 * DST_ARENA_FLOATS +
                                       h->wf_cap * (long long)(h->wf_state_bytes + 32 + 8 * DST_CHUNK + 4 + 8 + 4 + 4);
     return DST_OK;
 }
@@ -291,14 +291,14 @@ int dst_debug_round_counts(dst_handle* h, int32_t* counts, int32_t cap, void* st
     if (!h || !counts || cap < 0) return DST_E_ARG;
     if (!h->wf_counts) return dst_set_error(h, DST_E_STATE, "no trace call has run on this handle");
     DeviceGuard g(h->device);
-    const int n = cap < 50 ? cap : 50;      // DST_WF_ROUNDS + 2 list lengths
+    const int n = cap < 300 ? cap : 300;      // DST_WF_ROUNDS + 2 list lengths
     // one set of counters per slice of the last forward call (one set for every other call): the lengths add up
-    int32_t all[DST_MAX_SLICES * 100];
+    int32_t all[DST_MAX_SLICES * 300];
     const int sets = h->slices_used > 1 ? h->slices_used : 1;
-    DST_CUDA_TRY(h, cudaMemcpyAsync(all, h->wf_counts, sizeof(int32_t) * 100 * (size_t)sets, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    DST_CUDA_TRY(h, cudaMemcpyAsync(all, h->wf_counts, sizeof(int32_t) * 300 * (size_t)sets, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     DST_CUDA_TRY(h, cudaStreamSynchronize((cudaStream_t)stream));
     for (int i = 0; i < cap; i++) counts[i] = 0;
-    for (int g = 0; g < sets; g++) for (int i = 0; i < n; i++) counts[i] += all[g * 100 + i];
+    for (int g = 0; g < sets; g++) for (int i = 0; i < n; i++) counts[i] += all[g * 300 + i];
     return DST_OK;
 }
 

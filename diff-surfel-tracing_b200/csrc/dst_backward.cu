@@ -850,7 +850,7 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
                          h->log_depth == a->in.max_trace_depth;
     p.log_keys = h->log_keys; p.log_hdr = h->log_hdr; p.log_seg_head = h->log_seg_head; p.log_ray_ok = h->log_ray_ok;
     p.log_seg_stride = a->in.max_trace_depth + 1;
-    DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_counts, 0, 4 * 2 * (DST_WF_ROUNDS + 2), st));
+    DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_counts, 0, 4 * DST_COUNTS_STRIDE, st));
     h->slices_used = 1;
     const bool wave = slots >= h->wf_min_rays;
     rc = dst_live_lists(h, slots, &p.lv, st);
@@ -876,8 +876,8 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     const int g_enum = dst_wavefront_grid(h, slots, ENUM_THREADS, 10), g_shade = dst_wavefront_grid(h, slots, BWD_THREADS, 4);
     for (int r = 0; r < p.rounds; r++) {
         dst_prof_mark(h, 3, 0, st);
-        launch_gather(diag, g_enum, st, p.bvh, p.req, p.list[r & 1], p.counts + r, p.counts + DST_WF_ROUNDS + 2 + r, p.min_count, p.kbuf, p.kcnt,
-                      p.status, a->counters, r + 1, p.tiled != 0);
+        launch_gather(diag, g_enum, st, p.bvh, p.req, p.list[r & 1], p.counts + r, p.counts + r, p.min_count, p.kbuf, p.kcnt,
+                      p.status, a->counters, p.lv.tmp, p.list[(r + 1) & 1]);
         dst_prof_mark(h, 3, 1, st);
         if (dist) { if (diag) k_bwd_shade<true, true><<<g_shade, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, r); else k_bwd_shade<false, true><<<g_shade, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, r); }
         else { if (diag) k_bwd_shade<true, false><<<g_shade, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, r); else k_bwd_shade<false, false><<<g_shade, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, r); }
@@ -891,6 +891,6 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     k_unpack<<<(unsigned int)((P + 255) / 256), 256, 0, st>>>((int)P, h->arena, a->dL_drotations, a->dL_dmeans3D, a->dL_dopacities,
                                                               a->dL_dgrads3D, a->dL_dscales, a->dL_dothers, a->dL_dcolors);
     DST_CUDA_TRY(h, cudaGetLastError());
-    h->launches += 3 + (p.lv.stable ? 3 : 2) * p.rounds;       // logged re-composite or ray init, the rounds, tail, unpack
+    h->launches += 3 + (p.lv.stable ? 5 : 4) * p.rounds;       // logged re-composite or ray init, the rounds, tail, unpack
     return DST_OK;
 }

@@ -225,8 +225,7 @@ __device__ __forceinline__ int key_delta(const unsigned long long* __restrict__ 
 }
 
 __global__ void __launch_bounds__(256) k_karras(const unsigned long long* __restrict__ keys, int n, BvhNode* __restrict__ nodes,
-                                                int* __restrict__ leaf_parent, int* __restrict__ node_parent,
-                                                int* __restrict__ node_first, int* __restrict__ node_count) {
+                                                int* __restrict__ leaf_parent, int* __restrict__ node_parent) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     const unsigned long long ki = keys[i];
@@ -249,49 +248,19 @@ __global__ void __launch_bounds__(256) k_karras(const unsigned long long* __rest
     int c0, c1;
     if (lo == gamma) { c0 = ~gamma; leaf_parent[gamma] = i; } else { c0 = gamma; node_parent[gamma] = i; }
     if (hi == gamma + 1) { c1 = ~(gamma + 1); leaf_parent[gamma + 1] = i; } else { c1 = gamma + 1; node_parent[gamma + 1] = i; }
-    nodes[i].c0 = c0; nodes[i].c1 = c1;
-    node_first[i] = lo; node_count[i] = hi - lo + 1;
+    nodes[i].child[0].c = c0; nodes[i].child[1].c = c1;
     if (i == 0) node_parent[0] = -1;
 }
 
 // single-surfel scene: one node whose second child is an empty box
-__global__ void k_single_leaf(BvhNode* nodes, int* leaf_parent, int* node_parent, int* node_first, int* node_count, unsigned int* arrive) {
-    nodes[0].c0 = ~0; nodes[0].c1 = ~0; node_parent[0] = -1; node_first[0] = 0; node_count[0] = 1;
-    nodes[0].t0 = DST_LEAF_LINK(0, 1); nodes[0].t1 = DST_LEAF_LINK(0, 1);
-    for (int a = 0; a < 3; a++) { nodes[0].box[6 + a] = INFINITY; nodes[0].box[9 + a] = -INFINITY; }
+__global__ void k_single_leaf(BvhNode* nodes, int* leaf_parent, int* node_parent, unsigned int* arrive) {
+    nodes[0].child[0].c = ~0; nodes[0].child[1].c = ~0; node_parent[0] = -1;
+    for (int a = 0; a < 3; a++) { nodes[0].child[1].lo[a] = INFINITY; nodes[0].child[1].hi[a] = -INFINITY; }
     leaf_parent[0] = 0;
     arrive[0] = 1;      // the lone leaf acts as the second arrival
 }
 
 // ---- bottom-up pass: quad frames + leaf boxes, then boxes of all ancestors ----------------------
-// On the way up every node also gets the expected cost of walking its subtree (surface-area
-// heuristic) and decides whether the walk should treat it as ONE run of leaves: where boxes overlap
-// almost completely (large quads crossing each other) descending costs more than testing every quad.
-#ifndef DST_COST_NODE
-#define DST_COST_NODE 1.2f
-#endif
-// Cost of testing a leaf run of `count` quads, in units of one child-box test. The gather kernel tests a run of more
-// than DST_HULL_MIN quads with one quad per lane against the hull of its batch of rays (a fixed cost of a few node
-// steps for up to 32 quads) and hands only the survivors to all lanes for the exact test; shorter runs are tested
-// exactly right away. Where boxes overlap heavily (quads crossing each other in all directions) descending costs
-// far more than that and subtrees collapse into runs of up to DST_LEAF_MAX quads; where the children of a node
-// share little space (quads tiling a surface) the tree is kept down to single quads.
-#ifndef DST_RUN_FIXED
-#define DST_RUN_FIXED 3.5f
-#endif
-#ifndef DST_RUN_PER_QUAD
-#define DST_RUN_PER_QUAD 0.25f
-#endif
-#define DST_COST_QUAD 1.0f
-__device__ __forceinline__ float run_cost(int count) {
-    return count <= DST_HULL_MIN ? DST_COST_QUAD * (float)count : DST_RUN_FIXED + DST_RUN_PER_QUAD * (float)count;
-}
-__device__ __forceinline__ float box_area(const float* lo, const float* hi) {
-    const float dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
-    const float a = dx * dy + dy * dz + dz * dx;
-    return (a > 0.0f && a < INFINITY) ? a : 0.0f;
-}
-
 // The 4 corners of surfel g from its parameters, in the reference's expression order
 // (example/utils/gaussian_utils.py:176-210 with build_cov :286-296, build_scaling_rotation :273-282,
 // build_rotation :214-249): q = r / |r| in (w,x,y,z) order, tangent columns of R scaled by s_x and
@@ -338,15 +307,13 @@ __global__ void __launch_bounds__(256) k_surfel_quads(SurfelSource src, int P, i
     }
 }
 
-// Bottom-up pass over the hierarchy: leaf level from the quads, then boxes, costs and walk links of
-// every ancestor. FROM_SURFELS: the quad corners are computed from the surfel parameters here and
+// Bottom-up pass over the hierarchy: leaf level from the quads, then the boxes of every ancestor. FROM_SURFELS: the quad corners are computed from the surfel parameters here and
 // written to the caller's vertex buffer on the way (the refit then never reads the vertices).
 template <bool FROM_SURFELS>
 __global__ void __launch_bounds__(256) k_refit(const float* __restrict__ verts, SurfelSource src, int P, const unsigned int* __restrict__ vals,
                                                BvhNode* nodes, const int* __restrict__ leaf_parent, const int* __restrict__ node_parent,
-                                               const int* __restrict__ node_first, const int* __restrict__ node_count,
-                                               float* child_cost, unsigned int* arrive,
-                                               float4* __restrict__ quads, int* __restrict__ leaf_gid, float* header) {
+                                               unsigned int* arrive,
+                                               float4* __restrict__ quads, float* header) {
     const int pos = blockIdx.x * blockDim.x + threadIdx.x;
     if (pos >= P) return;
     const int gid = (int)vals[pos];
@@ -362,33 +329,27 @@ __global__ void __launch_bounds__(256) k_refit(const float* __restrict__ verts, 
         v[8] = c.x; v[9] = c.y; v[10] = c.z; v[11] = c.w;
     }
     const QuadFrame q = make_quad_frame(v);
-    quads[3 * (size_t)pos + 0] = make_float4(q.p0x, q.p0y, q.p0z, q.nx);
-    quads[3 * (size_t)pos + 1] = make_float4(q.ny, q.nz, q.wux, q.wuy);
-    quads[3 * (size_t)pos + 2] = make_float4(q.wuz, q.wvx, q.wvy, q.wvz);
-    leaf_gid[pos] = gid;
+    quads[4 * (size_t)pos + 0] = make_float4(q.p0x, q.p0y, q.p0z, q.nx);
+    quads[4 * (size_t)pos + 1] = make_float4(q.ny, q.nz, q.wux, q.wuy);
+    quads[4 * (size_t)pos + 2] = make_float4(q.wuz, q.wvx, q.wvy, q.wvz);
+    quads[4 * (size_t)pos + 3] = make_float4(__int_as_float(gid), 0.0f, 0.0f, 0.0f);
     float lo[3], hi[3];
     quad_box(v, lo, hi);
-    int child = ~pos;                           // topology id of the subtree being carried up
-    int link = DST_LEAF_LINK(pos, 1);           // how the walk reaches it
-    float cost = DST_COST_QUAD;
+    int child = ~pos;                           // link of the subtree being carried up
     int parent = leaf_parent[pos];
     // the depth of a Karras tree over 64-bit keys with index tie-breaks is below 128
     for (int guard = 0; guard < 128; guard++) {
         BvhNode* nd = nodes + parent;
-        const int slot = (nd->c0 == child) ? 0 : 1;
-        float2* dst = reinterpret_cast<float2*>(nd->box + 6 * slot);
-        dst[0] = make_float2(lo[0], lo[1]); dst[1] = make_float2(lo[2], hi[0]); dst[2] = make_float2(hi[1], hi[2]);
-        (&nd->t0)[slot] = link;
-        child_cost[2 * (size_t)parent + slot] = cost;
+        const int slot = (nd->child[0].c == child) ? 0 : 1;
+        float4* dst = reinterpret_cast<float4*>(nd->child + slot);
+        dst[0] = make_float4(lo[0], lo[1], lo[2], __int_as_float(child)); dst[1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
         __threadfence();
         if (atomicAdd(&arrive[parent], 1u) == 0u) return;      // the sibling subtree is not done yet
-        const float2* src = reinterpret_cast<const float2*>(nd->box + 6 * (1 - slot));
-        const float2 s0 = __ldcg(src), s1 = __ldcg(src + 1), s2 = __ldcg(src + 2);
-        const float sib_cost = __ldcg(child_cost + 2 * (size_t)parent + (1 - slot));
-        float slo[3] = { s0.x, s0.y, s1.x }, shi[3] = { s1.y, s2.x, s2.y };
-        const float a_me = box_area(lo, hi), a_sib = box_area(slo, shi);
-        lo[0] = fminf(lo[0], s0.x); lo[1] = fminf(lo[1], s0.y); lo[2] = fminf(lo[2], s1.x);
-        hi[0] = fmaxf(hi[0], s1.y); hi[1] = fmaxf(hi[1], s2.x); hi[2] = fmaxf(hi[2], s2.y);
+        const float4* src = reinterpret_cast<const float4*>(nd->child + (1 - slot));
+        const float4 s0 = __ldcg(src), s1 = __ldcg(src + 1);
+        const float slo[3] = { s0.x, s0.y, s0.z }, shi[3] = { s1.x, s1.y, s1.z };
+#pragma unroll
+        for (int a = 0; a < 3; a++) { lo[a] = fminf(lo[a], slo[a]); hi[a] = fmaxf(hi[a], shi[a]); }
         if (parent == 0) {
             float am = 0.0f;
 #pragma unroll
@@ -400,25 +361,17 @@ __global__ void __launch_bounds__(256) k_refit(const float* __restrict__ verts, 
             header[6] = am;
             return;
         }
-        const float a_all = box_area(lo, hi);
-        const float p_me = a_all > 0.0f ? fminf(a_me / a_all, 1.0f) : 1.0f, p_sib = a_all > 0.0f ? fminf(a_sib / a_all, 1.0f) : 1.0f;
-        const float cost_split = DST_COST_NODE + p_me * cost + p_sib * sib_cost;
-        const int count = node_count[parent];
-        const float cost_run = run_cost(count);
-        if (count <= DST_LEAF_MAX && cost_run <= cost_split) { link = DST_LEAF_LINK(node_first[parent], count); cost = cost_run; }
-        else { link = parent; cost = cost_split; }
         child = parent;
         parent = node_parent[parent];
     }
 }
 
 // plane frames back in surfel order, for tests
-__global__ void __launch_bounds__(256) k_export_frames(int P, const float4* __restrict__ quads, const int* __restrict__ leaf_gid,
-                                                       float* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_export_frames(int P, const float4* __restrict__ quads, float* __restrict__ out) {
     const int pos = blockIdx.x * blockDim.x + threadIdx.x;
     if (pos >= P) return;
-    const float4 a = quads[3 * (size_t)pos], b = quads[3 * (size_t)pos + 1], c = quads[3 * (size_t)pos + 2];
-    float* o = out + 12 * (size_t)leaf_gid[pos];
+    const float4 a = quads[4 * (size_t)pos], b = quads[4 * (size_t)pos + 1], c = quads[4 * (size_t)pos + 2];
+    float* o = out + 12 * (size_t)__float_as_int(quads[4 * (size_t)pos + 3].x);
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
     o[8] = c.x; o[9] = c.y; o[10] = c.z; o[11] = c.w;
 }
@@ -426,25 +379,20 @@ __global__ void __launch_bounds__(256) k_export_frames(int P, const float4* __re
 int ensure_capacity(dst_handle* h, int64_t P) {
     if (P <= h->cap) return DST_OK;
     // grow-only arena; the old buffers are released first (a rebuild does not need them)
-    cudaFree(h->nodes); cudaFree(h->quads); cudaFree(h->leaf_gid); cudaFree(h->leaf_parent); cudaFree(h->arrive);
-    cudaFree(h->node_parent); cudaFree(h->node_first); cudaFree(h->node_count); cudaFree(h->child_cost);
-    h->node_parent = h->node_first = h->node_count = nullptr; h->child_cost = nullptr;
+    cudaFree(h->nodes); cudaFree(h->quads); cudaFree(h->leaf_parent); cudaFree(h->arrive);
+    cudaFree(h->node_parent); h->node_parent = nullptr;
     cudaFree(h->keys); cudaFree(h->keys_alt); cudaFree(h->vals); cudaFree(h->vals_alt); cudaFree(h->block_hist);
-    h->nodes = nullptr; h->quads = nullptr; h->leaf_gid = nullptr; h->leaf_parent = nullptr; h->arrive = nullptr;
+    h->nodes = nullptr; h->quads = nullptr; h->leaf_parent = nullptr; h->arrive = nullptr;
     h->keys = h->keys_alt = nullptr; h->vals = h->vals_alt = nullptr; h->block_hist = nullptr;
     h->cap = 0; h->built = false;
     const int64_t cap = P + P / 8 + 1024;
     const int64_t nblocks = (cap + SORT_TILE - 1) / SORT_TILE;
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = cudaMalloc(&h->nodes, sizeof(BvhNode) * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->quads, 48 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->leaf_gid, 4 * cap);
+    if (e == cudaSuccess) e = cudaMalloc(&h->quads, 64 * cap);
     if (e == cudaSuccess) e = cudaMalloc(&h->leaf_parent, 4 * cap);
     if (e == cudaSuccess) e = cudaMalloc(&h->arrive, 4 * cap);
     if (e == cudaSuccess) e = cudaMalloc(&h->node_parent, 4 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->node_first, 4 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->node_count, 4 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->child_cost, 8 * cap);
     if (e == cudaSuccess) e = cudaMalloc(&h->keys, 8 * cap);
     if (e == cudaSuccess) e = cudaMalloc(&h->keys_alt, 8 * cap);
     if (e == cudaSuccess) e = cudaMalloc(&h->vals, 4 * cap);
@@ -462,7 +410,7 @@ int ensure_capacity(dst_handle* h, int64_t P) {
 
 int dst_surfel_quads_impl(dst_handle* h, const float* means, const float* scales, const float* rotations, int64_t P,
                           float* vertices, int32_t* triangles, cudaStream_t st) {
-    if (P <= 0 || P > (1ll << DST_LEAF_POS_BITS)) return dst_set_error(h, DST_E_ARG, "surfel count must be in [1, 2^26], got %lld", (long long)P);
+    if (P <= 0 || P > DST_MAX_SURFELS) return dst_set_error(h, DST_E_ARG, "surfel count must be in [1, 2^26], got %lld", (long long)P);
     if ((reinterpret_cast<uintptr_t>(vertices) & 15) || (reinterpret_cast<uintptr_t>(rotations) & 15) || (reinterpret_cast<uintptr_t>(scales) & 7) ||
         (reinterpret_cast<uintptr_t>(triangles) & 7))
         return dst_set_error(h, DST_E_ARG, "vertices and rotations must be 16-byte aligned, scales and triangles 8-byte aligned");
@@ -482,7 +430,7 @@ int dst_bvh_build_impl(dst_handle* h, const float* v, int64_t P, int rebuild, cu
     if (from_surfels && ((reinterpret_cast<uintptr_t>(rotations) & 15) || (reinterpret_cast<uintptr_t>(scales) & 7)))
         return dst_set_error(h, DST_E_ARG, "rotations must be 16-byte aligned and scales 8-byte aligned");
     if (P <= 0) return dst_set_error(h, DST_E_ARG, "vertices must hold at least one surfel (4 vertices)");
-    if (P > (1ll << DST_LEAF_POS_BITS)) return dst_set_error(h, DST_E_ARG, "at most 2^26 surfels are supported");
+    if (P > DST_MAX_SURFELS) return dst_set_error(h, DST_E_ARG, "at most 2^26 surfels are supported");
     if ((reinterpret_cast<uintptr_t>(v) & 15) != 0) return dst_set_error(h, DST_E_ARG, "vertices must be 16-byte aligned");
     if (!rebuild) {
         if (!h->built) return dst_set_error(h, DST_E_STATE, "refit (rebuild=0) requested before any build");
@@ -516,7 +464,7 @@ int dst_bvh_build_impl(dst_handle* h, const float* v, int64_t P, int rebuild, cu
             unsigned int* tv = vin; vin = vout; vout = tv;
         }
         // 8 passes: the sorted data is back in keys / vals
-        if (n > 1) k_karras<<<(n - 1 + tpb - 1) / tpb, tpb, 0, st>>>(h->keys, n, h->nodes, h->leaf_parent, h->node_parent, h->node_first, h->node_count);
+        if (n > 1) k_karras<<<(n - 1 + tpb - 1) / tpb, tpb, 0, st>>>(h->keys, n, h->nodes, h->leaf_parent, h->node_parent);
         h->P = P;
     } else if (from_surfels && !h->single_kernel_refit) {
         // measured at 3M surfels: the coalesced expansion pass (0.07 ms) plus the refit's gathered re-read of the
@@ -524,13 +472,11 @@ int dst_bvh_build_impl(dst_handle* h, const float* v, int64_t P, int rebuild, cu
         k_surfel_quads<<<grid, tpb, 0, st>>>(src, n, nullptr);
     }
     DST_CUDA_TRY(h, cudaMemsetAsync(h->arrive, 0, 4 * (size_t)(n > 1 ? n - 1 : 1), st));
-    if (n == 1) k_single_leaf<<<1, 1, 0, st>>>(h->nodes, h->leaf_parent, h->node_parent, h->node_first, h->node_count, h->arrive);
+    if (n == 1) k_single_leaf<<<1, 1, 0, st>>>(h->nodes, h->leaf_parent, h->node_parent, h->arrive);
     if (from_surfels && !rebuild && h->single_kernel_refit)
-        k_refit<true><<<grid, tpb, 0, st>>>(v, src, n, h->vals, h->nodes, h->leaf_parent, h->node_parent, h->node_first, h->node_count, h->child_cost,
-                                            h->arrive, h->quads, h->leaf_gid, h->header);
+        k_refit<true><<<grid, tpb, 0, st>>>(v, src, n, h->vals, h->nodes, h->leaf_parent, h->node_parent, h->arrive, h->quads, h->header);
     else
-        k_refit<false><<<grid, tpb, 0, st>>>(v, src, n, h->vals, h->nodes, h->leaf_parent, h->node_parent, h->node_first, h->node_count, h->child_cost,
-                                             h->arrive, h->quads, h->leaf_gid, h->header);
+        k_refit<false><<<grid, tpb, 0, st>>>(v, src, n, h->vals, h->nodes, h->leaf_parent, h->node_parent, h->arrive, h->quads, h->header);
     dst_prof_mark(h, 0, 1, st);
     DST_CUDA_TRY(h, cudaGetLastError());
     h->launches += (rebuild ? 27 + (n > 1 ? 1 : 0) : 0) + (from_surfels && (rebuild || !h->single_kernel_refit) ? 1 : 0) + (n == 1 ? 1 : 0) + 1;
@@ -540,7 +486,7 @@ int dst_bvh_build_impl(dst_handle* h, const float* v, int64_t P, int rebuild, cu
 
 int dst_export_frames_impl(dst_handle* h, float* out, cudaStream_t st) {
     if (!h->built) return dst_set_error(h, DST_E_STATE, "no hierarchy has been built");
-    k_export_frames<<<(unsigned int)((h->P + 255) / 256), 256, 0, st>>>((int)h->P, h->quads, h->leaf_gid, out);
+    k_export_frames<<<(unsigned int)((h->P + 255) / 256), 256, 0, st>>>((int)h->P, h->quads, out);
     DST_CUDA_TRY(h, cudaGetLastError());
     return DST_OK;
 }

@@ -7,36 +7,24 @@
 
 // ---------------------------------------------------------------------------------------------
 // Hierarchy layout in HBM
-//   nodes      (P-1) x 64 B : boxes of both children + child links (Aila-Laine style,
-//                             one 64-byte fetch = four 16-byte vector loads per visited node)
-//   quads      P x 48 B     : plane frame of each quad in LEAF ORDER (three 16-byte loads per test)
-//   leaf_gid   P x 4 B      : leaf position -> surfel id
-// A child link c >= 0 is an internal node, c < 0 is leaf position ~c.
+//   nodes      (P-1) x 64 B : 32 bytes per child: box and link, one 256-bit load
+//                             per child box (the walk tests one child box per lane)
+//   quads      P x 64 B     : plane frame of each quad and its surfel id in LEAF ORDER (two 256-bit loads per test)
 // ---------------------------------------------------------------------------------------------
-struct __align__(16) BvhNode {
-    float box[12];      // [0..2] lo of child 0, [3..5] hi of child 0, [6..8] lo of child 1, [9..11] hi of child 1
-    int c0, c1;         // topology of the Karras tree: child >= 0 internal node, < 0 leaf position ~c
-    int t0, t1;         // links the walk follows: >= 0 internal node, < 0 a run of leaves (DST_LEAF_* below);
-                        // a subtree whose boxes overlap so much that testing all its quads is cheaper is one run
+struct __align__(32) BvhChild {
+    float lo[3]; int c;     // box; child >= 0: internal node, < 0: the quad at leaf position ~c
+    float hi[3]; int pad;
 };
-#define DST_LEAF_FLAG 0x80000000u
-#define DST_LEAF_POS_BITS 26
-#ifndef DST_LEAF_MAX
-#define DST_LEAF_MAX 32               // most quads in one run (five count bits; the gather kernel tests a run with one quad per lane)
-#endif
-#define DST_HULL_MIN 2                 // runs of at most this many quads are tested exactly by every lane, longer ones go through the hull test first
-#define DST_LEAF_LINK(first, count) ((int)(DST_LEAF_FLAG | ((unsigned int)((count) - 1) << DST_LEAF_POS_BITS) | (unsigned int)(first)))
-#define DST_LEAF_FIRST(link) ((int)((unsigned int)(link) & ((1u << DST_LEAF_POS_BITS) - 1u)))
-#define DST_LEAF_COUNT(link) ((int)(((unsigned int)(link) >> DST_LEAF_POS_BITS) & 31u) + 1)
+struct __align__(64) BvhNode { BvhChild child[2]; };
+#define DST_MAX_SURFELS (1ll << 26)
 static_assert(sizeof(BvhNode) == 64, "node must be one 64-byte record");
 
 // header floats: [0..2] scene lo, [3..5] scene hi, [6] largest |coordinate|
 #define DST_HDR_FLOATS 8
 
 struct BvhView {
-    const float4* nodes;
-    const float4* quads;
-    const int* leaf_gid;
+    const BvhNode* nodes;
+    const float4* quads;    // 4 per quad: p0 n.x | n.yz wu.xy | wu.z wv | surfel id
     const float* header;
     int P;          // surfels = leaves
 };
@@ -61,12 +49,8 @@ struct dst_handle {
     int64_t cap;          // surfels the build buffers can hold
     BvhNode* nodes;
     float4* quads;
-    int* leaf_gid;
     int* leaf_parent;
     int* node_parent;             // -1 for the root
-    int* node_first;              // first leaf position under each node
-    int* node_count;              // leaves under each node
-    float* child_cost;            // 2 per node: expected walk cost of each child subtree (bottom-up pass)
     unsigned int* arrive;         // per-node arrival counters of the bottom-up pass
     unsigned long long *keys, *keys_alt;
     unsigned int *vals, *vals_alt;

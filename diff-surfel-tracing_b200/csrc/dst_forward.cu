@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_fwd_tail(const __grid_constant
 constexpr int WTAIL_THREADS = 128;
 template <bool DIAG>
 __global__ void __launch_bounds__(WTAIL_THREADS) k_fwd_tail_warp(const __grid_constant__ FwdParams p) {
-    __shared__ unsigned long long wstack[WTAIL_THREADS / 32][DST_WARP_STACK];
+    __shared__ WalkMem walk_mem[WTAIL_THREADS / 32];
     __shared__ unsigned long long wkeys[WTAIL_THREADS / 32][DST_CHUNK];
     constexpr unsigned int FULL = 0xffffffffu;
     const int round = first_skipped_round(p.counts, p.rounds, p.min_count);
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(WTAIL_THREADS) k_fwd_tail_warp(const __grid_co
             const float dx = __shfl_sync(FULL, q.dx, 0), dy = __shfl_sync(FULL, q.dy, 0), dz = __shfl_sync(FULL, q.dz, 0);
             const float k0 = __shfl_sync(FULL, q.kmax0, 0);
             unsigned long long key;
-            const int cnt = knearest_warp<DIAG>(p.bvh, ox, oy, oz, dx, dy, dz, k0, wstack[w], key, p.status, tc);
+            const int cnt = knearest_warp<DIAG>(p.bvh, ox, oy, oz, dx, dy, dz, k0, __ldg(p.bvh.header + 6), walk_mem[w], key, p.status, tc);
             if (lane < DST_CHUNK) wkeys[w][lane] = key;
             __syncwarp();
             bool go = false;
@@ -532,8 +532,8 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_knearest(BvhView bvh, const fl
 
 BvhView dst_bvh_view(const dst_handle* h) {
     BvhView b;
-    b.nodes = reinterpret_cast<const float4*>(h->nodes);
-    b.quads = h->quads; b.leaf_gid = h->leaf_gid; b.header = h->header; b.P = (int)h->P;
+    b.nodes = h->nodes;
+    b.quads = h->quads; b.header = h->header; b.P = (int)h->P;
     return b;
 }
 
@@ -838,8 +838,8 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
             const int g_enum = dst_wavefront_grid(h, sslots[g], ENUM_THREADS, DST_ENUM_GRID_PER_SM), g_shade = dst_wavefront_grid(h, sslots[g], SHADE_THREADS, DST_SHADE_GRID_PER_SM);
             const int g_compact = (int)((sslots[g] + DST_LIVE_BLOCK - 1) / DST_LIVE_BLOCK);
             dst_prof_mark(h, 3, 0, sst[g]);
-            launch_gather(diag, g_enum, sst[g], q.bvh, q.req, q.list[r & 1], q.counts + r, q.counts + DST_WF_ROUNDS + 2 + r, q.min_count, q.kbuf, q.kcnt,
-                          q.status, a->counters, r + 1, q.tiled != 0);
+            launch_gather(diag, g_enum, sst[g], q.bvh, q.req, q.list[r & 1], q.counts + r, q.counts + r, q.min_count, q.kbuf, q.kcnt,
+                          q.status, a->counters, q.lv.tmp, q.list[(r + 1) & 1]);
             dst_prof_mark(h, 3, 1, sst[g]);
             if (diag) k_fwd_shade<true><<<g_shade, SHADE_THREADS, 0, sst[g]>>>(q, r);
             else k_fwd_shade<false><<<g_shade, SHADE_THREADS, 0, sst[g]>>>(q, r);
@@ -866,7 +866,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     }
     dst_prof_mark(h, 1, 1, st);
     DST_CUDA_TRY(h, cudaGetLastError());
-    h->launches += (long long)nsl * (2 + (p.lv.stable ? 3 : 2) * p.rounds);       // per slice: ray init, the rounds, tail
+    h->launches += (long long)nsl * (2 + (p.lv.stable ? 5 : 4) * p.rounds);       // per slice: ray init, the rounds (three gather steps, composite, hand-over), tail
     if (wave) {
         if (!h->rounds_host) {
             if (cudaMallocHost(&h->rounds_host, 4 * (size_t)DST_COUNTS_STRIDE * DST_MAX_SLICES) != cudaSuccess) { cudaGetLastError(); h->rounds_host = nullptr; }
@@ -923,7 +923,7 @@ constexpr size_t ST_OFF_STATE = ST_OFF_CACHE + 64ull * DST_STATIC_MAX_SURFELS;  
 constexpr size_t ST_OFF_REQ = ST_OFF_STATE + sizeof(FwdState) * (size_t)DST_STATIC_MAX_RAYS;  // 32 B per ray
 constexpr size_t ST_OFF_LIST = ST_OFF_REQ + sizeof(EnumReq) * (size_t)DST_STATIC_MAX_RAYS;    // 4 B per slot
 constexpr size_t ST_OFF_COUNTS = ST_OFF_LIST + 4ull * ST_SLOTS;                               // round counters
-constexpr size_t ST_BYTES = ST_OFF_COUNTS + 4ull * 2 * (DST_WF_ROUNDS + 2) + 256;
+constexpr size_t ST_BYTES = ST_OFF_COUNTS + 4ull * DST_COUNTS_STRIDE + 256;
 }
 // In host code this name is only a handle for cudaGetSymbolAddress; kernels get the looked-up device pointer.
 static __device__ __align__(256) unsigned char g_static_scratch[ST_BYTES];
@@ -980,7 +980,7 @@ extern "C" int dst_forward_static(dst_handle* h, const dst_fwd_args* a, void* st
     p.log_keys = nullptr; p.log_hdr = nullptr; p.log_count = nullptr; p.log_seg_head = nullptr; p.log_ray_ok = nullptr;
     p.log_cap = 0; p.log_seg_stride = 0;
     // the array keeps the previous call's contents: the round counters must start at zero, everything else is rewritten
-    DST_CUDA_TRY(h, cudaMemsetAsync(p.counts, 0, 4 * 2 * (DST_WF_ROUNDS + 2), st));
+    DST_CUDA_TRY(h, cudaMemsetAsync(p.counts, 0, 4 * DST_COUNTS_STRIDE, st));
     if (a->training && a->a_weights) DST_CUDA_TRY(h, cudaMemsetAsync(a->a_weights, 0, 4 * (size_t)a->in.P, st));
     k_prepare_cache<<<(a->in.P + 255) / 256, 256, 0, st>>>(a->in.P, a->in.means3D, a->in.scales, a->in.rotations, a->in.opacities,
                                                              reinterpret_cast<float4*>(base + ST_OFF_CACHE));
@@ -999,12 +999,3 @@ extern "C" int dst_forward_static(dst_handle* h, const dst_fwd_args* a, void* st
     h->launches += 3;
     return DST_OK;
 }
-
-#ifdef DST_ROUND_STATS
-// build-time diagnostic (see dst_trace.cuh): copies and clears the per-round gather statistics of this translation unit
-extern "C" int dst_debug_round_stats(unsigned long long* out) {
-    if (cudaMemcpyFromSymbol(out, g_round_stats, sizeof(unsigned long long) * 64 * 8) != cudaSuccess) return DST_E_CUDA;
-    static unsigned long long zero[64 * 8];
-    return cudaMemcpyToSymbol(g_round_stats, zero, sizeof(zero)) == cudaSuccess ? DST_OK : DST_E_CUDA;
-}
-#endif

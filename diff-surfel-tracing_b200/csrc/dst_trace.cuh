@@ -7,21 +7,6 @@
 #define DST_STACK 96                 // >= depth bound of a Karras tree over 63-bit keys + 32-bit index tie-breaks
 #define DST_MAX_CHUNKS 4096          // bound on enumerations per ray segment (the reference loops without one)
 #define DST_MAX_INTERSECTION 256     // optix_tracer/config.h:23
-#define DST_NODE_VOTE 10                // lanes with node work needed to stay in the node phase of k_enum
-// The warp gives up walking together when fewer than this % of the lane tests are wanted. Pixel tiles: never. Measured on
-// tiled image grids (forward, 0 / 10 / 25 %): 3M-surfel reflective scene 61.6 / 62.7 / 67.1 ms, object-scale scene 9.0 / 10.7 /
-// 13.8 ms: even batches of reflected rays, whose directions have little in common, start from one small patch and find their
-// 16 nearest hits close to it. Linear ray lists (LiDAR sweeps: one origin, directions fanning out over metres of a sparse
-// scene) are the opposite case: 4.4 / 3.95 / 3.3 ms.
-#ifndef DST_SHARE_MIN_PCT_TILED
-#define DST_SHARE_MIN_PCT_TILED 0
-#endif
-#ifndef DST_SHARE_MIN_PCT_LINEAR
-#define DST_SHARE_MIN_PCT_LINEAR 25
-#endif
-#ifndef DST_SHARE_VOTE
-#define DST_SHARE_VOTE 1                // lanes that must want a subtree for the warp to walk it together (k_enum)
-#endif
 #define DST_PAD_FACTOR 4e-6f         // box padding per unit of coordinate magnitude, see knearest()
 
 struct TraceCounters { unsigned long long segs, enums, nodes, quads, evals, contribs; };
@@ -30,6 +15,29 @@ __device__ __forceinline__ unsigned long long make_key(float t, unsigned int pid
     return ((unsigned long long)__float_as_uint(t) << 32) | pidx;
 }
 __device__ __forceinline__ float hitkey_t(unsigned long long k) { return __uint_as_float((unsigned int)(k >> 32)); }
+
+// 256-bit read-only loads (one instruction per 32-byte record: what bounds the walk is the number of cache lines its load
+// instructions touch, and a record fetched in pieces touches its line once per piece)
+__device__ __forceinline__ void ldg256(const void* p, float4& lo, float4& hi) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w), "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w) : "l"(p));
+}
+__device__ __forceinline__ BvhChild load_child(const BvhView& bvh, int node, int k) {
+    float4 a, b;
+    ldg256(bvh.nodes[node].child + k, a, b);
+    BvhChild c;
+    c.lo[0] = a.x; c.lo[1] = a.y; c.lo[2] = a.z; c.c = __float_as_int(a.w);
+    c.hi[0] = b.x; c.hi[1] = b.y; c.hi[2] = b.z; c.pad = 0;
+    return c;
+}
+struct Quad { float4 a, b, c; unsigned int gid; };
+__device__ __forceinline__ Quad load_quad(const BvhView& bvh, int pos) {
+    Quad q;
+    float4 d;
+    const float4* p = bvh.quads + 4 * (size_t)pos;
+    ldg256(p, q.a, q.b); ldg256(p + 2, q.c, d);
+    q.gid = (unsigned int)__float_as_int(d.x);
+    return q;
+}
 
 // The DST_CHUNK smallest (t, primitive id) hits with 0 <= t < 1e16 from origin o, ascending, in
 // kb[0], kb[KS], kb[2 KS], ... (a column of a shared-memory array). Returns min(#hits, DST_CHUNK).
@@ -52,12 +60,11 @@ __device__ __forceinline__ int knearest(const BvhView& bvh, float ox, float oy, 
     if (bvh.P <= 0) return 0;
 
     auto offer = [&](int pos) {
-        const float4* qp = bvh.quads + 3 * (size_t)pos;
-        const float4 qa = __ldg(qp), qb = __ldg(qp + 1), qc = __ldg(qp + 2);
+        const Quad q = load_quad(bvh, pos);
         if (COUNT) tc.quads++;
         float t; int tri;
-        if (!ray_quad(qa, qb, qc, ox, oy, oz, dx, dy, dz, kmax, t, tri)) return;
-        const unsigned int gid = (unsigned int)__ldg(bvh.leaf_gid + pos);
+        if (!ray_quad(q.a, q.b, q.c, ox, oy, oz, dx, dy, dz, kmax, t, tri)) return;
+        const unsigned int gid = q.gid;
         const unsigned long long key = make_key(t, 2u * gid + (unsigned int)tri);
         if (n == DST_CHUNK && key >= kb[(DST_CHUNK - 1) * KS]) return;
         int j = n;
@@ -102,17 +109,14 @@ __device__ __forceinline__ int knearest(const BvhView& bvh, float ox, float oy, 
     for (;;) {
         // "while-while": lanes walk internal nodes until each holds a leaf (or is done), then test leaves together
         while ((unsigned int)cur < (unsigned int)DONE) {
-            const float4* np = bvh.nodes + 4 * (size_t)cur;
-            const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
-            const int4 lk = __ldg(reinterpret_cast<const int4*>(np + 3));
+            const BvhChild k0 = load_child(bvh, cur, 0), k1 = load_child(bvh, cur, 1);
             if (COUNT) tc.nodes++;
-            // child 0: lo (a.x a.y a.z) hi (a.w b.x b.y); child 1: lo (b.z b.w c.x) hi (c.y c.z c.w)
-            const float n0x = px ? a.x : a.w, f0x = px ? a.w : a.x;
-            const float n0y = py ? a.y : b.x, f0y = py ? b.x : a.y;
-            const float n0z = pz ? a.z : b.y, f0z = pz ? b.y : a.z;
-            const float n1x = px ? b.z : c.y, f1x = px ? c.y : b.z;
-            const float n1y = py ? b.w : c.z, f1y = py ? c.z : b.w;
-            const float n1z = pz ? c.x : c.w, f1z = pz ? c.w : c.x;
+            const float n0x = px ? k0.lo[0] : k0.hi[0], f0x = px ? k0.hi[0] : k0.lo[0];
+            const float n0y = py ? k0.lo[1] : k0.hi[1], f0y = py ? k0.hi[1] : k0.lo[1];
+            const float n0z = pz ? k0.lo[2] : k0.hi[2], f0z = pz ? k0.hi[2] : k0.lo[2];
+            const float n1x = px ? k1.lo[0] : k1.hi[0], f1x = px ? k1.hi[0] : k1.lo[0];
+            const float n1y = py ? k1.lo[1] : k1.hi[1], f1y = py ? k1.hi[1] : k1.lo[1];
+            const float n1z = pz ? k1.lo[2] : k1.hi[2], f1z = pz ? k1.hi[2] : k1.lo[2];
             const float tn0 = fmaxf(fmaxf(fmaf(n0x, ix, -onx), fmaf(n0y, iy, -ony)), fmaxf(fmaf(n0z, iz, -onz), 0.0f));
             const float tf0 = fminf(fminf(fmaf(f0x, ix, -ofx), fmaf(f0y, iy, -ofy)), fmaf(f0z, iz, -ofz));
             const float tn1 = fmaxf(fmaxf(fmaf(n1x, ix, -onx), fmaf(n1y, iy, -ony)), fmaxf(fmaf(n1z, iz, -onz), 0.0f));
@@ -121,20 +125,17 @@ __device__ __forceinline__ int knearest(const BvhView& bvh, float ox, float oy, 
             const bool h1 = (tn1 <= tf1) && (tn1 <= kmax);
             if (h0 && h1) {
                 const bool swap = tn1 < tn0 || (tn1 == tn0 && tf1 < tf0);      // entered first; on a tie (inside both boxes) left first
-                const int cf = swap ? lk.z : lk.w;
+                const int cf = swap ? k0.c : k1.c;
                 const float tfar = swap ? tn0 : tn1;
                 if (sp < DST_STACK) stack[sp++] = ((unsigned long long)__float_as_uint(tfar) << 32) | (unsigned int)cf;
                 else atomicOr(status, DST_STATUS_STACK_OVERFLOW);
-                cur = swap ? lk.w : lk.z;
-            } else if (h0) cur = lk.z;
-            else if (h1) cur = lk.w;
+                cur = swap ? k1.c : k0.c;
+            } else if (h0) cur = k0.c;
+            else if (h1) cur = k1.c;
             else cur = pop();
         }
         if (cur == DONE) break;
-        {   // a run of leaves: test every quad of it
-            const int first = DST_LEAF_FIRST(cur), count = DST_LEAF_COUNT(cur);
-            for (int q = 0; q < count; q++) offer(first + q);
-        }
+        offer(~cur);
         cur = pop();
     }
     return n;
@@ -279,62 +280,39 @@ constexpr int ENUM_THREADS = 128;
 #define DST_ENUM_MIN_BLOCKS 6         // resident blocks per SM the gather kernel is compiled for
 #endif
 #define DST_WF_ROUNDS 48
-#define DST_COUNTS_STRIDE (2 * (DST_WF_ROUNDS + 2))      // ints per set of round counters: list lengths, then batch cursors
+#define DST_COUNTS_STRIDE (6 * (DST_WF_ROUNDS + 2))      // ints per set of round counters: list lengths, batch cursors, rays given up by the batches, their cursor
 
-// Slab constants of one ray for the padded child-box test (see knearest()).
-struct RaySlab {
-    float ix, iy, iz, onx, ony, onz, ofx, ofy, ofz;
-    bool px, py, pz, valid;
-};
-__device__ __forceinline__ RaySlab make_slab(float ox, float oy, float oz, float dx, float dy, float dz, float absmax) {
-    RaySlab r;
-    const float omax = fmaxf(fabsf(ox), fmaxf(fabsf(oy), fabsf(oz)));
-    r.valid = omax < INFINITY;
-    const float pad = DST_PAD_FACTOR * (omax + absmax) + 1e-30f;
-    const float sdx = fabsf(dx) < 1e-20f ? copysignf(1e-20f, dx) : dx;
-    const float sdy = fabsf(dy) < 1e-20f ? copysignf(1e-20f, dy) : dy;
-    const float sdz = fabsf(dz) < 1e-20f ? copysignf(1e-20f, dz) : dz;
-    r.ix = 1.0f / sdx; r.iy = 1.0f / sdy; r.iz = 1.0f / sdz;
-    r.px = !(sdx < 0.0f); r.py = !(sdy < 0.0f); r.pz = !(sdz < 0.0f);
-    r.onx = fmaf(ox, r.ix, pad * fabsf(r.ix)); r.ofx = fmaf(ox, r.ix, -pad * fabsf(r.ix));
-    r.ony = fmaf(oy, r.iy, pad * fabsf(r.iy)); r.ofy = fmaf(oy, r.iy, -pad * fabsf(r.iy));
-    r.onz = fmaf(oz, r.iz, pad * fabsf(r.iz)); r.ofz = fmaf(oz, r.iz, -pad * fabsf(r.iz));
-    return r;
-}
-
-// Gather kernel: per live ray, the 16 nearest hits from the requested origin (same result as knearest()).
+// ---------------------------------------------------------------------------------------------
+// Gather: per live ray, the 16 nearest hits from the requested origin (same result as knearest()).
 //
-// A warp takes 32 consecutive entries of the live list: neighbouring pixels in the same stage (the lists keep their
-// tile order, see k_compact), whose rays start close to each other. Large overlapping quads put hundreds of boxes
-// around any origin, and every one of the 32 rays has to open them, so the walk is split in two:
-//   shared phase   the warp walks the hierarchy TOGETHER from the root with one stack; a node is fetched once (one
-//                  broadcast load instead of 32 scattered ones) and every lane tests its own ray against both
-//                  child boxes. A child wanted by at least DST_SHARE_VOTE lanes (1: any lane, measured best) stays
-//                  in the shared walk; a child wanted by fewer goes onto the private stacks of those lanes.
-//                  A leaf run reached here is NOT tested quad by quad by every lane: lane q fetches quad q and
-//                  decides, against the hull of the batch's rays (hull_quad), whether any ray of the batch can hit
-//                  it; only the survivors (a few of 32 for neighbouring rays) are handed round and tested exactly
-//                  by every lane. For linear ray lists only: when most lanes sit out most tests (after 64 nodes, under
-//                  share_min_pct % of the lane x test slots wanted) the warp gives the shared walk up and every lane
-//                  takes the pending subtrees onto its own stack (see DST_SHARE_MIN_PCT_TILED above).
-//   private phase  every lane drains its own stack as in knearest(), lanes alternating between a node phase (kept
-//                  while at least DST_NODE_VOTE lanes have node work) and a leaf phase.
-// Pruning uses each lane's own 16th-nearest distance throughout (before a lane has 16 hits: the bound its request carries,
-// see k_fwd_shade, or none) and the hull test is conservative, so the hit set is exactly that of an independent walk per
-// ray within that bound. Blocks are persistent and take batches from a shared cursor.
-#define DST_SHARED_STACK 64
-#define DST_ENUM_STACK 160       // private stack of k_enum: subtrees deferred by the shared walk + one depth-first descent
-#define DST_ENUM_DEFER 64        // the shared walk pauses to drain the private stacks when a lane holds this many entries
+// Large overlapping quads put hundreds of boxes around any origin: a walk for 16 hits opens 300 nodes in the dense scenes, and
+// neighbouring rays open the same ones. So a warp walks the hierarchy for the HULL of a set of rays (origins and
+// directions, component by component), and its lanes are 32 child boxes, then 32 quads, of one step, instead of 32
+// copies of nearly the same ray. Everything the hull test lets through is tested exactly, with each ray's own 16th-nearest distance;
+// the hull tests are conservative, so the hit set is that of an independent walk per ray. What a hull costs depends on how alike its rays are
+// (the hull of rays that fan out reaches quads none of them comes near), so a gather has three steps, each taking what the one before gave up:
+//   k_enum        32 consecutive live rays per warp (a pixel tile, or the survivors of neighbouring ones: the lists keep tile order, see
+//                 k_compact). Quads that pass the hull test are tested by every lane against its own ray. Given up past DST_BEAM_STEPS
+//                 steps or DST_BEAM_CANDS such quads.
+//   k_enum_group  8 rays per warp (a 4x2 patch of the tile); every lane holds one quad and tests the 8 rays in turn. Given up past DST_GROUP_STEPS.
+//   k_enum_ray    one ray per warp (the hull is the ray), one quad per lane.
+// Gather time of one forward, one launch after another (3M-surfel 1080p one-bounce scene / 6M-surfel two-bounce scene at 4 x 540 x 960), against
+// a walk in which every lane tested its own ray against each node's two boxes: 40 -> 16 ms and 250 -> 106 ms; a primary round of
+// 2.07M rays 4.0 -> 1.2 ms. Limits: half of DST_BEAM_* costs the two-bounce scene 20 ms, twice as much costs the
+// scenes with silhouettes 5-10 % (the slowest batch of a round gets longer). Groups of 4 or 16: 10-15 % slower on the two-bounce scene.
+// Runs of 2 or 4 quads as leaves of the walk: 2-9 % slower than single quads.
+// Blocks are persistent and take batches from a cursor; no block waits for another.
+// ---------------------------------------------------------------------------------------------
+#define DST_BEAM_STEPS 160
+#define DST_BEAM_CANDS 300
+#define DST_GROUP 8
+#define DST_GROUP_STEPS 192
+#define DST_GROUP_MIN_BLOCKS 8
+#define DST_WALK_STACK 320                 // one step adds at most 16 entries; see the width rule in beam_walk()
+#define DST_WALK_QUADS 64
+#define DST_WALK_STEP_LIMIT (1 << 20)      // bound on the steps of a walk that cannot be given up (status flag instead of a hang)
 // Hull of the rays of one batch (origins and directions, component by component), kept in shared memory per warp.
 struct BeamQ { float omin[3], omax[3], dmin[3], dmax[3], dabs[3], dsum; };      // dabs: largest |d| per axis, dsum: their sum
-
-__device__ __forceinline__ unsigned int f2ord_q(float f) {
-    const unsigned int u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ord2f_q(unsigned int u) { return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u); }
-__device__ __forceinline__ float wmin_f(float v) { return ord2f_q(__reduce_min_sync(0xffffffffu, f2ord_q(v))); }
-__device__ __forceinline__ float wmax_f(float v) { return ord2f_q(__reduce_max_sync(0xffffffffu, f2ord_q(v))); }
 
 // [rl, rh] += c * [lo, hi]
 __device__ __forceinline__ void ivmul(float c, float lo, float hi, float& rl, float& rh) {
@@ -385,97 +363,141 @@ __device__ __forceinline__ bool hull_quad(const BeamQ& bm, const float4 qa, cons
     return !(uh < -eu || ul > 1.f + eu || vh < -ev || vl > 1.f + ev);
 }
 
-#ifdef DST_ROUND_STATS
-// build-time diagnostic: per wavefront round [0] batches, [1] shared node steps, [2] shared quad steps, [3] private
-// node-phase warp steps, [4] private leaf-phase warp steps (quads), [5] batches that gave the shared walk up,
-// [6] lane tests wanted in the shared phase, [7] lanes active at batch start
-static __device__ unsigned long long g_round_stats[64][8];
-#define RSTAT(i, v) do { const unsigned long long v_ = (v); if (lane == 0) rs[i] += v_; } while (0)      // v may hold a warp vote: every lane evaluates it
-#else
-#define RSTAT(i, v) do { } while (0)
-#endif
+// Slab constants of the hull for the child-box test of the walk, four fused multiply-adds per axis and box. For every ray
+// of the hull, with origin in [omin, omax] and direction in [dmin, dmax] along an axis:
+//   entry  t >= (lo - omax) / dmax if the box lies ahead in +, t >= (omin - hi) / -dmin if it lies ahead in -, else t >= 0
+//   exit   t <= (hi - omin) / dmin if every ray travels in +, t <= (omax - lo) / -dmax if every ray travels in -, else unbounded
+// pa hi/lo factors and offsets are folded (entry = lo * ep + eo, hi * en + fo, ...); an impossible direction has a huge factor.
+struct BeamSlab { float4 entry[3], exit[3]; };       // (factor of lo, offset, factor of hi, offset)
+struct WalkMem {
+    unsigned long long stack[DST_WALK_STACK];        // subtrees: nearest possible t << 32 | link, nearest on top
+    unsigned long long quads[DST_WALK_QUADS];        // quads whose box the hull reaches: nearest possible t << 32 | leaf position
+    BeamSlab slab;
+    BeamQ beam;
+};
+
+// Walks the hierarchy for the hull in m.beam / m.slab: a step takes up to 16 nodes from the top of the stack and tests their 32
+// child boxes, one per lane. Single quads whose box passes go to a queue; whenever it holds 32 of them (or no node is
+// left) leaf_step(valid, position) gets one quad per lane. krun (uniform) is the largest distance any ray still searches;
+// leaf_step lowers it, and returns false to give the walk up. Returns false when given up or after max_steps steps.
+template <bool COUNT, class LeafStep>
+__device__ __forceinline__ bool beam_walk(const BvhView& bvh, WalkMem& m, float& krun, int max_steps, unsigned int* status, TraceCounters& tc, LeafStep leaf_step) {
+    constexpr unsigned int FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned int below = (1u << lane) - 1u;
+    int sp = 1, nq = 0;
+    if (lane == 0) m.stack[0] = 0ull;
+    __syncwarp();
+    for (int step = 0; step < max_steps; step++) {
+        if (nq >= 32 || sp == 0) {
+            if (nq == 0) return true;
+            const int take = nq < 32 ? nq : 32;
+            nq -= take;
+            const unsigned long long e = lane < take ? m.quads[nq + lane] : 0ull;
+            __syncwarp();
+            if (!leaf_step(lane < take && __uint_as_float((unsigned int)(e >> 32)) <= krun, (int)(unsigned int)e)) return false;
+            continue;
+        }
+        // lanes 30/31 take the top entry, lanes 28/29 the next, ...: lane order is then the order in which surviving children
+        // go back onto the stack (farthest first). A nearly full stack is walked one node at a time (it then grows by at most
+        // one entry per level of the tree).
+        const int width = sp > DST_WALK_STACK - 112 ? 1 : 16;
+        const int take = sp < width ? sp : width;
+        const int slot = 15 - (lane >> 1);
+        unsigned long long e = 0ull;
+        bool h = slot < take;
+        if (h) e = m.stack[sp - 1 - slot];
+        sp -= take;
+        __syncwarp();
+        h = h && __uint_as_float((unsigned int)(e >> 32)) <= krun;
+        float tn = 0.0f, tf = 0.0f;
+        int clink = 0;
+        if (h) {
+            if (COUNT && (lane & 1) == 0) tc.nodes++;
+            const BvhChild b = load_child(bvh, (int)(unsigned int)e, lane & 1);
+            clink = b.c;
+            const float4 ex = m.slab.entry[0], ey = m.slab.entry[1], ez = m.slab.entry[2];
+            const float4 fx = m.slab.exit[0], fy = m.slab.exit[1], fz = m.slab.exit[2];
+            tn = fmaxf(fmaxf(fmaf(b.lo[0], ex.x, ex.y), fmaf(b.hi[0], ex.z, ex.w)), 0.0f);
+            tn = fmaxf(fmaxf(fmaf(b.lo[1], ey.x, ey.y), fmaf(b.hi[1], ey.z, ey.w)), tn);
+            tn = fmaxf(fmaxf(fmaf(b.lo[2], ez.x, ez.y), fmaf(b.hi[2], ez.z, ez.w)), tn);
+            tf = fminf(fmaf(b.lo[0], fx.x, fx.y), fmaf(b.hi[0], fx.z, fx.w));
+            tf = fminf(fminf(fmaf(b.lo[1], fy.x, fy.y), fmaf(b.hi[1], fy.z, fy.w)), tf);
+            tf = fminf(fminf(fmaf(b.lo[2], fz.x, fz.y), fmaf(b.hi[2], fz.z, fz.w)), tf);
+            h = tn <= fminf(tf, krun);
+        }
+        {   // within a pair the farther child goes first (even lane), the nearer second (odd lane); nearer = entered first, on a
+            // tie (the rays start inside both boxes) left first
+            const float ptn = __shfl_xor_sync(FULL, tn, 1), ptf = __shfl_xor_sync(FULL, tf, 1);
+            const int plink = __shfl_xor_sync(FULL, clink, 1);
+            const bool ph = __shfl_xor_sync(FULL, h, 1);
+            const bool even = (lane & 1) == 0;
+            const bool mine_nearer = tn < ptn || (tn == ptn && (tf < ptf || (tf == ptf && even)));
+            if (h && ph && (even ? mine_nearer : !mine_nearer)) { tn = ptn; clink = plink; }
+        }
+        const unsigned int inner = __ballot_sync(FULL, h && clink >= 0);
+        const unsigned long long tword = (unsigned long long)__float_as_uint(tn) << 32;
+        if (sp + __popc(inner) > DST_WALK_STACK) { if (lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW); return true; }
+        if (h && clink >= 0) m.stack[sp + __popc(inner & below)] = tword | (unsigned int)clink;
+        sp += __popc(inner);
+        const unsigned int leaves = __ballot_sync(FULL, h && clink < 0);
+        if (h && clink < 0) m.quads[nq + __popc(leaves & below)] = tword | (unsigned int)~clink;
+        nq += __popc(leaves);
+        __syncwarp();
+    }
+    return false;
+}
+
+__device__ __forceinline__ float redux_min(float v) { float r; asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v)); return r; }
+__device__ __forceinline__ float redux_max(float v) { float r; asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v)); return r; }
+
+// hull of the rays of the lanes with `active` (at least one), into m.beam and m.slab
+__device__ __forceinline__ void make_beam(WalkMem& m, bool active, float ox, float oy, float oz, float dx, float dy, float dz, float absmax) {
+    const int lane = threadIdx.x & 31;
+    const float o3[3] = { ox, oy, oz }, d3[3] = { dx, dy, dz };
+    float olo[3], ohi[3], dlo[3], dhi[3], om = 0.0f;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        olo[a] = redux_min(active ? o3[a] : INFINITY); ohi[a] = redux_max(active ? o3[a] : -INFINITY);
+        dlo[a] = redux_min(active ? d3[a] : INFINITY); dhi[a] = redux_max(active ? d3[a] : -INFINITY);
+        om = fmaxf(om, fmaxf(fabsf(olo[a]), fabsf(ohi[a])));
+    }
+    if (lane < 3) {
+        const int a = lane;
+        const float ol = a == 0 ? olo[0] : a == 1 ? olo[1] : olo[2], oh = a == 0 ? ohi[0] : a == 1 ? ohi[1] : ohi[2];
+        const float dl = a == 0 ? dlo[0] : a == 1 ? dlo[1] : dlo[2], dh = a == 0 ? dhi[0] : a == 1 ? dhi[1] : dhi[2];
+        m.beam.omin[a] = ol; m.beam.omax[a] = oh; m.beam.dmin[a] = dl; m.beam.dmax[a] = dh; m.beam.dabs[a] = fmaxf(fabsf(dl), fabsf(dh));
+        // box padding as in knearest(), for the ray with the largest coordinates
+        const float pad = DST_PAD_FACTOR * (om + absmax) + 1e-30f;
+        const float lo = ol - pad, hi = oh + pad;
+        const float ip = 1.0f / fmaxf(dh, 1e-30f), in = 1.0f / fmaxf(-dl, 1e-30f);
+        m.slab.entry[a] = make_float4(ip, -hi * ip, -in, lo * in);
+        const float xp = dl > 1e-20f ? 1.0f / dl : 0.0f, xn = dh < -1e-20f ? 1.0f / dh : 0.0f;
+        m.slab.exit[a] = make_float4(xn, xn != 0.0f ? -hi * xn : 3e38f, xp, xp != 0.0f ? -lo * xp : 3e38f);
+    }
+    if (lane == 0) m.beam.dsum = fmaxf(fabsf(dlo[0]), fabsf(dhi[0])) + fmaxf(fabsf(dlo[1]), fabsf(dhi[1])) + fmaxf(fabsf(dlo[2]), fabsf(dhi[2]));
+    __syncwarp();
+}
+
+// First step of a gather: 32 consecutive entries of the live list per warp. A batch that is given up goes to `heavy` with its 32 slots, each ray
+// with the search bound it has found.
 template <bool COUNT>
-__global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhView bvh, const EnumReq* __restrict__ req, const int* __restrict__ list,
+__global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhView bvh, EnumReq* req, const int* __restrict__ list,
                                                        const int* __restrict__ count_ptr, int* cursor, int min_count,
                                                        unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
-                                                       unsigned int* status, unsigned long long* counters, int tag, int share_min_pct) {
+                                                       unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count) {
     __shared__ unsigned long long kshared[DST_CHUNK * ENUM_THREADS];
-    __shared__ int sstack[ENUM_THREADS / 32][DST_SHARED_STACK];
-    __shared__ BeamQ sbeam[ENUM_THREADS / 32];
+    __shared__ WalkMem walk_mem[ENUM_THREADS / 32];
     const int total = *count_ptr;
     if (total < min_count || bvh.P <= 0) return;
     constexpr int KS = ENUM_THREADS;
-    constexpr int DONE = 0x7fffffff;
     constexpr unsigned int FULL = 0xffffffffu;
     unsigned long long* kb = kshared + threadIdx.x;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    WalkMem& m = walk_mem[threadIdx.x >> 5];
     const float absmax = __ldg(bvh.header + 6);
     TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
-#ifdef DST_ROUND_STATS
-    unsigned long long rs[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
-#endif
-    unsigned long long stack[DST_ENUM_STACK];
-    int sp = 0, n = 0;
-    float kmax = -1.0f;
-    float ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f;
-    RaySlab sl = make_slab(0.f, 0.f, 0.f, 1.f, 1.f, 1.f, 0.f);
-
-    auto pop = [&]() -> int {
-        while (sp > 0) {
-            const unsigned long long e = stack[--sp];
-            if (__uint_as_float((unsigned int)(e >> 32)) <= kmax) return (int)(unsigned int)e;
-        }
-        return DONE;
-    };
-    auto push = [&](int link, float tn) {
-        if (sp < DST_ENUM_STACK) stack[sp++] = ((unsigned long long)__float_as_uint(tn) << 32) | (unsigned int)link;
-        else atomicOr(status, DST_STATUS_STACK_OVERFLOW);
-    };
-    // both child boxes of one node against this lane's ray
-    auto test_node = [&](int node, float& tn0, float& tn1, bool& h0, bool& h1, int& l0, int& l1, bool& near1) {
-        const float4* np = bvh.nodes + 4 * (size_t)node;
-        const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
-        const int4 lk = __ldg(reinterpret_cast<const int4*>(np + 3));
-        const float n0x = sl.px ? a.x : a.w, f0x = sl.px ? a.w : a.x;
-        const float n0y = sl.py ? a.y : b.x, f0y = sl.py ? b.x : a.y;
-        const float n0z = sl.pz ? a.z : b.y, f0z = sl.pz ? b.y : a.z;
-        const float n1x = sl.px ? b.z : c.y, f1x = sl.px ? c.y : b.z;
-        const float n1y = sl.py ? b.w : c.z, f1y = sl.py ? c.z : b.w;
-        const float n1z = sl.pz ? c.x : c.w, f1z = sl.pz ? c.w : c.x;
-        tn0 = fmaxf(fmaxf(fmaf(n0x, sl.ix, -sl.onx), fmaf(n0y, sl.iy, -sl.ony)), fmaxf(fmaf(n0z, sl.iz, -sl.onz), 0.0f));
-        const float tf0 = fminf(fminf(fmaf(f0x, sl.ix, -sl.ofx), fmaf(f0y, sl.iy, -sl.ofy)), fmaf(f0z, sl.iz, -sl.ofz));
-        tn1 = fmaxf(fmaxf(fmaf(n1x, sl.ix, -sl.onx), fmaf(n1y, sl.iy, -sl.ony)), fmaxf(fmaf(n1z, sl.iz, -sl.onz), 0.0f));
-        const float tf1 = fminf(fminf(fmaf(f1x, sl.ix, -sl.ofx), fmaf(f1y, sl.iy, -sl.ofy)), fmaf(f1z, sl.iz, -sl.ofz));
-        h0 = tn0 <= fminf(tf0, kmax);
-        h1 = tn1 <= fminf(tf1, kmax);
-        l0 = lk.z; l1 = lk.w;
-        // which child first when both are wanted: the one entered first; when the ray starts inside both boxes (entry 0 for
-        // both, the usual case among large overlapping quads) the one it leaves first, whose hits lie nearer on average.
-        // Without the second rule child 0 (the lower coordinates) always went first on a tie, which is the far child for
-        // every ray that travels towards lower coordinates: views along -x cost 50 % more than views along +x.
-        near1 = tn1 < tn0 || (tn1 == tn0 && tf1 < tf0);
-    };
-    // exact test of one quad and insertion into this lane's k-buffer
-    auto offer_quad = [&](const float4 qa, const float4 qb, const float4 qc, unsigned int gid) {
-        float t; int tri;
-        if (!ray_quad(qa, qb, qc, ox, oy, oz, dx, dy, dz, kmax, t, tri)) return;
-        const unsigned long long key = make_key(t, 2u * gid + (unsigned int)tri);
-        if (n == DST_CHUNK && key >= kb[(DST_CHUNK - 1) * KS]) return;
-        int j = n;
-        while (j > 0 && kb[(j - 1) * KS] > key) j--;
-        if (n == DST_CHUNK) n = DST_CHUNK - 1;
-        for (int i = n; i > j; i--) kb[i * KS] = kb[(i - 1) * KS];
-        kb[j * KS] = key;
-        n++;
-        if (n == DST_CHUNK) kmax = hitkey_t(kb[(DST_CHUNK - 1) * KS]);
-    };
-    auto offer = [&](int pos) {
-        const float4* qp = bvh.quads + 3 * (size_t)pos;
-        offer_quad(__ldg(qp), __ldg(qp + 1), __ldg(qp + 2), (unsigned int)__ldg(bvh.leaf_gid + pos));
-    };
-
     for (;;) {
-        // ---- next batch of 32 list entries for this warp ----
         int base = 0;
         if (lane == 0) base = atomicAdd(cursor, 32);
         base = __shfl_sync(FULL, base, 0);
@@ -483,313 +505,252 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
         // The list is taken from its end: rays on a reflected segment come last in it (k_compact) and their batches are
         // the slow ones, so they start first and the cheap batches of primary rays fill the end of the round.
         const int idx = (((total + 31) >> 5) - 1 - (base >> 5)) * 32 + lane;
-        int ray = idx < total ? list[idx] : -1;
+        const int ray = idx < total ? list[idx] : -1;
         bool active = false;
-        // takes up `ray`: request, slab constants, empty k-buffer and stack
-        auto begin_ray = [&]() {
-            n = 0; sp = 0; kmax = -1.0f;
-            active = false;
-            if (ray >= 0) {
-                const float4 r0 = __ldg(reinterpret_cast<const float4*>(req + ray)), r1 = __ldg(reinterpret_cast<const float4*>(req + ray) + 1);
-                ox = r0.x; oy = r0.y; oz = r0.z; dx = r0.w; dy = r1.x; dz = r1.y;
-                sl = make_slab(ox, oy, oz, dx, dy, dz, absmax);
-                active = sl.valid;
-                if (active) kmax = r1.z;
-                if (COUNT) tc.enums++;
+        int n = 0;
+        float kmax = -1.0f, ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f;
+        if (ray >= 0) {
+            const float4 r0 = __ldg(reinterpret_cast<const float4*>(req + ray)), r1 = __ldg(reinterpret_cast<const float4*>(req + ray) + 1);
+            ox = r0.x; oy = r0.y; oz = r0.z; dx = r0.w; dy = r1.x; dz = r1.y;
+            active = fabsf(ox) < INFINITY && fabsf(oy) < INFINITY && fabsf(oz) < INFINITY && fabsf(dx) < INFINITY && fabsf(dy) < INFINITY && fabsf(dz) < INFINITY;
+            if (active) kmax = r1.z;
+            if (COUNT) tc.enums++;
+        }
+        if (__any_sync(FULL, active)) {
+            make_beam(m, active, ox, oy, oz, dx, dy, dz, absmax);
+            float krun = redux_max(kmax);
+            int cands = 0;
+            const bool done = beam_walk<COUNT>(bvh, m, krun, DST_BEAM_STEPS, status, tc, [&](bool valid, int pos) {
+                bool pass = false;
+                if (valid) { const Quad q = load_quad(bvh, pos); pass = hull_quad(m.beam, q.a, q.b, q.c, krun); }
+                unsigned int maybe = __ballot_sync(FULL, pass);
+                cands += __popc(maybe);
+                if (cands > DST_BEAM_CANDS) return false;
+                while (maybe) {
+                    const int src = 31 - __clz(maybe);
+                    maybe &= ~(1u << src);
+                    const int p = __shfl_sync(FULL, pos, src);
+                    const Quad q = load_quad(bvh, p);
+                    if (COUNT && lane == 0) tc.quads++;
+                    float t; int tri;
+                    if (!ray_quad(q.a, q.b, q.c, ox, oy, oz, dx, dy, dz, kmax, t, tri)) continue;
+                    const unsigned long long key = make_key(t, 2u * q.gid + (unsigned int)tri);
+                    if (n == DST_CHUNK && key >= kb[(DST_CHUNK - 1) * KS]) continue;
+                    int j = n < DST_CHUNK ? n : DST_CHUNK - 1;
+                    while (j > 0) {
+                        const unsigned long long prev = kb[(j - 1) * KS];
+                        if (prev < key) break;
+                        kb[j * KS] = prev;
+                        j--;
+                    }
+                    kb[j * KS] = key;
+                    if (n < DST_CHUNK) n++;
+                    if (n == DST_CHUNK) kmax = hitkey_t(kb[(DST_CHUNK - 1) * KS]);
+                }
+                krun = redux_max(kmax);
+                return true;
+            });
+            if (!done) {
+                // (a bound below the request's can only have come from a full k-buffer: the repeated search finds 16 hits again)
+                int at = 0;
+                if (lane == 0) at = atomicAdd(heavy_count, 32);
+                heavy[__shfl_sync(FULL, at, 0) + lane] = active ? ray : -1;
+                if (active) { req[ray].kmax0 = kmax; continue; }
+                n = 0;
             }
-        };
-        // writes the chunk of `ray` and lets go of it
-        auto publish = [&]() {
-            if (ray >= 0) {
-                kcnt[ray] = n;
-                ulonglong2* out = reinterpret_cast<ulonglong2*>(kbuf + (size_t)ray * DST_CHUNK);
+        }
+        if (ray >= 0) {
+            kcnt[ray] = n;
+            ulonglong2* out = reinterpret_cast<ulonglong2*>(kbuf + (size_t)ray * DST_CHUNK);
 #pragma unroll
-                for (int k = 0; k < DST_CHUNK / 2; k++) {
-                    if (2 * k < n) out[k] = make_ulonglong2(kb[(2 * k) * KS], kb[(2 * k + 1) * KS]);
-                }
-            }
-            ray = -1;
-        };
-        begin_ray();
-        RSTAT(0, 1); RSTAT(7, __popc(__ballot_sync(FULL, active)));
-        {   // hull of the batch's rays, for culling the quads of leaf runs the warp reaches together
-            const float o3[3] = { ox, oy, oz }, d3[3] = { dx, dy, dz };
-#pragma unroll
-            for (int a = 0; a < 3; a++) {
-                const float lo = wmin_f(active ? o3[a] : INFINITY), hi = wmax_f(active ? o3[a] : -INFINITY);
-                const float dl = wmin_f(active ? d3[a] : INFINITY), dh = wmax_f(active ? d3[a] : -INFINITY);
-                if (lane == 0) { sbeam[wid].omin[a] = lo; sbeam[wid].omax[a] = hi; sbeam[wid].dmin[a] = dl; sbeam[wid].dmax[a] = dh; sbeam[wid].dabs[a] = fmaxf(fabsf(dl), fabsf(dh)); }
-            }
-            __syncwarp();
-            if (lane == 0) sbeam[wid].dsum = sbeam[wid].dabs[0] + sbeam[wid].dabs[1] + sbeam[wid].dabs[2];
-            __syncwarp();
-        }
-        int ssp = 0, scur = __any_sync(FULL, active) ? 0 : DONE;     // shared walk: stack pointer and current link (uniform)
-        int s_tests = 0, s_wanted = 0;                                // child tests made together / of them wanted by their lane
-        bool drain = false;                                           // (uniform) a private stack is about to fill up
-        for (;;) {
-        // ---- shared phase (left early when a private stack is about to fill up: deferred subtrees pile up there) ----
-        if (scur != DONE) {
-            for (;;) {
-                if (drain) { drain = false; break; }                  // drain the private stacks first, then come back to scur
-                if (share_min_pct > 0 && s_tests >= 64 * 32 && s_wanted * 100 < s_tests * share_min_pct && ssp + 1 <= DST_ENUM_STACK - DST_ENUM_DEFER - 40) {
-                    // these rays do not travel together (most lanes sit out most tests): every lane takes the
-                    // pending subtrees onto its own stack and the batch continues lane by lane
-                    if (active) {
-                        push(scur, 0.0f);
-                        for (int e = 0; e < ssp; e++) push(sstack[wid][e], 0.0f);
-                    }
-                    ssp = 0; scur = DONE;
-                    RSTAT(5, 1);
-                    break;
-                }
-                if (scur >= 0) {
-                    float tn0, tn1; bool h0, h1, near1; int l0, l1;
-                    test_node(scur, tn0, tn1, h0, h1, l0, l1, near1);
-                    if (COUNT && lane == 0) tc.nodes++;
-                    const bool w0 = h0, w1 = h1;           // (a lane without a ray has kmax = -1 and every tn is >= 0: it never wants a child)
-                    const unsigned int m0 = __ballot_sync(FULL, w0), m1 = __ballot_sync(FULL, w1);
-                    if (share_min_pct > 0) { s_tests += 64; s_wanted += __popc(m0) + __popc(m1); }
-                    RSTAT(1, 1); RSTAT(6, __popc(m0) + __popc(m1));
-                    const bool s0 = DST_SHARE_VOTE <= 1 ? m0 != 0u : __popc(m0) >= DST_SHARE_VOTE, s1 = DST_SHARE_VOTE <= 1 ? m1 != 0u : __popc(m1) >= DST_SHARE_VOTE;
-                    int next = DONE;
-                    if (s0 && s1) {
-                        // the majority of the lanes that want both decides which child comes first
-                        const unsigned int pref1 = __ballot_sync(FULL, w0 && w1 && near1);
-                        const bool first1 = 2 * __popc(pref1) > __popc(m0 & m1);
-                        const int other = first1 ? l0 : l1;
-                        if (ssp < DST_SHARED_STACK) { if (lane == 0) sstack[wid][ssp] = other; ssp++; }
-                        else {                                                            // shared stack full: defer privately
-                            if (first1 ? w0 : w1) push(other, first1 ? tn0 : tn1);
-                            drain = __any_sync(FULL, sp >= DST_ENUM_DEFER);
-                        }
-                        next = first1 ? l1 : l0;
-                    } else {
-                        if (DST_SHARE_VOTE > 1) {
-                            // children wanted by too few lanes go onto those lanes' own stacks (farther one first)
-                            const bool d0 = w0 && !s0, d1 = w1 && !s1;
-                            if (d0 && d1) { if (tn1 < tn0) { push(l0, tn0); push(l1, tn1); } else { push(l1, tn1); push(l0, tn0); } }
-                            else if (d0) push(l0, tn0);
-                            else if (d1) push(l1, tn1);
-                            drain = __any_sync(FULL, sp >= DST_ENUM_DEFER);
-                        }
-                        if (s0) next = l0; else if (s1) next = l1;
-                    }
-                    if (next != DONE) { scur = next; continue; }
-                } else {
-                    // A run of leaves reached together. Lane q fetches quad q of the run and decides for the whole batch whether
-                    // any of its rays can hit it (hull_quad); the few quads that pass are handed round and tested exactly
-                    // by every lane against its own ray.
-                    const int first = DST_LEAF_FIRST(scur), count = DST_LEAF_COUNT(scur);
-                    if (count <= DST_HULL_MIN) {
-                        for (int lq = 0; lq < count; lq++) {
-                            if (COUNT && lane == 0) tc.quads++;
-                            RSTAT(2, 1);
-                            if (active) offer(first + lq);
-                        }
-                    } else {
-                    const bool mine = lane < count;
-                    float4 qa = make_float4(0.f, 0.f, 0.f, 0.f), qb = qa, qc = qa;
-                    unsigned int qgid = 0u;
-                    if (mine) {
-                        const float4* qp = bvh.quads + 3 * (size_t)(first + lane);
-                        qa = __ldg(qp); qb = __ldg(qp + 1); qc = __ldg(qp + 2);
-                        qgid = (unsigned int)__ldg(bvh.leaf_gid + first + lane);
-                    }
-                    const float krun = wmax_f(kmax);        // (-1 on lanes without a ray)
-                    unsigned int maybe = __ballot_sync(FULL, mine && hull_quad(sbeam[wid], qa, qb, qc, krun));
-                    RSTAT(4, count);
-                    while (maybe) {
-                        const int src = __ffs(maybe) - 1;
-                        maybe &= maybe - 1u;
-                        const float4 sa = make_float4(__shfl_sync(FULL, qa.x, src), __shfl_sync(FULL, qa.y, src), __shfl_sync(FULL, qa.z, src), __shfl_sync(FULL, qa.w, src));
-                        const float4 sb = make_float4(__shfl_sync(FULL, qb.x, src), __shfl_sync(FULL, qb.y, src), __shfl_sync(FULL, qb.z, src), __shfl_sync(FULL, qb.w, src));
-                        const float4 sc = make_float4(__shfl_sync(FULL, qc.x, src), __shfl_sync(FULL, qc.y, src), __shfl_sync(FULL, qc.z, src), __shfl_sync(FULL, qc.w, src));
-                        const unsigned int sg = __shfl_sync(FULL, qgid, src);
-                        if (COUNT && lane == 0) tc.quads++;
-                        RSTAT(2, 1);
-                        if (active) offer_quad(sa, sb, sc, sg);
-                    }
-                    }
-                }
-                if (ssp == 0) { scur = DONE; break; }
-                __syncwarp();
-                scur = sstack[wid][--ssp];
-                __syncwarp();
+            for (int k = 0; k < DST_CHUNK / 2; k++) {
+                if (2 * k < n) out[k] = make_ulonglong2(kb[(2 * k) * KS], kb[(2 * k + 1) * KS]);
             }
         }
-        // ---- private phase ----
-        int cur = active ? pop() : DONE;
-        for (;;) {
-            const unsigned int busy = __ballot_sync(FULL, cur != DONE);
-            if (busy == 0u) break;
-            // node phase: kept while at least DST_NODE_VOTE lanes have node work or nobody holds a leaf
-            for (;;) {
-                const bool is_node = (unsigned int)cur < (unsigned int)DONE;
-                const unsigned int m = __ballot_sync(FULL, is_node);
-                if (m == 0u) break;
-                if (__popc(m) < DST_NODE_VOTE && __any_sync(FULL, cur < 0)) break;
-                RSTAT(3, 1);
-                if (!is_node) continue;
-                float tn0, tn1; bool h0, h1, near1; int l0, l1;
-                test_node(cur, tn0, tn1, h0, h1, l0, l1, near1);
-                if (COUNT) tc.nodes++;
-                if (h0 && h1) {
-                    const bool swap = near1;
-                    push(swap ? l0 : l1, swap ? tn0 : tn1);
-                    cur = swap ? l1 : l0;
-                } else if (h0) cur = l0;
-                else if (h1) cur = l1;
-                else cur = pop();
-            }
-            // leaf phase
-            if (cur < 0) {
-                const int first = DST_LEAF_FIRST(cur), count = DST_LEAF_COUNT(cur);
-                for (int lq = 0; lq < count; lq++) { if (COUNT) tc.quads++; offer(first + lq); }
-                cur = pop();
-            }
-        }
-        if (scur == DONE) break;
-        }
-        // ---- publish the chunks of this batch ----
-        publish();
     }
     if (COUNT && counters) { atomicAdd(counters + 1, tc.enums); atomicAdd(counters + 2, tc.nodes); atomicAdd(counters + 3, tc.quads); }
-#ifdef DST_ROUND_STATS
-    if (lane == 0) for (int k = 0; k < 8; k++) if (rs[k]) atomicAdd(&g_round_stats[tag & 63][k], rs[k]);
-#endif
 }
 
-// one gather launch of a wavefront round (diag: with traversal counters)
-static inline void launch_gather(bool diag, int grid, cudaStream_t st, const BvhView& bvh, const EnumReq* req, const int* list,
-                                 const int* count_ptr, int* cursor, int min_count, unsigned long long* kbuf, int* kcnt, unsigned int* status,
-                                 unsigned long long* counters, int tag, bool tiled) {
-    const int share_min_pct = tiled ? DST_SHARE_MIN_PCT_TILED : DST_SHARE_MIN_PCT_LINEAR;
-    if (diag) k_enum<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cursor, min_count, kbuf, kcnt, status, counters, tag, share_min_pct);
-    else k_enum<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cursor, min_count, kbuf, kcnt, status, nullptr, tag, share_min_pct);
-}
-
-// The 16 nearest hits of ONE ray, found by a whole warp (same result as knearest()). For the few rays the
-// wavefront leaves to the tail kernel, and for small calls, what counts is the latency of a single walk:
-// a thread on its own pays one dependent memory round trip per box and per quad. Here every step takes up
-// to 16 entries from the top of a stack in shared memory (nearest first); leaf runs among them are tested
-// 16 quads at a time, one quad per lane, and the nodes among them 32 child boxes at a time, one box per
-// lane. The k-buffer lives in registers, one key per lane (lanes 0..15, ascending); an insertion is a
-// ballot and a shuffle. All arguments are warp-uniform. `stack` holds DST_WARP_STACK entries.
-#define DST_WARP_STACK 512
-#define DST_WARP_STEP_LIMIT (1 << 20)      // bound on the steps of one walk (status flag instead of a hang)
+// The 16 nearest hits of ONE ray, found by a whole warp (same result as knearest()): the walk of a hull that is a single
+// ray, its quads tested exactly, one per lane. The k-buffer lives in registers, one key per lane (lanes 0..15, ascending);
+// an insertion is a ballot and a shuffle. All arguments are warp-uniform.
 template <bool COUNT>
-__device__ __forceinline__ int knearest_warp(const BvhView& bvh, float ox, float oy, float oz, float dx, float dy, float dz,
-                                             float kmax0, unsigned long long* stack, unsigned long long& mykey,
-                                             unsigned int* status, TraceCounters& tc) {
+__device__ __forceinline__ int knearest_warp(const BvhView& bvh, float ox, float oy, float oz, float dx, float dy, float dz, float kmax0, float absmax,
+                                             WalkMem& m, unsigned long long& mykey, unsigned int* status, TraceCounters& tc) {
     constexpr unsigned int FULL = 0xffffffffu;
-    constexpr unsigned long long EMPTY = ~0ull;
     const int lane = threadIdx.x & 31;
-    mykey = EMPTY;
+    mykey = ~0ull;
     int n = 0;
-    float kmax = kmax0;
     if (bvh.P <= 0) return 0;
-    const RaySlab sl = make_slab(ox, oy, oz, dx, dy, dz, __ldg(bvh.header + 6));
-    if (!sl.valid) return 0;
-    // inserts a hit (uniform key) into the sorted keys held by lanes 0..15
-    auto insert = [&](unsigned long long key) {
-        const unsigned long long last = __shfl_sync(FULL, mykey, DST_CHUNK - 1);
-        if (key >= last) return;                                            // not among the 16 nearest (or the buffer is full of nearer ones)
-        const int pos = __popc(__ballot_sync(FULL, lane < DST_CHUNK && mykey < key));
-        const unsigned long long up = __shfl_up_sync(FULL, mykey, 1);
-        if (lane < DST_CHUNK) mykey = lane < pos ? mykey : (lane == pos ? key : up);
-        if (n < DST_CHUNK) n++;
-        if (n == DST_CHUNK) kmax = hitkey_t(__shfl_sync(FULL, mykey, DST_CHUNK - 1));
-    };
-    int sp = 0;
-    if (lane == 0) stack[0] = 0ull;            // the root: nearest possible t 0, link 0
-    sp = 1;
-    __syncwarp();
-    for (int step = 0; sp > 0; step++) {
-        if (step >= DST_WARP_STEP_LIMIT) { if (lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW); break; }
-        // lanes 30/31 take the top entry, lanes 28/29 the next, ...: lane order is then the order in which
-        // surviving children go back onto the stack (farthest first)
-        const int take = sp < 16 ? sp : 16;
-        const int slot = 15 - (lane >> 1);                                  // 0 = top of the stack
-        unsigned long long e = 0ull;
-        bool valid = slot < take;
-        if (valid) e = stack[sp - 1 - slot];
-        sp -= take;
-        __syncwarp();
-        const int link = (int)(unsigned int)e;
-        valid = valid && __uint_as_float((unsigned int)(e >> 32)) <= kmax;
-        // ---- leaf runs among the entries, nearest first ----
-        unsigned int leaves = __ballot_sync(FULL, valid && link < 0 && (lane & 1) == 1);
-        while (leaves) {
-            const int src = 31 - __clz(leaves);                             // highest lane = nearest entry
-            leaves &= ~(1u << src);
-            const int lnk = __shfl_sync(FULL, link, src);
-            const float etn = __uint_as_float((unsigned int)(__shfl_sync(FULL, e, src) >> 32));
-            if (etn > kmax) continue;                                       // the bound has shrunk meanwhile
-            const int first = DST_LEAF_FIRST(lnk), count = DST_LEAF_COUNT(lnk);
-            for (int base = 0; base < count; base += 32) {
-                bool hit = false;
-                unsigned long long key = 0ull;
-                if (base + lane < count) {
-                    const int pos = first + base + lane;
-                    const float4* qp = bvh.quads + 3 * (size_t)pos;
-                    const float4 qa = __ldg(qp), qb = __ldg(qp + 1), qc = __ldg(qp + 2);
-                    float t; int tri;
-                    if (ray_quad(qa, qb, qc, ox, oy, oz, dx, dy, dz, kmax, t, tri)) {
-                        const unsigned int gid = (unsigned int)__ldg(bvh.leaf_gid + pos);
-                        key = make_key(t, 2u * gid + (unsigned int)tri);
-                        hit = true;
-                    }
-                }
-                if (COUNT && lane == 0) tc.quads += (unsigned long long)(count - base < 32 ? count - base : 32);
-                unsigned int hits = __ballot_sync(FULL, hit);
-                while (hits) {
-                    const int hl = __ffs(hits) - 1;
-                    hits &= hits - 1u;
-                    insert(__shfl_sync(FULL, key, hl));
-                }
+    if (!(fabsf(ox) < INFINITY && fabsf(oy) < INFINITY && fabsf(oz) < INFINITY && fabsf(dx) < INFINITY && fabsf(dy) < INFINITY && fabsf(dz) < INFINITY)) return 0;
+    make_beam(m, true, ox, oy, oz, dx, dy, dz, absmax);
+    float krun = kmax0;
+    const bool done = beam_walk<COUNT>(bvh, m, krun, DST_WALK_STEP_LIMIT, status, tc, [&](bool valid, int pos) {
+        bool hit = false;
+        unsigned long long key = 0ull;
+        if (valid) {
+            const Quad q = load_quad(bvh, pos);
+            float t; int tri;
+            if (COUNT) tc.quads++;
+            if (ray_quad(q.a, q.b, q.c, ox, oy, oz, dx, dy, dz, krun, t, tri)) {
+                key = make_key(t, 2u * q.gid + (unsigned int)tri);
+                hit = true;
             }
         }
-        // ---- nodes among the entries: one child box per lane ----
-        bool h = false;
-        float tn = 0.0f, tf = 0.0f;
-        int clink = 0;
-        if (valid && link >= 0 && __uint_as_float((unsigned int)(e >> 32)) <= kmax) {
-            const float4* np = bvh.nodes + 4 * (size_t)link;
-            const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
-            const int4 lk = __ldg(reinterpret_cast<const int4*>(np + 3));
-            float lox, loy, loz, hix, hiy, hiz;
-            if ((lane & 1) == 0) { lox = a.x; loy = a.y; loz = a.z; hix = a.w; hiy = b.x; hiz = b.y; clink = lk.z; }
-            else { lox = b.z; loy = b.w; loz = c.x; hix = c.y; hiy = c.z; hiz = c.w; clink = lk.w; }
-            const float nx = sl.px ? lox : hix, fx = sl.px ? hix : lox;
-            const float ny = sl.py ? loy : hiy, fy = sl.py ? hiy : loy;
-            const float nz = sl.pz ? loz : hiz, fz = sl.pz ? hiz : loz;
-            tn = fmaxf(fmaxf(fmaf(nx, sl.ix, -sl.onx), fmaf(ny, sl.iy, -sl.ony)), fmaxf(fmaf(nz, sl.iz, -sl.onz), 0.0f));
-            tf = fminf(fminf(fmaf(fx, sl.ix, -sl.ofx), fmaf(fy, sl.iy, -sl.ofy)), fmaf(fz, sl.iz, -sl.ofz));
-            h = (tn <= tf) && (tn <= kmax);
-            if (COUNT && (lane & 1) == 0) tc.nodes++;
+        unsigned int hits = __ballot_sync(FULL, hit);
+        unsigned long long last = __shfl_sync(FULL, mykey, DST_CHUNK - 1);
+        while (hits) {
+            const int hl = 31 - __clz(hits);
+            hits &= ~(1u << hl);
+            const unsigned long long k = __shfl_sync(FULL, key, hl);
+            if (k >= last) continue;                                        // not among the 16 nearest
+            const int at = __popc(__ballot_sync(FULL, lane < DST_CHUNK && mykey < k));
+            const unsigned long long up = __shfl_up_sync(FULL, mykey, 1);
+            if (lane < DST_CHUNK) mykey = lane < at ? mykey : (lane == at ? k : up);
+            last = __shfl_sync(FULL, mykey, DST_CHUNK - 1);
+            if (n < DST_CHUNK) n++;
         }
-        // within a pair the farther child goes first (even lane), the nearer second (odd lane)
-        {
-            const float ptn = __shfl_xor_sync(FULL, tn, 1), ptf = __shfl_xor_sync(FULL, tf, 1);
-            const int plink = __shfl_xor_sync(FULL, clink, 1);
-            const bool ph = __shfl_xor_sync(FULL, h, 1);
-            const bool even = (lane & 1) == 0;
-            // nearer = entered first, on a tie (the ray starts inside both boxes) left first
-            const bool mine_nearer = tn < ptn || (tn == ptn && (tf < ptf || (tf == ptf && even)));
-            if (h && ph && (even ? mine_nearer : !mine_nearer)) { tn = ptn; clink = plink; }
+        if (n == DST_CHUNK) krun = hitkey_t(last);
+        return true;
+    });
+    if (!done && lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW);
+    return n;
+}
+
+// Second step of a gather: the batches k_enum gave up, in groups of DST_GROUP rays, one warp per group. The walk is again
+// that of the group's hull; a quad step tests its 32 quads (one per lane) exactly against one ray of the group after the
+// other. The k-buffers are in shared memory; lanes 0..15 hold one of them at a time.
+template <bool COUNT>
+__global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_group(BvhView bvh, EnumReq* req, const int* __restrict__ list,
+                                                       const int* __restrict__ count_ptr, int* cursor,
+                                                       unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
+                                                       unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count) {
+    constexpr unsigned int FULL = 0xffffffffu;
+    __shared__ WalkMem walk_mem[ENUM_THREADS / 32];
+    __shared__ unsigned long long skeys[ENUM_THREADS / 32][DST_GROUP][DST_CHUNK];
+    __shared__ float4 srays[ENUM_THREADS / 32][DST_GROUP][2];
+    const int total = *count_ptr / DST_GROUP;
+    if (total <= 0) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    WalkMem& m = walk_mem[w];
+    const float absmax = __ldg(bvh.header + 6);
+    TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
+    for (;;) {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(cursor, 1);
+        i = __shfl_sync(FULL, i, 0);
+        if (i >= total) break;
+        const int ray = lane < DST_GROUP ? list[i * DST_GROUP + lane] : -1;
+        const unsigned int members = __ballot_sync(FULL, ray >= 0);
+        if (members == 0u) continue;
+        float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
+        if (ray >= 0) { r0 = *reinterpret_cast<const float4*>(req + ray); r1 = *(reinterpret_cast<const float4*>(req + ray) + 1); }
+        const float bound0 = ray >= 0 ? r1.z : -1.0f;
+        if (lane < DST_GROUP) { srays[w][lane][0] = r0; srays[w][lane][1] = make_float4(r1.x, r1.y, bound0, 0.0f); }
+        for (int k = lane; k < DST_GROUP * DST_CHUNK; k += 32) (&skeys[w][0][0])[k] = ~0ull;
+        make_beam(m, ray >= 0, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, absmax);
+        float krun = redux_max(bound0);
+        const bool done = beam_walk<COUNT>(bvh, m, krun, DST_GROUP_STEPS, status, tc, [&](bool valid, int pos) {
+            Quad q;
+            q.a = q.b = q.c = make_float4(0.f, 0.f, 0.f, 0.f); q.gid = 0u;
+            if (valid) { q = load_quad(bvh, pos); if (COUNT) tc.quads++; }
+            float kall = -1.0f;
+#pragma unroll 1
+            for (int r = 0; r < DST_GROUP; r++) {
+                const float4 ra = srays[w][r][0], rb = srays[w][r][1];
+                float t; int tri;
+                const bool hit = valid && ray_quad(q.a, q.b, q.c, ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, t, tri);
+                unsigned int hits = __ballot_sync(FULL, hit);
+                float kr = rb.z;
+                if (hits) {
+                    const unsigned long long key = make_key(t, 2u * q.gid + (unsigned int)tri);
+                    unsigned long long mine = skeys[w][r][lane & (DST_CHUNK - 1)];
+                    unsigned long long last = __shfl_sync(FULL, mine, DST_CHUNK - 1);
+                    while (hits) {
+                        const int hl = 31 - __clz(hits);
+                        hits &= ~(1u << hl);
+                        const unsigned long long k = __shfl_sync(FULL, key, hl);
+                        if (k >= last) continue;
+                        const int at = __popc(__ballot_sync(FULL, lane < DST_CHUNK && mine < k));
+                        const unsigned long long up = __shfl_up_sync(FULL, mine, 1);
+                        if (lane < DST_CHUNK) mine = lane < at ? mine : (lane == at ? k : up);
+                        last = __shfl_sync(FULL, mine, DST_CHUNK - 1);
+                    }
+                    if (lane < DST_CHUNK) skeys[w][r][lane] = mine;
+                    if (last != ~0ull) { kr = hitkey_t(last); if (lane == 0) srays[w][r][1].z = kr; }
+                }
+                kall = fmaxf(kall, kr);
+            }
+            krun = kall;
+            __syncwarp();
+            return true;
+        });
+        __syncwarp();
+        if (done) {
+#pragma unroll 1
+            for (int r = 0; r < DST_GROUP; r++) {
+                if (!((members >> r) & 1u)) continue;
+                const int rr = __shfl_sync(FULL, ray, r);
+                const unsigned long long mine = skeys[w][r][lane & (DST_CHUNK - 1)];
+                const int n = __popc(__ballot_sync(FULL, lane < DST_CHUNK && mine != ~0ull));
+                if (lane < n) kbuf[(size_t)rr * DST_CHUNK + lane] = mine;
+                if (lane == 0) kcnt[rr] = n;
+            }
+        } else {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(heavy_count, __popc(members));
+            at = __shfl_sync(FULL, at, 0) + __popc(members & ((1u << lane) - 1u));
+            if (ray >= 0) { heavy[at] = ray; req[ray].kmax0 = srays[w][lane][1].z; }
         }
-        const unsigned int pushes = __ballot_sync(FULL, h);
-        const int npush = __popc(pushes);
-        if (sp + npush > DST_WARP_STACK) {
-            if (lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW);
-            break;
-        }
-        if (h) stack[sp + __popc(pushes & ((1u << lane) - 1u))] = ((unsigned long long)__float_as_uint(tn) << 32) | (unsigned int)clink;
-        sp += npush;
         __syncwarp();
     }
-    return n;
+    if (COUNT && counters) { atomicAdd(counters + 2, tc.nodes); atomicAdd(counters + 3, tc.quads); }
+}
+
+// Last step of a gather: the rays whose batch was given up by k_enum, one warp per ray.
+template <bool COUNT>
+__global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray(BvhView bvh, const EnumReq* __restrict__ req, const int* __restrict__ list,
+                                                       const int* __restrict__ count_ptr, int* cursor,
+                                                       unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
+                                                       unsigned int* status, unsigned long long* counters) {
+    __shared__ WalkMem walk_mem[ENUM_THREADS / 32];
+    const int total = *count_ptr;
+    if (total <= 0) return;
+    const int lane = threadIdx.x & 31;
+    WalkMem& m = walk_mem[threadIdx.x >> 5];
+    const float absmax = __ldg(bvh.header + 6);
+    TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
+    for (;;) {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(cursor, 1);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= total) break;
+        const int ray = list[i];
+        const float4 r0 = __ldg(reinterpret_cast<const float4*>(req + ray)), r1 = __ldg(reinterpret_cast<const float4*>(req + ray) + 1);
+        unsigned long long key;
+        const int n = knearest_warp<COUNT>(bvh, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, absmax, m, key, status, tc);
+        if (lane < n) kbuf[(size_t)ray * DST_CHUNK + lane] = key;
+        if (lane == 0) kcnt[ray] = n;
+        __syncwarp();
+    }
+    if (COUNT && counters) { atomicAdd(counters + 2, tc.nodes); atomicAdd(counters + 3, tc.quads); }
+}
+
+// the gather launches of a wavefront round (diag: with traversal counters). cnt: the round's entry in the set of round counters;
+// heavy, heavy2: lists of as many rays as the round has slots
+static inline void launch_gather(bool diag, int grid, cudaStream_t st, const BvhView& bvh, EnumReq* req, const int* list,
+                                 const int* count_ptr, int* cnt, int min_count, unsigned long long* kbuf, int* kcnt, unsigned int* status,
+                                 unsigned long long* counters, int* heavy, int* heavy2) {
+    constexpr int R = DST_WF_ROUNDS + 2;
+    if (diag) {
+        k_enum<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, counters, heavy, cnt + 2 * R);
+        k_enum_group<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, counters, heavy2, cnt + 4 * R);
+        k_enum_ray<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy2, cnt + 4 * R, cnt + 5 * R, kbuf, kcnt, status, counters);
+    } else {
+        k_enum<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, nullptr, heavy, cnt + 2 * R);
+        k_enum_group<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, nullptr, heavy2, cnt + 4 * R);
+        k_enum_ray<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy2, cnt + 4 * R, cnt + 5 * R, kbuf, kcnt, status, nullptr);
+    }
 }
 
 // List entry i of round 0 -> ray index (or -1). Image-like grids are walked in 8x4 pixel tiles (one tile = the 32
@@ -817,8 +778,8 @@ __device__ __forceinline__ int ray_of_slot(long long i, int H, int W, bool tiled
         tx = (int)(blk % blocks_x) * DST_TILE_BLOCK + (int)zx;
         ty = (int)(blk / blocks_x) * DST_TILE_BLOCK + (int)zy;
     } else { tx = (int)(tile % tiles_x); ty = (int)(tile / tiles_x); }
-    const int x = tx * 8 + (lane & 7);
-    const int y = ty * 4 + (lane >> 3);
+    const int x = tx * 8 + ((lane & 1) | ((lane >> 1) & 2) | ((lane >> 2) & 4));      // Z order inside the tile too: 8 consecutive lanes are a 4x2 patch
+    const int y = ty * 4 + (((lane >> 1) & 1) | ((lane >> 2) & 2));
     if (x >= W || y >= H) return -1;
     return y * W + x;
 }
