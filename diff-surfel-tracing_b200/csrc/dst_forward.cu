@@ -205,8 +205,62 @@ __device__ __forceinline__ void fwd_request(const FwdState& s, EnumReq& q) {
     q.dx = s.sdx; q.dy = s.sdy; q.dz = s.sdz; q.kmax0 = DST_T_MAX; q.pad = s.bounce > 0 ? 1.f : 0.f;       // pad: the ray is on a reflected segment
 }
 
-// Composites one gathered chunk (forward.cu:197-306) and, when the segment ends, finishes it
-// (forward.cu:309-314, tracePath 378-422). Returns true while the ray needs another enumeration.
+// After the hits of a chunk: the segment goes on (returns true), or it is finished (forward.cu:309-314, tracePath 378-422) and
+// the ray starts the reflected segment (true) or is done (false). opaque: the transmittance limit or the hit limit was reached.
+__device__ __forceinline__ bool fwd_end_chunk(const FwdParams& p, int ray, FwdState& s, bool opaque, int cnt, bool diag) {
+    const dst_trace_inputs& in = p.a.in;
+    s.chunk++;
+    bool seg_done = opaque || cnt < DST_CHUNK || s.contributor > DST_MAX_INTERSECTION;   // :299
+    if (!seg_done && s.chunk >= DST_MAX_CHUNKS) { atomicOr(p.status, DST_STATUS_CHUNK_LIMIT); seg_done = true; }
+    if (!seg_done) {
+        s.offset = (float)((double)s.dpt + 0.00001);                                     // :303
+        return true;
+    }
+    // ---- end of the segment (forward.cu:309-314) ----
+    const float bg0 = __ldg(in.background), bg1 = __ldg(in.background + 1), bg2 = __ldg(in.background + 2);
+    const float C0 = xadd(s.C0, xmul(s.T_prev, bg0)), C1 = xadd(s.C1, xmul(s.T_prev, bg1)), C2 = xadd(s.C2, xmul(s.T_prev, bg2));
+    const float A = xsub(1.0f, s.T_prev);
+    // tracePath, forward.cu:378-412
+    if (s.bounce == 0) {
+        p.a.out_dpt[ray] = s.D; p.a.out_acc[ray] = A;
+        p.a.out_norm[3 * (size_t)ray] = s.Nx; p.a.out_norm[3 * (size_t)ray + 1] = s.Ny; p.a.out_norm[3 * (size_t)ray + 2] = s.Nz;
+        p.a.out_aux[2 * (size_t)ray] = s.O0; p.a.out_aux[2 * (size_t)ray + 1] = s.O1;
+        // zeros as the reference, or (extension) the distortion and the two moments its gradient needs
+        p.a.out_dist[3 * (size_t)ray] = s.dist; p.a.out_dist[3 * (size_t)ray + 1] = s.m1; p.a.out_dist[3 * (size_t)ray + 2] = s.m2;
+    }
+    const float f_this = (s.bounce == in.max_trace_depth) ? 1.0f : xsub(1.0f, s.O0);
+    s.rgb0 = xadd(s.rgb0, xmul(xmul(C0, f_this), s.s_prod));
+    s.rgb1 = xadd(s.rgb1, xmul(xmul(C1, f_this), s.s_prod));
+    s.rgb2 = xadd(s.rgb2, xmul(xmul(C2, f_this), s.s_prod));
+    s.s_prod = xmul(s.s_prod, s.O0);
+    float* mid = p.a.mid_val + (size_t)ray * in.mid_stride;
+    float4* m4 = reinterpret_cast<float4*>(mid + s.bounce * DST_MID_CHANNELS);
+    m4[0] = make_float4(s.sox, s.soy, s.soz, s.sdx);
+    m4[1] = make_float4(s.sdy, s.sdz, s.D, A);
+    m4[2] = make_float4(s.Nx, s.Ny, s.Nz, s.O0);
+    m4[3] = make_float4(s.O1, C0, C1, C2);
+    const float nlen = xsqrt(rdot3(s.Nx, s.Ny, s.Nz, s.Nx, s.Ny, s.Nz));
+    if (nlen == 0.0f || s.O0 <= in.specular_threshold || s.bounce == in.max_trace_depth) {        // :416
+        // the ray is finished; bounces that were never traced read as zeros (the reference leaves them uninitialised, forward.cu:446)
+        for (int k = (s.bounce + 1) * DST_MID_CHANNELS; k < in.mid_stride; k += 4)
+            *reinterpret_cast<float4*>(mid + k) = make_float4(0.f, 0.f, 0.f, 0.f);
+        p.a.out_rgb[3 * (size_t)ray] = s.rgb0; p.a.out_rgb[3 * (size_t)ray + 1] = s.rgb1; p.a.out_rgb[3 * (size_t)ray + 2] = s.rgb2;
+        if (diag && p.a.hit_cnt) p.a.hit_cnt[ray] = s.hit_count;
+        return false;
+    }
+    // reflect about the accumulated normal, restart 0.06 along the new direction (:420-422);
+    // exactly rounded, because the bounce ray decides which quads the next segment sees
+    const float nx = xdiv(s.Nx, nlen), ny = xdiv(s.Ny, nlen), nz = xdiv(s.Nz, nlen);
+    const float k = xmul(2.0f, rdot3(nx, ny, nz, s.sdx, s.sdy, s.sdz));
+    const float Ex = xadd(s.sox, xmul(s.D, s.sdx)), Ey = xadd(s.soy, xmul(s.D, s.sdy)), Ez = xadd(s.soz, xmul(s.D, s.sdz));
+    s.sdx = xsub(s.sdx, xmul(k, nx)); s.sdy = xsub(s.sdy, xmul(k, ny)); s.sdz = xsub(s.sdz, xmul(k, nz));
+    s.sox = xadd(Ex, xmul(0.06f, s.sdx)); s.soy = xadd(Ey, xmul(0.06f, s.sdy)); s.soz = xadd(Ez, xmul(0.06f, s.sdz));
+    s.bounce++;
+    fwd_begin_segment(s);
+    return true;
+}
+
+// Composites one gathered chunk (forward.cu:197-306), one thread per ray. Returns true while the ray needs another enumeration.
 // kb: the chunk's keys with stride KS; cnt: how many.
 template <bool DIAG, int KS>
 __device__ __forceinline__ bool fwd_shade(const FwdParams& p, int ray, FwdState& s, const unsigned long long* kb, int cnt, TraceCounters& tc) {
@@ -288,55 +342,7 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, int ray, FwdState&
             s.hit_count++;
         }
     }
-    s.chunk++;
-    bool seg_done = stop || T_next < T_threshold || cnt < DST_CHUNK || s.contributor > DST_MAX_INTERSECTION;   // :299
-    if (!seg_done && s.chunk >= DST_MAX_CHUNKS) { atomicOr(p.status, DST_STATUS_CHUNK_LIMIT); seg_done = true; }
-    if (!seg_done) {
-        s.offset = (float)((double)s.dpt + 0.00001);                                     // :303
-        return true;
-    }
-    // ---- end of the segment (forward.cu:309-314) ----
-    const float bg0 = __ldg(in.background), bg1 = __ldg(in.background + 1), bg2 = __ldg(in.background + 2);
-    const float C0 = xadd(s.C0, xmul(s.T_prev, bg0)), C1 = xadd(s.C1, xmul(s.T_prev, bg1)), C2 = xadd(s.C2, xmul(s.T_prev, bg2));
-    const float A = xsub(1.0f, s.T_prev);
-    // tracePath, forward.cu:378-412
-    if (s.bounce == 0) {
-        p.a.out_dpt[ray] = s.D; p.a.out_acc[ray] = A;
-        p.a.out_norm[3 * (size_t)ray] = s.Nx; p.a.out_norm[3 * (size_t)ray + 1] = s.Ny; p.a.out_norm[3 * (size_t)ray + 2] = s.Nz;
-        p.a.out_aux[2 * (size_t)ray] = s.O0; p.a.out_aux[2 * (size_t)ray + 1] = s.O1;
-        // zeros as the reference, or (extension) the distortion and the two moments its gradient needs
-        p.a.out_dist[3 * (size_t)ray] = s.dist; p.a.out_dist[3 * (size_t)ray + 1] = s.m1; p.a.out_dist[3 * (size_t)ray + 2] = s.m2;
-    }
-    const float f_this = (s.bounce == in.max_trace_depth) ? 1.0f : xsub(1.0f, s.O0);
-    s.rgb0 = xadd(s.rgb0, xmul(xmul(C0, f_this), s.s_prod));
-    s.rgb1 = xadd(s.rgb1, xmul(xmul(C1, f_this), s.s_prod));
-    s.rgb2 = xadd(s.rgb2, xmul(xmul(C2, f_this), s.s_prod));
-    s.s_prod = xmul(s.s_prod, s.O0);
-    float* mid = p.a.mid_val + (size_t)ray * in.mid_stride;
-    float4* m4 = reinterpret_cast<float4*>(mid + s.bounce * DST_MID_CHANNELS);
-    m4[0] = make_float4(s.sox, s.soy, s.soz, s.sdx);
-    m4[1] = make_float4(s.sdy, s.sdz, s.D, A);
-    m4[2] = make_float4(s.Nx, s.Ny, s.Nz, s.O0);
-    m4[3] = make_float4(s.O1, C0, C1, C2);
-    const float nlen = xsqrt(rdot3(s.Nx, s.Ny, s.Nz, s.Nx, s.Ny, s.Nz));
-    if (nlen == 0.0f || s.O0 <= in.specular_threshold || s.bounce == in.max_trace_depth) {        // :416
-        // the ray is finished; bounces that were never traced read as zeros (the reference leaves them uninitialised, forward.cu:446)
-        for (int k = (s.bounce + 1) * DST_MID_CHANNELS; k < in.mid_stride; k += 4)
-            *reinterpret_cast<float4*>(mid + k) = make_float4(0.f, 0.f, 0.f, 0.f);
-        p.a.out_rgb[3 * (size_t)ray] = s.rgb0; p.a.out_rgb[3 * (size_t)ray + 1] = s.rgb1; p.a.out_rgb[3 * (size_t)ray + 2] = s.rgb2;
-        if (DIAG && p.a.hit_cnt) p.a.hit_cnt[ray] = s.hit_count;
-        return false;
-    }
-    // reflect about the accumulated normal, restart 0.06 along the new direction (:420-422);
-    // exactly rounded, because the bounce ray decides which quads the next segment sees
-    const float nx = xdiv(s.Nx, nlen), ny = xdiv(s.Ny, nlen), nz = xdiv(s.Nz, nlen);
-    const float k = xmul(2.0f, rdot3(nx, ny, nz, s.sdx, s.sdy, s.sdz));
-    const float Ex = xadd(s.sox, xmul(s.D, s.sdx)), Ey = xadd(s.soy, xmul(s.D, s.sdy)), Ez = xadd(s.soz, xmul(s.D, s.sdz));
-    s.sdx = xsub(s.sdx, xmul(k, nx)); s.sdy = xsub(s.sdy, xmul(k, ny)); s.sdz = xsub(s.sdz, xmul(k, nz));
-    s.sox = xadd(Ex, xmul(0.06f, s.sdx)); s.soy = xadd(Ey, xmul(0.06f, s.sdy)); s.soz = xadd(Ez, xmul(0.06f, s.sdz));
-    s.bounce++;
-    fwd_begin_segment(s);
-    return true;
+    return fwd_end_chunk(p, ray, s, stop || T_next < T_threshold, cnt, DIAG);
 }
 
 __device__ __forceinline__ void load_state(const void* base, int ray, FwdState& s) {
@@ -469,43 +475,149 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_fwd_tail(const __grid_constant
     if (DIAG) flush_counters(p.a.counters, tc);
 }
 
-// The same for few rays (what the wavefront leaves over, or a small call): one WARP per ray. The warp gathers
-// the chunk together (knearest_warp), lane 0 composites it. The longest ray, whose serial work is what this
-// kernel takes, gets through its walks several times faster than a thread on its own.
-constexpr int WTAIL_THREADS = 128;
+// fwd_shade() by a whole warp for one ray, lane i on hit i: the records and colour rows of the 16 hits are loaded and evaluated side by
+// side instead of one dependent load after another. What has an order keeps it: the transmittance is a chain of uniform
+// products, and the nine running sums (C, D, N, O: neighbours in FwdState) are added up hit by hit, one sum per lane, so every bit is
+// that of the serial loop. s and terms are shared memory of the warp; key: lane i's hit.
+struct WarpShade { FwdState s; float terms[DST_CHUNK][9]; };
 template <bool DIAG>
-__global__ void __launch_bounds__(WTAIL_THREADS) k_fwd_tail_warp(const __grid_constant__ FwdParams p) {
-    __shared__ WalkMem walk_mem[WTAIL_THREADS / 32];
-    __shared__ unsigned long long wkeys[WTAIL_THREADS / 32][DST_CHUNK];
+__device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int ray, WarpShade& ws, unsigned long long key, int cnt, TraceCounters& tc) {
     constexpr unsigned int FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const dst_trace_inputs& in = p.a.in;
+    FwdState& s = ws.s;
+    const bool have = lane < cnt;
+    if (p.log_keys) {
+        int idx = 0;
+        if (lane == 0) idx = atomicAdd(p.log_count, 1);
+        idx = __shfl_sync(FULL, idx, 0);
+        if (idx >= 0 && idx < p.log_cap) {
+            if (have) p.log_keys[(size_t)idx * DST_CHUNK + lane] = key;
+            if (lane == 0) {
+                p.log_hdr[idx] = make_int2(-1, cnt);
+                if (s.log_prev < 0) p.log_seg_head[(size_t)ray * p.log_seg_stride + s.bounce] = idx;
+                else p.log_hdr[s.log_prev].x = idx;
+                s.log_prev = idx;
+            }
+        } else if (lane == 0) p.log_ray_ok[ray] = 0;
+    }
+    const float min_depth = s.bounce == 0 ? (in.start_from_first ? 0.2f : 0.0f) : 0.06f;       // forward.cu:353
+    const int gidx = (int)((unsigned int)key >> 1);
+    SlotEval e;
+    e.dpt = 0.f; e.alpha = 0.f;
+    const bool ok = have && eval_slot(key, s.offset, s.sox, s.soy, s.soz, s.sdx, s.sdy, s.sdz, min_depth, p.cache, gidx, e);
+    unsigned int okm = __ballot_sync(FULL, ok);
+    // forward.cu:207: a hit on the surfel that contributed last is passed over. Within a chunk every surfel occurs once, so that can
+    // only be the last contributor of the chunk before, as long as nothing has contributed in this one.
+    const unsigned int again = __ballot_sync(FULL, have && gidx == s.last_gidx);
+    const unsigned int skip = (okm & (again - 1u)) == 0u ? again : 0u;
+    okm &= ~skip;
+    float T = s.T_prev, my_T = 0.f;
+    int contributor = s.contributor, last = DST_CHUNK;          // last: slot at which compositing stops
+    for (unsigned int m = okm; m; m &= m - 1u) {
+        const int i = __ffs(m) - 1;
+        const float T_next = xmul(T, xsub(1.0f, __shfl_sync(FULL, e.alpha, i)));
+        if (T_next < 0.0001f) { last = i; break; }
+        contributor++;
+        if (contributor > DST_MAX_INTERSECTION) { last = i; break; }
+        if (lane == i) my_T = T;
+        T = T_next;
+    }
+    const bool stop = last < DST_CHUNK;
+    const unsigned int contrib = okm & ((1u << last) - 1u);
+    const unsigned int evaluated = ((1u << cnt) - 1u) & ~skip & (stop ? (2u << last) - 1u : FULL);
+    const float w = xmul(e.alpha, my_T);
+    if ((contrib >> lane) & 1u) {
+        float* t = ws.terms[lane];
+        if (in.colors_precomp == nullptr) {
+            const int ncoef = (in.sh_degree + 1) * (in.sh_degree + 1);
+            const bool sh_aligned = ((in.sh_coeffs * 3) & 3) == 0 && ((reinterpret_cast<uintptr_t>(in.shs) & 15) == 0);
+            float sb[16], c[48];
+            load_sh_row(in.shs + 3 * (size_t)gidx * in.sh_coeffs, 3 * ncoef, sh_aligned, c);
+            sh_basis(in.sh_degree, s.sdx, s.sdy, s.sdz, sb);
+            t[0] = xmul(w, fmaxf(sh_channel(ncoef, sb, c, 0), 0.f)); t[1] = xmul(w, fmaxf(sh_channel(ncoef, sb, c, 1), 0.f));
+            t[2] = xmul(w, fmaxf(sh_channel(ncoef, sb, c, 2), 0.f));
+        } else {
+            const float* cp = in.colors_precomp + 3 * (size_t)gidx;
+            t[0] = xmul(w, __ldg(cp)); t[1] = xmul(w, __ldg(cp + 1)); t[2] = xmul(w, __ldg(cp + 2));
+        }
+        t[3] = xmul(w, e.dpt);
+        t[4] = xmul(w, e.nsign * e.r2.x); t[5] = xmul(w, e.nsign * e.r2.y); t[6] = xmul(w, e.nsign * e.r2.z);
+        float2 ax = make_float2(0.f, 0.f);
+        if (in.others_precomp) ax = __ldg(reinterpret_cast<const float2*>(in.others_precomp) + gidx);
+        t[7] = xmul(w, ax.x); t[8] = xmul(w, ax.y);
+        if (p.a.training && p.a.a_weights) atomicAdd(p.a.a_weights + gidx, w);          // forward.cu:295
+        if (DIAG && p.a.hit_log) {
+            const int at = s.hit_count + __popc(contrib & ((1u << lane) - 1u));
+            if (at < p.a.hit_cap) p.a.hit_log[(size_t)ray * p.a.hit_cap + at] = (int)(unsigned int)key;
+        }
+    }
+    if (p.dist_on && s.bounce == 0 && contrib) {      // see fwd_shade()
+        float m0 = s.m0, m1 = s.m1, m2 = s.m2, dist = s.dist;
+        bool first = s.contributor == 0;
+        for (unsigned int mm = contrib; mm; mm &= mm - 1u) {
+            const int i = __ffs(mm) - 1;
+            const float wi = __shfl_sync(FULL, w, i), Ti = __shfl_sync(FULL, my_T, i);
+            const float m_abs = DST_DIST_K * (1.0f - DST_DIST_NEAR / __shfl_sync(FULL, e.dpt, i));
+            if (first) { m0 = m_abs; first = false; }
+            const float m = m_abs - m0;
+            dist += wi * (m * m * (1.0f - Ti) + m2 - 2.0f * m * m1);
+            m1 += m * wi; m2 += m * m * wi;
+        }
+        __syncwarp();
+        if (lane == 0) { s.m0 = m0; s.m1 = m1; s.m2 = m2; s.dist = dist; }
+    }
+    const float dpt = evaluated ? __shfl_sync(FULL, e.dpt, 31 - __clz(evaluated)) : s.dpt;       // forward.cu:211 (kept even when the slot is skipped)
+    const int last_gidx = contrib ? __shfl_sync(FULL, gidx, 31 - __clz(contrib)) : s.last_gidx;
+    __syncwarp();
+    if (lane < 9) {
+        float* sum = &s.C0 + lane;
+        float acc = *sum;
+        for (unsigned int m = contrib; m; m &= m - 1u) acc = xadd(acc, ws.terms[__ffs(m) - 1][lane]);
+        *sum = acc;
+    }
+    __syncwarp();
+    bool go = false;
+    if (lane == 0) {
+        if (DIAG) { if (s.chunk == 0) tc.segs++; tc.enums++; tc.evals += __popc(evaluated); tc.contribs += __popc(contrib); s.hit_count += __popc(contrib); }
+        s.T_prev = T; s.contributor = contributor; s.dpt = dpt; s.last_gidx = last_gidx;
+        go = fwd_end_chunk(p, ray, s, stop, cnt, DIAG);
+    }
+    return __shfl_sync(FULL, go, 0);
+}
+
+// Few rays (what the wavefront leaves over, or a small call): one WARP per ray to completion. The warp gathers the chunk together
+// (knearest_warp) and composites it together (fwd_shade_warp): what such a call takes is the serial work of its longest rays.
+constexpr int WTAIL_THREADS = 128;
+#ifndef DST_WTAIL_BLOCKS
+#define DST_WTAIL_BLOCKS 10
+#endif
+template <bool DIAG>
+__global__ void __launch_bounds__(WTAIL_THREADS, DST_WTAIL_BLOCKS) k_fwd_tail_warp(const __grid_constant__ FwdParams p) {
+    __shared__ WalkMem walk_mem[WTAIL_THREADS / 32];
+    __shared__ __align__(16) WarpShade shade_mem[WTAIL_THREADS / 32];
     const int round = first_skipped_round(p.counts, p.rounds, p.min_count);
     const int n = p.counts[round];
     const int* list = p.list[round & 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int warps = gridDim.x * (WTAIL_THREADS / 32);
+    const float absmax = __ldg(p.bvh.header + 6);
+    WarpShade& ws = shade_mem[w];
     TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
     for (int i = blockIdx.x * (WTAIL_THREADS / 32) + w; i < n; i += warps) {
         const int ray = list[i];
         if (ray < 0) continue;
-        FwdState s;
-        if (lane == 0) load_state(p.state, ray, s);
+        if (lane < (int)(sizeof(FwdState) / 16))
+            reinterpret_cast<float4*>(&ws.s)[lane] = reinterpret_cast<const float4*>(reinterpret_cast<const FwdState*>(p.state) + ray)[lane];
+        __syncwarp();
         bool alive = true;
         while (alive) {
             EnumReq q;
-            if (lane == 0) fwd_request(s, q);
-            const float ox = __shfl_sync(FULL, q.ox, 0), oy = __shfl_sync(FULL, q.oy, 0), oz = __shfl_sync(FULL, q.oz, 0);
-            const float dx = __shfl_sync(FULL, q.dx, 0), dy = __shfl_sync(FULL, q.dy, 0), dz = __shfl_sync(FULL, q.dz, 0);
-            const float k0 = __shfl_sync(FULL, q.kmax0, 0);
+            fwd_request(ws.s, q);
             unsigned long long key;
-            const int cnt = knearest_warp<DIAG>(p.bvh, ox, oy, oz, dx, dy, dz, k0, __ldg(p.bvh.header + 6), walk_mem[w], key, p.status, tc);
-            if (lane < DST_CHUNK) wkeys[w][lane] = key;
+            const int cnt = knearest_warp<DIAG>(p.bvh, q.ox, q.oy, q.oz, q.dx, q.dy, q.dz, q.kmax0, absmax, walk_mem[w], key, p.status, tc);
+            alive = fwd_shade_warp<DIAG>(p, ray, ws, key, cnt, tc);
             __syncwarp();
-            bool go = false;
-            if (lane == 0) {
-                if (DIAG) tc.enums++;
-                go = fwd_shade<DIAG, 1>(p, ray, s, wkeys[w], cnt, tc);
-            }
-            alive = __shfl_sync(FULL, go, 0);
         }
     }
     if (DIAG) flush_counters(p.a.counters, tc);
