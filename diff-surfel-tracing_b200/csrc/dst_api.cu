@@ -108,7 +108,7 @@ int dst_destroy(dst_handle* h) {
     if (h->log_needed_event) cudaEventDestroy(h->log_needed_event);
     if (h->rounds_host) cudaFreeHost(h->rounds_host);
     if (h->rounds_event) cudaEventDestroy(h->rounds_event);
-    cudaFree(h->log_keys); cudaFree(h->log_hdr); cudaFree(h->log_count); cudaFree(h->log_seg_head); cudaFree(h->log_ray_ok);
+    cudaFree(h->log_keys); cudaFree(h->log_next); cudaFree(h->log_count); cudaFree(h->log_head); cudaFree(h->log_num); cudaFree(h->log_ok);
     cudaFree(h->wf_state); cudaFree(h->wf_req); cudaFree(h->wf_kbuf); cudaFree(h->wf_kcnt); cudaFree(h->wf_list[0]); cudaFree(h->wf_list[1]); cudaFree(h->wf_counts);
     cudaFree(h->wf_tmp); cudaFree(h->wf_wcnt); cudaFree(h->wf_bcnt);
     cudaFree(h->bound_stats);
@@ -333,7 +333,7 @@ int dst_debug_chunk_log(const dst_handle* h, int64_t* records_wanted, int64_t* r
     if (!h) return DST_E_ARG;
     if (records_wanted) *records_wanted = (h->log_needed_host && h->log_needed_event && cudaEventQuery(h->log_needed_event) == cudaSuccess) ? *h->log_needed_host : -1;
     if (records_held) *records_held = h->log_cap;
-    if (bytes_per_record) *bytes_per_record = 8 * DST_CHUNK + (int64_t)sizeof(int2);
+    if (bytes_per_record) *bytes_per_record = 8 * DST_CHUNK + (int64_t)sizeof(int);
     return DST_OK;
 }
 

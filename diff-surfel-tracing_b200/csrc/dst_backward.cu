@@ -16,8 +16,8 @@ namespace {
 #define DST_BWD_THREADS 128
 #endif
 constexpr int BWD_THREADS = DST_BWD_THREADS;
-#ifndef DST_BWD_LOGGED_BLOCKS
-#define DST_BWD_LOGGED_BLOCKS 1      // resident blocks per SM the logged backward is compiled for
+#ifndef DST_BWD_BLOCKS
+#define DST_BWD_BLOCKS 4               // resident blocks per SM the backward kernels are compiled for
 #endif
 
 struct BwdParams {
@@ -29,8 +29,8 @@ struct BwdParams {
     int tiled, grid_h, grid_w;      // ray order, as in the forward
     int dist_on;                    // depth-distortion extension
     // wavefront scratch
-    void* state;
-    EnumReq* req;
+    float4* state;
+    float4* req;
     unsigned long long* kbuf;
     int* kcnt;
     int* list[2];
@@ -38,17 +38,15 @@ struct BwdParams {
     int min_count;
     int rounds;
     LiveLists lv;
-    // chunk log of the matching forward call (null: not available)
-    const unsigned long long* log_keys; const int2* log_hdr; const int* log_seg_head; const unsigned char* log_ray_ok;
-    int log_seg_stride;
+    // contribution log of the matching forward call, see dst_ensure_log()
+    const unsigned long long* log_keys; const int* log_next; const int* log_head; const int* log_num; const unsigned char* log_ok;
+    long long log_slots;
 };
 
 struct __align__(16) BwdState {
     float sox, soy, soz, sdx;
     float sdy, sdz, offset, dpt;
-    float T_prev, C0, C1, C2;
-    float D, Nx, Ny, Nz;
-    float O0, O1, s_prod, Cp0;
+    float T_prev, rem, s_prod, Cp0;       // rem: what lies behind the hits composited so far, weighted with the upstream gradients (see bwd_chunk)
     float Cp1, Cp2, cp0, cp1;
     float cp2, t_rgb0, t_rgb1, t_rgb2;
     float t_dpt, t_acc, t_aux0, t_aux1;
@@ -59,124 +57,141 @@ struct __align__(16) BwdState {
     int dir_gidx;
     float dm0, dvs, dws;        // distortion term on the primary segment: mapped depth of the first contribution, running sums of w c^2 and w
 };
-static_assert(sizeof(BwdState) == 208, "ray state is thirteen 16-byte words");
-
-__device__ __forceinline__ void red4(float* addr, float a, float b, float c, float d) {
-    atomicAdd(reinterpret_cast<float4*>(addr), make_float4(a, b, c, d));
-}
+static_assert(sizeof(BwdState) == 176, "ray state is eleven 16-byte words");
 
 // ---------------------------------------------------------------------------------------------
 // Gradient rows leave the SM as bulk reductions. A contribution adds an 80-byte row to the packed arena and (with
-// SH colours) a 48- or 192-byte row of coefficient gradients. As vector reductions that is 5 + 12 red.global.add.v4.f32
-// per contribution and lane, and the L2's reduction path is what the kernel then waits for (without the reductions the
-// logged backward of the headline workload takes 13 ms instead of 42). Instead every thread stages its rows in shared
-// memory and hands each to the bulk copy engine as ONE cp.reduce.async.bulk (shared -> global, add.f32): a 192-byte row
-// is one request instead of twelve. Two staging buffers per thread: a row is rewritten only after the engine has read
-// the one staged two contributions earlier (cp.async.bulk.wait_group.read 1). Bulk operations want 16-byte aligned
-// addresses and sizes that are multiples of 16 bytes: arena rows always qualify, SH rows when the gradient tensor is
-// 16-byte aligned and 12 * (degree + 1)^2 is a multiple of 16 (degrees 1 and 3); other rows keep the vector reductions.
+// SH colours) a row of coefficient gradients. As vector reductions those are 5 + 12 red.global.add.v4.f32 per contribution
+// and lane, and the L2's reduction path is what the kernel then waits for. Instead a row is staged in shared memory and handed
+// to the bulk copy engine as ONE cp.reduce.async.bulk (shared -> global, add.f32). Bulk operations want 16-byte aligned
+// addresses and sizes that are multiples of 16 bytes: arena rows always qualify, SH rows when the gradient tensor is 16-byte
+// aligned and 12 * (degree + 1)^2 is a multiple of 16 (degrees 1 and 3); other SH rows are added with scalar reductions.
+//
+// The lanes of a warp are neighbouring pixels that composite their chunks in step, so at one point of the hit loop most of
+// them hold one of a handful of surfels. Their rows are summed in shared memory and leave as one. An SH row is the product of the 16
+// basis values of the ray's direction, which stay the same for a whole segment, and three colour gradients: a lane stages the three,
+// and the sum over the lanes of a group is formed from them and the basis values in shared memory.
 // ---------------------------------------------------------------------------------------------
-#ifndef DST_BWD_BULK
-#define DST_BWD_BULK 1
-#endif
 constexpr int STAGE_FLOATS = DST_ARENA_FLOATS + 48;                       // arena row + the longest SH row
-constexpr size_t BWD_STAGE_BYTES = 2ull * BWD_THREADS * STAGE_FLOATS * 4;  // dynamic shared memory of every backward kernel
-
-struct BulkStage {
-    float* base;        // this thread's two staging rows (shared memory), STAGE_FLOATS each
-    unsigned int n;     // rows handed over so far
+struct BwdWarp {
+    float rows[32][STAGE_FLOATS];       // lane's arena row; SH row of the lanes that send one
+    float4 colour[32];                  // colour gradients of the lane's contribution (clamped channels 0)
+    float basis[16][33];                // SH basis of the lane's segment direction, one column per lane
 };
-__device__ __forceinline__ BulkStage bulk_stage_init(unsigned char* dyn_smem) {
-    BulkStage b;
-    b.base = reinterpret_cast<float*>(dyn_smem) + (size_t)threadIdx.x * STAGE_FLOATS;
-    b.n = 0;
-    return b;
-}
-// the row to fill next (waits until the engine has read what it held)
-__device__ __forceinline__ float* bulk_stage_row(BulkStage& b) {
-    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-    return b.base + (size_t)(b.n & 1u) * BWD_THREADS * STAGE_FLOATS;
-}
+constexpr size_t BWD_STAGE_BYTES = sizeof(BwdWarp) * (BWD_THREADS / 32);   // dynamic shared memory of every backward kernel
+
 // adds `bytes` bytes of floats at shared-memory `src` to global `dst` (both 16-byte aligned, bytes a multiple of 16)
 __device__ __forceinline__ void bulk_add(float* dst, const float* src, int bytes) {
     const unsigned int s = (unsigned int)__cvta_generic_to_shared(src);
     asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" :: "l"(dst), "r"(s), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void bulk_stage_commit(BulkStage& b) {
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    b.n++;
-}
-// Rows of the same surfel staged by several lanes of a warp are summed in shared memory before they leave, and only
-// the lowest lane of each group hands its (summed) row to the engine. The lanes of a warp are neighbouring pixels that
-// walk their chunk logs in step, so at one point of the loop most of them hold one of a handful of surfels; without the
-// summing every lane's row is an addition of its own at the L2, which serialises additions to one address (the
-// reductions were 11 of the backward's 26 ms on the 3M-surfel 1080p workload). The lanes that are here together split the
-// 17 float4 columns of a row between them and each sums its columns over the rows of a group, in lane order.
-// gidx < 0: this lane has no row. Returns true for the lanes that send their row.
-#ifndef DST_BWD_AGGREGATE
-#define DST_BWD_AGGREGATE 1
-#endif
-__device__ __forceinline__ bool bulk_stage_aggregate(const BulkStage& b, int gidx) {
-#if DST_BWD_AGGREGATE
-    const unsigned int act = __activemask();
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }      // the engine has read this lane's rows
+__device__ __forceinline__ void bulk_drain() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }               // ... and added them: before the kernel ends
+__device__ __forceinline__ void bulk_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }            // staged values become visible to the engine
+
+struct RowTarget { float* arena; float* dsh; int coeffs, ncoef; bool bulk; };       // dsh null: no SH colours
+
+// Sends the contributions staged by the lanes with gidx >= 0 (the others pass -1); called by all 32 lanes. `group`: sum the rows of
+// lanes with the same surfel where neighbours do hold the same ones: when fewer than three quarters of the rows have the surfel of
+// the lane next door, every lane sends its own (grouping costs more than it saves where surfels are small against the pixel spacing).
+__device__ __forceinline__ void send_rows(const RowTarget& t, BwdWarp& ws, int gidx, bool group) {
+    constexpr unsigned int FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const unsigned int staged = __ballot_sync(act, gidx >= 0);           // lanes without a row pass -1 and form a group that is skipped
-    // Worth it only where neighbouring pixels do hold the same surfels: when fewer than three quarters of the rows have the
-    // surfel of the lane next door, every lane sends its own row (grouping costs more than it saves on scenes whose
-    // surfels are small against the pixel spacing).
-    const int next_door = __shfl_xor_sync(act, gidx, 1);
-    const unsigned int paired = __ballot_sync(act, gidx >= 0 && ((act >> (lane ^ 1)) & 1u) != 0u && next_door == gidx);
-    if (4 * __popc(paired) < 3 * __popc(staged)) return gidx >= 0;
-    const unsigned int peers = __match_any_sync(act, gidx);
-    const int first = __ffs(peers) - 1;
-    const unsigned int leaders = __ballot_sync(act, lane == first) & staged;
-    const unsigned int parity = __ballot_sync(act, (b.n & 1u) != 0u);
-    __syncwarp(act);                                                     // every lane's row is staged
-    if (leaders != staged) {                                              // some surfel is held by more than one lane
-        float* warp_rows = b.base - (size_t)lane * STAGE_FLOATS;         // buffer 0 of lane 0
-        const int rank = __popc(act & ((1u << lane) - 1u)), nact = __popc(act);
-        for (unsigned int todo = leaders; todo; todo &= todo - 1u) {
-            const int lead = __ffs(todo) - 1;
-            const unsigned int grp = __shfl_sync(act, peers, lead);
-            if ((grp & (grp - 1u)) == 0u) continue;                      // a lane alone with its surfel
-            for (int col = rank; col < STAGE_FLOATS / 4; col += nact) {
-                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const unsigned int staged = __ballot_sync(FULL, gidx >= 0);
+    if (staged == 0u) return;
+    unsigned int peers = 1u << lane;
+    if (group) {
+        const int next_door = __shfl_xor_sync(FULL, gidx, 1);
+        const unsigned int paired = __ballot_sync(FULL, gidx >= 0 && next_door == gidx);
+        if (4 * __popc(paired) >= 3 * __popc(staged)) peers = __match_any_sync(FULL, gidx);
+    }
+    const bool alone = gidx >= 0 && (peers & (peers - 1u)) == 0u;
+    if (t.dsh && alone) {       // a row of its own
+        const float4 m = ws.colour[lane];
+        if (t.bulk) {
+            float4* o = reinterpret_cast<float4*>(ws.rows[lane] + DST_ARENA_FLOATS);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {       // four basis values are three float4 of the row
+                if (4 * q < t.ncoef) {
+                    const float b0 = ws.basis[4 * q][lane], b1 = ws.basis[4 * q + 1][lane], b2 = ws.basis[4 * q + 2][lane], b3 = ws.basis[4 * q + 3][lane];
+                    o[3 * q] = make_float4(b0 * m.x, b0 * m.y, b0 * m.z, b1 * m.x);
+                    o[3 * q + 1] = make_float4(b1 * m.y, b1 * m.z, b2 * m.x, b2 * m.y);
+                    o[3 * q + 2] = make_float4(b2 * m.z, b3 * m.x, b3 * m.y, b3 * m.z);
+                }
+            }
+        } else {
+            float* d = t.dsh + 3 * (size_t)gidx * t.coeffs;
+            for (int j = 0; j < t.ncoef; j++) {
+                const float b = ws.basis[j][lane];
+                atomicAdd(d + 3 * j, b * m.x); atomicAdd(d + 3 * j + 1, b * m.y); atomicAdd(d + 3 * j + 2, b * m.z);
+            }
+        }
+    }
+    const bool leader = gidx >= 0 && lane == __ffs(peers) - 1;
+    __syncwarp();                                                        // every lane's row is staged
+    for (unsigned int todo = __ballot_sync(FULL, leader && !alone); todo; todo &= todo - 1u) {
+        const int lead = __ffs(todo) - 1;
+        const unsigned int grp = __shfl_sync(FULL, peers, lead);
+        {   // arena row: lane c sums float c of the group's rows
+            float acc = 0.0f;
+            const float* col = &ws.rows[0][lane < DST_ARENA_FLOATS ? lane : 0];
+            if (grp == FULL) {
+#pragma unroll 8
+                for (int r = 0; r < 32; r++) acc += col[r * STAGE_FLOATS];
+            } else {
                 for (unsigned int q = grp; q;) {                         // four rows per pass, so that their loads are in flight together
                     const int r0 = __ffs(q) - 1; q &= q - 1u;
                     const int r1 = __ffs(q) - 1; q &= q - 1u;
                     const int r2 = __ffs(q) - 1; q &= q - 1u;
                     const int r3 = __ffs(q) - 1; q &= q - 1u;
-#define DST_STAGED(r) reinterpret_cast<const float4*>(warp_rows + ((r) + (int)((parity >> (r)) & 1u) * BWD_THREADS) * STAGE_FLOATS)[col]
-                    const float4 x0 = DST_STAGED(r0);
-                    const float4 x1 = r1 >= 0 ? DST_STAGED(r1) : zero;
-                    const float4 x2 = r2 >= 0 ? DST_STAGED(r2) : zero;
-                    const float4 x3 = r3 >= 0 ? DST_STAGED(r3) : zero;
-#undef DST_STAGED
-                    acc.x += (x0.x + x1.x) + (x2.x + x3.x); acc.y += (x0.y + x1.y) + (x2.y + x3.y);
-                    acc.z += (x0.z + x1.z) + (x2.z + x3.z); acc.w += (x0.w + x1.w) + (x2.w + x3.w);
+                    const float x0 = col[r0 * STAGE_FLOATS], x1 = r1 >= 0 ? col[r1 * STAGE_FLOATS] : 0.0f;
+                    const float x2 = r2 >= 0 ? col[r2 * STAGE_FLOATS] : 0.0f, x3 = r3 >= 0 ? col[r3 * STAGE_FLOATS] : 0.0f;
+                    acc += (x0 + x1) + (x2 + x3);
                 }
-                reinterpret_cast<float4*>(warp_rows + (lead + (int)((parity >> lead) & 1u) * BWD_THREADS) * STAGE_FLOATS)[col] = acc;
+            }
+            if (lane < DST_ARENA_FLOATS) ws.rows[lead][lane] = acc;
+        }
+        if (t.dsh) {   // SH row: lane (j, half) sums coefficient j over the lanes 16 half .. 16 half + 15 of the group
+            const int j = lane & 15, g = __shfl_sync(FULL, gidx, lead);
+            float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
+            const unsigned int half = (lane >> 4) * 16;
+            unsigned int q = (grp >> half) & 0xffffu;
+            if (grp == FULL) {
+#pragma unroll 8
+                for (int r = 0; r < 16; r++) {
+                    const float4 m = ws.colour[half + r];
+                    const float b = ws.basis[j][half + r];
+                    a0 = fmaf(b, m.x, a0); a1 = fmaf(b, m.y, a1); a2 = fmaf(b, m.z, a2);
+                }
+            } else {
+                while (q) {
+                    const int r = __ffs(q) - 1; q &= q - 1u;
+                    const float4 m = ws.colour[half + r];
+                    const float b = ws.basis[j][half + r];
+                    a0 = fmaf(b, m.x, a0); a1 = fmaf(b, m.y, a1); a2 = fmaf(b, m.z, a2);
+                }
+                __syncwarp();
+            }
+            a0 += __shfl_xor_sync(FULL, a0, 16); a1 += __shfl_xor_sync(FULL, a1, 16); a2 += __shfl_xor_sync(FULL, a2, 16);
+            if (lane < t.ncoef) {       // (ncoef <= 16: lanes of half 0)
+                if (t.bulk) {
+                    float* o = ws.rows[lead] + DST_ARENA_FLOATS + 3 * j;
+                    o[0] = a0; o[1] = a1; o[2] = a2;
+                } else {
+                    float* d = t.dsh + 3 * ((size_t)g * t.coeffs + j);
+                    atomicAdd(d, a0); atomicAdd(d + 1, a1); atomicAdd(d + 2, a2);
+                }
             }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp(act);                                                 // the sums are in place
     }
-    return lane == first && gidx >= 0;
-#else
-    return true;
-#endif
-}
-// before the kernel ends: every row has been read from shared memory and added
-__device__ __forceinline__ void bulk_stage_drain() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
-// The colour of a contribution as the backward needs it: a factor of gradients, not an input of a decision, so the sum
-// may be fused (the forward's sh_channel() rounds every product and sum as the reference does: twice the instructions).
-__device__ __forceinline__ float sh_channel_fused(int ncoef, const float* b, const float* c, int ch) {
-    float r = b[0] * c[ch];
-#pragma unroll
-    for (int j = 1; j < 16; j++) if (j < ncoef) r = fmaf(b[j], c[3 * j + ch], r);
-    return r + 0.5f;
+    bulk_fence();
+    __syncwarp();                                                        // the sums are in place
+    if (leader) {
+        bulk_add(t.arena + (size_t)gidx * DST_ARENA_FLOATS, ws.rows[lane], DST_ARENA_FLOATS * 4);
+        if (t.bulk) bulk_add(t.dsh + 3 * (size_t)gidx * t.coeffs, ws.rows[lane] + DST_ARENA_FLOATS, 12 * t.ncoef);
+        bulk_commit();
+    }
 }
 
 struct V3 { float x, y, z; };
@@ -232,17 +247,15 @@ __device__ __forceinline__ V3 sh_dir_grad(int deg, const float* s, float x, floa
 }
 
 
-__device__ __forceinline__ void bwd_load_state(const void* base, int ray, BwdState& s) {
-    const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const BwdState*>(base) + ray);
+__device__ __forceinline__ void bwd_load_state(const float4* base, int slot, BwdState& s) {
     float4* dst = reinterpret_cast<float4*>(&s);
 #pragma unroll
-    for (int i = 0; i < 13; i++) dst[i] = src[i];
+    for (int i = 0; i < 11; i++) dst[i] = base[soa(slot, i, 11)];
 }
-__device__ __forceinline__ void bwd_store_state(void* base, int ray, const BwdState& s) {
-    float4* dst = reinterpret_cast<float4*>(reinterpret_cast<BwdState*>(base) + ray);
+__device__ __forceinline__ void bwd_store_state(float4* base, int slot, const BwdState& s) {
     const float4* src = reinterpret_cast<const float4*>(&s);
 #pragma unroll
-    for (int i = 0; i < 13; i++) dst[i] = src[i];
+    for (int i = 0; i < 11; i++) base[soa(slot, i, 11)] = src[i];
 }
 
 __device__ __forceinline__ void bwd_request(const BwdState& s, EnumReq& q) {
@@ -303,7 +316,10 @@ __device__ __forceinline__ bool bwd_next_segment(const BwdParams& p, int ray, Bw
         s.drd_x = drd.x; s.drd_y = drd.y; s.drd_z = drd.z;
         s.sox = m0.x; s.soy = m0.y; s.soz = m0.z; s.sdx = sdx; s.sdy = sdy; s.sdz = sdz;
         s.offset = 0.f; s.dpt = 0.f; s.T_prev = 1.f;
-        s.C0 = s.C1 = s.C2 = 0.f; s.D = 0.f; s.Nx = s.Ny = s.Nz = 0.f; s.O0 = s.O1 = 0.f;
+        // everything the segment composited, and the background seen through it (counted a second time, as the reference does, :545-548)
+        s.rem = s.t_rgb0 * tot_c0 + s.t_rgb1 * tot_c1 + s.t_rgb2 * tot_c2 + s.t_aux0 * tot_o0 + s.t_aux1 * m3.x + s.t_dpt * tot_dpt +
+                (t_norm.x * tot_n.x + t_norm.y * tot_n.y + t_norm.z * tot_n.z) + s.t_acc * m1.w +
+                (1.0f - m1.w) * (s.t_rgb0 * __ldg(in.background) + s.t_rgb1 * __ldg(in.background + 1) + s.t_rgb2 * __ldg(in.background + 2));
         s.last_gidx = -1; s.contributor = 0; s.chunk = 0; s.seg = i; s.dir_gidx = -1;
         s.dm0 = s.dvs = s.dws = 0.f;
         return true;
@@ -332,380 +348,248 @@ __device__ __forceinline__ bool bwd_init_state(const BwdParams& p, int ray, BwdS
     return bwd_next_segment(p, ray, s, in.max_trace_depth);
 }
 
-// b[j] for a run-time j without indexing the array (which would move it from registers to local memory)
-__device__ __forceinline__ float basis_at(const float* b, int j) {
-    float r = b[0];
-#pragma unroll
-    for (int k = 1; k < 16; k++) r = (j == k) ? b[k] : r;
-    return r;
-}
+// what the hits of one ray segment have in common
+struct BwdSegment { bool use_sh, has_aux, sh_aligned, dist_on; int ncoef; float tot_acc, t_dist, dist_mu, dist_V; };
 
-// Re-composites one gathered chunk of segment s.seg and accumulates the gradients of every
-// contributing hit (backward.cu:429-655). Returns true while the ray needs another enumeration.
-template <bool DIAG, int KS, bool DIST>
-__device__ __forceinline__ bool bwd_shade(const BwdParams& p, int ray, BwdState& s, const unsigned long long* kb, int cnt, TraceCounters& tc, BulkStage& stage) {
+// Called by the lanes with `in` at the start of a chunk / segment; writes the lane's SH basis.
+template <bool DIST>
+__device__ __forceinline__ BwdSegment bwd_segment(const BwdParams& p, bool in_seg, int ray, const BwdState& s, BwdWarp& ws) {
     const dst_trace_inputs& in = p.a.in;
-    const bool use_sh = in.colors_precomp == nullptr;
-    const bool has_aux = in.others_precomp != nullptr;
-    const int ncoef = (in.sh_degree + 1) * (in.sh_degree + 1);
-    const bool sh_aligned = ((in.sh_coeffs * 3) & 3) == 0 && ((reinterpret_cast<uintptr_t>(in.shs) & 15) == 0);
-    const bool dsh_aligned = ((in.sh_coeffs * 3) & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.a.dL_dshs) & 15) == 0);
-    const float bg0 = __ldg(in.background), bg1 = __ldg(in.background + 1), bg2 = __ldg(in.background + 2);
-    const float4* mp = reinterpret_cast<const float4*>(p.a.mid_val + (size_t)ray * in.mid_stride + s.seg * DST_MID_CHANNELS);
-    const float4 m1 = __ldg(mp + 1), m2 = __ldg(mp + 2), m3 = __ldg(mp + 3);
-    const float tot_dpt = m1.z, tot_acc = m1.w;
-    const V3 tot_n = v3(m2.x, m2.y, m2.z);
-    const float tot_o0 = m2.w, tot_o1 = m3.x, tot_c0 = m3.y, tot_c1 = m3.z, tot_c2 = m3.w;
-    const float sox = s.sox, soy = s.soy, soz = s.soz, sdx = s.sdx, sdy = s.sdy, sdz = s.sdz;
-    const float t_rgb0 = s.t_rgb0, t_rgb1 = s.t_rgb1, t_rgb2 = s.t_rgb2, t_dpt = s.t_dpt, t_acc = s.t_acc, t_aux0 = s.t_aux0, t_aux1 = s.t_aux1;
-    const V3 t_norm = v3(s.t_nx, s.t_ny, s.t_nz);
-    const float min_depth = s.seg == 0 ? (in.start_from_first ? 0.2f : 0.0f) : 0.06f;
-    const float T_threshold = 0.0001f;
-    const float T_final = 1.0f - tot_acc;
-    float C0 = s.C0, C1 = s.C1, C2 = s.C2, D = s.D, O0 = s.O0, O1 = s.O1;
-    V3 N = v3(s.Nx, s.Ny, s.Nz);
-    float T_prev = s.T_prev, T_next = 1.0f, dpt = s.dpt;
-    const float offset = s.offset;
-    int last_gidx = s.last_gidx, contributor = s.contributor;
-    V3 dL_dray_o = v3(s.dro_x, s.dro_y, s.dro_z), dL_dray_d = v3(s.drd_x, s.drd_y, s.drd_z);
-    int dir_gidx = s.dir_gidx; float dir_g0 = s.dir_g0, dir_g1 = s.dir_g1, dir_g2 = s.dir_g2;
-    float sb[16];
-    if (use_sh) sh_basis(in.sh_degree, sdx, sdy, sdz, sb);
-    if (DIAG) { if (s.chunk == 0) tc.segs++; }
+    BwdSegment x;
+    x.use_sh = in.colors_precomp == nullptr;
+    x.has_aux = in.others_precomp != nullptr;
+    x.ncoef = (in.sh_degree + 1) * (in.sh_degree + 1);
+    x.sh_aligned = (in.sh_coeffs & 3) == 0 && ((reinterpret_cast<uintptr_t>(in.shs) & 15) == 0);
+    x.dist_on = false; x.tot_acc = x.t_dist = x.dist_mu = x.dist_V = 0.f;
+    if (x.use_sh && in_seg) {
+        float sb[16];
+        sh_basis(in.sh_degree, s.sdx, s.sdy, s.sdz, sb);
+#pragma unroll
+        for (int j = 0; j < 16; j++) if (j < x.ncoef) ws.basis[j][threadIdx.x & 31] = sb[j];
+    }
     // Distortion extension (primary segment only; see fwd_shade): upstream gradient, the totals the forward saved, the
     // running sums. With W = sum w (the accumulated opacity), mu = M1 / W, c_k = m_k - mu, V = M2 - M1^2 / W = sum w c^2:
     // d dist / d m_k = 2 w_k W c_k, d dist / d w_k = W c_k^2 + V, and what lies behind hit k enters through the
     // transmittance: sum_{i>k} (d dist / d w_i) w_i = W (V - V_k) + V (W - W_k) with the running sums through k.
-    const bool dist_on = DIST && s.seg == 0 && p.a.dL_ddist && p.a.out_dist && tot_acc > 0.0f;
-    const float t_dist = dist_on ? __ldg(p.a.dL_ddist + ray) : 0.f;
-    const float dist_mu = dist_on ? __ldg(p.a.out_dist + 3 * (size_t)ray + 1) / tot_acc : 0.f;
-    const float dist_V = dist_on ? __ldg(p.a.out_dist + 3 * (size_t)ray + 2) - __ldg(p.a.out_dist + 3 * (size_t)ray + 1) * dist_mu : 0.f;
-    float dm0 = s.dm0, dvs = s.dvs, dws = s.dws;
-
-    bool stop = false;
-    for (int sl = 0; sl < cnt; sl++) {
-        // One pass of the body per hit; a hit that does not contribute leaves it early. The lanes of the warp meet again
-        // behind it, where the rows of the lanes that did contribute are summed per surfel and sent.
-        bool staged = false;
-        int gsent = -1;
-        float4* st = nullptr;
-        do {
-        const unsigned long long key = kb[sl * KS];
-        const int pidx = (int)(unsigned int)key;
-        const int gidx = pidx >> 1;
-        if (gidx == last_gidx) break;
-        if (DIAG) tc.evals++;
-        SlotEval e;
-        const bool ok = eval_slot(key, offset, sox, soy, soz, sdx, sdy, sdz, min_depth, p.cache, gidx, e);
-        dpt = e.dpt;
-        if (!ok) break;
-        const float alpha = e.alpha;
-        T_next = xmul(T_prev, xsub(1.0f, alpha));
-        if (T_next < T_threshold) { stop = true; break; }
-        contributor++;
-        if (contributor > DST_MAX_INTERSECTION) { stop = true; break; }
-        last_gidx = gidx;
-        if (DIAG) tc.contribs++;
-        const float w = xmul(alpha, T_prev);
-        const V3 normal = v3(e.nsign * e.r2.x, e.nsign * e.r2.y, e.nsign * e.r2.z);
-        float c0, c1, c2, k0 = 1.f, k1 = 1.f, k2 = 1.f;       // colour and its clamp mask
-        float csh[48];
-        float pc0 = 0.f, pc1 = 0.f, pc2 = 0.f;
-        if (use_sh) load_sh_row(in.shs + 3 * (size_t)gidx * in.sh_coeffs, 3 * ncoef, sh_aligned, csh);
-        else { const float* cp = in.colors_precomp + 3 * (size_t)gidx; pc0 = __ldg(cp); pc1 = __ldg(cp + 1); pc2 = __ldg(cp + 2); }
-        float2 ax = make_float2(0.f, 0.f);
-        if (has_aux) ax = __ldg(reinterpret_cast<const float2*>(in.others_precomp) + gidx);
-        const float4* vq = reinterpret_cast<const float4*>(in.vertices + 12 * (size_t)gidx);
-        const float4 va = __ldg(vq), vb = __ldg(vq + 1), vc = __ldg(vq + 2);
-        const V3 pm = v3(__ldg(in.means3D + 3 * (size_t)gidx), __ldg(in.means3D + 3 * (size_t)gidx + 1), __ldg(in.means3D + 3 * (size_t)gidx + 2));
-        const float4 q = __ldg(reinterpret_cast<const float4*>(in.rotations) + gidx);
-        if (use_sh) {
-            c0 = sh_channel_fused(ncoef, sb, csh, 0); c1 = sh_channel_fused(ncoef, sb, csh, 1); c2 = sh_channel_fused(ncoef, sb, csh, 2);
-            k0 = c0 < 0.f ? 0.f : 1.f; k1 = c1 < 0.f ? 0.f : 1.f; k2 = c2 < 0.f ? 0.f : 1.f;
-            c0 = fmaxf(c0, 0.f); c1 = fmaxf(c1, 0.f); c2 = fmaxf(c2, 0.f);
-        } else { c0 = pc0; c1 = pc1; c2 = pc2; }
-        C0 = xadd(C0, xmul(w, c0)); C1 = xadd(C1, xmul(w, c1)); C2 = xadd(C2, xmul(w, c2));
-        float ox0 = 0.f, ox1 = 0.f;
-        if (has_aux) {
-            ox0 = ax.x; ox1 = ax.y;
-            O0 = xadd(O0, xmul(w, ox0)); O1 = xadd(O1, xmul(w, ox1));
+    if (DIST && in_seg && s.seg == 0 && p.a.dL_ddist && p.a.out_dist) {
+        x.tot_acc = __ldg(p.a.mid_val + (size_t)ray * in.mid_stride + 7);
+        if (x.tot_acc > 0.0f) {
+            x.dist_on = true;
+            x.t_dist = __ldg(p.a.dL_ddist + ray);
+            x.dist_mu = __ldg(p.a.out_dist + 3 * (size_t)ray + 1) / x.tot_acc;
+            x.dist_V = __ldg(p.a.out_dist + 3 * (size_t)ray + 2) - __ldg(p.a.out_dist + 3 * (size_t)ray + 1) * x.dist_mu;
         }
-        D = xadd(D, xmul(w, dpt));
-        N.x = xadd(N.x, xmul(w, normal.x)); N.y = xadd(N.y, xmul(w, normal.y)); N.z = xadd(N.z, xmul(w, normal.z));
+    }
+    return x;
+}
+__device__ __forceinline__ RowTarget row_target(const BwdParams& p) {
+    const dst_trace_inputs& in = p.a.in;
+    RowTarget t;
+    t.arena = p.arena; t.dsh = in.colors_precomp == nullptr ? p.a.dL_dshs : nullptr; t.coeffs = in.sh_coeffs;
+    t.ncoef = (in.sh_degree + 1) * (in.sh_degree + 1);
+    t.bulk = t.dsh && (in.sh_coeffs & 3) == 0 && (t.ncoef & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.a.dL_dshs) & 15) == 0);
+    return t;
+}
 
-        // gradient w.r.t. alpha from every composited quantity (backward.cu:529-568)
-        const float inv = 1.0f / (1.0f - alpha);
-        float dL_dalpha = t_rgb0 * (T_prev * c0 - (tot_c0 - C0) * inv) + t_rgb1 * (T_prev * c1 - (tot_c1 - C1) * inv) +
-                          t_rgb2 * (T_prev * c2 - (tot_c2 - C2) * inv);
-        dL_dalpha += (t_rgb0 * bg0 + t_rgb1 * bg1 + t_rgb2 * bg2) * (-T_final * inv);   // background counted a second time, as the reference does
-        if (has_aux) dL_dalpha += t_aux0 * (T_prev * ox0 - (tot_o0 - O0) * inv) + t_aux1 * (T_prev * ox1 - (tot_o1 - O1) * inv);
-        dL_dalpha += t_dpt * (T_prev * dpt - (tot_dpt - D) * inv);
-        dL_dalpha += t_norm.x * (T_prev * normal.x - (tot_n.x - N.x) * inv) + t_norm.y * (T_prev * normal.y - (tot_n.y - N.y) * inv) +
-                     t_norm.z * (T_prev * normal.z - (tot_n.z - N.z) * inv);
-        dL_dalpha += t_acc * (T_prev - tot_acc * inv);      // the reference's running weight sum stays 0 (backward.cu:359, 568)
-        float dist_dd = 0.f;       // gradient of the distortion with respect to this hit's depth
-        if (DIST && dist_on) {
-            const float m_abs = DST_DIST_K * (1.0f - DST_DIST_NEAR / dpt);
-            if (contributor == 1) dm0 = m_abs;
-            const float cm = (m_abs - dm0) - dist_mu;
-            dws += w; dvs += w * cm * cm;
-            const float d_dw = tot_acc * cm * cm + dist_V;
-            const float behind = tot_acc * (dist_V - dvs) + dist_V * (tot_acc - dws);
-            dL_dalpha += t_dist * (d_dw * T_prev - behind * inv);
-            dist_dd = t_dist * 2.0f * w * tot_acc * cm * DST_DIST_K * DST_DIST_NEAR / (dpt * dpt);
-        }
-
-        const float opac = e.r2.w, G = e.G;
-        const float dL_dG = dL_dalpha * opac;
-        const float pc = (opac * G) > 0.99f ? 0.0f : 1.0f;
-        const float dL_dopac = dL_dalpha * G * pc;
-
-        // geometry (backward.cu:201-287, 581-607)
-        const float sx = e.r3.x, sy = e.r3.y, u = e.u, v = e.v;
-        const V3 R0 = v3(e.r0.x, e.r0.y, e.r0.z), R1 = v3(e.r1.x, e.r1.y, e.r1.z);
-        const V3 rel = v3(e.X - pm.x, e.Y - pm.y, e.Z - pm.z);
-        const float kk = dL_dG * pc;
-        const float dL_du = kk * -G * u, dL_dv = kk * -G * v;
-        V3 dR0 = (dL_du / sx) * rel, dR1 = (dL_dv / sy) * rel;
-        const V3 dR2 = v3(t_norm.x * w * e.nsign, t_norm.y * w * e.nsign, t_norm.z * w * e.nsign);
-        float dsx = kk * (G * u * u / sx), dsy = kk * (G * v * v / sy);
-        V3 dmean = (kk * G) * ((u / sx) * R0 + (v / sy) * R1);
-        const V3 dxyz = (dL_du / sx) * R0 + (dL_dv / sy) * R1;
-        const V3 rd = v3(sdx, sdy, sdz), ro = v3(sox, soy, soz);
-        const float dL_dd = t_dpt * w + dist_dd + dot(dxyz, rd);
-        V3 p1, p2, p3; float h1x, h1y, h2x, h2y, h3x, h3y;
-        {
-            if ((pidx & 1) == 0) {
-                p1 = v3(va.x, va.y, va.z); p2 = v3(va.w, vb.x, vb.y); p3 = v3(vb.z, vb.w, vc.x);
-                h1x = -3.f; h1y = 3.f; h2x = -3.f; h2y = -3.f; h3x = 3.f; h3y = 3.f;
-            } else {
-                p1 = v3(va.w, vb.x, vb.y); p2 = v3(vb.z, vb.w, vc.x); p3 = v3(vc.y, vc.z, vc.w);
-                h1x = -3.f; h1y = -3.f; h2x = 3.f; h2y = 3.f; h3x = 3.f; h3y = -3.f;
-            }
-        }
-        const V3 n = cross(p2 - p1, p3 - p1);
-        const V3 cvec = p1 - ro;
-        const float pp = dot(n, cvec), qq = dot(n, rd);
-        const float iq = 1.0f / qq;
-        const V3 dn = iq * (cvec - (pp * iq) * rd);
-        const V3 dv1 = dL_dd * cross(p2 - p3, dn) + (dL_dd * iq) * n;
-        const V3 dv2 = dL_dd * cross(p3 - p1, dn);
-        const V3 dv3 = dL_dd * cross(p1 - p2, dn);
-        dL_dray_o = dL_dray_o + dxyz - (dL_dd * iq) * n;
-        if (!use_sh) dL_dray_d = dL_dray_d + dpt * dxyz - (dL_dd * pp * iq * iq) * n;   // with SH the value is replaced below
-        const V3 shx = h1x * dv1 + h2x * dv2 + h3x * dv3, shy = h1y * dv1 + h2y * dv2 + h3y * dv3;
-        dR0 = dR0 + sx * shx; dR1 = dR1 + sy * shy;
-        dsx += dot(R0, shx); dsy += dot(R1, shy);
-        dmean = dmean + dv1 + dv2 + dv3;
-        // quaternion (auxiliary.h:433-477; no gradient through the normalisation)
-        const float qs = rsqrtf(q.w * q.w + q.x * q.x + q.y * q.y + q.z * q.z);
-        const float qw = q.x * qs, qx = q.y * qs, qy = q.z * qs, qz = q.w * qs;
-        const float dq0 = 2.f * (qx * (dR1.z - dR2.y) + qy * (dR2.x - dR0.z) + qz * (dR0.y - dR1.x));
-        const float dq1 = 2.f * (-2.f * qx * (dR1.y + dR2.z) + qy * (dR0.y + dR1.x) + qz * (dR0.z + dR2.x) + qw * (dR1.z - dR2.y));
-        const float dq2 = 2.f * (qx * (dR0.y + dR1.x) - 2.f * qy * (dR0.x + dR2.z) + qz * (dR1.z + dR2.y) + qw * (dR2.x - dR0.z));
-        const float dq3 = 2.f * (qx * (dR0.z + dR2.x) + qy * (dR1.z + dR2.y) - 2.f * qz * (dR0.x + dR1.y) + qw * (dR0.y - dR1.x));
-
-        // per-surfel accumulation (backward.cu:543, 557, 578, 610-626)
-#if !DST_BWD_BULK
-        float* row = p.arena + (size_t)gidx * DST_ARENA_FLOATS;
-#endif
-        const float hd = 0.5f * dpt;
-        const float dc0 = t_rgb0 * w, dc1 = t_rgb1 * w, dc2 = t_rgb2 * w;
-        const float m0c = dc0 * k0, m1c = dc1 * k1, m2c = dc2 * k2;
-        const int nf = 3 * ncoef, nv = nf >> 2;
-        float* dsh = use_sh ? p.a.dL_dshs + 3 * (size_t)gidx * in.sh_coeffs : nullptr;
-#if DST_BWD_BULK
-        {
-            st = reinterpret_cast<float4*>(bulk_stage_row(stage));
-            st[0] = make_float4(dq0, dq1, dq2, dq3);
-            st[1] = make_float4(dmean.x, dmean.y, dmean.z, dL_dopac);
-            st[2] = make_float4(dmean.x * hd, dmean.y * hd, dmean.z * hd, 0.f);
-            st[3] = make_float4(dsx, dsy, has_aux ? t_aux0 * w : 0.f, has_aux ? t_aux1 * w : 0.f);
-            st[4] = make_float4(dc0, dc1, dc2, 0.f);
-            const bool sh_bulk = use_sh && dsh_aligned && (nf & 3) == 0;
-            if (sh_bulk) {
+// Gradients of one contributing hit (backward.cu:529-632), staged in ws for send_rows(). e: the evaluated hit.
+//
+// The reference differentiates each composited quantity on its own. All of them are sums of w f over the hits, so the gradient of a hit's alpha
+// needs only F = (upstream gradients) . (what the hit contributes) and the one running value s.rem = (upstream gradients) . (totals of the
+// segment, background and opacity included) - sum of w F so far: dL/dalpha = T (F + t_acc) - rem / (1 - alpha). The vertex terms are
+// written in the edges e1, e2 of the triangle at one corner: the gradients of the three corners add up to E n, and their
+// moments with the corner signs (the gradients of the scaled tangents) to 6 E e x h -+ 3 E n. Both are the reference's
+// sums in exact arithmetic with a fraction of the operations.
+template <bool DIST>
+__device__ __forceinline__ void bwd_hit(const BwdParams& p, BwdState& s, const BwdSegment& x, const SlotEval& e, int pidx, bool first, BwdWarp& ws) {
+    const dst_trace_inputs& in = p.a.in;
+    const int lane = threadIdx.x & 31, gidx = pidx >> 1;
+    const float alpha = e.alpha, T_prev = s.T_prev, dpt = e.dpt;
+    const float w = xmul(alpha, T_prev);
+    float F = s.t_dpt * dpt + e.nsign * (s.t_nx * e.r2.x + s.t_ny * e.r2.y + s.t_nz * e.r2.z);
+    float m0 = s.t_rgb0 * w, m1 = s.t_rgb1 * w, m2 = s.t_rgb2 * w;
+    float4* row = reinterpret_cast<float4*>(ws.rows[lane]);
+    bulk_wait_read();                                          // the engine has read what this lane's row held
+    row[4] = make_float4(m0, m1, m2, 0.f);
+    if (x.use_sh) {
+        float c0 = 0.5f, c1 = 0.5f, c2 = 0.5f;
+        const float* sh = in.shs + 3 * (size_t)gidx * in.sh_coeffs;
 #pragma unroll
-                for (int q4 = 0; q4 < 12; q4++) {
-                    if (q4 < nv) {
-                        float o4[4];
+        for (int q = 0; q < 4; q++) {
+            if (4 * q < x.ncoef) {
+                float c[12];
+                if (x.sh_aligned) {
 #pragma unroll
-                        for (int l = 0; l < 4; l++) { const int f = 4 * q4 + l; const int j = f / 3, ch = f - 3 * j; o4[l] = sb[j] * (ch == 0 ? m0c : ch == 1 ? m1c : m2c); }
-                        st[DST_ARENA_FLOATS / 4 + q4] = make_float4(o4[0], o4[1], o4[2], o4[3]);
+                    for (int l = 0; l < 3; l++) {
+                        const float4 v = __ldg(reinterpret_cast<const float4*>(sh) + 3 * q + l);
+                        c[4 * l] = v.x; c[4 * l + 1] = v.y; c[4 * l + 2] = v.z; c[4 * l + 3] = v.w;
                     }
-                }
-            }
-            staged = true; gsent = gidx;
-            if (use_sh && !sh_bulk) {
-                if (dsh_aligned) {
-#pragma unroll
-                    for (int q4 = 0; q4 < 12; q4++) {
-                        if (q4 < nv) {
-                            float o4[4];
-#pragma unroll
-                            for (int l = 0; l < 4; l++) { const int f = 4 * q4 + l; const int j = f / 3, ch = f - 3 * j; o4[l] = sb[j] * (ch == 0 ? m0c : ch == 1 ? m1c : m2c); }
-                            red4(dsh + 4 * q4, o4[0], o4[1], o4[2], o4[3]);
-                        }
-                    }
-                    for (int f = nv << 2; f < nf; f++) { const int j = f / 3, ch = f - 3 * j; atomicAdd(dsh + f, basis_at(sb, j) * (ch == 0 ? m0c : ch == 1 ? m1c : m2c)); }
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 16; j++) {
-                        if (j < ncoef) { atomicAdd(dsh + 3 * j, sb[j] * m0c); atomicAdd(dsh + 3 * j + 1, sb[j] * m1c); atomicAdd(dsh + 3 * j + 2, sb[j] * m2c); }
+                    for (int l = 0; l < 12; l++) c[l] = 12 * q + l < 3 * x.ncoef ? __ldg(sh + 12 * q + l) : 0.0f;
+                }
+#pragma unroll
+                for (int l = 0; l < 4; l++) {
+                    if (4 * q + l < x.ncoef) {
+                        const float b = ws.basis[4 * q + l][lane];
+                        c0 = fmaf(b, c[3 * l], c0); c1 = fmaf(b, c[3 * l + 1], c1); c2 = fmaf(b, c[3 * l + 2], c2);
                     }
                 }
             }
         }
-#else
-        red4(row, dq0, dq1, dq2, dq3);
-        red4(row + 4, dmean.x, dmean.y, dmean.z, dL_dopac);
-        red4(row + 8, dmean.x * hd, dmean.y * hd, dmean.z * hd, 0.f);
-        red4(row + 12, dsx, dsy, has_aux ? t_aux0 * w : 0.f, has_aux ? t_aux1 * w : 0.f);
-        red4(row + 16, dc0, dc1, dc2, 0.f);
-        if (use_sh) {
-            if (dsh_aligned) {
-                // 3*ncoef floats as 4-float reductions (ncoef = 4, 16 -> 3, 12 vectors; 1, 9 leave a scalar tail)
-#pragma unroll
-                for (int q4 = 0; q4 < 12; q4++) {
-                    if (q4 < nv) {
-                        float o4[4];
-#pragma unroll
-                        for (int l = 0; l < 4; l++) { const int f = 4 * q4 + l; const int j = f / 3, ch = f - 3 * j; o4[l] = sb[j] * (ch == 0 ? m0c : ch == 1 ? m1c : m2c); }
-                        red4(dsh + 4 * q4, o4[0], o4[1], o4[2], o4[3]);
-                    }
-                }
-                for (int f = nv << 2; f < nf; f++) { const int j = f / 3, ch = f - 3 * j; atomicAdd(dsh + f, basis_at(sb, j) * (ch == 0 ? m0c : ch == 1 ? m1c : m2c)); }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    if (j < ncoef) { atomicAdd(dsh + 3 * j, sb[j] * m0c); atomicAdd(dsh + 3 * j + 1, sb[j] * m1c); atomicAdd(dsh + 3 * j + 2, sb[j] * m2c); }
-                }
-            }
-        }
-#endif
-        if (use_sh) {
-            dir_gidx = gidx; dir_g0 = m0c; dir_g1 = m1c; dir_g2 = m2c;
-        }
-        T_prev = T_next;
-        } while (false);
-#if DST_BWD_BULK
-        if ((p.tiled ? bulk_stage_aggregate(stage, gsent) : true) && staged) {       // linear ray lists: neighbours in the list are not neighbours on a surface
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the staged values become visible to the bulk copy engine
-            bulk_add(p.arena + (size_t)gsent * DST_ARENA_FLOATS, reinterpret_cast<const float*>(st), DST_ARENA_FLOATS * 4);
-            if (use_sh && dsh_aligned && ((3 * ncoef) & 3) == 0)
-                bulk_add(p.a.dL_dshs + 3 * (size_t)gsent * in.sh_coeffs, reinterpret_cast<const float*>(st + DST_ARENA_FLOATS / 4), 3 * ncoef * 4);
-            bulk_stage_commit(stage);
-        }
-#endif
-        if (stop) break;
+        if (c0 < 0.f) { c0 = 0.f; m0 = 0.f; }                 // clamped channels take no gradient
+        if (c1 < 0.f) { c1 = 0.f; m1 = 0.f; }
+        if (c2 < 0.f) { c2 = 0.f; m2 = 0.f; }
+        F += s.t_rgb0 * c0 + s.t_rgb1 * c1 + s.t_rgb2 * c2;
+        ws.colour[lane] = make_float4(m0, m1, m2, 0.f);
+        s.dir_gidx = gidx; s.dir_g0 = m0; s.dir_g1 = m1; s.dir_g2 = m2;
+    } else {
+        const float* cp = in.colors_precomp + 3 * (size_t)gidx;
+        F += s.t_rgb0 * __ldg(cp) + s.t_rgb1 * __ldg(cp + 1) + s.t_rgb2 * __ldg(cp + 2);
     }
-    s.C0 = C0; s.C1 = C1; s.C2 = C2; s.D = D; s.O0 = O0; s.O1 = O1; s.Nx = N.x; s.Ny = N.y; s.Nz = N.z;
-    s.T_prev = T_prev; s.dpt = dpt; s.last_gidx = last_gidx; s.contributor = contributor;
-    s.dro_x = dL_dray_o.x; s.dro_y = dL_dray_o.y; s.dro_z = dL_dray_o.z;
-    s.drd_x = dL_dray_d.x; s.drd_y = dL_dray_d.y; s.drd_z = dL_dray_d.z;
-    s.dir_gidx = dir_gidx; s.dir_g0 = dir_g0; s.dir_g1 = dir_g1; s.dir_g2 = dir_g2;
-    s.dm0 = dm0; s.dvs = dvs; s.dws = dws;
-    s.chunk++;
-    bool seg_done = stop || T_next < T_threshold || cnt < DST_CHUNK || contributor > DST_MAX_INTERSECTION;
-    if (!seg_done && s.chunk >= DST_MAX_CHUNKS) { atomicOr(p.status, DST_STATUS_CHUNK_LIMIT); seg_done = true; }
-    if (!seg_done) {
-        s.offset = (float)((double)dpt + 0.00001);
-        return true;
+    if (x.has_aux) {
+        const float2 ax = __ldg(reinterpret_cast<const float2*>(in.others_precomp) + gidx);
+        F += s.t_aux0 * ax.x + s.t_aux1 * ax.y;
     }
+    const float inv = 1.0f / (1.0f - alpha);
+    s.rem = fmaf(-w, F, s.rem);
+    float dL_dalpha = T_prev * (F + s.t_acc) - s.rem * inv;
+    float dist_dd = 0.f;       // gradient of the distortion with respect to this hit's depth
+    if (DIST && x.dist_on) {
+        const float m_abs = DST_DIST_K * (1.0f - DST_DIST_NEAR / dpt);
+        if (first) s.dm0 = m_abs;
+        const float cm = (m_abs - s.dm0) - x.dist_mu;
+        s.dws += w; s.dvs += w * cm * cm;
+        const float d_dw = x.tot_acc * cm * cm + x.dist_V;
+        const float behind = x.tot_acc * (x.dist_V - s.dvs) + x.dist_V * (x.tot_acc - s.dws);
+        dL_dalpha += x.t_dist * (d_dw * T_prev - behind * inv);
+        dist_dd = x.t_dist * 2.0f * w * x.tot_acc * cm * DST_DIST_K * DST_DIST_NEAR / (dpt * dpt);
+    }
+    // geometry (backward.cu:201-287, 581-607)
+    const float opac = e.r2.w;
+    const float gG = (opac * e.G) > 0.99f ? 0.0f : dL_dalpha * e.G;         // no gradient through a clamped alpha
+    const float kG = gG * opac;
+    const float sx = e.r3.x, sy = e.r3.y, u = e.u, v = e.v;
+    const float au = -kG * u * e.r3.z, av = -kG * v * e.r3.w;               // dL/du / sx, dL/dv / sy
+    const V3 R0 = v3(e.r0.x, e.r0.y, e.r0.z), R1 = v3(e.r1.x, e.r1.y, e.r1.z);
+    const V3 rd = v3(s.sdx, s.sdy, s.sdz);
+    const V3 dxyz = au * R0 + av * R1;
+    const float dL_dd = s.t_dpt * w + dist_dd + dot(dxyz, rd);
+    const float4* vq = reinterpret_cast<const float4*>(in.vertices + 12 * (size_t)gidx);
+    const float4 va = __ldg(vq), vb = __ldg(vq + 1), vc = __ldg(vq + 2);
+    const bool t0 = (pidx & 1) == 0;
+    const V3 v1 = v3(va.w, vb.x, vb.y), v2 = v3(vb.z, vb.w, vc.x);
+    const V3 pa = t0 ? v3(va.x, va.y, va.z) : v3(vc.y, vc.z, vc.w), pb = t0 ? v1 : v2, pc = t0 ? v2 : v1;
+    const V3 e1 = pa - pb, e2 = pa - pc;
+    const V3 nn = cross(e1, e2);
+    const V3 cvec = (t0 ? pa : v1) - v3(s.sox, s.soy, s.soz);
+    const float iq = 1.0f / dot(nn, rd), depth = dot(nn, cvec) * iq;
+    const V3 h = cvec - depth * rd;
+    const float E = dL_dd * iq;
+    const V3 En = E * nn;
+    const float E6 = t0 ? 6.0f * E : -6.0f * E, En3 = t0 ? 3.0f : -3.0f;
+    const V3 shx = E6 * cross(e1, h) - 3.0f * En, shy = E6 * cross(e2, h) + En3 * En;
+    const V3 dmean = En - dxyz;
+    s.dro_x -= dmean.x; s.dro_y -= dmean.y; s.dro_z -= dmean.z;
+    if (!x.use_sh) {   // with SH the value is replaced below
+        s.drd_x += dpt * dxyz.x - depth * En.x; s.drd_y += dpt * dxyz.y - depth * En.y; s.drd_z += dpt * dxyz.z - depth * En.z;
+    }
+    const float hd = 0.5f * dpt;
+    row[1] = make_float4(dmean.x, dmean.y, dmean.z, gG);
+    row[2] = make_float4(dmean.x * hd, dmean.y * hd, dmean.z * hd, 0.f);
+    row[3] = make_float4(dot(R0, shx) - au * u, dot(R1, shy) - av * v, x.has_aux ? s.t_aux0 * w : 0.f, x.has_aux ? s.t_aux1 * w : 0.f);
+    // quaternion (auxiliary.h:433-477; no gradient through the normalisation)
+    const V3 rel = v3(e.X - __ldg(in.means3D + 3 * (size_t)gidx), e.Y - __ldg(in.means3D + 3 * (size_t)gidx + 1), e.Z - __ldg(in.means3D + 3 * (size_t)gidx + 2));
+    const V3 dR0 = au * rel + sx * shx, dR1 = av * rel + sy * shy;
+    const float wn = w * e.nsign;
+    const V3 dR2 = v3(s.t_nx * wn, s.t_ny * wn, s.t_nz * wn);
+    const float4 q = __ldg(reinterpret_cast<const float4*>(in.rotations) + gidx);
+    const float qs = 2.0f * rsqrtf(q.w * q.w + q.x * q.x + q.y * q.y + q.z * q.z);
+    const float qw = q.x * qs, qx = q.y * qs, qy = q.z * qs, qz = q.w * qs;          // twice the unit quaternion
+    const float a = dR1.z - dR2.y, b = dR2.x - dR0.z, c = dR0.y - dR1.x;
+    const float d = dR0.y + dR1.x, f = dR0.z + dR2.x, g = dR1.z + dR2.y;
+    row[0] = make_float4(qx * a + qy * b + qz * c, qw * a + qy * d + qz * f - 2.f * qx * (dR1.y + dR2.z),
+                         qw * b + qx * d + qz * g - 2.f * qy * (dR0.x + dR2.z), qw * c + qx * f + qy * g - 2.f * qz * (dR0.x + dR1.y));
+    s.T_prev = xmul(T_prev, xsub(1.0f, alpha));
+}
+
+// After the last contribution of a segment: true if an earlier one is left to differentiate.
+__device__ __forceinline__ bool bwd_end_segment(const BwdParams& p, int ray, BwdState& s, const BwdSegment& x) {
+    const dst_trace_inputs& in = p.a.in;
     // With SH colours the reference ASSIGNS the SH direction gradient to the ray-direction
     // accumulator at every contribution (backward.cu:165, 631-632), so what survives a segment
     // is the value of its last contribution.
-    if (use_sh && dir_gidx >= 0) {
+    if (x.use_sh && s.dir_gidx >= 0) {
         float csh[48], sj[16];
-        load_sh_row(in.shs + 3 * (size_t)dir_gidx * in.sh_coeffs, 3 * ncoef, sh_aligned, csh);
+        load_sh_row(in.shs + 3 * (size_t)s.dir_gidx * in.sh_coeffs, 3 * x.ncoef, x.sh_aligned, csh);
 #pragma unroll
-        for (int j = 0; j < 16; j++) sj[j] = j < ncoef ? csh[3 * j] * dir_g0 + csh[3 * j + 1] * dir_g1 + csh[3 * j + 2] * dir_g2 : 0.f;
-        const V3 g = sh_dir_grad(in.sh_degree, sj, sdx, sdy, sdz);
+        for (int j = 0; j < 16; j++) sj[j] = j < x.ncoef ? csh[3 * j] * s.dir_g0 + csh[3 * j + 1] * s.dir_g1 + csh[3 * j + 2] * s.dir_g2 : 0.f;
+        const V3 g = sh_dir_grad(in.sh_degree, sj, s.sdx, s.sdy, s.sdz);
         s.drd_x = g.x; s.drd_y = g.y; s.drd_z = g.z;
     }
     return bwd_next_segment(p, ray, s, s.seg - 1);
+}
+
+// Re-composites one gathered chunk of segment s.seg (backward.cu:429-655) for the rays of a warp in step: all 32 lanes call it, `in_chunk`
+// marks those with a chunk. key_at(i): the lane's i-th hit of cnt. Returns true for rays that need another enumeration.
+template <bool DIAG, bool DIST, class KeyAt>
+__device__ __forceinline__ bool bwd_chunk(const BwdParams& p, bool in_chunk, int ray, BwdState& s, KeyAt key_at, int cnt, BwdWarp& ws, TraceCounters& tc) {
+    const BwdSegment x = bwd_segment<DIST>(p, in_chunk, ray, s, ws);
+    const RowTarget target = row_target(p);
+    const float min_depth = s.seg == 0 ? (p.a.in.start_from_first ? 0.2f : 0.0f) : 0.06f;
+    if (DIAG && in_chunk && s.chunk == 0) tc.segs++;
+    bool stop = !in_chunk;
+    const int n = __reduce_max_sync(0xffffffffu, in_chunk ? cnt : 0);
+    for (int sl = 0; sl < n; sl++) {
+        int gsent = -1;
+        if (!stop && sl < cnt) {
+            const unsigned long long key = key_at(sl);
+            const int pidx = (int)(unsigned int)key;
+            const int gidx = pidx >> 1;
+            SlotEval e;
+            bool ok = false;
+            if (gidx != s.last_gidx) {
+                if (DIAG) tc.evals++;
+                ok = eval_slot(key, s.offset, s.sox, s.soy, s.soz, s.sdx, s.sdy, s.sdz, min_depth, p.cache, gidx, e);
+                s.dpt = e.dpt;
+            }
+            if (ok && (xmul(s.T_prev, xsub(1.0f, e.alpha)) < 0.0001f || ++s.contributor > DST_MAX_INTERSECTION)) { stop = true; ok = false; }
+            if (ok) {
+                s.last_gidx = gidx;
+                if (DIAG) tc.contribs++;
+                bwd_hit<DIST>(p, s, x, e, pidx, s.contributor == 1, ws);
+                gsent = gidx;
+            }
+        }
+        send_rows(target, ws, gsent, p.tiled != 0);       // linear ray lists: neighbours in the list are not neighbours on a surface
+    }
+    if (!in_chunk) return false;
+    s.chunk++;
+    bool seg_done = stop || cnt < DST_CHUNK || s.contributor > DST_MAX_INTERSECTION;
+    if (!seg_done && s.chunk >= DST_MAX_CHUNKS) { atomicOr(p.status, DST_STATUS_CHUNK_LIMIT); seg_done = true; }
+    if (!seg_done) {
+        s.offset = (float)((double)s.dpt + 0.00001);
+        return true;
+    }
+    return bwd_end_segment(p, ray, s, x);
 }
 
 __global__ void __launch_bounds__(256) k_bwd_init(const __grid_constant__ BwdParams p, long long slots) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= slots) return;
     if (i == 0) p.counts[0] = (int)slots;
-    int ray = ray_of_slot(i, p.grid_h, p.grid_w, p.tiled != 0);
+    const int ray = slot_ray(i, p.grid_h, p.grid_w, p.tiled != 0);
+    bool alive = false;
     if (ray >= 0) {
         BwdState s;
-        if (bwd_init_state(p, ray, s)) {
-            bwd_store_state(p.state, ray, s);
+        alive = bwd_init_state(p, ray, s);
+        if (alive) {
+            bwd_store_state(p.state, (int)i, s);
             EnumReq q;
             bwd_request(s, q);
-            p.req[ray] = q;
-        } else ray = -1;       // no segment to differentiate: the (zero) ray gradients are already written
+            store_req(p.req, (int)i, q);
+        }       // else no segment to differentiate: the (zero) ray gradients are already written
     }
-    p.list[0][i] = ray;
-}
-
-template <bool DIAG, bool DIST>
-__global__ void __launch_bounds__(BWD_THREADS) k_bwd_shade(const __grid_constant__ BwdParams p, int round) {
-    const int n = p.counts[round];
-    if (n < p.min_count) return;
-    const int* list = p.list[round & 1];
-    int* next_list = p.list[(round + 1) & 1];
-    TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
-    extern __shared__ __align__(128) unsigned char dyn_smem[];
-    BulkStage stage = bulk_stage_init(dyn_smem);
-    const int n_pad = (n + 31) & ~31;
-    for (int i = blockIdx.x * BWD_THREADS + threadIdx.x; i < n_pad; i += gridDim.x * BWD_THREADS) {
-        const int ray = i < n ? list[i] : -1;
-        bool alive = false;
-        int cls = 0;
-        if (ray >= 0) {
-            BwdState s;
-            bwd_load_state(p.state, ray, s);
-            alive = bwd_shade<DIAG, 1, DIST>(p, ray, s, p.kbuf + (size_t)ray * DST_CHUNK, p.kcnt[ray], tc, stage);
-            if (alive) {
-                bwd_store_state(p.state, ray, s);
-                EnumReq q;
-                bwd_request(s, q);
-                p.req[ray] = q;
-                cls = s.seg > 0;
-            }
-        }
-        if (p.lv.stable) live_out(p.lv, round, i, alive, ray, cls);
-        else append_alive(alive, ray, next_list, p.counts + round + 1);
-    }
-    bulk_stage_drain();
-    if (DIAG && p.a.counters) {
-        atomicAdd(p.a.counters + 0, tc.segs); atomicAdd(p.a.counters + 4, tc.evals); atomicAdd(p.a.counters + 5, tc.contribs);
-    }
-}
-
-template <bool DIAG, bool DIST>
-__global__ void __launch_bounds__(BWD_THREADS) k_bwd_tail(const __grid_constant__ BwdParams p) {
-    __shared__ unsigned long long kshared[DST_CHUNK * BWD_THREADS];
-    const int round = first_skipped_round(p.counts, p.rounds, p.min_count);
-    const int n = p.counts[round];
-    const int* list = p.list[round & 1];
-    unsigned long long* kb = kshared + threadIdx.x;
-    TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
-    extern __shared__ __align__(128) unsigned char dyn_smem[];
-    BulkStage stage = bulk_stage_init(dyn_smem);
-    for (int i = blockIdx.x * BWD_THREADS + threadIdx.x; i < n; i += gridDim.x * BWD_THREADS) {
-        const int ray = list[i];
-        if (ray < 0) continue;
-        BwdState s;
-        bwd_load_state(p.state, ray, s);
-        bool alive = true;
-        while (alive) {
-            EnumReq q;
-            bwd_request(s, q);
-            const int cnt = knearest<false, DIAG, BWD_THREADS>(p.bvh, q.ox, q.oy, q.oz, q.dx, q.dy, q.dz, kb, p.status, tc, q.kmax0);
-            if (DIAG) tc.enums++;
-            alive = bwd_shade<DIAG, BWD_THREADS, DIST>(p, ray, s, kb, cnt, tc, stage);
-        }
-    }
-    bulk_stage_drain();
-    if (DIAG && p.a.counters) {
-        atomicAdd(p.a.counters + 0, tc.segs); atomicAdd(p.a.counters + 1, tc.enums); atomicAdd(p.a.counters + 2, tc.nodes);
-        atomicAdd(p.a.counters + 3, tc.quads); atomicAdd(p.a.counters + 4, tc.evals); atomicAdd(p.a.counters + 5, tc.contribs);
-    }
+    p.list[0][i] = alive ? (int)i : -1;
 }
 
 __device__ __forceinline__ void bwd_flush_counters(unsigned long long* counters, const TraceCounters& tc) {
@@ -718,54 +602,149 @@ __device__ __forceinline__ void bwd_flush_counters(unsigned long long* counters,
     if (tc.contribs) atomicAdd(counters + 5, tc.contribs);
 }
 
-// Backward over the chunk log of the matching forward call: every ray re-composites the chunks the
-// forward composited (chained per segment), so no hierarchy walk is needed; one thread per ray, all
-// segments. Rays whose log is incomplete (log full during the forward) are initialised and queued
-// for k_bwd_tail, which re-traces them.
-template <bool DIAG, bool DIST>
-__global__ void __launch_bounds__(BWD_THREADS, DST_BWD_LOGGED_BLOCKS) k_bwd_logged(const __grid_constant__ BwdParams p, long long slots) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int ray = i < slots ? ray_of_slot(i, p.grid_h, p.grid_w, p.tiled != 0) : -1;
-    TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
+__device__ __forceinline__ BwdWarp& bwd_warp_mem() {
     extern __shared__ __align__(128) unsigned char dyn_smem[];
-    BulkStage stage = bulk_stage_init(dyn_smem);
-    bool requeue = false, active = false;
-    BwdState s;
-    s.seg = -1;
-    const int* heads = nullptr;
-    int idx = -1;
-    if (ray >= 0 && bwd_init_state(p, ray, s)) {
-        if (!p.log_ray_ok[ray]) {
-            bwd_store_state(p.state, ray, s);
+    return reinterpret_cast<BwdWarp*>(dyn_smem)[threadIdx.x >> 5];
+}
+
+// one round of the re-trace: composites the gathered chunk of every ray on the list
+template <bool DIAG, bool DIST>
+__global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_shade(const __grid_constant__ BwdParams p, int round) {
+    const int n = p.counts[round];
+    if (n < p.min_count) return;
+    const int* list = p.list[round & 1];
+    int* next_list = p.list[(round + 1) & 1];
+    TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
+    BwdWarp& ws = bwd_warp_mem();
+    const int n_pad = (n + 31) & ~31;
+    for (int i = blockIdx.x * BWD_THREADS + threadIdx.x; i < n_pad; i += gridDim.x * BWD_THREADS) {
+        const int slot = i < n ? list[i] : -1;
+        const int ray = slot >= 0 ? slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0) : -1;
+        BwdState s;
+        int cnt = 0;
+        if (slot >= 0) { bwd_load_state(p.state, slot, s); cnt = p.kcnt[slot]; }
+        const unsigned long long* kb = p.kbuf + soa(slot >= 0 ? slot : 0, 0, DST_CHUNK);
+        const bool alive = bwd_chunk<DIAG, DIST>(p, slot >= 0, ray, s, [&](int k) { return kb[k * 32]; }, cnt, ws, tc);
+        int cls = 0;
+        if (alive) {
+            bwd_store_state(p.state, slot, s);
             EnumReq q;
             bwd_request(s, q);
-            p.req[ray] = q;
-            requeue = true;
-        } else {
-            heads = p.log_seg_head + (size_t)ray * p.log_seg_stride;
-            idx = heads[s.seg];
-            active = true;
+            store_req(p.req, slot, q);
+            cls = s.seg > 0;
         }
+        if (p.lv.stable) live_out(p.lv, round, i, alive, slot, cls);
+        else append_alive(alive, slot, next_list, p.counts + round + 1);
     }
-    // The warp walks its rays' chunk chains in step: one chunk per pass, and only the lanes whose ray is in the
-    // latest segment still open in the warp (the backward visits a ray's segments last to first). Neighbouring pixels then
-    // composite the same surfels in the same pass of the hit loop, which is what bulk_stage_aggregate() feeds on, and
-    // the lanes run one instruction stream instead of drifting apart chunk by chunk.
-    for (;;) {
-        const int cur = __reduce_max_sync(0xffffffffu, active ? s.seg : -1);
-        if (cur < 0) break;
-        if (active && s.seg == cur) {
-            if (idx < 0) { atomicOr(p.status, DST_STATUS_LOG_MISMATCH); active = false; }
-            else {
-                const int2 hdr = __ldg(p.log_hdr + idx);
-                if (DIAG) tc.enums++;
-                if (!bwd_shade<DIAG, 1, DIST>(p, ray, s, p.log_keys + (size_t)idx * DST_CHUNK, hdr.y, tc, stage)) active = false;
-                else idx = (s.chunk == 0) ? heads[s.seg] : hdr.x;      // chunk == 0: an earlier segment has begun
+    bulk_drain();
+    if (DIAG) bwd_flush_counters(p.a.counters, tc);
+}
+
+// Runs every ray of the first list the rounds left alone to completion: a warp takes as many rays as it takes to keep all warps busy (one, for the
+// few rays the rounds leave), gathers the chunk of one after the other together (knearest_warp) and composites them in step.
+template <bool DIAG, bool DIST>
+__global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_tail(const __grid_constant__ BwdParams p) {
+    constexpr unsigned int FULL = 0xffffffffu;
+    __shared__ WalkMem walk_mem[BWD_THREADS / 32];
+    __shared__ unsigned long long skeys[BWD_THREADS / 32][32][DST_CHUNK];
+    const int round = first_skipped_round(p.counts, p.rounds, p.min_count);
+    const int n = p.counts[round];
+    const int* list = p.list[round & 1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int warps = gridDim.x * (BWD_THREADS / 32);
+    const int share = (n + warps - 1) / warps, per = share < 1 ? 1 : share > 32 ? 32 : share;
+    const float absmax = __ldg(p.bvh.header + 6);
+    BwdWarp& ws = bwd_warp_mem();
+    TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
+    for (long long i0 = (long long)(blockIdx.x * (BWD_THREADS / 32) + w) * per; i0 < n; i0 += (long long)warps * per) {
+        const int slot = lane < per && i0 + lane < n ? list[i0 + lane] : -1;
+        const int ray = slot >= 0 ? slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0) : -1;
+        BwdState s;
+        bool alive = slot >= 0;
+        if (alive) bwd_load_state(p.state, slot, s);
+        for (;;) {
+            const unsigned int todo = __ballot_sync(FULL, alive);
+            if (todo == 0u) break;
+            EnumReq q = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
+            if (alive) { bwd_request(s, q); if (DIAG) tc.enums++; }
+            int cnt = 0;
+            for (unsigned int m = todo; m; m &= m - 1u) {
+                const int r = __ffs(m) - 1;
+                unsigned long long key;
+                const int c = knearest_warp<DIAG>(p.bvh, __shfl_sync(FULL, q.ox, r), __shfl_sync(FULL, q.oy, r), __shfl_sync(FULL, q.oz, r), __shfl_sync(FULL, q.dx, r),
+                                                  __shfl_sync(FULL, q.dy, r), __shfl_sync(FULL, q.dz, r), DST_T_MAX, absmax, walk_mem[w], key, p.status, tc);
+                if (lane < c) skeys[w][r][lane] = key;
+                if (lane == r) cnt = c;
+                __syncwarp();
             }
+            const bool go = bwd_chunk<DIAG, DIST>(p, alive, ray, s, [&](int k) { return skeys[w][lane][k]; }, cnt, ws, tc);
+            alive = alive && go;
+            __syncwarp();
         }
     }
-    bulk_stage_drain();
-    append_alive(requeue, ray, p.list[0], p.counts);
+    bulk_drain();
+    if (DIAG) bwd_flush_counters(p.a.counters, tc);
+}
+
+// Backward over the contribution log of the matching forward call: every ray composites its logged contributions again, so no
+// hierarchy walk is needed; one thread per ray, all segments. Rays whose log is incomplete (log full during the forward) are
+// initialised and queued for the re-trace.
+//
+// A warp composites its rays' contributions in step, entry by entry, and only the lanes whose ray is in the latest segment still
+// open in the warp (the backward visits a ray's segments last to first): neighbouring pixels then composite the same surfels in
+// the same pass, which is what send_rows() feeds on.
+template <bool DIAG, bool DIST>
+__global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_logged(const __grid_constant__ BwdParams p, long long slots) {
+    constexpr unsigned int FULL = 0xffffffffu;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int slot = i < slots ? (int)i : -1;
+    const int ray = slot >= 0 ? slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0) : -1;
+    TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
+    BwdWarp& ws = bwd_warp_mem();
+    const RowTarget target = row_target(p);
+    bool requeue = false;
+    BwdState s;
+    bool active = ray >= 0 && bwd_init_state(p, ray, s);
+    if (active && !p.log_ok[slot]) {
+        bwd_store_state(p.state, slot, s);
+        EnumReq q;
+        bwd_request(s, q);
+        store_req(p.req, slot, q);
+        requeue = true; active = false;
+    }
+    for (;;) {
+        const int cur = __reduce_max_sync(FULL, active ? s.seg : -1);
+        if (cur < 0) break;
+        const bool in = active && s.seg == cur;
+        int num = 0, rec = -1;
+        if (in) {
+            num = __ldg(p.log_num + cur * p.log_slots + slot);
+            if (num > 0) rec = __ldg(p.log_head + cur * p.log_slots + slot);
+            if (DIAG) { tc.segs++; tc.contribs += num; tc.evals += num; }
+        }
+        const BwdSegment x = bwd_segment<DIST>(p, in, ray, s, ws);
+        const float min_depth = cur == 0 ? (p.a.in.start_from_first ? 0.2f : 0.0f) : 0.06f;
+        unsigned long long key = num > 0 ? __ldg(p.log_keys + soa(rec, 0, DST_CHUNK)) : 0ull;
+        const int n = __reduce_max_sync(FULL, num);
+        for (int at = 0; at < n; at++) {
+            int gsent = -1;
+            if (at < num) {
+                const int pidx = (int)(unsigned int)key;
+                SlotEval e;
+                eval_slot(key, 0.0f, s.sox, s.soy, s.soz, s.sdx, s.sdy, s.sdz, min_depth, p.cache, pidx >> 1, e);      // (accepted, as in the forward)
+                if (at + 1 < num) {
+                    if (((at + 1) & (DST_CHUNK - 1)) == 0) rec = __ldg(p.log_next + rec);
+                    key = __ldg(p.log_keys + soa(rec, (at + 1) & (DST_CHUNK - 1), DST_CHUNK));
+                }
+                bwd_hit<DIST>(p, s, x, e, pidx, at == 0, ws);
+                gsent = pidx >> 1;
+            }
+            send_rows(target, ws, gsent, p.tiled != 0);
+        }
+        if (in) active = bwd_end_segment(p, ray, s, x);
+    }
+    bulk_drain();
+    append_alive(requeue, slot, p.list[0], p.counts);
     if (DIAG) bwd_flush_counters(p.a.counters, tc);
 }
 
@@ -842,14 +821,14 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     const long long slots = slots_of_grid(p.grid_h, p.grid_w, p.tiled != 0);
     rc = dst_ensure_wavefront(h, slots, sizeof(BwdState));
     if (rc != DST_OK) return rc;
-    p.state = h->wf_state; p.req = static_cast<EnumReq*>(h->wf_req); p.kbuf = h->wf_kbuf; p.kcnt = h->wf_kcnt;
+    p.state = static_cast<float4*>(h->wf_state); p.req = static_cast<float4*>(h->wf_req); p.kbuf = h->wf_kbuf; p.kcnt = h->wf_kcnt;
     p.list[0] = h->wf_list[0]; p.list[1] = h->wf_list[1]; p.counts = h->wf_counts;
     const bool diag = a->counters != nullptr;
     const bool dist = h->distortion != 0 && a->dL_ddist != nullptr && a->out_dist != nullptr;
     const bool use_log = a->forward_serial != 0 && a->forward_serial == h->log_serial && h->log_H == a->in.H && h->log_W == a->in.W &&
                          h->log_depth == a->in.max_trace_depth;
-    p.log_keys = h->log_keys; p.log_hdr = h->log_hdr; p.log_seg_head = h->log_seg_head; p.log_ray_ok = h->log_ray_ok;
-    p.log_seg_stride = a->in.max_trace_depth + 1;
+    p.log_keys = h->log_keys; p.log_next = h->log_next; p.log_head = h->log_head; p.log_num = h->log_num; p.log_ok = h->log_ok;
+    p.log_slots = slots;
     DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_counts, 0, 4 * DST_COUNTS_STRIDE, st));
     h->slices_used = 1;
     const bool wave = slots >= h->wf_min_rays;
@@ -865,7 +844,7 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
         p.rounds = 12;
     dst_prof_mark(h, 2, 0, st);
     if (use_log) {
-        // the forward kept its chunks: re-composite them; rays the log could not hold are queued as round 0 of the
+        // the forward logged its contributions: composite them again; rays the log could not hold are queued as round 0 of the
         // re-trace below (normally none: the rounds then find an empty list and return at once)
         const unsigned int blocks = (unsigned int)((slots + BWD_THREADS - 1) / BWD_THREADS);
         if (dist) { if (diag) k_bwd_logged<true, true><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots); else k_bwd_logged<false, true><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots); }
@@ -883,7 +862,7 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
         else { if (diag) k_bwd_shade<true, false><<<g_shade, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, r); else k_bwd_shade<false, false><<<g_shade, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, r); }
         if (p.lv.stable) k_compact<<<g_compact, 256, 0, st>>>(p.lv, p.counts + r, p.counts + r + 1, p.min_count, p.list[(r + 1) & 1], r);
     }
-    const int g_tail = dst_wavefront_grid(h, wave ? p.min_count : slots, BWD_THREADS, 4);
+    const int g_tail = dst_wavefront_grid(h, (wave ? p.min_count : slots) * 32, BWD_THREADS, DST_BWD_BLOCKS);
     if (dist) { if (diag) k_bwd_tail<true, true><<<g_tail, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p); else k_bwd_tail<false, true><<<g_tail, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p); }
     else { if (diag) k_bwd_tail<true, false><<<g_tail, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p); else k_bwd_tail<false, false><<<g_tail, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p); }
     dst_prof_mark(h, 2, 1, st);

@@ -32,13 +32,13 @@ struct BvhView {
 // Per-surfel shading record rebuilt at the start of every trace call (parameters change each
 // training step): rows of the tangent frame, the frame origin, opacity and scales, 64 B so that
 // one evaluated hit costs two 32-byte sectors instead of four scattered gathers.
-//   f4[0] = (R0.xyz, T.x)  f4[1] = (R1.xyz, T.y)  f4[2] = (R2.xyz, opacity)  f4[3] = (sx, sy, 0, 0)
+//   f4[0] = (R0.xyz, T.x)  f4[1] = (R1.xyz, T.y)  f4[2] = (R2.xyz, opacity)  f4[3] = (sx, sy, 1/sx, 1/sy)
 struct SurfelCacheView { const float4* rec; };
 
 // packed per-surfel gradient rows (16-byte aligned so that 4-float vector reductions apply):
 //   [0..3] rotation  [4..6] mean  [7] opacity  [8..10] grads3D  [11] -  [12..13] scale  [14..15] others  [16..18] colour  [19] -
 #define DST_ARENA_FLOATS 20
-#define DST_LOG_MAX_RECORDS (320ll << 20)     // 136 B each: at most 43.5 GB of chunk log
+#define DST_LOG_MAX_RECORDS (320ll << 20)     // 132 B each: at most 44.3 GB of contribution log
 
 #define DST_MAX_SLICES 8
 struct dst_handle {
@@ -82,11 +82,11 @@ struct dst_handle {
     // the current call, their pinned read-back, and how many coming calls leave the prediction off after a call in which it
     // failed too often.
     int* bound_stats; int* bound_host; cudaEvent_t bound_event; bool bound_pending; int bound_off_calls;
-    // chunk log: the 16-hit chunks every ray composited in the last training forward, chained per ray and segment,
-    // so that the backward re-composites them without walking the hierarchy again
-    unsigned long long* log_keys; int2* log_hdr; int* log_count; int* log_seg_head; unsigned char* log_ray_ok;
+    // contribution log of the last training forward (dst_ensure_log), so that the backward re-composites it without walking the
+    // hierarchy again
+    unsigned long long* log_keys; int* log_next; int* log_count; int* log_head; int* log_num; unsigned char* log_ok;
     long long log_cap;            // records
-    long long log_rays_cap; int log_seg_stride_cap;
+    long long log_index_cap;      // slots x segments of log_head / log_num
     unsigned long long log_serial;      // serial of the forward call the log belongs to (0 = none)
     unsigned long long serial_counter;
     int log_H, log_W, log_depth;
@@ -135,7 +135,7 @@ int dst_knearest_impl(dst_handle* h, const float* ro, const float* rd, int64_t n
 int dst_prepare_cache(dst_handle* h, const dst_trace_inputs* in, cudaStream_t st);
 int dst_export_frames_impl(dst_handle* h, float* out, cudaStream_t st);
 int dst_ensure_wavefront(dst_handle* h, long long slots, size_t state_bytes);
-int dst_ensure_chunk_log(dst_handle* h, long long rays, int segs);
+int dst_ensure_log(dst_handle* h, long long rays, long long slots, int segs);
 int dst_wavefront_grid(const dst_handle* h, long long slots, int threads, int per_sm);
 
 #ifdef __CUDACC__

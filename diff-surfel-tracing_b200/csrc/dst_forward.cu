@@ -63,8 +63,8 @@ struct FwdParams {
     int* bound_stats;               // {bounded searches issued, of them failed} in this call, or null: no predicted bounds
     float bound_factor;
     // wavefront scratch
-    void* state;
-    EnumReq* req;
+    float4* state;
+    float4* req;        // null: no gather kernels run
     unsigned long long* kbuf;
     int* kcnt;
     int* list[2];
@@ -72,9 +72,9 @@ struct FwdParams {
     int min_count;
     int rounds;
     LiveLists lv;
-    // chunk log (null log_keys: disabled)
-    unsigned long long* log_keys; int2* log_hdr; int* log_count; int* log_seg_head; unsigned char* log_ray_ok;
-    int log_cap, log_seg_stride;
+    // contribution log (null log_keys: disabled), see dst_ensure_log()
+    unsigned long long* log_keys; int* log_next; int* log_count; int* log_head; int* log_num; unsigned char* log_ok;
+    int log_cap; long long log_slots;       // records; slots per segment of log_head / log_num
 };
 
 struct __align__(16) FwdState {
@@ -84,11 +84,13 @@ struct __align__(16) FwdState {
     float D, Nx, Ny, Nz;
     float O0, O1, s_prod, rgb0;
     float rgb1, rgb2; int last_gidx, contributor;
-    int bounce, chunk, hit_count; float m0;      // m0: mapped depth of the first contribution (distortion extension)
-    int log_prev;       // last chunk-log record of the current segment, -1 at a segment start
+    short bounce; unsigned short chunk;
+    int hit_count, log_spare; float m0;          // log_spare: log record reserved and not yet used, or -1; m0: mapped depth of the first contribution (distortion extension)
+    int log_rec;        // log record the current segment's last contribution is in
     float dist, m1, m2; // depth distortion of the primary segment and the two moments of the mapped depth (extension)
 };
-static_assert(sizeof(FwdState) == 128, "ray state is one 128-byte record");
+static_assert(sizeof(FwdState) == 128, "ray state is eight 16-byte words");
+static_assert(DST_MAX_CHUNKS < 65536, "chunk counter of the ray state");
 
 // Per-surfel shading record: tangent-frame rows from the quaternion exactly as
 // quat_to_rotmat_transpose does on an IEEE host (optix_tracer/auxiliary.h:403-429, with rsqrtf
@@ -116,7 +118,8 @@ __global__ void __launch_bounds__(256) k_prepare_cache(int P, const float* __res
     o[0] = make_float4(r0x, r0y, r0z, tx);
     o[1] = make_float4(r1x, r1y, r1z, ty);
     o[2] = make_float4(r2x, r2y, r2z, opac[g]);
-    o[3] = make_float4(scales[2 * (size_t)g], scales[2 * (size_t)g + 1], 0.f, 0.f);
+    const float sx = scales[2 * (size_t)g], sy = scales[2 * (size_t)g + 1];
+    o[3] = make_float4(sx, sy, xdiv(1.0f, sx), xdiv(1.0f, sy));
 }
 
 // a_weights[gidx] += w (optix_tracer/forward.cu:295), aggregated over the lanes of the warp that are here together.
@@ -145,7 +148,7 @@ __device__ __forceinline__ void add_weight(float* __restrict__ a_weights, int gi
 __device__ __forceinline__ void fwd_begin_segment(FwdState& s) {
     s.offset = 0.f; s.dpt = 0.f; s.T_prev = 1.f;
     s.C0 = s.C1 = s.C2 = 0.f; s.D = 0.f; s.Nx = s.Ny = s.Nz = 0.f; s.O0 = s.O1 = 0.f;
-    s.last_gidx = -1; s.contributor = 0; s.chunk = 0; s.log_prev = -1;
+    s.last_gidx = -1; s.contributor = 0; s.chunk = 0;
 }
 
 // Ray of pixel (i, j) as get_rays_from_ij computes it (example/utils/ray_utils.py:121-133): camera point
@@ -193,7 +196,7 @@ __device__ __forceinline__ void fwd_init_state(const FwdParams& p, int ray, FwdS
         s.sox = __ldg(in.ray_o + 3 * (size_t)ray); s.soy = __ldg(in.ray_o + 3 * (size_t)ray + 1); s.soz = __ldg(in.ray_o + 3 * (size_t)ray + 2);
         s.sdx = __ldg(in.ray_d + 3 * (size_t)ray); s.sdy = __ldg(in.ray_d + 3 * (size_t)ray + 1); s.sdz = __ldg(in.ray_d + 3 * (size_t)ray + 2);
     }
-    s.s_prod = 1.f; s.rgb0 = s.rgb1 = s.rgb2 = 0.f; s.bounce = 0; s.hit_count = 0;
+    s.s_prod = 1.f; s.rgb0 = s.rgb1 = s.rgb2 = 0.f; s.bounce = 0; s.hit_count = 0; s.log_spare = s.log_rec = -1;
     s.dist = s.m1 = s.m2 = 0.f; s.m0 = -1.f;
     fwd_begin_segment(s);
 }
@@ -207,7 +210,7 @@ __device__ __forceinline__ void fwd_request(const FwdState& s, EnumReq& q) {
 
 // After the hits of a chunk: the segment goes on (returns true), or it is finished (forward.cu:309-314, tracePath 378-422) and
 // the ray starts the reflected segment (true) or is done (false). opaque: the transmittance limit or the hit limit was reached.
-__device__ __forceinline__ bool fwd_end_chunk(const FwdParams& p, int ray, FwdState& s, bool opaque, int cnt, bool diag) {
+__device__ __forceinline__ bool fwd_end_chunk(const FwdParams& p, int slot, FwdState& s, bool opaque, int cnt, bool diag) {
     const dst_trace_inputs& in = p.a.in;
     s.chunk++;
     bool seg_done = opaque || cnt < DST_CHUNK || s.contributor > DST_MAX_INTERSECTION;   // :299
@@ -217,6 +220,8 @@ __device__ __forceinline__ bool fwd_end_chunk(const FwdParams& p, int ray, FwdSt
         return true;
     }
     // ---- end of the segment (forward.cu:309-314) ----
+    const int ray = slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0);
+    if (p.log_keys) p.log_num[s.bounce * p.log_slots + slot] = s.contributor < DST_MAX_INTERSECTION ? s.contributor : DST_MAX_INTERSECTION;
     const float bg0 = __ldg(in.background), bg1 = __ldg(in.background + 1), bg2 = __ldg(in.background + 2);
     const float C0 = xadd(s.C0, xmul(s.T_prev, bg0)), C1 = xadd(s.C1, xmul(s.T_prev, bg1)), C2 = xadd(s.C2, xmul(s.T_prev, bg2));
     const float A = xsub(1.0f, s.T_prev);
@@ -260,10 +265,23 @@ __device__ __forceinline__ bool fwd_end_chunk(const FwdParams& p, int ray, FwdSt
     return true;
 }
 
+// Logs a contribution (depth along the segment, primitive) as entry number `at` of its segment: 16 entries per record, records chained.
+__device__ __forceinline__ void log_entry(const FwdParams& p, int slot, FwdState& s, int at, float dpt, unsigned int pidx) {
+    if ((at & (DST_CHUNK - 1)) == 0) {
+        const int rec = s.log_spare;
+        s.log_spare = -1;
+        if (rec >= 0) {
+            if (at == 0) p.log_head[s.bounce * p.log_slots + slot] = rec; else if (s.log_rec >= 0) p.log_next[s.log_rec] = rec;
+        }
+        s.log_rec = rec;
+    }
+    if (s.log_rec >= 0) p.log_keys[soa(s.log_rec, at & (DST_CHUNK - 1), DST_CHUNK)] = make_key(dpt, pidx);
+}
+
 // Composites one gathered chunk (forward.cu:197-306), one thread per ray. Returns true while the ray needs another enumeration.
 // kb: the chunk's keys with stride KS; cnt: how many.
 template <bool DIAG, int KS>
-__device__ __forceinline__ bool fwd_shade(const FwdParams& p, int ray, FwdState& s, const unsigned long long* kb, int cnt, TraceCounters& tc) {
+__device__ __forceinline__ bool fwd_shade(const FwdParams& p, int slot, FwdState& s, const unsigned long long* kb, int cnt, TraceCounters& tc) {
     const dst_trace_inputs& in = p.a.in;
     const bool use_sh = in.colors_precomp == nullptr;
     const bool has_aux = in.others_precomp != nullptr;
@@ -274,18 +292,12 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, int ray, FwdState&
     float sb[16];
     if (use_sh) sh_basis(in.sh_degree, s.sdx, s.sdy, s.sdz, sb);
     if (DIAG) { if (s.chunk == 0) tc.segs++; }
-    if (p.log_keys) {
-        // keep this chunk for the backward: one record per chunk, chained per segment
-        const int idx = atomicAdd(p.log_count, 1);
-        if (idx >= 0 && idx < p.log_cap) {
-            ulonglong2* dst = reinterpret_cast<ulonglong2*>(p.log_keys + (size_t)idx * DST_CHUNK);
-#pragma unroll
-            for (int k = 0; k < DST_CHUNK / 2; k++) if (2 * k < cnt) dst[k] = make_ulonglong2(kb[(2 * k) * KS], kb[(2 * k + 1) * KS]);
-            p.log_hdr[idx] = make_int2(-1, cnt);
-            if (s.log_prev < 0) p.log_seg_head[(size_t)ray * p.log_seg_stride + s.bounce] = idx;
-            else p.log_hdr[s.log_prev].x = idx;
-            s.log_prev = idx;
-        } else p.log_ray_ok[ray] = 0;       // log full: this ray's backward walks the hierarchy again
+    if (p.log_keys && s.log_spare < 0 && ((s.contributor & (DST_CHUNK - 1)) == 0 || (s.contributor & (DST_CHUNK - 1)) + cnt > DST_CHUNK)) {
+        // a chunk can fill at most one further record: it is reserved here, where the lanes of a warp that need one get neighbouring ones,
+        // and kept for the next chunk or segment when it is not used
+        const int rec = atomicAdd(p.log_count, 1);
+        if (rec >= 0 && rec < p.log_cap) s.log_spare = rec;
+        else p.log_ok[slot] = 0;       // log full: this ray's backward walks the hierarchy again
     }
 
     float T_next = 1.0f;
@@ -308,6 +320,7 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, int ray, FwdState&
         if (s.contributor > DST_MAX_INTERSECTION) { stop = true; break; }
         s.last_gidx = gidx;
         const float w = xmul(alpha, s.T_prev);
+        if (p.log_keys) log_entry(p, slot, s, s.contributor - 1, s.dpt, (unsigned int)pidx);
         if (use_sh) {
             float c[48];
             load_sh_row(in.shs + 3 * (size_t)gidx * in.sh_coeffs, 3 * ncoef, sh_aligned, c);
@@ -338,24 +351,22 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, int ray, FwdState&
         if (p.a.training && p.a.a_weights) add_weight(p.a.a_weights, gidx, w);          // forward.cu:295
         if (DIAG) {
             tc.contribs++;
-            if (p.a.hit_log && s.hit_count < p.a.hit_cap) p.a.hit_log[(size_t)ray * p.a.hit_cap + s.hit_count] = pidx;
+            if (p.a.hit_log && s.hit_count < p.a.hit_cap) p.a.hit_log[(size_t)slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0) * p.a.hit_cap + s.hit_count] = pidx;
             s.hit_count++;
         }
     }
-    return fwd_end_chunk(p, ray, s, stop || T_next < T_threshold, cnt, DIAG);
+    return fwd_end_chunk(p, slot, s, stop || T_next < T_threshold, cnt, DIAG);
 }
 
-__device__ __forceinline__ void load_state(const void* base, int ray, FwdState& s) {
-    const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const FwdState*>(base) + ray);
+__device__ __forceinline__ void load_state(const float4* base, int slot, FwdState& s) {
     float4* dst = reinterpret_cast<float4*>(&s);
 #pragma unroll
-    for (int i = 0; i < 8; i++) dst[i] = src[i];
+    for (int i = 0; i < 8; i++) dst[i] = base[soa(slot, i, 8)];
 }
-__device__ __forceinline__ void store_state(void* base, int ray, const FwdState& s) {
-    float4* dst = reinterpret_cast<float4*>(reinterpret_cast<FwdState*>(base) + ray);
+__device__ __forceinline__ void store_state(float4* base, int slot, const FwdState& s) {
     const float4* src = reinterpret_cast<const float4*>(&s);
 #pragma unroll
-    for (int i = 0; i < 8; i++) dst[i] = src[i];
+    for (int i = 0; i < 8; i++) base[soa(slot, i, 8)] = src[i];
 }
 
 __device__ __forceinline__ void flush_counters(unsigned long long* counters, const TraceCounters& tc) {
@@ -373,23 +384,26 @@ __global__ void __launch_bounds__(256) k_fwd_init(const __grid_constant__ FwdPar
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= slots) return;
     if (i == 0) p.counts[0] = (int)slots;
-    const int ray = ray_of_slot(p.slot0 + i, p.grid_h, p.grid_w, p.tiled != 0);
-    p.list[0][i] = ray;
+    const int slot = (int)(p.slot0 + i);
+    const int ray = slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0);
+    p.list[0][i] = ray < 0 ? -1 : slot;
     if (ray < 0) return;
     FwdState s;
     fwd_init_state(p, ray, s);
     if (p.log_keys) {
-        p.log_ray_ok[ray] = 1;
-        for (int k = 0; k < p.log_seg_stride; k++) p.log_seg_head[(size_t)ray * p.log_seg_stride + k] = -1;
+        p.log_ok[slot] = 1;
+        for (int k = 0; k <= p.a.in.max_trace_depth; k++) p.log_num[k * p.log_slots + slot] = 0;
     }
-    store_state(p.state, ray, s);
-    EnumReq q;
-    fwd_request(s, q);
-    p.req[ray] = q;
+    store_state(p.state, slot, s);
+    if (p.req) {
+        EnumReq q;
+        fwd_request(s, q);
+        store_req(p.req, slot, q);
+    }
 }
 
 template <bool DIAG>
-__global__ void __launch_bounds__(SHADE_THREADS) k_fwd_shade(const __grid_constant__ FwdParams p, int round) {
+__global__ void __launch_bounds__(SHADE_THREADS, DST_SHADE_GRID_PER_SM) k_fwd_shade(const __grid_constant__ FwdParams p, int round) {
     const int n = p.counts[round];
     if (n < p.min_count) return;
     const int* list = p.list[round & 1];
@@ -404,26 +418,26 @@ __global__ void __launch_bounds__(SHADE_THREADS) k_fwd_shade(const __grid_consta
         bound_on = issued < 4096 || fails * 12 < issued;
     }
     for (int i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < n_pad; i += gridDim.x * SHADE_THREADS) {
-        const int ray = i < n ? list[i] : -1;
+        const int slot = i < n ? list[i] : -1;
         bool alive = false, bounded = false, failed = false;
         int cls = 0;
-        if (ray >= 0) {
+        if (slot >= 0) {
             FwdState s;
-            load_state(p.state, ray, s);
-            const unsigned long long* kb = p.kbuf + (size_t)ray * DST_CHUNK;
-            const int cnt = p.kcnt[ray];
-            if (cnt < DST_CHUNK && p.req[ray].kmax0 < DST_T_MAX) {
+            load_state(p.state, slot, s);
+            const unsigned long long* kb = p.kbuf + soa(slot, 0, DST_CHUNK);
+            const int cnt = p.kcnt[slot];
+            if (cnt < DST_CHUNK && req_bound(p.req, slot) < DST_T_MAX) {
                 // The gather searched within a predicted distance (below) and found fewer than 16 hits there: that says nothing
                 // about what lies beyond. Nothing is composited; the same request goes out again without a bound.
-                p.req[ray].kmax0 = DST_T_MAX;
+                req_bound(p.req, slot) = DST_T_MAX;
                 alive = true;
                 cls = s.bounce > 0;
                 failed = true;
                 if (DIAG && p.a.counters) atomicAdd(p.a.counters + 1, ~0ull);        // (the counter reports completed enumerations)
             } else {
-                alive = fwd_shade<DIAG, 1>(p, ray, s, kb, cnt, tc);
+                alive = fwd_shade<DIAG, 32>(p, slot, s, kb, cnt, tc);
                 if (alive) {
-                    store_state(p.state, ray, s);
+                    store_state(p.state, slot, s);
                     EnumReq q;
                     fwd_request(s, q);
                     // A segment that goes on: its next 16 hits are searched within bound_factor times the distance the last 16
@@ -431,10 +445,10 @@ __global__ void __launch_bounds__(SHADE_THREADS) k_fwd_shade(const __grid_consta
                     // learns it from its 16th hit; the spans of consecutive chunks differ by less than that factor for all but
                     // a per cent of the rays of a dense scene, and those search again.
                     if (bound_on && s.chunk > 0 && cnt == DST_CHUNK) {
-                        q.kmax0 = fmaxf(p.bound_factor * (hitkey_t(kb[DST_CHUNK - 1]) - hitkey_t(kb[0])), 1e-4f);
+                        q.kmax0 = fmaxf(p.bound_factor * (hitkey_t(kb[(DST_CHUNK - 1) * 32]) - hitkey_t(kb[0])), 1e-4f);
                         bounded = true;
                     }
-                    p.req[ray] = q;
+                    store_req(p.req, slot, q);
                     cls = s.bounce > 0;
                 }
             }
@@ -443,8 +457,8 @@ __global__ void __launch_bounds__(SHADE_THREADS) k_fwd_shade(const __grid_consta
             const unsigned int mb = __ballot_sync(0xffffffffu, bounded), mf = __ballot_sync(0xffffffffu, failed);
             if ((threadIdx.x & 31) == 0) { if (mb) atomicAdd(p.bound_stats, __popc(mb)); if (mf) atomicAdd(p.bound_stats + 1, __popc(mf)); }
         }
-        if (p.lv.stable) live_out(p.lv, round, i, alive, ray, cls);
-        else append_alive(alive, ray, next_list, p.counts + round + 1);
+        if (p.lv.stable) live_out(p.lv, round, i, alive, slot, cls);
+        else append_alive(alive, slot, next_list, p.counts + round + 1);
     }
     if (DIAG) flush_counters(p.a.counters, tc);
 }
@@ -459,17 +473,17 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_fwd_tail(const __grid_constant
     unsigned long long* kb = kshared + threadIdx.x;
     TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
     for (int i = blockIdx.x * TAIL_THREADS + threadIdx.x; i < n; i += gridDim.x * TAIL_THREADS) {
-        const int ray = list[i];
-        if (ray < 0) continue;
+        const int slot = list[i];
+        if (slot < 0) continue;
         FwdState s;
-        load_state(p.state, ray, s);
+        load_state(p.state, slot, s);
         bool alive = true;
         while (alive) {
             EnumReq q;
             fwd_request(s, q);
             const int cnt = knearest<BRUTE, DIAG, TAIL_THREADS>(p.bvh, q.ox, q.oy, q.oz, q.dx, q.dy, q.dz, kb, p.status, tc, q.kmax0);
             if (DIAG) tc.enums++;
-            alive = fwd_shade<DIAG, TAIL_THREADS>(p, ray, s, kb, cnt, tc);
+            alive = fwd_shade<DIAG, TAIL_THREADS>(p, slot, s, kb, cnt, tc);
         }
     }
     if (DIAG) flush_counters(p.a.counters, tc);
@@ -481,26 +495,12 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_fwd_tail(const __grid_constant
 // that of the serial loop. s and terms are shared memory of the warp; key: lane i's hit.
 struct WarpShade { FwdState s; float terms[DST_CHUNK][9]; };
 template <bool DIAG>
-__device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int ray, WarpShade& ws, unsigned long long key, int cnt, TraceCounters& tc) {
+__device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int slot, WarpShade& ws, unsigned long long key, int cnt, TraceCounters& tc) {
     constexpr unsigned int FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const dst_trace_inputs& in = p.a.in;
     FwdState& s = ws.s;
     const bool have = lane < cnt;
-    if (p.log_keys) {
-        int idx = 0;
-        if (lane == 0) idx = atomicAdd(p.log_count, 1);
-        idx = __shfl_sync(FULL, idx, 0);
-        if (idx >= 0 && idx < p.log_cap) {
-            if (have) p.log_keys[(size_t)idx * DST_CHUNK + lane] = key;
-            if (lane == 0) {
-                p.log_hdr[idx] = make_int2(-1, cnt);
-                if (s.log_prev < 0) p.log_seg_head[(size_t)ray * p.log_seg_stride + s.bounce] = idx;
-                else p.log_hdr[s.log_prev].x = idx;
-                s.log_prev = idx;
-            }
-        } else if (lane == 0) p.log_ray_ok[ray] = 0;
-    }
     const float min_depth = s.bounce == 0 ? (in.start_from_first ? 0.2f : 0.0f) : 0.06f;       // forward.cu:353
     const int gidx = (int)((unsigned int)key >> 1);
     SlotEval e;
@@ -527,6 +527,26 @@ __device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int ray, Warp
     const unsigned int contrib = okm & ((1u << last) - 1u);
     const unsigned int evaluated = ((1u << cnt) - 1u) & ~skip & (stop ? (2u << last) - 1u : FULL);
     const float w = xmul(e.alpha, my_T);
+    if (p.log_keys && contrib) {      // see log_entry(); at most one new record per chunk
+        const int c0 = s.contributor, num = __popc(contrib), fresh = (c0 + DST_CHUNK - 1) & ~(DST_CHUNK - 1);      // fresh: first entry that needs a new record
+        int rec = -1;
+        if (c0 + num > fresh) {
+            rec = s.log_spare;
+            if (rec < 0) {
+                if (lane == 0) rec = atomicAdd(p.log_count, 1);
+                rec = __shfl_sync(FULL, rec, 0);
+                if (rec < 0 || rec >= p.log_cap) { rec = -1; if (lane == 0) p.log_ok[slot] = 0; }
+            }
+        }
+        const int at = c0 + __popc(contrib & ((1u << lane) - 1u)), prev = s.log_rec;
+        const int mine = at < fresh ? prev : rec;
+        if (((contrib >> lane) & 1u) && mine >= 0) p.log_keys[soa(mine, at & (DST_CHUNK - 1), DST_CHUNK)] = make_key(e.dpt, (unsigned int)key);
+        __syncwarp();
+        if (lane == 0 && c0 + num > fresh) {
+            if (rec >= 0) { if (fresh == 0) p.log_head[s.bounce * p.log_slots + slot] = rec; else if (prev >= 0) p.log_next[prev] = rec; }
+            s.log_rec = rec; s.log_spare = -1;
+        }
+    }
     if ((contrib >> lane) & 1u) {
         float* t = ws.terms[lane];
         if (in.colors_precomp == nullptr) {
@@ -549,7 +569,7 @@ __device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int ray, Warp
         if (p.a.training && p.a.a_weights) atomicAdd(p.a.a_weights + gidx, w);          // forward.cu:295
         if (DIAG && p.a.hit_log) {
             const int at = s.hit_count + __popc(contrib & ((1u << lane) - 1u));
-            if (at < p.a.hit_cap) p.a.hit_log[(size_t)ray * p.a.hit_cap + at] = (int)(unsigned int)key;
+            if (at < p.a.hit_cap) p.a.hit_log[(size_t)slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0) * p.a.hit_cap + at] = (int)(unsigned int)key;
         }
     }
     if (p.dist_on && s.bounce == 0 && contrib) {      // see fwd_shade()
@@ -581,7 +601,7 @@ __device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int ray, Warp
     if (lane == 0) {
         if (DIAG) { if (s.chunk == 0) tc.segs++; tc.enums++; tc.evals += __popc(evaluated); tc.contribs += __popc(contrib); s.hit_count += __popc(contrib); }
         s.T_prev = T; s.contributor = contributor; s.dpt = dpt; s.last_gidx = last_gidx;
-        go = fwd_end_chunk(p, ray, s, stop, cnt, DIAG);
+        go = fwd_end_chunk(p, slot, s, stop, cnt, DIAG);
     }
     return __shfl_sync(FULL, go, 0);
 }
@@ -605,10 +625,10 @@ __global__ void __launch_bounds__(WTAIL_THREADS, DST_WTAIL_BLOCKS) k_fwd_tail_wa
     WarpShade& ws = shade_mem[w];
     TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
     for (int i = blockIdx.x * (WTAIL_THREADS / 32) + w; i < n; i += warps) {
-        const int ray = list[i];
-        if (ray < 0) continue;
+        const int slot = list[i];
+        if (slot < 0) continue;
         if (lane < (int)(sizeof(FwdState) / 16))
-            reinterpret_cast<float4*>(&ws.s)[lane] = reinterpret_cast<const float4*>(reinterpret_cast<const FwdState*>(p.state) + ray)[lane];
+            reinterpret_cast<float4*>(&ws.s)[lane] = p.state[soa(slot, lane, 8)];
         __syncwarp();
         bool alive = true;
         while (alive) {
@@ -616,7 +636,7 @@ __global__ void __launch_bounds__(WTAIL_THREADS, DST_WTAIL_BLOCKS) k_fwd_tail_wa
             fwd_request(ws.s, q);
             unsigned long long key;
             const int cnt = knearest_warp<DIAG>(p.bvh, q.ox, q.oy, q.oz, q.dx, q.dy, q.dz, q.kmax0, absmax, walk_mem[w], key, p.status, tc);
-            alive = fwd_shade_warp<DIAG>(p, ray, ws, key, cnt, tc);
+            alive = fwd_shade_warp<DIAG>(p, slot, ws, key, cnt, tc);
             __syncwarp();
         }
     }
@@ -683,7 +703,7 @@ int dst_prepare_cache(dst_handle* h, const dst_trace_inputs* in, cudaStream_t st
 // state record replaces the buffers with ones that hold the larger of the old and the new value of each)
 int dst_ensure_wavefront(dst_handle* h, long long slots, size_t state_bytes) {
     if (slots <= h->wf_cap && state_bytes <= h->wf_state_bytes) return DST_OK;
-    const long long cap = slots > h->wf_cap ? slots + slots / 16 + 1024 : h->wf_cap;
+    const long long cap = slots > h->wf_cap ? (slots + slots / 16 + 1024 + 31) / 32 * 32 : h->wf_cap;
     const size_t sb = state_bytes > h->wf_state_bytes ? state_bytes : h->wf_state_bytes;
     cudaFree(h->wf_state); cudaFree(h->wf_req); cudaFree(h->wf_kbuf); cudaFree(h->wf_kcnt); cudaFree(h->wf_list[0]); cudaFree(h->wf_list[1]);
     cudaFree(h->wf_counts); cudaFree(h->wf_tmp); cudaFree(h->wf_wcnt); cudaFree(h->wf_bcnt);
@@ -728,10 +748,12 @@ long long dst_call_signature(const dst_trace_inputs* in) {
     return ((long long)in->H * 1000003ll + in->W) * 1000033ll + (long long)in->P * 131ll + in->max_trace_depth + 1;
 }
 
-// chunk-log buffers for `rays` rays of up to `segs` segments (grow-only)
-int dst_ensure_chunk_log(dst_handle* h, long long rays, int segs) {
-    // first guess 12 chunks per ray; afterwards what the previous training forward actually needed (read back
-    // asynchronously, see dst_forward_impl), within DST_LOG_MAX_RECORDS. Rays beyond the log re-trace in the backward.
+// Contribution log for `slots` list slots of up to `segs` segments (grow-only). A training forward logs every contribution (depth along
+// the segment, primitive) so that the backward can composite them again without walking the hierarchy: records of 16 entries,
+// chained per segment, 32 records interleaved (soa()); per segment and slot the first record and the number of entries.
+int dst_ensure_log(dst_handle* h, long long rays, long long slots, int segs) {
+    // first guess 12 records per ray; afterwards what the previous training forward actually needed (read back
+    // asynchronously, see forward_common), within DST_LOG_MAX_RECORDS. Rays beyond the log re-trace in the backward.
     long long want = rays * 12 + 4096;
     if (h->log_needed_host && h->log_needed_event && cudaEventQuery(h->log_needed_event) == cudaSuccess) {
         const long long seen = *h->log_needed_host;
@@ -740,22 +762,23 @@ int dst_ensure_chunk_log(dst_handle* h, long long rays, int segs) {
     } else cudaGetLastError();
     if (want > DST_LOG_MAX_RECORDS) want = DST_LOG_MAX_RECORDS;
     if (h->log_max_records > 0 && want > h->log_max_records) want = h->log_max_records;
-    if (want > h->log_cap || (h->log_max_records > 0 && h->log_cap > h->log_max_records)) {
-        cudaFree(h->log_keys); cudaFree(h->log_hdr); h->log_keys = nullptr; h->log_hdr = nullptr; h->log_cap = 0;
+    want = (want + 31) / 32 * 32;
+    if (want > h->log_cap || (h->log_max_records > 0 && h->log_cap > want)) {
+        cudaFree(h->log_keys); cudaFree(h->log_next); h->log_keys = nullptr; h->log_next = nullptr; h->log_cap = 0;
         cudaError_t e = cudaMalloc(&h->log_keys, 8 * DST_CHUNK * (size_t)want);
-        if (e == cudaSuccess) e = cudaMalloc(&h->log_hdr, sizeof(int2) * (size_t)want);
-        if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "chunk log allocation failed: %s", cudaGetErrorString(e)); }
+        if (e == cudaSuccess) e = cudaMalloc(&h->log_next, sizeof(int) * (size_t)want);
+        if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed: %s", cudaGetErrorString(e)); }
         h->log_cap = want;
     }
-    if (!h->log_count && cudaMalloc(&h->log_count, 4) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "chunk log allocation failed"); }
-    if (rays > h->log_rays_cap || segs > h->log_seg_stride_cap) {
-        cudaFree(h->log_seg_head); cudaFree(h->log_ray_ok); h->log_seg_head = nullptr; h->log_ray_ok = nullptr;
-        const long long rc = rays > h->log_rays_cap ? rays + rays / 16 + 1024 : h->log_rays_cap;
-        const int sc = segs > h->log_seg_stride_cap ? segs : h->log_seg_stride_cap;
-        cudaError_t e = cudaMalloc(&h->log_seg_head, 4 * (size_t)rc * sc);
-        if (e == cudaSuccess) e = cudaMalloc(&h->log_ray_ok, (size_t)rc);
-        if (e != cudaSuccess) { cudaGetLastError(); h->log_rays_cap = 0; h->log_seg_stride_cap = 0; return dst_set_error(h, DST_E_NOMEM, "chunk log allocation failed: %s", cudaGetErrorString(e)); }
-        h->log_rays_cap = rc; h->log_seg_stride_cap = sc;
+    if (!h->log_count && cudaMalloc(&h->log_count, 4) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed"); }
+    if (slots * segs > h->log_index_cap) {
+        cudaFree(h->log_head); cudaFree(h->log_num); cudaFree(h->log_ok); h->log_head = h->log_num = nullptr; h->log_ok = nullptr; h->log_index_cap = 0;
+        const long long cap = slots * segs + slots / 16 + 1024;
+        cudaError_t e = cudaMalloc(&h->log_head, 4 * (size_t)cap);
+        if (e == cudaSuccess) e = cudaMalloc(&h->log_num, 4 * (size_t)cap);
+        if (e == cudaSuccess) e = cudaMalloc(&h->log_ok, (size_t)cap);
+        if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed: %s", cudaGetErrorString(e)); }
+        h->log_index_cap = cap;
     }
     return DST_OK;
 }
@@ -836,17 +859,17 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     if (rc != DST_OK) return rc;
     p.cache = h->cache;
     if (a->training && a->a_weights) DST_CUDA_TRY(h, cudaMemsetAsync(a->a_weights, 0, 4 * (size_t)a->in.P, st));
-    p.state = h->wf_state; p.req = static_cast<EnumReq*>(h->wf_req); p.kbuf = h->wf_kbuf; p.kcnt = h->wf_kcnt;
+    p.state = static_cast<float4*>(h->wf_state); p.req = static_cast<float4*>(h->wf_req); p.kbuf = h->wf_kbuf; p.kcnt = h->wf_kcnt;
     p.list[0] = h->wf_list[0]; p.list[1] = h->wf_list[1]; p.counts = h->wf_counts;
-    // chunk log for the backward (training calls only)
-    p.log_keys = nullptr; p.log_hdr = nullptr; p.log_count = nullptr; p.log_seg_head = nullptr; p.log_ray_ok = nullptr;
-    p.log_cap = 0; p.log_seg_stride = a->in.max_trace_depth + 1;
+    // contribution log for the backward (training calls only)
+    p.log_keys = nullptr; p.log_next = nullptr; p.log_count = nullptr; p.log_head = p.log_num = nullptr; p.log_ok = nullptr;
+    p.log_cap = 0; p.log_slots = slots;
     h->log_serial = 0;
     if (a->training && h->log_enabled) {
-        rc = dst_ensure_chunk_log(h, (long long)a->in.H * a->in.W, a->in.max_trace_depth + 1);
+        rc = dst_ensure_log(h, (long long)a->in.H * a->in.W, slots, a->in.max_trace_depth + 1);
         if (rc != DST_OK) return rc;
-        p.log_keys = h->log_keys; p.log_hdr = h->log_hdr; p.log_count = h->log_count; p.log_seg_head = h->log_seg_head;
-        p.log_ray_ok = h->log_ray_ok; p.log_cap = (int)h->log_cap;
+        p.log_keys = h->log_keys; p.log_next = h->log_next; p.log_count = h->log_count; p.log_head = h->log_head; p.log_num = h->log_num;
+        p.log_ok = h->log_ok; p.log_cap = (int)h->log_cap;
         DST_CUDA_TRY(h, cudaMemsetAsync(h->log_count, 0, 4, st));
         h->log_serial = ++h->serial_counter;
         h->log_H = a->in.H; h->log_W = a->in.W; h->log_depth = a->in.max_trace_depth;
@@ -1031,9 +1054,8 @@ int dst_knearest_impl(dst_handle* h, const float* ro, const float* rd, int64_t n
 namespace {
 constexpr long long ST_SLOTS = 98304;                        // list entries: rays rounded up to whole 8x4 tiles
 constexpr size_t ST_OFF_CACHE = 0;                                                        // 64 B per surfel
-constexpr size_t ST_OFF_STATE = ST_OFF_CACHE + 64ull * DST_STATIC_MAX_SURFELS;            // 128 B per ray
-constexpr size_t ST_OFF_REQ = ST_OFF_STATE + sizeof(FwdState) * (size_t)DST_STATIC_MAX_RAYS;  // 32 B per ray
-constexpr size_t ST_OFF_LIST = ST_OFF_REQ + sizeof(EnumReq) * (size_t)DST_STATIC_MAX_RAYS;    // 4 B per slot
+constexpr size_t ST_OFF_STATE = ST_OFF_CACHE + 64ull * DST_STATIC_MAX_SURFELS;            // 128 B per slot
+constexpr size_t ST_OFF_LIST = ST_OFF_STATE + sizeof(FwdState) * (size_t)ST_SLOTS;            // 4 B per slot
 constexpr size_t ST_OFF_COUNTS = ST_OFF_LIST + 4ull * ST_SLOTS;                               // round counters
 constexpr size_t ST_BYTES = ST_OFF_COUNTS + 4ull * DST_COUNTS_STRIDE + 256;
 }
@@ -1082,15 +1104,14 @@ extern "C" int dst_forward_static(dst_handle* h, const dst_fwd_args* a, void* st
     p.slot0 = 0; p.bound_stats = nullptr; p.bound_factor = 0.0f;
     p.dist_on = h->distortion;
     p.cache = reinterpret_cast<const float4*>(base + ST_OFF_CACHE);
-    p.state = base + ST_OFF_STATE;
-    p.req = reinterpret_cast<EnumReq*>(base + ST_OFF_REQ);
-    p.kbuf = nullptr; p.kcnt = nullptr;                          // only the per-ray kernel runs: no round buffers
+    p.state = reinterpret_cast<float4*>(base + ST_OFF_STATE);
+    p.req = nullptr; p.kbuf = nullptr; p.kcnt = nullptr;                          // only the per-ray kernel runs: no round buffers
     p.list[0] = reinterpret_cast<int*>(base + ST_OFF_LIST); p.list[1] = p.list[0];
     p.counts = reinterpret_cast<int*>(base + ST_OFF_COUNTS);
     p.rounds = 0; p.min_count = 1;
     memset(&p.lv, 0, sizeof(p.lv));                              // no rounds, no list hand-over
-    p.log_keys = nullptr; p.log_hdr = nullptr; p.log_count = nullptr; p.log_seg_head = nullptr; p.log_ray_ok = nullptr;
-    p.log_cap = 0; p.log_seg_stride = 0;
+    p.log_keys = nullptr; p.log_next = nullptr; p.log_count = nullptr; p.log_head = p.log_num = nullptr; p.log_ok = nullptr;
+    p.log_cap = 0; p.log_slots = 0;
     // the array keeps the previous call's contents: the round counters must start at zero, everything else is rewritten
     DST_CUDA_TRY(h, cudaMemsetAsync(p.counts, 0, 4 * DST_COUNTS_STRIDE, st));
     if (a->training && a->a_weights) DST_CUDA_TRY(h, cudaMemsetAsync(a->a_weights, 0, 4 * (size_t)a->in.P, st));

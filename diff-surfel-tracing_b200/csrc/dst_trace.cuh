@@ -275,6 +275,23 @@ __device__ __forceinline__ bool eval_slot(unsigned long long key, float offset, 
 // ---------------------------------------------------------------------------------------------
 struct __align__(16) EnumReq { float ox, oy, oz, dx, dy, dz, kmax0, pad; };
 
+// Everything a ray keeps between kernels is indexed by its list slot (its place in the tile-ordered list of round 0, see slot_ray()), in blocks of
+// 32 slots with the words of a record one after the other and the 32 slots of a block side by side. The rays of a warp are (survivors of)
+// neighbouring slots, so a warp's access to one word of its rays' records touches a few cache lines; as one record per ray it touched
+// 32, and the composite kernel, whose loads those mostly were, was bound by them.
+__device__ __forceinline__ size_t soa(int slot, int word, int words) { return ((size_t)(slot >> 5) * words + word) * 32 + (slot & 31); }
+__device__ __forceinline__ EnumReq load_req(const float4* req, int slot) {
+    const float4 a = req[soa(slot, 0, 2)], b = req[soa(slot, 1, 2)];
+    EnumReq q;
+    q.ox = a.x; q.oy = a.y; q.oz = a.z; q.dx = a.w; q.dy = b.x; q.dz = b.y; q.kmax0 = b.z; q.pad = b.w;
+    return q;
+}
+__device__ __forceinline__ void store_req(float4* req, int slot, const EnumReq& q) {
+    req[soa(slot, 0, 2)] = make_float4(q.ox, q.oy, q.oz, q.dx);
+    req[soa(slot, 1, 2)] = make_float4(q.dy, q.dz, q.kmax0, q.pad);
+}
+__device__ __forceinline__ float& req_bound(float4* req, int slot) { return req[soa(slot, 1, 2)].z; }
+
 constexpr int ENUM_THREADS = 128;
 #ifndef DST_ENUM_MIN_BLOCKS
 #define DST_ENUM_MIN_BLOCKS 6         // resident blocks per SM the gather kernel is compiled for
@@ -482,7 +499,7 @@ __device__ __forceinline__ void make_beam(WalkMem& m, bool active, float ox, flo
 // First step of a gather: 32 consecutive entries of the live list per warp. A batch that is given up goes to `heavy` with its 32 slots, each ray
 // with the search bound it has found.
 template <bool COUNT>
-__global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhView bvh, EnumReq* req, const int* __restrict__ list,
+__global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhView bvh, float4* req, const int* __restrict__ list,
                                                        const int* __restrict__ count_ptr, int* cursor, int min_count,
                                                        unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
                                                        unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count) {
@@ -505,15 +522,15 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
         // The list is taken from its end: rays on a reflected segment come last in it (k_compact) and their batches are
         // the slow ones, so they start first and the cheap batches of primary rays fill the end of the round.
         const int idx = (((total + 31) >> 5) - 1 - (base >> 5)) * 32 + lane;
-        const int ray = idx < total ? list[idx] : -1;
+        const int slot = idx < total ? list[idx] : -1;
         bool active = false;
         int n = 0;
         float kmax = -1.0f, ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f;
-        if (ray >= 0) {
-            const float4 r0 = __ldg(reinterpret_cast<const float4*>(req + ray)), r1 = __ldg(reinterpret_cast<const float4*>(req + ray) + 1);
-            ox = r0.x; oy = r0.y; oz = r0.z; dx = r0.w; dy = r1.x; dz = r1.y;
+        if (slot >= 0) {
+            const EnumReq q = load_req(req, slot);
+            ox = q.ox; oy = q.oy; oz = q.oz; dx = q.dx; dy = q.dy; dz = q.dz;
             active = fabsf(ox) < INFINITY && fabsf(oy) < INFINITY && fabsf(oz) < INFINITY && fabsf(dx) < INFINITY && fabsf(dy) < INFINITY && fabsf(dz) < INFINITY;
-            if (active) kmax = r1.z;
+            if (active) kmax = q.kmax0;
             if (COUNT) tc.enums++;
         }
         if (__any_sync(FULL, active)) {
@@ -554,18 +571,15 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
                 // (a bound below the request's can only have come from a full k-buffer: the repeated search finds 16 hits again)
                 int at = 0;
                 if (lane == 0) at = atomicAdd(heavy_count, 32);
-                heavy[__shfl_sync(FULL, at, 0) + lane] = active ? ray : -1;
-                if (active) { req[ray].kmax0 = kmax; continue; }
+                heavy[__shfl_sync(FULL, at, 0) + lane] = active ? slot : -1;
+                if (active) { req_bound(req, slot) = kmax; continue; }
                 n = 0;
             }
         }
-        if (ray >= 0) {
-            kcnt[ray] = n;
-            ulonglong2* out = reinterpret_cast<ulonglong2*>(kbuf + (size_t)ray * DST_CHUNK);
+        if (slot >= 0) {
+            kcnt[slot] = n;
 #pragma unroll
-            for (int k = 0; k < DST_CHUNK / 2; k++) {
-                if (2 * k < n) out[k] = make_ulonglong2(kb[(2 * k) * KS], kb[(2 * k + 1) * KS]);
-            }
+            for (int i = 0; i < DST_CHUNK; i++) if (i < n) kbuf[soa(slot, i, DST_CHUNK)] = kb[i * KS];
         }
     }
     if (COUNT && counters) { atomicAdd(counters + 1, tc.enums); atomicAdd(counters + 2, tc.nodes); atomicAdd(counters + 3, tc.quads); }
@@ -621,7 +635,7 @@ __device__ __forceinline__ int knearest_warp(const BvhView& bvh, float ox, float
 // that of the group's hull; a quad step tests its 32 quads (one per lane) exactly against one ray of the group after the
 // other. The k-buffers are in shared memory; lanes 0..15 hold one of them at a time.
 template <bool COUNT>
-__global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_group(BvhView bvh, EnumReq* req, const int* __restrict__ list,
+__global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_group(BvhView bvh, float4* req, const int* __restrict__ list,
                                                        const int* __restrict__ count_ptr, int* cursor,
                                                        unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
                                                        unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count) {
@@ -640,15 +654,15 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
         if (lane == 0) i = atomicAdd(cursor, 1);
         i = __shfl_sync(FULL, i, 0);
         if (i >= total) break;
-        const int ray = lane < DST_GROUP ? list[i * DST_GROUP + lane] : -1;
-        const unsigned int members = __ballot_sync(FULL, ray >= 0);
+        const int slot = lane < DST_GROUP ? list[i * DST_GROUP + lane] : -1;
+        const unsigned int members = __ballot_sync(FULL, slot >= 0);
         if (members == 0u) continue;
         float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
-        if (ray >= 0) { r0 = *reinterpret_cast<const float4*>(req + ray); r1 = *(reinterpret_cast<const float4*>(req + ray) + 1); }
-        const float bound0 = ray >= 0 ? r1.z : -1.0f;
+        if (slot >= 0) { r0 = req[soa(slot, 0, 2)]; r1 = req[soa(slot, 1, 2)]; }
+        const float bound0 = slot >= 0 ? r1.z : -1.0f;
         if (lane < DST_GROUP) { srays[w][lane][0] = r0; srays[w][lane][1] = make_float4(r1.x, r1.y, bound0, 0.0f); }
         for (int k = lane; k < DST_GROUP * DST_CHUNK; k += 32) (&skeys[w][0][0])[k] = ~0ull;
-        make_beam(m, ray >= 0, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, absmax);
+        make_beam(m, slot >= 0, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, absmax);
         float krun = redux_max(bound0);
         const bool done = beam_walk<COUNT>(bvh, m, krun, DST_GROUP_STEPS, status, tc, [&](bool valid, int pos) {
             Quad q;
@@ -690,17 +704,17 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
 #pragma unroll 1
             for (int r = 0; r < DST_GROUP; r++) {
                 if (!((members >> r) & 1u)) continue;
-                const int rr = __shfl_sync(FULL, ray, r);
+                const int to = __shfl_sync(FULL, slot, r);
                 const unsigned long long mine = skeys[w][r][lane & (DST_CHUNK - 1)];
                 const int n = __popc(__ballot_sync(FULL, lane < DST_CHUNK && mine != ~0ull));
-                if (lane < n) kbuf[(size_t)rr * DST_CHUNK + lane] = mine;
-                if (lane == 0) kcnt[rr] = n;
+                if (lane < n) kbuf[soa(to, lane, DST_CHUNK)] = mine;
+                if (lane == 0) kcnt[to] = n;
             }
         } else {
             int at = 0;
             if (lane == 0) at = atomicAdd(heavy_count, __popc(members));
             at = __shfl_sync(FULL, at, 0) + __popc(members & ((1u << lane) - 1u));
-            if (ray >= 0) { heavy[at] = ray; req[ray].kmax0 = srays[w][lane][1].z; }
+            if (slot >= 0) { heavy[at] = slot; req_bound(req, slot) = srays[w][lane][1].z; }
         }
         __syncwarp();
     }
@@ -709,7 +723,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
 
 // Last step of a gather: the rays whose batch was given up by k_enum, one warp per ray.
 template <bool COUNT>
-__global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray(BvhView bvh, const EnumReq* __restrict__ req, const int* __restrict__ list,
+__global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray(BvhView bvh, const float4* __restrict__ req, const int* __restrict__ list,
                                                        const int* __restrict__ count_ptr, int* cursor,
                                                        unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
                                                        unsigned int* status, unsigned long long* counters) {
@@ -725,12 +739,12 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray
         if (lane == 0) i = atomicAdd(cursor, 1);
         i = __shfl_sync(0xffffffffu, i, 0);
         if (i >= total) break;
-        const int ray = list[i];
-        const float4 r0 = __ldg(reinterpret_cast<const float4*>(req + ray)), r1 = __ldg(reinterpret_cast<const float4*>(req + ray) + 1);
+        const int slot = list[i];
+        const float4 r0 = req[soa(slot, 0, 2)], r1 = req[soa(slot, 1, 2)];
         unsigned long long key;
         const int n = knearest_warp<COUNT>(bvh, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, absmax, m, key, status, tc);
-        if (lane < n) kbuf[(size_t)ray * DST_CHUNK + lane] = key;
-        if (lane == 0) kcnt[ray] = n;
+        if (lane < n) kbuf[soa(slot, lane, DST_CHUNK)] = key;
+        if (lane == 0) kcnt[slot] = n;
         __syncwarp();
     }
     if (COUNT && counters) { atomicAdd(counters + 2, tc.nodes); atomicAdd(counters + 3, tc.quads); }
@@ -738,7 +752,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray
 
 // the gather launches of a wavefront round (diag: with traversal counters). cnt: the round's entry in the set of round counters;
 // heavy, heavy2: lists of as many rays as the round has slots
-static inline void launch_gather(bool diag, int grid, cudaStream_t st, const BvhView& bvh, EnumReq* req, const int* list,
+static inline void launch_gather(bool diag, int grid, cudaStream_t st, const BvhView& bvh, float4* req, const int* list,
                                  const int* count_ptr, int* cnt, int min_count, unsigned long long* kbuf, int* kcnt, unsigned int* status,
                                  unsigned long long* counters, int* heavy, int* heavy2) {
     constexpr int R = DST_WF_ROUNDS + 2;
@@ -753,7 +767,7 @@ static inline void launch_gather(bool diag, int grid, cudaStream_t st, const Bvh
     }
 }
 
-// List entry i of round 0 -> ray index (or -1). Image-like grids are walked in 8x4 pixel tiles (one tile = the 32
+// List slot i -> ray index (or -1). Image-like grids are walked in 8x4 pixel tiles (one tile = the 32
 // rays a warp of the gather kernel takes), and the tiles in Z order inside blocks of 8x8 tiles (64x32 pixels): any
 // aligned run of 2 or 4 consecutive tiles is a compact 16x4 or 16x8 pixel patch. That matters once rays have
 // dropped out: the lists keep this order, so a warp of a later round holds the survivors of a few consecutive
@@ -762,7 +776,7 @@ static inline void launch_gather(bool diag, int grid, cudaStream_t st, const Bvh
 #ifndef DST_TILE_BLOCK
 #define DST_TILE_BLOCK 8              // tiles per side of a Z-ordered block (1: row-major tile order)
 #endif
-__device__ __forceinline__ int ray_of_slot(long long i, int H, int W, bool tiled) {
+__device__ __forceinline__ int slot_ray(long long i, int H, int W, bool tiled) {
     if (!tiled) return i < (long long)H * W ? (int)i : -1;
     const int tiles_x = (W + 7) >> 3;
     long long tile = i >> 5;
