@@ -72,9 +72,9 @@ static_assert(sizeof(BwdState) == 176, "ray state is eleven 16-byte words");
 // basis values of the ray's direction, which stay the same for a whole segment, and three colour gradients: a lane stages the three,
 // and the sum over the lanes of a group is formed from them and the basis values in shared memory.
 // ---------------------------------------------------------------------------------------------
-constexpr int STAGE_FLOATS = DST_ARENA_FLOATS + 48;                       // arena row + the longest SH row
 struct BwdWarp {
-    float rows[32][STAGE_FLOATS];       // lane's arena row; SH row of the lanes that send one
+    float rows[32][DST_ARENA_FLOATS];   // lane's arena row
+    float sh[32][48];                   // SH row of the lanes that send one
     float4 colour[32];                  // colour gradients of the lane's contribution (clamped channels 0)
     float basis[16][33];                // SH basis of the lane's segment direction, one column per lane
 };
@@ -110,7 +110,7 @@ __device__ __forceinline__ void send_rows(const RowTarget& t, BwdWarp& ws, int g
     if (t.dsh && alone) {       // a row of its own
         const float4 m = ws.colour[lane];
         if (t.bulk) {
-            float4* o = reinterpret_cast<float4*>(ws.rows[lane] + DST_ARENA_FLOATS);
+            float4* o = reinterpret_cast<float4*>(ws.sh[lane]);
 #pragma unroll
             for (int q = 0; q < 4; q++) {       // four basis values are three float4 of the row
                 if (4 * q < t.ncoef) {
@@ -128,69 +128,55 @@ __device__ __forceinline__ void send_rows(const RowTarget& t, BwdWarp& ws, int g
             }
         }
     }
-    const bool leader = gidx >= 0 && lane == __ffs(peers) - 1;
-    __syncwarp();                                                        // every lane's row is staged
-    for (unsigned int todo = __ballot_sync(FULL, leader && !alone); todo; todo &= todo - 1u) {
-        const int lead = __ffs(todo) - 1;
-        const unsigned int grp = __shfl_sync(FULL, peers, lead);
-        {   // arena row: lane c sums float c of the group's rows
-            float acc = 0.0f;
-            const float* col = &ws.rows[0][lane < DST_ARENA_FLOATS ? lane : 0];
-            if (grp == FULL) {
-#pragma unroll 8
-                for (int r = 0; r < 32; r++) acc += col[r * STAGE_FLOATS];
-            } else {
-                for (unsigned int q = grp; q;) {                         // four rows per pass, so that their loads are in flight together
-                    const int r0 = __ffs(q) - 1; q &= q - 1u;
-                    const int r1 = __ffs(q) - 1; q &= q - 1u;
-                    const int r2 = __ffs(q) - 1; q &= q - 1u;
-                    const int r3 = __ffs(q) - 1; q &= q - 1u;
-                    const float x0 = col[r0 * STAGE_FLOATS], x1 = r1 >= 0 ? col[r1 * STAGE_FLOATS] : 0.0f;
-                    const float x2 = r2 >= 0 ? col[r2 * STAGE_FLOATS] : 0.0f, x3 = r3 >= 0 ? col[r3 * STAGE_FLOATS] : 0.0f;
-                    acc += (x0 + x1) + (x2 + x3);
-                }
-            }
-            if (lane < DST_ARENA_FLOATS) ws.rows[lead][lane] = acc;
-        }
-        if (t.dsh) {   // SH row: lane (j, half) sums coefficient j over the lanes 16 half .. 16 half + 15 of the group
-            const int j = lane & 15, g = __shfl_sync(FULL, gidx, lead);
-            float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
-            const unsigned int half = (lane >> 4) * 16;
-            unsigned int q = (grp >> half) & 0xffffu;
-            if (grp == FULL) {
-#pragma unroll 8
-                for (int r = 0; r < 16; r++) {
-                    const float4 m = ws.colour[half + r];
-                    const float b = ws.basis[j][half + r];
-                    a0 = fmaf(b, m.x, a0); a1 = fmaf(b, m.y, a1); a2 = fmaf(b, m.z, a2);
-                }
-            } else {
-                while (q) {
-                    const int r = __ffs(q) - 1; q &= q - 1u;
-                    const float4 m = ws.colour[half + r];
-                    const float b = ws.basis[j][half + r];
-                    a0 = fmaf(b, m.x, a0); a1 = fmaf(b, m.y, a1); a2 = fmaf(b, m.z, a2);
-                }
-                __syncwarp();
-            }
-            a0 += __shfl_xor_sync(FULL, a0, 16); a1 += __shfl_xor_sync(FULL, a1, 16); a2 += __shfl_xor_sync(FULL, a2, 16);
-            if (lane < t.ncoef) {       // (ncoef <= 16: lanes of half 0)
-                if (t.bulk) {
-                    float* o = ws.rows[lead] + DST_ARENA_FLOATS + 3 * j;
-                    o[0] = a0; o[1] = a1; o[2] = a2;
-                } else {
-                    float* d = t.dsh + 3 * ((size_t)g * t.coeffs + j);
-                    atomicAdd(d, a0); atomicAdd(d + 1, a1); atomicAdd(d + 2, a2);
-                }
-            }
-        }
-    }
     bulk_fence();
-    __syncwarp();                                                        // the sums are in place
-    if (leader) {
+    __syncwarp();                                                        // every lane's row is staged
+    if (alone) {
         bulk_add(t.arena + (size_t)gidx * DST_ARENA_FLOATS, ws.rows[lane], DST_ARENA_FLOATS * 4);
-        if (t.bulk) bulk_add(t.dsh + 3 * (size_t)gidx * t.coeffs, ws.rows[lane] + DST_ARENA_FLOATS, 12 * t.ncoef);
+        if (t.bulk) bulk_add(t.dsh + 3 * (size_t)gidx * t.coeffs, ws.sh[lane], 12 * t.ncoef);
         bulk_commit();
+    }
+    // Groups, one after the other. The lanes share the sums of a row out: floats 0..15 to lanes 16..31, 16..19 to lanes 0..3; SH
+    // coefficient j, channels 0 and 1 to lane j, channel 2 to lane 16 + j.
+    const int j = lane & 15, upper = lane >> 4;
+    const float* col = &ws.rows[0][upper ? j : 16 + (lane & 3)];
+    const float* bas = &ws.basis[j][0];
+    const float2* clr = reinterpret_cast<const float2*>(ws.colour) + upper;
+    for (unsigned int todo = __ballot_sync(FULL, gidx >= 0 && !alone && lane == __ffs(peers) - 1); todo; todo &= todo - 1u) {
+        const int lead = __ffs(todo) - 1;
+        unsigned int q = __shfl_sync(FULL, peers, lead);
+        const int g = __shfl_sync(FULL, gidx, lead);
+        float a = 0.0f, c0 = 0.0f, c1 = 0.0f;
+        do {                                                             // two rows per pass (the second with weight 0 where there is none)
+            const int r0 = __ffs(q) - 1;
+            q &= q - 1u;
+            const int r1 = q ? __ffs(q) - 1 : r0;
+            const float w1 = q ? 1.0f : 0.0f;
+            q &= q - 1u;
+            a += fmaf(w1, col[r1 * DST_ARENA_FLOATS], col[r0 * DST_ARENA_FLOATS]);
+            if (t.dsh) {
+                const float2 m0 = clr[2 * r0], m1 = clr[2 * r1];
+                const float b0 = bas[r0], b1 = w1 * bas[r1];
+                c0 = fmaf(b0, m0.x, c0); c1 = fmaf(b0, m0.y, c1);
+                c0 = fmaf(b1, m1.x, c0); c1 = fmaf(b1, m1.y, c1);
+            }
+        } while (q);
+        __syncwarp();
+        if (upper) ws.rows[lead][j] = a; else if (lane < 4) ws.rows[lead][16 + lane] = a;
+        if (t.dsh && j < t.ncoef) {
+            if (t.bulk) {
+                if (upper) ws.sh[lead][3 * j + 2] = c0; else { ws.sh[lead][3 * j] = c0; ws.sh[lead][3 * j + 1] = c1; }
+            } else {
+                float* d = t.dsh + 3 * ((size_t)g * t.coeffs + j);
+                if (upper) atomicAdd(d + 2, c0); else { atomicAdd(d, c0); atomicAdd(d + 1, c1); }
+            }
+        }
+        bulk_fence();
+        __syncwarp();
+        if (lane == lead) {
+            bulk_add(t.arena + (size_t)g * DST_ARENA_FLOATS, ws.rows[lane], DST_ARENA_FLOATS * 4);
+            if (t.bulk) bulk_add(t.dsh + 3 * (size_t)g * t.coeffs, ws.sh[lane], 12 * t.ncoef);
+            bulk_commit();
+        }
     }
 }
 

@@ -122,27 +122,21 @@ __global__ void __launch_bounds__(256) k_prepare_cache(int P, const float* __res
     o[3] = make_float4(sx, sy, xdiv(1.0f, sx), xdiv(1.0f, sy));
 }
 
-// a_weights[gidx] += w (optix_tracer/forward.cu:295), aggregated over the lanes of the warp that are here together.
-// The lanes of a warp are neighbouring pixels walking their chunks in step, and they composite the same surfels at the
-// same time: the lanes that hold the same surfel add their weights up with shuffles and one of them issues the atomic.
-// As one atomic per contribution this was 7 of the 16 ms the composite kernel takes on the 3M-surfel 1080p workload
-// (the L2 serialises additions to one address, and surfels near the camera are hit by thousands of rays).
+// a_weights[gidx] += w (optix_tracer/forward.cu:295), aggregated over the warp: neighbouring pixels composite the same surfels
+// at the same time, and as one atomic per contribution this was half of what the composite kernel takes (the L2 serialises additions to
+// one address). Lanes hold a partial sum for a surfel (gidx < 0: none); in five butterfly steps a lane whose partner holds
+// the same surfel takes or hands over the sum, which leaves one lane per patch of the tile (35 instructions; grouping all lanes with
+// the same surfel by match_any and a shuffle loop leaves a few atomics less and took 4 ms more on the 3M-surfel 1080p workload).
+// Called by all 32 lanes.
 __device__ __forceinline__ void add_weight(float* __restrict__ a_weights, int gidx, float w) {
-    const unsigned int act = __activemask();
-    unsigned int peers = __match_any_sync(act, gidx);
     const int lane = threadIdx.x & 31;
-    const int first = __ffs(peers) - 1;
-    int rel_pos = __popc(peers << (32 - lane)) * (lane != 0);        // my rank among the peers (a shift by 32 is undefined: lane 0 has rank 0)
-    peers &= (0xfffffffeu << lane);                                  // peers above me
-    while (__any_sync(act, peers != 0u)) {
-        const int next = __ffs(peers);
-        const float t = __shfl_sync(act, w, next ? next - 1 : lane);
-        if (next) w += t;
-        const bool done = rel_pos & 1;                               // my value was taken in this step
-        peers &= __ballot_sync(act, !done);
-        rel_pos >>= 1;
+#pragma unroll
+    for (int step = 1; step < 32; step <<= 1) {
+        const int pg = __shfl_xor_sync(0xffffffffu, gidx, step);
+        const float pw = __shfl_xor_sync(0xffffffffu, w, step);
+        if (pg == gidx) { w += pw; if (lane & step) gidx = -1; }
     }
-    if (lane == first) atomicAdd(a_weights + gidx, w);
+    if (gidx >= 0) atomicAdd(a_weights + gidx, w);
 }
 
 __device__ __forceinline__ void fwd_begin_segment(FwdState& s) {
@@ -278,10 +272,10 @@ __device__ __forceinline__ void log_entry(const FwdParams& p, int slot, FwdState
     if (s.log_rec >= 0) p.log_keys[soa(s.log_rec, at & (DST_CHUNK - 1), DST_CHUNK)] = make_key(dpt, pidx);
 }
 
-// Composites one gathered chunk (forward.cu:197-306), one thread per ray. Returns true while the ray needs another enumeration.
-// kb: the chunk's keys with stride KS; cnt: how many.
+// Composites one gathered chunk (forward.cu:197-306), one thread per ray, the rays of a warp in step: all 32 lanes call
+// it, `in_chunk` marks those with a chunk. Returns true while the ray needs another enumeration. kb: the chunk's keys with stride KS; cnt: how many.
 template <bool DIAG, int KS>
-__device__ __forceinline__ bool fwd_shade(const FwdParams& p, int slot, FwdState& s, const unsigned long long* kb, int cnt, TraceCounters& tc) {
+__device__ __forceinline__ bool fwd_shade(const FwdParams& p, bool in_chunk, int slot, FwdState& s, const unsigned long long* kb, int cnt, TraceCounters& tc) {
     const dst_trace_inputs& in = p.a.in;
     const bool use_sh = in.colors_precomp == nullptr;
     const bool has_aux = in.others_precomp != nullptr;
@@ -291,8 +285,8 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, int slot, FwdState
     const float T_threshold = 0.0001f;
     float sb[16];
     if (use_sh) sh_basis(in.sh_degree, s.sdx, s.sdy, s.sdz, sb);
-    if (DIAG) { if (s.chunk == 0) tc.segs++; }
-    if (p.log_keys && s.log_spare < 0 && ((s.contributor & (DST_CHUNK - 1)) == 0 || (s.contributor & (DST_CHUNK - 1)) + cnt > DST_CHUNK)) {
+    if (DIAG) { if (in_chunk && s.chunk == 0) tc.segs++; }
+    if (p.log_keys && in_chunk && s.log_spare < 0 && ((s.contributor & (DST_CHUNK - 1)) == 0 || (s.contributor & (DST_CHUNK - 1)) + cnt > DST_CHUNK)) {
         // a chunk can fill at most one further record: it is reserved here, where the lanes of a warp that need one get neighbouring ones,
         // and kept for the next chunk or segment when it is not used
         const int rec = atomicAdd(p.log_count, 1);
@@ -301,17 +295,23 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, int slot, FwdState
     }
 
     float T_next = 1.0f;
-    bool stop = false;
-    for (int i = 0; i < cnt; i++) {
+    bool stop = !in_chunk;
+    const bool weights = p.a.training && p.a.a_weights;
+    const int n = __reduce_max_sync(0xffffffffu, in_chunk ? cnt : 0);
+    for (int i = 0; i < n; i++) {
+        int wg = -1;
+        float w = 0.f;
+        do {
+        if (stop || i >= cnt) break;
         const unsigned long long key = kb[i * KS];
         const int pidx = (int)(unsigned int)key;
         const int gidx = pidx >> 1;
-        if (gidx == s.last_gidx) continue;                                // forward.cu:207
+        if (gidx == s.last_gidx) break;                                // forward.cu:207
         if (DIAG) tc.evals++;
         SlotEval e;
         const bool ok = eval_slot(key, s.offset, s.sox, s.soy, s.soz, s.sdx, s.sdy, s.sdz, min_depth, p.cache, gidx, e);
         s.dpt = e.dpt;                                                    // :211 (kept even when the slot is skipped)
-        if (!ok) continue;
+        if (!ok) break;
         const float alpha = e.alpha, nsign = e.nsign;
         const float4 r2 = e.r2;
         T_next = xmul(s.T_prev, xsub(1.0f, alpha));
@@ -319,7 +319,7 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, int slot, FwdState
         s.contributor++;
         if (s.contributor > DST_MAX_INTERSECTION) { stop = true; break; }
         s.last_gidx = gidx;
-        const float w = xmul(alpha, s.T_prev);
+        w = xmul(alpha, s.T_prev);
         if (p.log_keys) log_entry(p, slot, s, s.contributor - 1, s.dpt, (unsigned int)pidx);
         if (use_sh) {
             float c[48];
@@ -348,13 +348,16 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, int slot, FwdState
         s.D = xadd(s.D, xmul(w, s.dpt));
         s.Nx = xadd(s.Nx, xmul(w, nsign * r2.x)); s.Ny = xadd(s.Ny, xmul(w, nsign * r2.y)); s.Nz = xadd(s.Nz, xmul(w, nsign * r2.z));
         s.T_prev = T_next;
-        if (p.a.training && p.a.a_weights) add_weight(p.a.a_weights, gidx, w);          // forward.cu:295
+        wg = gidx;
         if (DIAG) {
             tc.contribs++;
             if (p.a.hit_log && s.hit_count < p.a.hit_cap) p.a.hit_log[(size_t)slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0) * p.a.hit_cap + s.hit_count] = pidx;
             s.hit_count++;
         }
+        } while (false);
+        if (weights) add_weight(p.a.a_weights, wg, w);          // forward.cu:295
     }
+    if (!in_chunk) return false;
     return fwd_end_chunk(p, slot, s, stop || T_next < T_threshold, cnt, DIAG);
 }
 
@@ -420,38 +423,36 @@ __global__ void __launch_bounds__(SHADE_THREADS, DST_SHADE_GRID_PER_SM) k_fwd_sh
     for (int i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < n_pad; i += gridDim.x * SHADE_THREADS) {
         const int slot = i < n ? list[i] : -1;
         bool alive = false, bounded = false, failed = false;
-        int cls = 0;
+        int cls = 0, cnt = 0;
+        FwdState s;
+        const unsigned long long* kb = p.kbuf + soa(slot >= 0 ? slot : 0, 0, DST_CHUNK);
         if (slot >= 0) {
-            FwdState s;
+            cnt = p.kcnt[slot];
             load_state(p.state, slot, s);
-            const unsigned long long* kb = p.kbuf + soa(slot, 0, DST_CHUNK);
-            const int cnt = p.kcnt[slot];
-            if (cnt < DST_CHUNK && req_bound(p.req, slot) < DST_T_MAX) {
-                // The gather searched within a predicted distance (below) and found fewer than 16 hits there: that says nothing
-                // about what lies beyond. Nothing is composited; the same request goes out again without a bound.
-                req_bound(p.req, slot) = DST_T_MAX;
-                alive = true;
-                cls = s.bounce > 0;
-                failed = true;
-                if (DIAG && p.a.counters) atomicAdd(p.a.counters + 1, ~0ull);        // (the counter reports completed enumerations)
-            } else {
-                alive = fwd_shade<DIAG, 32>(p, slot, s, kb, cnt, tc);
-                if (alive) {
-                    store_state(p.state, slot, s);
-                    EnumReq q;
-                    fwd_request(s, q);
-                    // A segment that goes on: its next 16 hits are searched within bound_factor times the distance the last 16
-                    // spanned (first to last). A walk that knows its bound from the start opens a fifth fewer nodes than one that
-                    // learns it from its 16th hit; the spans of consecutive chunks differ by less than that factor for all but
-                    // a per cent of the rays of a dense scene, and those search again.
-                    if (bound_on && s.chunk > 0 && cnt == DST_CHUNK) {
-                        q.kmax0 = fmaxf(p.bound_factor * (hitkey_t(kb[(DST_CHUNK - 1) * 32]) - hitkey_t(kb[0])), 1e-4f);
-                        bounded = true;
-                    }
-                    store_req(p.req, slot, q);
-                    cls = s.bounce > 0;
-                }
+            // Fewer than 16 hits within a predicted distance (below) say nothing about what lies beyond. Nothing is composited; the
+            // same request goes out again without a bound.
+            failed = cnt < DST_CHUNK && req_bound(p.req, slot) < DST_T_MAX;
+        }
+        alive = fwd_shade<DIAG, 32>(p, slot >= 0 && !failed, slot, s, kb, cnt, tc);
+        if (failed) {
+            req_bound(p.req, slot) = DST_T_MAX;
+            alive = true;
+            cls = s.bounce > 0;
+            if (DIAG && p.a.counters) atomicAdd(p.a.counters + 1, ~0ull);        // (the counter reports completed enumerations)
+        } else if (alive) {
+            store_state(p.state, slot, s);
+            EnumReq q;
+            fwd_request(s, q);
+            // A segment that goes on: its next 16 hits are searched within bound_factor times the distance the last 16
+            // spanned (first to last). A walk that knows its bound from the start opens a fifth fewer nodes than one that
+            // learns it from its 16th hit; the spans of consecutive chunks differ by less than that factor for all but
+            // a per cent of the rays of a dense scene, and those search again.
+            if (bound_on && s.chunk > 0 && cnt == DST_CHUNK) {
+                q.kmax0 = fmaxf(p.bound_factor * (hitkey_t(kb[(DST_CHUNK - 1) * 32]) - hitkey_t(kb[0])), 1e-4f);
+                bounded = true;
             }
+            store_req(p.req, slot, q);
+            cls = s.bounce > 0;
         }
         if (p.bound_stats) {
             const unsigned int mb = __ballot_sync(0xffffffffu, bounded), mf = __ballot_sync(0xffffffffu, failed);
@@ -472,18 +473,21 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_fwd_tail(const __grid_constant
     const int* list = p.list[round & 1];
     unsigned long long* kb = kshared + threadIdx.x;
     TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
-    for (int i = blockIdx.x * TAIL_THREADS + threadIdx.x; i < n; i += gridDim.x * TAIL_THREADS) {
-        const int slot = list[i];
-        if (slot < 0) continue;
+    for (int i = blockIdx.x * TAIL_THREADS + threadIdx.x; i - (int)(threadIdx.x & 31) < n; i += gridDim.x * TAIL_THREADS) {
+        const int slot = i < n ? list[i] : -1;
         FwdState s;
-        load_state(p.state, slot, s);
-        bool alive = true;
-        while (alive) {
-            EnumReq q;
-            fwd_request(s, q);
-            const int cnt = knearest<BRUTE, DIAG, TAIL_THREADS>(p.bvh, q.ox, q.oy, q.oz, q.dx, q.dy, q.dz, kb, p.status, tc, q.kmax0);
-            if (DIAG) tc.enums++;
-            alive = fwd_shade<DIAG, TAIL_THREADS>(p, slot, s, kb, cnt, tc);
+        bool alive = slot >= 0;
+        if (alive) load_state(p.state, slot, s);
+        while (__any_sync(0xffffffffu, alive)) {
+            int cnt = 0;
+            if (alive) {
+                EnumReq q;
+                fwd_request(s, q);
+                cnt = knearest<BRUTE, DIAG, TAIL_THREADS>(p.bvh, q.ox, q.oy, q.oz, q.dx, q.dy, q.dz, kb, p.status, tc, q.kmax0);
+                if (DIAG) tc.enums++;
+            }
+            __syncwarp();
+            alive = fwd_shade<DIAG, TAIL_THREADS>(p, alive, slot, s, kb, cnt, tc);
         }
     }
     if (DIAG) flush_counters(p.a.counters, tc);

@@ -162,6 +162,16 @@ __device__ __forceinline__ void load_sh_row(const float* __restrict__ row, int n
     if (aligned) {
         const float4* r4 = reinterpret_cast<const float4*>(row);
         const int nv = nfloat >> 2;
+        if (nv == 12 && (reinterpret_cast<uintptr_t>(row) & 31) == 0) {       // degree 3, the usual layout: six 256-bit loads
+#pragma unroll
+            for (int i = 0; i < 6; i++) {
+                float4 q, r;
+                ldg256(r4 + 2 * i, q, r);
+                c[8 * i] = q.x; c[8 * i + 1] = q.y; c[8 * i + 2] = q.z; c[8 * i + 3] = q.w;
+                c[8 * i + 4] = r.x; c[8 * i + 5] = r.y; c[8 * i + 6] = r.z; c[8 * i + 7] = r.w;
+            }
+            return;
+        }
 #pragma unroll
         for (int i = 0; i < 12; i++) {
             if (i < nv) { const float4 q = __ldg(r4 + i); c[4 * i] = q.x; c[4 * i + 1] = q.y; c[4 * i + 2] = q.z; c[4 * i + 3] = q.w; }
@@ -247,7 +257,7 @@ __device__ __forceinline__ bool eval_slot(unsigned long long key, float offset, 
     e.dpt = xadd(hitkey_t(key), offset);
     e.X = xadd(sox, xmul(e.dpt, sdx)); e.Y = xadd(soy, xmul(e.dpt, sdy)); e.Z = xadd(soz, xmul(e.dpt, sdz));
     const float4* rec = cache + 4 * (size_t)gidx;
-    e.r0 = __ldg(rec); e.r1 = __ldg(rec + 1); e.r2 = __ldg(rec + 2); e.r3 = __ldg(rec + 3);
+    ldg256(rec, e.r0, e.r1); ldg256(rec + 2, e.r2, e.r3);
     const float u1 = xadd(rdot3(e.r0.x, e.r0.y, e.r0.z, e.X, e.Y, e.Z), -e.r0.w);
     const float v1 = xadd(rdot3(e.r1.x, e.r1.y, e.r1.z, e.X, e.Y, e.Z), -e.r1.w);
     e.u = xdiv(u1, e.r3.x); e.v = xdiv(v1, e.r3.y);
