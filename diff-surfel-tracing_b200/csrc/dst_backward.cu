@@ -247,7 +247,7 @@ __device__ __forceinline__ void bwd_store_state(float4* base, int slot, const Bw
 __device__ __forceinline__ void bwd_request(const BwdState& s, EnumReq& q) {
     if (s.chunk == 0) { q.ox = s.sox; q.oy = s.soy; q.oz = s.soz; }
     else { q.ox = xadd(s.sox, xmul(s.offset, s.sdx)); q.oy = xadd(s.soy, xmul(s.offset, s.sdy)); q.oz = xadd(s.soz, xmul(s.offset, s.sdz)); }
-    q.dx = s.sdx; q.dy = s.sdy; q.dz = s.sdz; q.kmax0 = DST_T_MAX; q.pad = s.seg > 0 ? 1.f : 0.f;       // pad: the ray is on a reflected segment
+    q.dx = s.sdx; q.dy = s.sdy; q.dz = s.sdz; q.kmax0 = DST_T_MAX; q.step = 0.0f;
 }
 
 // Finds the next segment to differentiate, from segment `start` downwards (backward.cu:706-802):
@@ -609,6 +609,8 @@ __global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_shade(const
         BwdState s;
         int cnt = 0;
         if (slot >= 0) { bwd_load_state(p.state, slot, s); cnt = p.kcnt[slot]; }
+        const bool wide = (cnt & DST_KCNT_WIDE) != 0;
+        cnt &= DST_KCNT_WIDE - 1;
         const unsigned long long* kb = p.kbuf + soa(slot >= 0 ? slot : 0, 0, DST_CHUNK);
         const bool alive = bwd_chunk<DIAG, DIST>(p, slot >= 0, ray, s, [&](int k) { return kb[k * 32]; }, cnt, ws, tc);
         int cls = 0;
@@ -616,6 +618,7 @@ __global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_shade(const
             bwd_store_state(p.state, slot, s);
             EnumReq q;
             bwd_request(s, q);
+            q.step = wide && s.chunk > 0 ? 1.0f : 0.0f;
             store_req(p.req, slot, q);
             cls = s.seg > 0;
         }
@@ -823,11 +826,11 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     const int g_compact = (int)((slots + DST_LIVE_BLOCK - 1) / DST_LIVE_BLOCK);
     p.rounds = wave ? DST_WF_ROUNDS : 0;
     p.min_count = wave ? (int)(slots / 512 > 2048 ? slots / 512 : 2048) : 1;
-    // With the chunk log the rounds only serve rays the log could not hold. When the last completed read-back of a
-    // forward of this shape shows that everything fitted, a dozen rounds are enqueued instead of all of them
-    // (scheduling only: whatever is left after them is finished by the tail kernel).
+    // With the log the rounds only serve rays it could not hold. When the last completed read-back of a forward of this shape
+    // shows that everything fitted, none are enqueued (scheduling only: whatever is left after them is finished by the tail
+    // kernel). A dozen rounds of empty launches took 0.15 ms.
     if (wave && use_log && h->log_known_needed > 0 && h->log_known_sig == dst_call_signature(&a->in) && h->log_known_needed <= h->log_cap)
-        p.rounds = 12;
+        p.rounds = 0;
     dst_prof_mark(h, 2, 0, st);
     if (use_log) {
         // the forward logged its contributions: composite them again; rays the log could not hold are queued as round 0 of the

@@ -255,7 +255,8 @@ __global__ void __launch_bounds__(256) k_karras(const unsigned long long* __rest
 // single-surfel scene: one node whose second child is an empty box
 __global__ void k_single_leaf(BvhNode* nodes, int* leaf_parent, int* node_parent, unsigned int* arrive) {
     nodes[0].child[0].c = ~0; nodes[0].child[1].c = ~0; node_parent[0] = -1;
-    for (int a = 0; a < 3; a++) { nodes[0].child[1].lo[a] = INFINITY; nodes[0].child[1].hi[a] = -INFINITY; }
+    nodes[0].child[1].lox = nodes[0].child[1].loy = nodes[0].child[1].loz = INFINITY;
+    nodes[0].child[1].hix = nodes[0].child[1].hiy = nodes[0].child[1].hiz = -INFINITY;
     leaf_parent[0] = 0;
     arrive[0] = 1;      // the lone leaf acts as the second arrival
 }
@@ -342,12 +343,12 @@ __global__ void __launch_bounds__(256) k_refit(const float* __restrict__ verts, 
         BvhNode* nd = nodes + parent;
         const int slot = (nd->child[0].c == child) ? 0 : 1;
         float4* dst = reinterpret_cast<float4*>(nd->child + slot);
-        dst[0] = make_float4(lo[0], lo[1], lo[2], __int_as_float(child)); dst[1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        dst[0] = make_float4(lo[0], lo[1], hi[0], hi[1]); dst[1] = make_float4(lo[2], hi[2], __int_as_float(child), 0.0f);
         __threadfence();
         if (atomicAdd(&arrive[parent], 1u) == 0u) return;      // the sibling subtree is not done yet
         const float4* src = reinterpret_cast<const float4*>(nd->child + (1 - slot));
         const float4 s0 = __ldcg(src), s1 = __ldcg(src + 1);
-        const float slo[3] = { s0.x, s0.y, s0.z }, shi[3] = { s1.x, s1.y, s1.z };
+        const float slo[3] = { s0.x, s0.y, s1.x }, shi[3] = { s0.z, s0.w, s1.y };
 #pragma unroll
         for (int a = 0; a < 3; a++) { lo[a] = fminf(lo[a], slo[a]); hi[a] = fmaxf(hi[a], shi[a]); }
         if (parent == 0) {

@@ -12,8 +12,9 @@
 //   quads      P x 64 B     : plane frame of each quad and its surfel id in LEAF ORDER (two 256-bit loads per test)
 // ---------------------------------------------------------------------------------------------
 struct __align__(32) BvhChild {
-    float lo[3]; int c;     // box; child >= 0: internal node, < 0: the quad at leaf position ~c
-    float hi[3]; int pad;
+    float lox, loy, hix, hiy, loz, hiz;      // box, in the pairs the walk's packed multiply-adds take
+    int c;                                   // child >= 0: internal node, < 0: the quad at leaf position ~c
+    int pad;
 };
 struct __align__(64) BvhNode { BvhChild child[2]; };
 #define DST_MAX_SURFELS (1ll << 26)

@@ -199,7 +199,7 @@ __device__ __forceinline__ void fwd_init_state(const FwdParams& p, int ray, FwdS
 __device__ __forceinline__ void fwd_request(const FwdState& s, EnumReq& q) {
     if (s.chunk == 0) { q.ox = s.sox; q.oy = s.soy; q.oz = s.soz; }
     else { q.ox = xadd(s.sox, xmul(s.offset, s.sdx)); q.oy = xadd(s.soy, xmul(s.offset, s.sdy)); q.oz = xadd(s.soz, xmul(s.offset, s.sdz)); }
-    q.dx = s.sdx; q.dy = s.sdy; q.dz = s.sdz; q.kmax0 = DST_T_MAX; q.pad = s.bounce > 0 ? 1.f : 0.f;       // pad: the ray is on a reflected segment
+    q.dx = s.sdx; q.dy = s.sdy; q.dz = s.sdz; q.kmax0 = DST_T_MAX; q.step = 0.0f;
 }
 
 // After the hits of a chunk: the segment goes on (returns true), or it is finished (forward.cu:309-314, tracePath 378-422) and
@@ -422,12 +422,14 @@ __global__ void __launch_bounds__(SHADE_THREADS, DST_SHADE_GRID_PER_SM) k_fwd_sh
     }
     for (int i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < n_pad; i += gridDim.x * SHADE_THREADS) {
         const int slot = i < n ? list[i] : -1;
-        bool alive = false, bounded = false, failed = false;
+        bool alive = false, bounded = false, failed = false, wide = false;
         int cls = 0, cnt = 0;
         FwdState s;
         const unsigned long long* kb = p.kbuf + soa(slot >= 0 ? slot : 0, 0, DST_CHUNK);
         if (slot >= 0) {
             cnt = p.kcnt[slot];
+            wide = (cnt & DST_KCNT_WIDE) != 0;
+            cnt &= DST_KCNT_WIDE - 1;
             load_state(p.state, slot, s);
             // Fewer than 16 hits within a predicted distance (below) say nothing about what lies beyond. Nothing is composited; the
             // same request goes out again without a bound.
@@ -443,6 +445,7 @@ __global__ void __launch_bounds__(SHADE_THREADS, DST_SHADE_GRID_PER_SM) k_fwd_sh
             store_state(p.state, slot, s);
             EnumReq q;
             fwd_request(s, q);
+            q.step = wide && s.chunk > 0 ? 1.0f : 0.0f;
             // A segment that goes on: its next 16 hits are searched within bound_factor times the distance the last 16
             // spanned (first to last). A walk that knows its bound from the start opens a fifth fewer nodes than one that
             // learns it from its 16th hit; the spans of consecutive chunks differ by less than that factor for all but
@@ -922,7 +925,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
             h->rounds_known = used; h->rounds_known_sig = h->rounds_pending_sig;
         } else cudaGetLastError();
         if (h->rounds_known > 0 && h->rounds_known_sig == sig) {
-            const int want = h->rounds_known + (h->rounds_known / 2 > 4 ? h->rounds_known / 2 : 4);
+            const int want = h->rounds_known + (h->rounds_known / 4 > 2 ? h->rounds_known / 4 : 2);
             p.rounds = want < DST_WF_ROUNDS ? want : DST_WF_ROUNDS;
         }
     }

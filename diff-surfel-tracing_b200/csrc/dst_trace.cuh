@@ -25,8 +25,7 @@ __device__ __forceinline__ BvhChild load_child(const BvhView& bvh, int node, int
     float4 a, b;
     ldg256(bvh.nodes[node].child + k, a, b);
     BvhChild c;
-    c.lo[0] = a.x; c.lo[1] = a.y; c.lo[2] = a.z; c.c = __float_as_int(a.w);
-    c.hi[0] = b.x; c.hi[1] = b.y; c.hi[2] = b.z; c.pad = 0;
+    c.lox = a.x; c.loy = a.y; c.hix = a.z; c.hiy = a.w; c.loz = b.x; c.hiz = b.y; c.c = __float_as_int(b.z); c.pad = 0;
     return c;
 }
 struct Quad { float4 a, b, c; unsigned int gid; };
@@ -111,12 +110,12 @@ __device__ __forceinline__ int knearest(const BvhView& bvh, float ox, float oy, 
         while ((unsigned int)cur < (unsigned int)DONE) {
             const BvhChild k0 = load_child(bvh, cur, 0), k1 = load_child(bvh, cur, 1);
             if (COUNT) tc.nodes++;
-            const float n0x = px ? k0.lo[0] : k0.hi[0], f0x = px ? k0.hi[0] : k0.lo[0];
-            const float n0y = py ? k0.lo[1] : k0.hi[1], f0y = py ? k0.hi[1] : k0.lo[1];
-            const float n0z = pz ? k0.lo[2] : k0.hi[2], f0z = pz ? k0.hi[2] : k0.lo[2];
-            const float n1x = px ? k1.lo[0] : k1.hi[0], f1x = px ? k1.hi[0] : k1.lo[0];
-            const float n1y = py ? k1.lo[1] : k1.hi[1], f1y = py ? k1.hi[1] : k1.lo[1];
-            const float n1z = pz ? k1.lo[2] : k1.hi[2], f1z = pz ? k1.hi[2] : k1.lo[2];
+            const float n0x = px ? k0.lox : k0.hix, f0x = px ? k0.hix : k0.lox;
+            const float n0y = py ? k0.loy : k0.hiy, f0y = py ? k0.hiy : k0.loy;
+            const float n0z = pz ? k0.loz : k0.hiz, f0z = pz ? k0.hiz : k0.loz;
+            const float n1x = px ? k1.lox : k1.hix, f1x = px ? k1.hix : k1.lox;
+            const float n1y = py ? k1.loy : k1.hiy, f1y = py ? k1.hiy : k1.loy;
+            const float n1z = pz ? k1.loz : k1.hiz, f1z = pz ? k1.hiz : k1.loz;
             const float tn0 = fmaxf(fmaxf(fmaf(n0x, ix, -onx), fmaf(n0y, iy, -ony)), fmaxf(fmaf(n0z, iz, -onz), 0.0f));
             const float tf0 = fminf(fminf(fmaf(f0x, ix, -ofx), fmaf(f0y, iy, -ofy)), fmaf(f0z, iz, -ofz));
             const float tn1 = fmaxf(fmaxf(fmaf(n1x, ix, -onx), fmaf(n1y, iy, -ony)), fmaxf(fmaf(n1z, iz, -onz), 0.0f));
@@ -283,7 +282,7 @@ __device__ __forceinline__ bool eval_slot(unsigned long long key, float offset, 
 // `min_count` is skipped by both kernels and left to the tail kernel, which runs the remaining
 // rays to completion one thread per ray.
 // ---------------------------------------------------------------------------------------------
-struct __align__(16) EnumReq { float ox, oy, oz, dx, dy, dz, kmax0, pad; };
+struct __align__(16) EnumReq { float ox, oy, oz, dx, dy, dz, kmax0, step; };      // step: gather step that answered the ray's last request (0: k_enum)
 
 // Everything a ray keeps between kernels is indexed by its list slot (its place in the tile-ordered list of round 0, see slot_ray()), in blocks of
 // 32 slots with the words of a record one after the other and the 32 slots of a block side by side. The rays of a warp are (survivors of)
@@ -293,12 +292,12 @@ __device__ __forceinline__ size_t soa(int slot, int word, int words) { return ((
 __device__ __forceinline__ EnumReq load_req(const float4* req, int slot) {
     const float4 a = req[soa(slot, 0, 2)], b = req[soa(slot, 1, 2)];
     EnumReq q;
-    q.ox = a.x; q.oy = a.y; q.oz = a.z; q.dx = a.w; q.dy = b.x; q.dz = b.y; q.kmax0 = b.z; q.pad = b.w;
+    q.ox = a.x; q.oy = a.y; q.oz = a.z; q.dx = a.w; q.dy = b.x; q.dz = b.y; q.kmax0 = b.z; q.step = b.w;
     return q;
 }
 __device__ __forceinline__ void store_req(float4* req, int slot, const EnumReq& q) {
     req[soa(slot, 0, 2)] = make_float4(q.ox, q.oy, q.oz, q.dx);
-    req[soa(slot, 1, 2)] = make_float4(q.dy, q.dz, q.kmax0, q.pad);
+    req[soa(slot, 1, 2)] = make_float4(q.dy, q.dz, q.kmax0, q.step);
 }
 __device__ __forceinline__ float& req_bound(float4* req, int slot) { return req[soa(slot, 1, 2)].z; }
 
@@ -330,72 +329,80 @@ constexpr int ENUM_THREADS = 128;
 // Runs of 2 or 4 quads as leaves of the walk: 2-9 % slower than single quads.
 // Blocks are persistent and take batches from a cursor; no block waits for another.
 // ---------------------------------------------------------------------------------------------
+#ifndef DST_BEAM_STEPS
 #define DST_BEAM_STEPS 160
+#endif
+#ifndef DST_BEAM_CANDS
 #define DST_BEAM_CANDS 300
+#endif
 #define DST_GROUP 8
+#ifndef DST_GROUP_STEPS
 #define DST_GROUP_STEPS 192
+#endif
 #define DST_GROUP_MIN_BLOCKS 8
 #define DST_WALK_STACK 320                 // one step adds at most 16 entries; see the width rule in beam_walk()
 #define DST_WALK_QUADS 64
 #define DST_WALK_STEP_LIMIT (1 << 20)      // bound on the steps of a walk that cannot be given up (status flag instead of a hang)
-// Hull of the rays of one batch (origins and directions, component by component), kept in shared memory per warp.
-struct BeamQ { float omin[3], omax[3], dmin[3], dmax[3], dabs[3], dsum; };      // dabs: largest |d| per axis, dsum: their sum
+// Hull of a set of rays, component by component: origins oc +- orad, directions dc +- drad.
+struct BeamQ { float oc[3], orad[3], dc[3], drad[3], dsum, dmax; };      // dsum: sum of the largest |d| per axis, dmax: largest of them
 
-// [rl, rh] += c * [lo, hi]
-__device__ __forceinline__ void ivmul(float c, float lo, float hi, float& rl, float& rh) {
-    const bool pos = c >= 0.f;
-    rl = fmaf(c, pos ? lo : hi, rl); rh = fmaf(c, pos ? hi : lo, rh);
-}
-// Conservative test of one quad against the hull of a batch of rays, in interval arithmetic over the hull's origins
-// and directions: can ANY ray of the batch pass ray_quad() with a hit no farther than kmaxb? The steps are those of
-// ray_quad(): t = n.(p0 - o) / n.d, h = t d - (p0 - o), u = wu.h, v = wv.h, accepted iff 0 <= t <= kmax and u, v in
-// [0, 1]. Every interval is widened by margins orders of magnitude above the rounding of either computation, so a
-// quad some ray hits is never rejected. For neighbouring rays (close origins, directions a degree apart) the
-// intervals are narrow: nearly every quad that no ray hits is rejected here by ONE lane, and the lanes of a warp
-// do that for 32 quads at a time, instead of every lane testing every quad against its own ray.
+// Conservative test of one quad against the hull, in interval arithmetic (centre and radius): can ANY ray of the set pass ray_quad() with a hit no
+// farther than kmaxb? The steps are those of ray_quad(): t = n.(p0 - o) / n.d, h = t d - (p0 - o), u = wu.h, v = wv.h,
+// accepted iff 0 <= t <= kmax and u, v in [0, 1]. Every interval is widened by margins orders of magnitude above the
+// rounding of either computation, so a quad some ray hits is never rejected. For neighbouring rays (close origins, directions a
+// degree apart) the intervals are narrow, and nearly every quad that no ray hits is rejected here by ONE lane.
 __device__ __forceinline__ bool hull_quad(const BeamQ& bm, const float4 qa, const float4 qb, const float4 qc, float kmaxb) {
     const float p0[3] = { qa.x, qa.y, qa.z }, nn[3] = { qa.w, qb.x, qb.y }, wu[3] = { qb.z, qb.w, qc.x }, wv[3] = { qc.y, qc.z, qc.w };
-    float rl[3], rh[3];
-    float bl = 0.f, bh = 0.f, al = 0.f, ah = 0.f, scale = 0.f;
+    float rc[3], bc = 0.f, br = 0.f, ac = 0.f, ar = 0.f, scale = 0.f;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        rl[a] = p0[a] - bm.omax[a]; rh[a] = p0[a] - bm.omin[a];
-        ivmul(nn[a], bm.dmin[a], bm.dmax[a], bl, bh);
-        ivmul(nn[a], rl[a], rh[a], al, ah);
-        scale = fmaxf(scale, fmaxf(fabsf(rl[a]), fabsf(rh[a])));
+        rc[a] = p0[a] - bm.oc[a];
+        bc = fmaf(nn[a], bm.dc[a], bc); br = fmaf(fabsf(nn[a]), bm.drad[a], br);
+        ac = fmaf(nn[a], rc[a], ac); ar = fmaf(fabsf(nn[a]), bm.orad[a], ar);
+        scale = fmaxf(scale, fabsf(rc[a]) + bm.orad[a]);
     }
     const float nmag = fabsf(nn[0]) + fabsf(nn[1]) + fabsf(nn[2]);
-    const float eb = 4e-6f * nmag * bm.dsum, ea = 12e-6f * nmag * scale;
-    bl -= eb; bh += eb; al -= ea; ah += ea;
-    if (!(bl > 1e-30f || bh < -1e-30f)) return true;        // some direction of the hull is (all but) parallel to the plane: no bound
+    br = fmaf(4e-6f * nmag, bm.dsum, br); ar = fmaf(12e-6f * nmag, scale, ar);
+    const float bs = fabsf(bc), as = bc < 0.f ? -ac : ac;
+    if (!(bs - br > 1e-30f)) return true;        // some direction of the hull is (all but) parallel to the plane: no bound
     // quotients by approximate reciprocals (two units in the last place; the interval is widened by 1e-5 relative below)
-    const float ibl = __fdividef(1.0f, bl), ibh = __fdividef(1.0f, bh);
-    const float t1 = al * ibl, t2 = al * ibh, t3 = ah * ibl, t4 = ah * ibh;
-    float tl = fminf(fminf(t1, t2), fminf(t3, t4)), th = fmaxf(fmaxf(t1, t2), fmaxf(t3, t4));
+    const float al = as - ar, ah = as + ar;
+    float tl = __fdividef(al, al >= 0.f ? bs + br : bs - br), th = __fdividef(ah, ah >= 0.f ? bs - br : bs + br);
     tl -= 1e-5f * fabsf(tl) + 1e-30f; th += 1e-5f * fabsf(th) + 1e-30f;
-    if (th < 0.f || tl > kmaxb) return false;
+    if (!(th >= 0.f && tl <= kmaxb)) return false;
     tl = fmaxf(tl, 0.f); th = fminf(th, kmaxb);
-    float ul = 0.f, uh = 0.f, vl = 0.f, vh = 0.f, hmag = 0.f;
+    const float tc = 0.5f * (tl + th), tr = 0.5f * (th - tl) + 1e-6f * th;
+    float uc = -0.5f, ur = 0.5f + 1e-5f, vc = -0.5f, vr = 0.5f + 1e-5f;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        // t in [tl, th] with 0 <= tl <= th, d in [dmin, dmax]: the smallest t d is at (tl, dmin) or (th, dmin), the largest at (th, dmax) or (tl, dmax)
-        const float hl = bm.dmin[a] * (bm.dmin[a] >= 0.f ? tl : th) - rh[a], hh = bm.dmax[a] * (bm.dmax[a] >= 0.f ? th : tl) - rl[a];
-        ivmul(wu[a], hl, hh, ul, uh);
-        ivmul(wv[a], hl, hh, vl, vh);
-        hmag = fmaxf(hmag, fmaxf(fabsf(hl), fabsf(hh)) + scale + th * bm.dabs[a]);
+        const float hc = fmaf(tc, bm.dc[a], -rc[a]), hr = fmaf(tr, fabsf(bm.dc[a]) + bm.drad[a], fmaf(tc, bm.drad[a], bm.orad[a]));
+        uc = fmaf(wu[a], hc, uc); ur = fmaf(fabsf(wu[a]), hr, ur);
+        vc = fmaf(wv[a], hc, vc); vr = fmaf(fabsf(wv[a]), hr, vr);
     }
     // u and v are of order 1; their rounding error is that of h (cancellation of t d against p0 - o) times |w|
-    const float eu = 1e-5f + 8e-6f * hmag * (fabsf(wu[0]) + fabsf(wu[1]) + fabsf(wu[2]));
-    const float ev = 1e-5f + 8e-6f * hmag * (fabsf(wv[0]) + fabsf(wv[1]) + fabsf(wv[2]));
-    return !(uh < -eu || ul > 1.f + eu || vh < -ev || vl > 1.f + ev);
+    const float eh = 16e-6f * fmaf(th, bm.dmax, scale);
+    ur = fmaf(eh, fabsf(wu[0]) + fabsf(wu[1]) + fabsf(wu[2]), ur);
+    vr = fmaf(eh, fabsf(wv[0]) + fabsf(wv[1]) + fabsf(wv[2]), vr);
+    return !(fabsf(uc) > ur || fabsf(vc) > vr);
 }
 
-// Slab constants of the hull for the child-box test of the walk, four fused multiply-adds per axis and box. For every ray
-// of the hull, with origin in [omin, omax] and direction in [dmin, dmax] along an axis:
+// Three-operand minimum / maximum and packed multiply-add, instructions sm_100 has and the compiler does not form here.
+__device__ __forceinline__ float min3(float a, float b, float c) { float r; asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
+__device__ __forceinline__ float max3(float a, float b, float c) { float r; asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
+__device__ __forceinline__ float2 fma2(float ax, float ay, float4 fo) {      // (ax, ay) * (fo.x, fo.y) + (fo.z, fo.w)
+    float2 r;
+    asm("{ .reg .b64 a, b, c, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mov.b64 c, {%6, %7}; fma.rn.f32x2 d, a, b, c; mov.b64 {%0, %1}, d; }"
+        : "=f"(r.x), "=f"(r.y) : "f"(ax), "f"(ay), "f"(fo.x), "f"(fo.y), "f"(fo.z), "f"(fo.w));
+    return r;
+}
+
+// Slab constants of the hull for the child-box test of the walk. For every ray of the hull, with origin in [omin, omax] and direction
+// in [dmin, dmax] along an axis:
 //   entry  t >= (lo - omax) / dmax if the box lies ahead in +, t >= (omin - hi) / -dmin if it lies ahead in -, else t >= 0
 //   exit   t <= (hi - omin) / dmin if every ray travels in +, t <= (omax - lo) / -dmax if every ray travels in -, else unbounded
-// pa hi/lo factors and offsets are folded (entry = lo * ep + eo, hi * en + fo, ...); an impossible direction has a huge factor.
-struct BeamSlab { float4 entry[3], exit[3]; };       // (factor of lo, offset, factor of hi, offset)
+// Each is one multiply-add of a box coordinate, taken two at a time (factors x, y and offsets z, w); an impossible direction has a huge factor.
+struct BeamSlab { float4 in_lo, in_hi, out_lo, out_hi, in_z, out_z; };       // x and y of lo, x and y of hi, z of lo and hi
+#define DST_KCNT_WIDE 0x100                // flag in a ray's hit count: answered by a later step than k_enum
 struct WalkMem {
     unsigned long long stack[DST_WALK_STACK];        // subtrees: nearest possible t << 32 | link, nearest on top
     unsigned long long quads[DST_WALK_QUADS];        // quads whose box the hull reaches: nearest possible t << 32 | leaf position
@@ -411,7 +418,7 @@ template <bool COUNT, class LeafStep>
 __device__ __forceinline__ bool beam_walk(const BvhView& bvh, WalkMem& m, float& krun, int max_steps, unsigned int* status, TraceCounters& tc, LeafStep leaf_step) {
     constexpr unsigned int FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const unsigned int below = (1u << lane) - 1u;
+    const unsigned int below = (1u << lane) - 1u, pair_below = (1u << (lane & 30)) - 1u;
     int sp = 1, nq = 0;
     if (lane == 0) m.stack[0] = 0ull;
     __syncwarp();
@@ -428,47 +435,33 @@ __device__ __forceinline__ bool beam_walk(const BvhView& bvh, WalkMem& m, float&
         // lanes 30/31 take the top entry, lanes 28/29 the next, ...: lane order is then the order in which surviving children
         // go back onto the stack (farthest first). A nearly full stack is walked one node at a time (it then grows by at most
         // one entry per level of the tree).
-        const int width = sp > DST_WALK_STACK - 112 ? 1 : 16;
+        int width = 16;
+        if (sp > DST_WALK_STACK - 112) {
+            width = 1;
+            if (sp > DST_WALK_STACK - 2) { if (lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW); return true; }
+        }
         const int take = sp < width ? sp : width;
-        const int slot = 15 - (lane >> 1);
-        unsigned long long e = 0ull;
-        bool h = slot < take;
-        if (h) e = m.stack[sp - 1 - slot];
+        const bool valid = 15 - (lane >> 1) < take;
+        const unsigned long long e = valid ? m.stack[sp - 16 + (lane >> 1)] : 0ull;
         sp -= take;
         __syncwarp();
-        h = h && __uint_as_float((unsigned int)(e >> 32)) <= krun;
-        float tn = 0.0f, tf = 0.0f;
-        int clink = 0;
+        const BvhChild b = load_child(bvh, (int)(unsigned int)e, lane & 1);          // (lanes without an entry read the root)
+        if (COUNT && valid && (lane & 1) == 0) tc.nodes++;
+        const float2 il = fma2(b.lox, b.loy, m.slab.in_lo), ih = fma2(b.hix, b.hiy, m.slab.in_hi), iz = fma2(b.loz, b.hiz, m.slab.in_z);
+        const float2 ol = fma2(b.lox, b.loy, m.slab.out_lo), oh = fma2(b.hix, b.hiy, m.slab.out_hi), oz = fma2(b.loz, b.hiz, m.slab.out_z);
+        const float tn = max3(max3(il.x, il.y, ih.x), max3(ih.y, iz.x, iz.y), 0.0f);
+        const float tf = min3(min3(ol.x, ol.y, oh.x), oh.y, fminf(oz.x, oz.y));
+        const bool h = valid && __uint_as_float((unsigned int)(e >> 32)) <= krun && tn <= fminf(tf, krun);
+        // Of a pair the nearer child goes on top: entered first, on a tie (the rays start inside both boxes) left first.
+        const float ptn = __shfl_xor_sync(FULL, tn, 1), ptf = __shfl_xor_sync(FULL, tf, 1);
+        const bool on_top = tn < ptn || (tn == ptn && (tf < ptf || (tf == ptf && !(lane & 1))));
+        const unsigned int inner = __ballot_sync(FULL, h && b.c >= 0), leaves = __ballot_sync(FULL, h && b.c < 0);
+        const unsigned long long entry = ((unsigned long long)__float_as_uint(tn) << 32) | (unsigned int)(b.c ^ (b.c >> 31));      // (~c for a quad)
         if (h) {
-            if (COUNT && (lane & 1) == 0) tc.nodes++;
-            const BvhChild b = load_child(bvh, (int)(unsigned int)e, lane & 1);
-            clink = b.c;
-            const float4 ex = m.slab.entry[0], ey = m.slab.entry[1], ez = m.slab.entry[2];
-            const float4 fx = m.slab.exit[0], fy = m.slab.exit[1], fz = m.slab.exit[2];
-            tn = fmaxf(fmaxf(fmaf(b.lo[0], ex.x, ex.y), fmaf(b.hi[0], ex.z, ex.w)), 0.0f);
-            tn = fmaxf(fmaxf(fmaf(b.lo[1], ey.x, ey.y), fmaf(b.hi[1], ey.z, ey.w)), tn);
-            tn = fmaxf(fmaxf(fmaf(b.lo[2], ez.x, ez.y), fmaf(b.hi[2], ez.z, ez.w)), tn);
-            tf = fminf(fmaf(b.lo[0], fx.x, fx.y), fmaf(b.hi[0], fx.z, fx.w));
-            tf = fminf(fminf(fmaf(b.lo[1], fy.x, fy.y), fmaf(b.hi[1], fy.z, fy.w)), tf);
-            tf = fminf(fminf(fmaf(b.lo[2], fz.x, fz.y), fmaf(b.hi[2], fz.z, fz.w)), tf);
-            h = tn <= fminf(tf, krun);
+            if (b.c >= 0) m.stack[sp + __popc(inner & pair_below) + (on_top ? (int)((inner >> (lane ^ 1)) & 1u) : 0)] = entry;
+            else m.quads[nq + __popc(leaves & below)] = entry;
         }
-        {   // within a pair the farther child goes first (even lane), the nearer second (odd lane); nearer = entered first, on a
-            // tie (the rays start inside both boxes) left first
-            const float ptn = __shfl_xor_sync(FULL, tn, 1), ptf = __shfl_xor_sync(FULL, tf, 1);
-            const int plink = __shfl_xor_sync(FULL, clink, 1);
-            const bool ph = __shfl_xor_sync(FULL, h, 1);
-            const bool even = (lane & 1) == 0;
-            const bool mine_nearer = tn < ptn || (tn == ptn && (tf < ptf || (tf == ptf && even)));
-            if (h && ph && (even ? mine_nearer : !mine_nearer)) { tn = ptn; clink = plink; }
-        }
-        const unsigned int inner = __ballot_sync(FULL, h && clink >= 0);
-        const unsigned long long tword = (unsigned long long)__float_as_uint(tn) << 32;
-        if (sp + __popc(inner) > DST_WALK_STACK) { if (lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW); return true; }
-        if (h && clink >= 0) m.stack[sp + __popc(inner & below)] = tword | (unsigned int)clink;
         sp += __popc(inner);
-        const unsigned int leaves = __ballot_sync(FULL, h && clink < 0);
-        if (h && clink < 0) m.quads[nq + __popc(leaves & below)] = tword | (unsigned int)~clink;
         nq += __popc(leaves);
         __syncwarp();
     }
@@ -493,16 +486,27 @@ __device__ __forceinline__ void make_beam(WalkMem& m, bool active, float ox, flo
         const int a = lane;
         const float ol = a == 0 ? olo[0] : a == 1 ? olo[1] : olo[2], oh = a == 0 ? ohi[0] : a == 1 ? ohi[1] : ohi[2];
         const float dl = a == 0 ? dlo[0] : a == 1 ? dlo[1] : dlo[2], dh = a == 0 ? dhi[0] : a == 1 ? dhi[1] : dhi[2];
-        m.beam.omin[a] = ol; m.beam.omax[a] = oh; m.beam.dmin[a] = dl; m.beam.dmax[a] = dh; m.beam.dabs[a] = fmaxf(fabsf(dl), fabsf(dh));
+        m.beam.oc[a] = 0.5f * (ol + oh); m.beam.orad[a] = 0.5f * (oh - ol) + 2e-7f * fmaxf(fabsf(ol), fabsf(oh));      // (the centre is rounded)
+        m.beam.dc[a] = 0.5f * (dl + dh); m.beam.drad[a] = 0.5f * (dh - dl) + 2e-7f * fmaxf(fabsf(dl), fabsf(dh));
         // box padding as in knearest(), for the ray with the largest coordinates
         const float pad = DST_PAD_FACTOR * (om + absmax) + 1e-30f;
         const float lo = ol - pad, hi = oh + pad;
         const float ip = 1.0f / fmaxf(dh, 1e-30f), in = 1.0f / fmaxf(-dl, 1e-30f);
-        m.slab.entry[a] = make_float4(ip, -hi * ip, -in, lo * in);
         const float xp = dl > 1e-20f ? 1.0f / dl : 0.0f, xn = dh < -1e-20f ? 1.0f / dh : 0.0f;
-        m.slab.exit[a] = make_float4(xn, xn != 0.0f ? -hi * xn : 3e38f, xp, xp != 0.0f ? -lo * xp : 3e38f);
+        const float f_in_lo = ip, o_in_lo = -hi * ip, f_in_hi = -in, o_in_hi = lo * in;
+        const float f_out_lo = xn, o_out_lo = xn != 0.0f ? -hi * xn : 3e38f, f_out_hi = xp, o_out_hi = xp != 0.0f ? -lo * xp : 3e38f;
+        if (a < 2) {
+            (&m.slab.in_lo.x)[a] = f_in_lo; (&m.slab.in_lo.z)[a] = o_in_lo; (&m.slab.in_hi.x)[a] = f_in_hi; (&m.slab.in_hi.z)[a] = o_in_hi;
+            (&m.slab.out_lo.x)[a] = f_out_lo; (&m.slab.out_lo.z)[a] = o_out_lo; (&m.slab.out_hi.x)[a] = f_out_hi; (&m.slab.out_hi.z)[a] = o_out_hi;
+        } else {
+            m.slab.in_z = make_float4(f_in_lo, f_in_hi, o_in_lo, o_in_hi);
+            m.slab.out_z = make_float4(f_out_lo, f_out_hi, o_out_lo, o_out_hi);
+        }
     }
-    if (lane == 0) m.beam.dsum = fmaxf(fabsf(dlo[0]), fabsf(dhi[0])) + fmaxf(fabsf(dlo[1]), fabsf(dhi[1])) + fmaxf(fabsf(dlo[2]), fabsf(dhi[2]));
+    if (lane == 0) {
+        const float a0 = fmaxf(fabsf(dlo[0]), fabsf(dhi[0])), a1 = fmaxf(fabsf(dlo[1]), fabsf(dhi[1])), a2 = fmaxf(fabsf(dlo[2]), fabsf(dhi[2]));
+        m.beam.dsum = a0 + a1 + a2; m.beam.dmax = fmaxf(a0, fmaxf(a1, a2));
+    }
     __syncwarp();
 }
 
@@ -533,31 +537,36 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
         // the slow ones, so they start first and the cheap batches of primary rays fill the end of the round.
         const int idx = (((total + 31) >> 5) - 1 - (base >> 5)) * 32 + lane;
         const int slot = idx < total ? list[idx] : -1;
-        bool active = false;
+        bool active = false, wide = false;
         int n = 0;
         float kmax = -1.0f, ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f;
         if (slot >= 0) {
             const EnumReq q = load_req(req, slot);
             ox = q.ox; oy = q.oy; oz = q.oz; dx = q.dx; dy = q.dy; dz = q.dz;
             active = fabsf(ox) < INFINITY && fabsf(oy) < INFINITY && fabsf(oz) < INFINITY && fabsf(dx) < INFINITY && fabsf(dy) < INFINITY && fabsf(dz) < INFINITY;
-            if (active) kmax = q.kmax0;
+            if (active) { kmax = q.kmax0; wide = q.step > 0.0f; }
             if (COUNT) tc.enums++;
         }
-        if (__any_sync(FULL, active)) {
+        const unsigned int am = __ballot_sync(FULL, active);
+        if (am != 0u) {
+            // most of these rays' last requests were not answered here: their hull is still as wide, and trying it first is wasted
+            bool done = 2 * __popc(__ballot_sync(FULL, wide)) <= __popc(am);
+            if (done) {
             make_beam(m, active, ox, oy, oz, dx, dy, dz, absmax);
             float krun = redux_max(kmax);
             int cands = 0;
-            const bool done = beam_walk<COUNT>(bvh, m, krun, DST_BEAM_STEPS, status, tc, [&](bool valid, int pos) {
+            done = beam_walk<COUNT>(bvh, m, krun, DST_BEAM_STEPS, status, tc, [&](bool valid, int pos) {
                 bool pass = false;
                 if (valid) { const Quad q = load_quad(bvh, pos); pass = hull_quad(m.beam, q.a, q.b, q.c, krun); }
                 unsigned int maybe = __ballot_sync(FULL, pass);
                 cands += __popc(maybe);
                 if (cands > DST_BEAM_CANDS) return false;
+                Quad next;       // (the next quad is on its way while this one is tested)
+                if (maybe) next = load_quad(bvh, __shfl_sync(FULL, pos, 31 - __clz(maybe)));
                 while (maybe) {
-                    const int src = 31 - __clz(maybe);
-                    maybe &= ~(1u << src);
-                    const int p = __shfl_sync(FULL, pos, src);
-                    const Quad q = load_quad(bvh, p);
+                    const Quad q = next;
+                    maybe &= ~(1u << (31 - __clz(maybe)));
+                    if (maybe) next = load_quad(bvh, __shfl_sync(FULL, pos, 31 - __clz(maybe)));
                     if (COUNT && lane == 0) tc.quads++;
                     float t; int tri;
                     if (!ray_quad(q.a, q.b, q.c, ox, oy, oz, dx, dy, dz, kmax, t, tri)) continue;
@@ -577,6 +586,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
                 krun = redux_max(kmax);
                 return true;
             });
+            }
             if (!done) {
                 // (a bound below the request's can only have come from a full k-buffer: the repeated search finds 16 hits again)
                 int at = 0;
@@ -718,7 +728,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
                 const unsigned long long mine = skeys[w][r][lane & (DST_CHUNK - 1)];
                 const int n = __popc(__ballot_sync(FULL, lane < DST_CHUNK && mine != ~0ull));
                 if (lane < n) kbuf[soa(to, lane, DST_CHUNK)] = mine;
-                if (lane == 0) kcnt[to] = n;
+                if (lane == 0) kcnt[to] = n | DST_KCNT_WIDE;
             }
         } else {
             int at = 0;
@@ -754,7 +764,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray
         unsigned long long key;
         const int n = knearest_warp<COUNT>(bvh, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, absmax, m, key, status, tc);
         if (lane < n) kbuf[soa(slot, lane, DST_CHUNK)] = key;
-        if (lane == 0) kcnt[slot] = n;
+        if (lane == 0) kcnt[slot] = n | DST_KCNT_WIDE;
         __syncwarp();
     }
     if (COUNT && counters) { atomicAdd(counters + 2, tc.nodes); atomicAdd(counters + 3, tc.quads); }
