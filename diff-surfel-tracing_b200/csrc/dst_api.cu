@@ -83,6 +83,7 @@ int dst_create(int device, dst_handle** out) {
     h->wf_min_rays = 1 << 15;
     h->log_enabled = 1;
     h->stable_lists = 1;
+    h->logs_keep = 1;
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) { delete h; dst_global_error("dst_create: cudaGetDeviceProperties failed"); return DST_E_CUDA; }
     h->sm_count = prop.multiProcessorCount;
@@ -108,7 +109,8 @@ int dst_destroy(dst_handle* h) {
     if (h->log_needed_event) cudaEventDestroy(h->log_needed_event);
     if (h->rounds_host) cudaFreeHost(h->rounds_host);
     if (h->rounds_event) cudaEventDestroy(h->rounds_event);
-    cudaFree(h->log_keys); cudaFree(h->log_next); cudaFree(h->log_count); cudaFree(h->log_head); cudaFree(h->log_num); cudaFree(h->log_ok);
+    cudaFree(h->log_keys); cudaFree(h->log_next); cudaFree(h->log_count);
+    for (int k = 0; k < DST_MAX_LOGS; k++) { cudaFree(h->logs[k].head); cudaFree(h->logs[k].num); cudaFree(h->logs[k].ok); }
     cudaFree(h->wf_state); cudaFree(h->wf_req); cudaFree(h->wf_kbuf); cudaFree(h->wf_kcnt); cudaFree(h->wf_list[0]); cudaFree(h->wf_list[1]); cudaFree(h->wf_counts);
     cudaFree(h->wf_tmp); cudaFree(h->wf_wcnt); cudaFree(h->wf_bcnt);
     cudaFree(h->bound_stats);
@@ -137,7 +139,7 @@ int dst_build(dst_handle* h, const float* vertices, int64_t n_vertices, const in
         return dst_set_error(h, DST_E_ARG, "triangles must hold 2 per surfel: %lld triangles for %lld vertices", (long long)n_triangles, (long long)n_vertices);
     DeviceGuard g(h->device);
     if (!g.ok) return dst_set_error(h, DST_E_CUDA, "cudaSetDevice(%d) failed", h->device);
-    h->log_serial = 0;      // the logged chunks refer to the hierarchy that is about to change
+    dst_drop_logs(h);      // the logged contributions refer to the quads that are about to change
     return dst_bvh_build_impl(h, vertices, n_vertices / 4, rebuild, (cudaStream_t)stream);
 }
 
@@ -157,7 +159,7 @@ int dst_build_from_surfels(dst_handle* h, const float* means3D, const float* sca
     if (!means3D || !scales || !rotations || !vertices) return dst_set_error(h, DST_E_ARG, "a required pointer is null");
     DeviceGuard g(h->device);
     if (!g.ok) return dst_set_error(h, DST_E_CUDA, "cudaSetDevice(%d) failed", h->device);
-    h->log_serial = 0;
+    dst_drop_logs(h);
     return dst_bvh_build_impl(h, vertices, n_surfels, rebuild, (cudaStream_t)stream, means3D, scales, rotations);
 }
 
@@ -227,13 +229,14 @@ int dst_set_option(dst_handle* h, int option, int64_t value) {
     if (!h) return DST_E_ARG;
     switch (option) {
         case DST_OPT_WAVEFRONT_MIN_RAYS: h->wf_min_rays = value < 0 ? 0 : value; return DST_OK;
-        case DST_OPT_CHUNK_LOG_MAX_RECORDS: h->log_max_records = value < 0 ? 0 : value; h->log_serial = 0; return DST_OK;
-        case DST_OPT_IMAGE_WIDTH: h->image_width = value < 0 ? 0 : value; h->log_serial = 0; return DST_OK;
+        case DST_OPT_CHUNK_LOG_MAX_RECORDS: h->log_max_records = value < 0 ? 0 : value; dst_drop_logs(h); return DST_OK;
+        case DST_OPT_IMAGE_WIDTH: h->image_width = value < 0 ? 0 : value; return DST_OK;
         case DST_OPT_SINGLE_KERNEL_REFIT: h->single_kernel_refit = value != 0; return DST_OK;
         case DST_OPT_DISTORTION: h->distortion = value != 0; return DST_OK;
         case DST_OPT_STABLE_LISTS: h->stable_lists = value != 0; return DST_OK;
         case DST_OPT_FORWARD_SLICES: h->fwd_slices = value < 0 ? 0 : (value > DST_MAX_SLICES ? DST_MAX_SLICES : (int)value); return DST_OK;
-        case DST_OPT_CHUNK_LOG: h->log_enabled = value != 0; if (!h->log_enabled) h->log_serial = 0; return DST_OK;
+        case DST_OPT_CHUNK_LOG: h->log_enabled = value != 0; if (!h->log_enabled) dst_drop_logs(h); return DST_OK;
+        case DST_OPT_KEPT_LOGS: h->logs_keep = value < 1 ? 1 : (value > DST_MAX_LOGS ? DST_MAX_LOGS : (int)value); return DST_OK;
         default: return dst_set_error(h, DST_E_ARG, "unknown option %d", option);
     }
 }
@@ -331,7 +334,7 @@ int dst_debug_read_bandwidth(dst_handle* h, int64_t bytes, int reps, float* gb_p
 
 int dst_debug_chunk_log(const dst_handle* h, int64_t* records_wanted, int64_t* records_held, int64_t* bytes_per_record) {
     if (!h) return DST_E_ARG;
-    if (records_wanted) *records_wanted = (h->log_needed_host && h->log_needed_event && cudaEventQuery(h->log_needed_event) == cudaSuccess) ? *h->log_needed_host : -1;
+    if (records_wanted) *records_wanted = (h->log_needed_host && h->log_needed_event && cudaEventQuery(h->log_needed_event) == cudaSuccess) ? h->log_needed_host[0] - h->log_needed_host[1] : -1;
     if (records_held) *records_held = h->log_cap;
     if (bytes_per_record) *bytes_per_record = 8 * DST_CHUNK + (int64_t)sizeof(int);
     return DST_OK;

@@ -38,7 +38,7 @@ struct BwdParams {
     int min_count;
     int rounds;
     LiveLists lv;
-    // contribution log of the matching forward call, see dst_ensure_log()
+    // contribution log of the matching forward call, see dst_begin_log()
     const unsigned long long* log_keys; const int* log_next; const int* log_head; const int* log_num; const unsigned char* log_ok;
     long long log_slots;
 };
@@ -267,7 +267,9 @@ __device__ __forceinline__ bool bwd_next_segment(const BwdParams& p, int ray, Bw
         const float s_prev = i > 0 ? __ldg(mid + (i - 1) * DST_MID_CHANNELS + 11) : 1.0f;
         if (sqrtf(sdx * sdx + sdy * sdy + sdz * sdz) == 0.0f || s_prev <= in.specular_threshold) continue;    // :724
 
-        const float g_rgb0 = __ldg(p.a.dL_drgb + 3 * (size_t)ray), g_rgb1 = __ldg(p.a.dL_drgb + 3 * (size_t)ray + 1), g_rgb2 = __ldg(p.a.dL_drgb + 3 * (size_t)ray + 2);
+        // (an upstream gradient that is not given is zero)
+        const float* up_rgb = p.a.dL_drgb ? p.a.dL_drgb + 3 * (size_t)ray : nullptr;
+        const float g_rgb0 = up_rgb ? __ldg(up_rgb) : 0.f, g_rgb1 = up_rgb ? __ldg(up_rgb + 1) : 0.f, g_rgb2 = up_rgb ? __ldg(up_rgb + 2) : 0.f;
         const float f_this = (i == depth) ? 1.0f : 1.0f - tot_o0;
         s.t_rgb0 = g_rgb0 * f_this * s.s_prod; s.t_rgb1 = g_rgb1 * f_this * s.s_prod; s.t_rgb2 = g_rgb2 * f_this * s.s_prod;   // :760
         s.s_prod /= s_prev;                                                                                   // :762
@@ -294,9 +296,10 @@ __device__ __forceinline__ bool bwd_next_segment(const BwdParams& p, int ray, Bw
             }
         }
         if (i == 0) {                                                                                         // :793-802
-            s.t_dpt += __ldg(p.a.dL_ddpt + ray); s.t_acc += __ldg(p.a.dL_dacc + ray);
-            t_norm = t_norm + v3(__ldg(p.a.dL_dnorm + 3 * (size_t)ray), __ldg(p.a.dL_dnorm + 3 * (size_t)ray + 1), __ldg(p.a.dL_dnorm + 3 * (size_t)ray + 2));
-            s.t_aux0 += __ldg(p.a.dL_daux + 2 * (size_t)ray); s.t_aux1 += __ldg(p.a.dL_daux + 2 * (size_t)ray + 1);
+            if (p.a.dL_ddpt) s.t_dpt += __ldg(p.a.dL_ddpt + ray);
+            if (p.a.dL_dacc) s.t_acc += __ldg(p.a.dL_dacc + ray);
+            if (p.a.dL_dnorm) t_norm = t_norm + v3(__ldg(p.a.dL_dnorm + 3 * (size_t)ray), __ldg(p.a.dL_dnorm + 3 * (size_t)ray + 1), __ldg(p.a.dL_dnorm + 3 * (size_t)ray + 2));
+            if (p.a.dL_daux) { s.t_aux0 += __ldg(p.a.dL_daux + 2 * (size_t)ray); s.t_aux1 += __ldg(p.a.dL_daux + 2 * (size_t)ray + 1); }
         }
         s.t_nx = t_norm.x; s.t_ny = t_norm.y; s.t_nz = t_norm.z;
         s.drd_x = drd.x; s.drd_y = drd.y; s.drd_z = drd.z;
@@ -737,14 +740,20 @@ __global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_logged(cons
     if (DIAG) bwd_flush_counters(p.a.counters, tc);
 }
 
-// arena rows -> the caller's gradient tensors
-__global__ void __launch_bounds__(256) k_unpack(int P, const float* __restrict__ arena, float* __restrict__ d_rot, float* __restrict__ d_mean,
+// Arena rows -> the caller's gradient tensors. The rows that hold anything are zeroed on the way, so the arena is clean for the next call: a
+// call with few rays leaves most of it untouched, and clearing all 80 bytes per surfel first was a fifth of what such a call writes.
+__global__ void __launch_bounds__(256) k_unpack(int P, float* __restrict__ arena, float* __restrict__ d_rot, float* __restrict__ d_mean,
                                                 float* __restrict__ d_opac, float* __restrict__ d_g3d, float* __restrict__ d_scale,
                                                 float* __restrict__ d_others, float* __restrict__ d_color) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= P) return;
-    const float4* r = reinterpret_cast<const float4*>(arena + (size_t)g * DST_ARENA_FLOATS);
+    float4* r = reinterpret_cast<float4*>(arena + (size_t)g * DST_ARENA_FLOATS);
     const float4 a = r[0], b = r[1], c = r[2], d = r[3], e = r[4];
+    auto used = [](const float4& v) { return v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f; };
+    if (used(a) || used(b) || used(c) || used(d) || used(e)) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        r[0] = zero; r[1] = zero; r[2] = zero; r[3] = zero; r[4] = zero;
+    }
     reinterpret_cast<float4*>(d_rot)[g] = a;
     d_mean[3 * (size_t)g] = b.x; d_mean[3 * (size_t)g + 1] = b.y; d_mean[3 * (size_t)g + 2] = b.z;
     d_opac[g] = b.w;
@@ -782,8 +791,7 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     if (rc != DST_OK) return rc;
     rc = backward_kernel_setup(h);
     if (rc != DST_OK) return rc;
-    if (!a->out_rgb || !a->mid_val || !a->dL_drgb || !a->dL_ddpt || !a->dL_dacc || !a->dL_dnorm || !a->dL_daux)
-        return dst_set_error(h, DST_E_ARG, "a saved forward output or upstream gradient pointer is null");
+    if (!a->out_rgb || !a->mid_val) return dst_set_error(h, DST_E_ARG, "a saved forward output pointer is null");
     if (!a->dL_dray_o || !a->dL_dray_d || !a->dL_dmeans3D || !a->dL_dgrads3D || !a->dL_dcolors || !a->dL_dothers ||
         !a->dL_dopacities || !a->dL_dscales || !a->dL_drotations || (a->in.shs && !a->dL_dshs))
         return dst_set_error(h, DST_E_ARG, "a gradient output pointer is null");
@@ -796,17 +804,31 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
         cudaFree(h->arena); h->arena = nullptr; h->arena_cap = 0;
         const int64_t cap = P + P / 8 + 1024;
         if (cudaMalloc(&h->arena, 4 * DST_ARENA_FLOATS * cap) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "gradient arena allocation failed"); }
-        h->arena_cap = cap;
+        h->arena_cap = cap; h->arena_clean = false;
     }
-    rc = dst_prepare_cache(h, &a->in, st);
-    if (rc != DST_OK) return rc;
-    DST_CUDA_TRY(h, cudaMemsetAsync(h->arena, 0, 4 * DST_ARENA_FLOATS * (size_t)P, st));
+    if (!h->arena_clean) DST_CUDA_TRY(h, cudaMemsetAsync(h->arena, 0, 4 * DST_ARENA_FLOATS * (size_t)h->arena_cap, st));
+    h->arena_clean = false;      // until k_unpack has been enqueued
+    // the records of the forward this belongs to, when they are still there
+    const bool same = a->forward_serial != 0 && a->forward_serial == h->cache_serial && h->cache_src[0] == a->in.means3D && h->cache_src[1] == a->in.scales &&
+                      h->cache_src[2] == a->in.rotations && h->cache_src[3] == a->in.opacities && h->cache_P == P;
+    if (!same) { rc = dst_prepare_cache(h, &a->in, st); if (rc != DST_OK) return rc; }
     if (a->dL_dshs) DST_CUDA_TRY(h, cudaMemsetAsync(a->dL_dshs, 0, 12 * (size_t)P * a->in.sh_coeffs, st));
     BwdParams p;
     p.a = *a; p.bvh = dst_bvh_view(h); p.cache = h->cache; p.arena = h->arena; p.status = h->status;
     p.dist_on = h->distortion;
+    dst_handle::Log* log = nullptr;
+    if (a->forward_serial != 0) {
+        for (int k = 0; k < h->logs_used; k++) {
+            dst_handle::Log& l = h->logs[k];
+            if (l.serial == a->forward_serial && l.H == a->in.H && l.W == a->in.W && l.depth == a->in.max_trace_depth) log = &l;
+        }
+        // a log that was overwritten before its backward came: room for the forwards since then next time
+        const unsigned long long since = h->serial_counter - a->forward_serial + 1;
+        if (!log && h->logs_keep > 1 && since > 1) h->logs_wanted = since < (unsigned long long)h->logs_keep ? (int)since : h->logs_keep;
+    }
     dst_slot_grid(h, &a->in, &p.grid_h, &p.grid_w);
     p.tiled = p.grid_h >= 16;
+    if (log) { p.grid_h = log->grid_h; p.grid_w = log->grid_w; p.tiled = log->tiled; log->consumed = true; }       // the log is indexed by its forward's slots
     const long long slots = slots_of_grid(p.grid_h, p.grid_w, p.tiled != 0);
     rc = dst_ensure_wavefront(h, slots, sizeof(BwdState));
     if (rc != DST_OK) return rc;
@@ -814,9 +836,8 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     p.list[0] = h->wf_list[0]; p.list[1] = h->wf_list[1]; p.counts = h->wf_counts;
     const bool diag = a->counters != nullptr;
     const bool dist = h->distortion != 0 && a->dL_ddist != nullptr && a->out_dist != nullptr;
-    const bool use_log = a->forward_serial != 0 && a->forward_serial == h->log_serial && h->log_H == a->in.H && h->log_W == a->in.W &&
-                         h->log_depth == a->in.max_trace_depth;
-    p.log_keys = h->log_keys; p.log_next = h->log_next; p.log_head = h->log_head; p.log_num = h->log_num; p.log_ok = h->log_ok;
+    const bool use_log = log != nullptr;
+    p.log_keys = h->log_keys; p.log_next = h->log_next; p.log_head = log ? log->head : nullptr; p.log_num = log ? log->num : nullptr; p.log_ok = log ? log->ok : nullptr;
     p.log_slots = slots;
     DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_counts, 0, 4 * DST_COUNTS_STRIDE, st));
     h->slices_used = 1;
@@ -829,7 +850,7 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     // With the log the rounds only serve rays it could not hold. When the last completed read-back of a forward of this shape
     // shows that everything fitted, none are enqueued (scheduling only: whatever is left after them is finished by the tail
     // kernel). A dozen rounds of empty launches took 0.15 ms.
-    if (wave && use_log && h->log_known_needed > 0 && h->log_known_sig == dst_call_signature(&a->in) && h->log_known_needed <= h->log_cap)
+    if (wave && use_log && h->log_known_needed > 0 && h->log_known_sig == dst_call_signature(&a->in) && h->log_use <= h->log_cap)
         p.rounds = 0;
     dst_prof_mark(h, 2, 0, st);
     if (use_log) {
@@ -859,6 +880,7 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     k_unpack<<<(unsigned int)((P + 255) / 256), 256, 0, st>>>((int)P, h->arena, a->dL_drotations, a->dL_dmeans3D, a->dL_dopacities,
                                                               a->dL_dgrads3D, a->dL_dscales, a->dL_dothers, a->dL_dcolors);
     DST_CUDA_TRY(h, cudaGetLastError());
+    h->arena_clean = true;
     h->launches += 3 + (p.lv.stable ? 5 : 4) * p.rounds;       // logged re-composite or ray init, the rounds, tail, unpack
     return DST_OK;
 }

@@ -42,6 +42,7 @@ struct SurfelCacheView { const float4* rec; };
 #define DST_LOG_MAX_RECORDS (320ll << 20)     // 132 B each: at most 44.3 GB of contribution log
 
 #define DST_MAX_SLICES 8
+#define DST_MAX_LOGS 4                 // forwards whose contribution logs a handle can keep at once
 struct dst_handle {
     int device;
     char err[512];
@@ -60,7 +61,8 @@ struct dst_handle {
     float* header;                // DST_HDR_FLOATS floats + 8 uint bounds words
     unsigned int* status;         // device status word
     float4* cache; int64_t cache_cap;
-    float* arena;  int64_t arena_cap;
+    unsigned long long cache_serial; const float* cache_src[4]; int64_t cache_P;      // training forward (serial) and tensors the records were built from
+    float* arena;  int64_t arena_cap; bool arena_clean;       // clean: all zeros once the work enqueued so far has run
     void* cam_dev;      // camera constants of the last ray-generation call
     long long image_width;     // hint: rays given as (B, h*w, 3) are whole images of this width (0: unknown)
     int single_kernel_refit;   // dst_build_from_surfels(rebuild = 0): expand the quads inside the refit kernel
@@ -83,17 +85,25 @@ struct dst_handle {
     // the current call, their pinned read-back, and how many coming calls leave the prediction off after a call in which it
     // failed too often.
     int* bound_stats; int* bound_host; cudaEvent_t bound_event; bool bound_pending; int bound_off_calls;
-    // contribution log of the last training forward (dst_ensure_log), so that the backward re-composites it without walking the
+    // contribution log of training forwards (dst_begin_log), so that the backward re-composites it without walking the
     // hierarchy again
-    unsigned long long* log_keys; int* log_next; int* log_count; int* log_head; int* log_num; unsigned char* log_ok;
+    unsigned long long* log_keys; int* log_next; int* log_count;      // records of all logs; log_count: {records in use, of them before the last forward}
     long long log_cap;            // records
-    long long log_index_cap;      // slots x segments of log_head / log_num
-    unsigned long long log_serial;      // serial of the forward call the log belongs to (0 = none)
+    unsigned long long log_serial;      // serial of the last forward call if it left a log (0 = none)
     unsigned long long serial_counter;
-    int log_H, log_W, log_depth;
+    // Logs of the last forwards, in the order of the calls. More than one only where the caller asks for it (DST_OPT_KEPT_LOGS): a step
+    // that traces several views before its backward then needs no re-trace. log_use: records the logs are expected to hold.
+    struct Log {
+        unsigned long long serial;      // 0: none
+        bool consumed;                  // a backward has used it: the next forward may overwrite it
+        int H, W, depth, grid_h, grid_w, tiled;
+        long long slots;
+        int* head; int* num; unsigned char* ok; long long index_cap;       // per slot and segment: first record, entries; per slot: complete
+    } logs[DST_MAX_LOGS];
+    int logs_used, logs_keep, logs_wanted; long long log_use;       // logs_wanted: logs a backward has asked for at the same time
     int log_enabled;
     long long log_max_records;    // user limit on the log size (0: only the built-in limit)
-    int* log_needed_host; cudaEvent_t log_needed_event;     // pinned read-back of the record count of the last forward
+    int* log_needed_host; cudaEvent_t log_needed_event;     // pinned read-back of log_count after the last forward
     long long log_known_sig, log_known_needed;              // last completed read-back: call shape and records wanted (0: none yet)
     long long log_pending_sig;                              // call shape of the forward whose read-back is in flight
     // pinned read-back of the per-round list lengths of the last wavefront forward, for the round count of the next one
@@ -136,7 +146,8 @@ int dst_knearest_impl(dst_handle* h, const float* ro, const float* rd, int64_t n
 int dst_prepare_cache(dst_handle* h, const dst_trace_inputs* in, cudaStream_t st);
 int dst_export_frames_impl(dst_handle* h, float* out, cudaStream_t st);
 int dst_ensure_wavefront(dst_handle* h, long long slots, size_t state_bytes);
-int dst_ensure_log(dst_handle* h, long long rays, long long slots, int segs);
+int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int grid_w, int tiled, long long slots, dst_handle::Log** log, cudaStream_t st);
+void dst_drop_logs(dst_handle* h);
 int dst_wavefront_grid(const dst_handle* h, long long slots, int threads, int per_sm);
 
 #ifdef __CUDACC__

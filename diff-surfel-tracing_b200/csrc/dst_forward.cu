@@ -72,7 +72,7 @@ struct FwdParams {
     int min_count;
     int rounds;
     LiveLists lv;
-    // contribution log (null log_keys: disabled), see dst_ensure_log()
+    // contribution log (null log_keys: disabled), see dst_begin_log()
     unsigned long long* log_keys; int* log_next; int* log_count; int* log_head; int* log_num; unsigned char* log_ok;
     int log_cap; long long log_slots;       // records; slots per segment of log_head / log_num
 };
@@ -702,6 +702,8 @@ int dst_prepare_cache(dst_handle* h, const dst_trace_inputs* in, cudaStream_t st
     }
     k_prepare_cache<<<(in->P + 255) / 256, 256, 0, st>>>(in->P, in->means3D, in->scales, in->rotations, in->opacities, h->cache);
     h->launches += 1;
+    h->cache_serial = 0;
+    h->cache_src[0] = in->means3D; h->cache_src[1] = in->scales; h->cache_src[2] = in->rotations; h->cache_src[3] = in->opacities; h->cache_P = in->P;
     DST_CUDA_TRY(h, cudaGetLastError());
     return DST_OK;
 }
@@ -755,38 +757,63 @@ long long dst_call_signature(const dst_trace_inputs* in) {
     return ((long long)in->H * 1000003ll + in->W) * 1000033ll + (long long)in->P * 131ll + in->max_trace_depth + 1;
 }
 
-// Contribution log for `slots` list slots of up to `segs` segments (grow-only). A training forward logs every contribution (depth along
-// the segment, primitive) so that the backward can composite them again without walking the hierarchy: records of 16 entries,
-// chained per segment, 32 records interleaved (soa()); per segment and slot the first record and the number of entries.
-int dst_ensure_log(dst_handle* h, long long rays, long long slots, int segs) {
-    // first guess 12 records per ray; afterwards what the previous training forward actually needed (read back
-    // asynchronously, see forward_common), within DST_LOG_MAX_RECORDS. Rays beyond the log re-trace in the backward.
-    long long want = rays * 12 + 4096;
+void dst_drop_logs(dst_handle* h) {
+    for (int k = 0; k < DST_MAX_LOGS; k++) h->logs[k].serial = 0;
+    h->logs_used = 0; h->log_use = 0; h->log_serial = 0;
+}
+
+// Starts the contribution log of a training forward. The forward logs every contribution (depth along the segment, primitive) so that
+// the backward can composite them again without walking the hierarchy: records of 16 entries, chained per segment, 32 records
+// interleaved (soa()); per segment and slot the first record and the number of entries. Buffers are grow-only.
+//
+// The log of the forward before is overwritten, unless its backward has not come yet and the caller wants logs kept: then this
+// one is appended, if the records both are expected to need fit.
+int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int grid_w, int tiled, long long slots, dst_handle::Log** log, cudaStream_t st) {
+    const long long rays = (long long)in->H * in->W, sig = dst_call_signature(in);
+    const int segs = in->max_trace_depth + 1;
     if (h->log_needed_host && h->log_needed_event && cudaEventQuery(h->log_needed_event) == cudaSuccess) {
-        const long long seen = *h->log_needed_host;
-        if (seen > 0 && seen + seen / 8 > want) want = seen + seen / 8;
+        const long long seen = (long long)h->log_needed_host[0] - h->log_needed_host[1];
         if (seen > 0) { h->log_known_needed = seen; h->log_known_sig = h->log_pending_sig; }
     } else cudaGetLastError();
-    if (want > DST_LOG_MAX_RECORDS) want = DST_LOG_MAX_RECORDS;
-    if (h->log_max_records > 0 && want > h->log_max_records) want = h->log_max_records;
-    want = (want + 31) / 32 * 32;
-    if (want > h->log_cap || (h->log_max_records > 0 && h->log_cap > want)) {
-        cudaFree(h->log_keys); cudaFree(h->log_next); h->log_keys = nullptr; h->log_next = nullptr; h->log_cap = 0;
-        cudaError_t e = cudaMalloc(&h->log_keys, 8 * DST_CHUNK * (size_t)want);
-        if (e == cudaSuccess) e = cudaMalloc(&h->log_next, sizeof(int) * (size_t)want);
-        if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed: %s", cudaGetErrorString(e)); }
-        h->log_cap = want;
-    }
-    if (!h->log_count && cudaMalloc(&h->log_count, 4) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed"); }
-    if (slots * segs > h->log_index_cap) {
-        cudaFree(h->log_head); cudaFree(h->log_num); cudaFree(h->log_ok); h->log_head = h->log_num = nullptr; h->log_ok = nullptr; h->log_index_cap = 0;
+    // first guess 12 records per ray; then what the last forward of this shape needed (read back asynchronously), within
+    // DST_LOG_MAX_RECORDS. Rays beyond the log re-trace in the backward.
+    const long long guess = rays * 12 + 4096;
+    const long long need = h->log_known_needed > 0 && h->log_known_sig == sig ? h->log_known_needed + h->log_known_needed / 8 + 1024 : guess;
+    bool pending = false;
+    for (int k = 0; k < h->logs_used; k++) pending |= h->logs[k].serial != 0 && !h->logs[k].consumed;
+    if (!(pending && h->logs_used < h->logs_keep && h->log_use + need <= h->log_cap)) {
+        dst_drop_logs(h);
+        long long want = need > guess ? need : guess;
+        if (h->logs_wanted > 1 && need * h->logs_wanted > want) want = need * h->logs_wanted;
+        if (want > DST_LOG_MAX_RECORDS) want = DST_LOG_MAX_RECORDS;
+        if (h->log_max_records > 0 && want > h->log_max_records) want = h->log_max_records;
+        want = (want + 31) / 32 * 32;
+        if (want > h->log_cap || (h->log_max_records > 0 && h->log_cap > want)) {
+            cudaFree(h->log_keys); cudaFree(h->log_next); h->log_keys = nullptr; h->log_next = nullptr; h->log_cap = 0;
+            cudaError_t e = cudaMalloc(&h->log_keys, 8 * DST_CHUNK * (size_t)want);
+            if (e == cudaSuccess) e = cudaMalloc(&h->log_next, sizeof(int) * (size_t)want);
+            if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed: %s", cudaGetErrorString(e)); }
+            h->log_cap = want;
+        }
+        if (!h->log_count && cudaMalloc(&h->log_count, 8) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed"); }
+        DST_CUDA_TRY(h, cudaMemsetAsync(h->log_count, 0, 8, st));
+    } else DST_CUDA_TRY(h, cudaMemcpyAsync(h->log_count + 1, h->log_count, 4, cudaMemcpyDeviceToDevice, st));
+    dst_handle::Log& l = h->logs[h->logs_used];
+    if (slots * segs > l.index_cap) {
+        cudaFree(l.head); cudaFree(l.num); cudaFree(l.ok); l.head = l.num = nullptr; l.ok = nullptr; l.index_cap = 0;
         const long long cap = slots * segs + slots / 16 + 1024;
-        cudaError_t e = cudaMalloc(&h->log_head, 4 * (size_t)cap);
-        if (e == cudaSuccess) e = cudaMalloc(&h->log_num, 4 * (size_t)cap);
-        if (e == cudaSuccess) e = cudaMalloc(&h->log_ok, (size_t)cap);
+        cudaError_t e = cudaMalloc(&l.head, 4 * (size_t)cap);
+        if (e == cudaSuccess) e = cudaMalloc(&l.num, 4 * (size_t)cap);
+        if (e == cudaSuccess) e = cudaMalloc(&l.ok, (size_t)cap);
         if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed: %s", cudaGetErrorString(e)); }
-        h->log_index_cap = cap;
+        l.index_cap = cap;
     }
+    h->logs_used++;
+    h->log_use += need;
+    l.serial = h->log_serial = ++h->serial_counter;
+    l.consumed = false;
+    l.H = in->H; l.W = in->W; l.depth = in->max_trace_depth; l.grid_h = grid_h; l.grid_w = grid_w; l.tiled = tiled; l.slots = slots;
+    *log = &l;
     return DST_OK;
 }
 
@@ -873,13 +900,12 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     p.log_cap = 0; p.log_slots = slots;
     h->log_serial = 0;
     if (a->training && h->log_enabled) {
-        rc = dst_ensure_log(h, (long long)a->in.H * a->in.W, slots, a->in.max_trace_depth + 1);
+        dst_handle::Log* log = nullptr;
+        rc = dst_begin_log(h, &a->in, p.grid_h, p.grid_w, p.tiled, slots, &log, st);
         if (rc != DST_OK) return rc;
-        p.log_keys = h->log_keys; p.log_next = h->log_next; p.log_count = h->log_count; p.log_head = h->log_head; p.log_num = h->log_num;
-        p.log_ok = h->log_ok; p.log_cap = (int)h->log_cap;
-        DST_CUDA_TRY(h, cudaMemsetAsync(h->log_count, 0, 4, st));
-        h->log_serial = ++h->serial_counter;
-        h->log_H = a->in.H; h->log_W = a->in.W; h->log_depth = a->in.max_trace_depth;
+        p.log_keys = h->log_keys; p.log_next = h->log_next; p.log_count = h->log_count; p.log_head = log->head; p.log_num = log->num;
+        p.log_ok = log->ok; p.log_cap = (int)h->log_cap;
+        h->cache_serial = log->serial;
     }
     // small launches go straight to the per-ray kernel; large ones run wavefront rounds until few rays are left
     const bool wave = slots >= h->wf_min_rays;
@@ -1030,12 +1056,12 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     if (p.log_keys) {
         // how many records this call wanted, for sizing the log of the next one (no synchronisation here)
         if (!h->log_needed_host) {
-            if (cudaMallocHost(&h->log_needed_host, sizeof(int)) != cudaSuccess) { cudaGetLastError(); h->log_needed_host = nullptr; }
-            else *h->log_needed_host = 0;
+            if (cudaMallocHost(&h->log_needed_host, 8) != cudaSuccess) { cudaGetLastError(); h->log_needed_host = nullptr; }
+            else h->log_needed_host[0] = h->log_needed_host[1] = 0;
             if (h->log_needed_host && cudaEventCreateWithFlags(&h->log_needed_event, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); h->log_needed_event = nullptr; }
         }
         if (h->log_needed_host && h->log_needed_event) {
-            cudaMemcpyAsync(h->log_needed_host, h->log_count, sizeof(int), cudaMemcpyDeviceToHost, st);
+            cudaMemcpyAsync(h->log_needed_host, h->log_count, 8, cudaMemcpyDeviceToHost, st);
             cudaEventRecord(h->log_needed_event, st);
             h->log_pending_sig = dst_call_signature(&a->in);      // (the backward compares with the plain shape: slices are the forward's business)
         }

@@ -203,6 +203,11 @@ class OptiXStateWrapper:
         ray count, 1: no slicing). Scheduling only."""
         _check(self, lib().dst_set_option(self.handle, 9, int(n)))
 
+    def set_kept_logs(self, n):
+        """Training forwards whose contribution logs are kept until their backward comes (default 1: a forward replaces the log of
+        the one before, whose backward then re-traces)."""
+        _check(self, lib().dst_set_option(self.handle, 10, int(n)))
+
     def profile(self, on=True):
         """Records CUDA events around the build, forward and backward kernels of later calls; on=2 also around
         every launch of the gather kernel."""
@@ -369,7 +374,7 @@ def trace_surfels_backward(state, start_from_first, ray_o, ray_d, vertices, back
                            others_precomp, opacities, scales, scale_modifier, rotations, transMat_precomp, viewmatrix,
                            projmatrix, campos, prefiltered, debug, max_trace_depth, specular_threshold,
                            out_rgb, out_dpt, out_acc, out_norm, out_dist, out_aux, mid_val,
-                           dL_drgb, dL_ddpt, dL_dacc, dL_dnorm, dL_ddist, dL_daux, _diag=None, _forward_serial=None):
+                           dL_drgb, dL_ddpt, dL_dacc, dL_dnorm, dL_ddist, dL_daux, _diag=None, _forward_serial=None, _zeros=True):
     """trace_surfels.cpp:307-464. Returns the 12 gradients in the reference's order:
     ray_o, ray_d, means3D, grads3D, grads3D_abs (zeros), shs, colors_precomp, others_precomp,
     opacities, scales, rotations, transMat_precomp (zeros).
@@ -378,7 +383,9 @@ def trace_surfels_backward(state, start_from_first, ray_o, ray_d, vertices, back
     tensors come from; when it still names the handle's chunk log the backward re-composites the logged
     chunks instead of walking the hierarchy again (same result). When it is not given (None), the call is
     recognised by its `mid_val` tensor: if that is the one the state's last training forward returned, its
-    serial is used. Pass 0 to force a re-trace."""
+    serial is used. Pass 0 to force a re-trace.
+
+    `_zeros`: False returns None for the two gradients that are always zero."""
     if _forward_serial is None:
         key = (mid_val.data_ptr(), tuple(mid_val.shape))
         _forward_serial = state.last_forward_serial if getattr(state, "_logged_mid", None) == key else 0
@@ -392,9 +399,9 @@ def trace_surfels_backward(state, start_from_first, ray_o, ray_d, vertices, back
     sv = [_cuda_f32(t, n, state) for t, n in ((out_rgb, "out_rgb"), (out_dpt, "out_dpt"), (out_acc, "out_acc"), (out_norm, "out_norm"),
                                          (out_dist, "out_dist"), (out_aux, "out_aux"), (mid_val, "mid_val"))]
 
-    def up(g, shape, name):
+    def up(g, shape, name):       # an upstream gradient that is not given is zero
         if g is None:
-            return torch.zeros(shape, **f32)
+            return None
         return _cuda_f32(g.expand(shape) if g.shape != torch.Size(shape) else g, name, state)
 
     ug = [up(dL_drgb, (H, W, 3), "dL_drgb"), up(dL_ddpt, (H, W, 1), "dL_ddpt"), up(dL_dacc, (H, W, 1), "dL_dacc"),
@@ -430,13 +437,13 @@ def trace_surfels_backward(state, start_from_first, ray_o, ray_d, vertices, back
     g_others = view("others", P * AUX_CHANNELS, (P, AUX_CHANNELS))
     g_opac = view("opac", P, (P, 1))
     g_scales = view("scales", P * 2, (P, 2))
-    g_g3d_abs = torch.zeros((P, 3), **f32)
+    g_g3d_abs = torch.zeros((P, 3), **f32) if _zeros else None
     state.grad_bucket = bucket
-    g_trans = torch.zeros((P, 9), **f32)
+    g_trans = torch.zeros((P, 9), **f32) if _zeros else None
     a = _BwdArgs()
     a.inp = i
     (a.out_rgb, a.out_dpt, a.out_acc, a.out_norm, a.out_dist, a.out_aux, a.mid_val) = [t.data_ptr() for t in sv]
-    (a.dL_drgb, a.dL_ddpt, a.dL_dacc, a.dL_dnorm, a.dL_ddist, a.dL_daux) = [t.data_ptr() for t in ug]
+    (a.dL_drgb, a.dL_ddpt, a.dL_dacc, a.dL_dnorm, a.dL_ddist, a.dL_daux) = [_ptr(t) for t in ug]
     a.dL_dray_o, a.dL_dray_d, a.dL_dmeans3D, a.dL_dgrads3D = g_ray_o.data_ptr(), g_ray_d.data_ptr(), g_means.data_ptr(), g_g3d.data_ptr()
     a.dL_dshs = _ptr(g_shs)
     a.dL_dcolors, a.dL_dothers, a.dL_dopacities = g_colors.data_ptr(), g_others.data_ptr(), g_opac.data_ptr()

@@ -53,6 +53,7 @@ class _TraceSurfels(torch.autograd.Function):
             out = _C.trace_surfels(*args)
         out_rgb, out_dpt, out_acc, out_norm, out_dist, out_aux, mid_val, a_weights = out
 
+        ctx.set_materialize_grads(False)       # outputs the loss does not use: None instead of a tensor of zeros
         ctx.tracer_settings = tracer_settings
         ctx.optix_context = optix_context
         ctx.start_from_first = start_from_first
@@ -76,13 +77,13 @@ class _TraceSurfels(torch.autograd.Function):
         if s.debug:
             cpu_args = cpu_deep_copy_tuple(args[1:])
             try:
-                grads = _C.trace_surfels_backward(*args, _forward_serial=ctx.forward_serial)
+                grads = _C.trace_surfels_backward(*args, _forward_serial=ctx.forward_serial, _zeros=False)
             except Exception as ex:
                 torch.save(cpu_args, "snapshot_bw.dump")
                 print("\nAn error occured in backward. Writing snapshot_bw.dump for debugging.\n")
                 raise ex
         else:
-            grads = _C.trace_surfels_backward(*args, _forward_serial=ctx.forward_serial)
+            grads = _C.trace_surfels_backward(*args, _forward_serial=ctx.forward_serial, _zeros=False)
         (grad_ray_o, grad_ray_d, grad_means3D, grad_grads3D, grad_grads3D_abs, grad_shs, grad_colors_precomp,
          grad_others_precomp, grad_opacities, grad_scales, grad_rotations, grad_cov3Ds_precomp) = grads
 
@@ -91,7 +92,7 @@ class _TraceSurfels(torch.autograd.Function):
 
         return (None, None, None, grad_ray_o, grad_ray_d, None, grad_means3D, grad_grads3D, fit(grad_shs, shs),
                 fit(grad_colors_precomp, colors_precomp), fit(grad_others_precomp, others_precomp), grad_opacities,
-                grad_scales, grad_rotations, fit(grad_cov3Ds_precomp, cov3Ds_precomp), None)
+                grad_scales, grad_rotations, None, None)
 
 
 class SurfelTracingSettings(NamedTuple):
@@ -117,6 +118,7 @@ class SurfelTracer(nn.Module):
         self.pkg_dir = _C._PKG
         # name kept from the reference; the object owns the hierarchy and scratch memory of this GPU
         self.optix_context = _C.OptiXStateWrapper(self.pkg_dir)
+        self.optix_context.set_kept_logs(4)       # several views traced before one backward: autograd names the forward it belongs to
 
     def build_acceleration_structure(self, vertices: torch.Tensor, triangles: torch.Tensor, rebuild: bool = 1):
         return _C.build_acceleration_structure(self.optix_context, vertices, triangles, rebuild)

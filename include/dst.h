@@ -246,6 +246,9 @@ int dst_bvh_info(const dst_handle* h, int64_t* surfels, int64_t* nodes, int64_t*
  * joined into it before the call returns, so that the slow last batches of one slice's round overlap with the other
  * slices' work. 0 (default): 4 for calls of a million rays and more, fewer for smaller ones; 1: no slicing; at most 8. */
 #define DST_OPT_FORWARD_SLICES 9
+/* Training forwards whose contribution logs the handle keeps until their backward comes (1, the default, to 4). With 1 a
+ * forward replaces the log of the one before, whose backward then re-traces. */
+#define DST_OPT_KEPT_LOGS 10
 int dst_set_option(dst_handle* h, int option, int64_t value);
 
 /* Timing of the main kernels with CUDA events on the launching stream. While enabled, every
