@@ -686,10 +686,11 @@ __global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_tail(const 
 // open in the warp (the backward visits a ray's segments last to first): neighbouring pixels then composite the same surfels in
 // the same pass, which is what send_rows() feeds on.
 template <bool DIAG, bool DIST>
-__global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_logged(const __grid_constant__ BwdParams p, long long slots) {
+__global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_logged(const __grid_constant__ BwdParams p, long long slots, int per) {
     constexpr unsigned int FULL = 0xffffffffu;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int slot = i < slots ? (int)i : -1;
+    const int lane = threadIdx.x & 31;
+    const long long i = ((long long)blockIdx.x * (BWD_THREADS / 32) + (threadIdx.x >> 5)) * per + lane;
+    const int slot = lane < per && i < slots ? (int)i : -1;
     const int ray = slot >= 0 ? slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0) : -1;
     TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
     BwdWarp& ws = bwd_warp_mem();
@@ -856,9 +857,14 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     if (use_log) {
         // the forward logged its contributions: composite them again; rays the log could not hold are queued as round 0 of the
         // re-trace below (normally none: the rounds then find an empty list and return at once)
-        const unsigned int blocks = (unsigned int)((slots + BWD_THREADS - 1) / BWD_THREADS);
-        if (dist) { if (diag) k_bwd_logged<true, true><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots); else k_bwd_logged<false, true><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots); }
-        else { if (diag) k_bwd_logged<true, false><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots); else k_bwd_logged<false, false><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots); }
+        // Rays per warp: 32, or 16 or 8 (4x4 and 4x2 patches of a tile) where 32 would leave warp slots of the GPU empty. What a small call takes
+        // is the chain of one warp's hits, and adding the rows of 8 rays up is shorter than those of 32.
+        int per = 32;
+        while (per > 8 && slots / per * 2 <= (long long)h->sm_count * DST_BWD_BLOCKS * (BWD_THREADS / 32)) per >>= 1;
+        const long long per_block = per * (BWD_THREADS / 32);
+        const unsigned int blocks = (unsigned int)((slots + per_block - 1) / per_block);
+        if (dist) { if (diag) k_bwd_logged<true, true><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); else k_bwd_logged<false, true><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); }
+        else { if (diag) k_bwd_logged<true, false><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); else k_bwd_logged<false, false><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); }
     } else {
         k_bwd_init<<<(unsigned int)((slots + 255) / 256), 256, 0, st>>>(p, slots);
     }

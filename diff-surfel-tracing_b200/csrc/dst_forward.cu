@@ -386,7 +386,7 @@ __device__ __forceinline__ void flush_counters(unsigned long long* counters, con
 __global__ void __launch_bounds__(256) k_fwd_init(const __grid_constant__ FwdParams p, long long slots) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= slots) return;
-    if (i == 0) p.counts[0] = (int)slots;
+    if (i == 0) { p.counts[0] = (int)slots; p.counts[DST_TAIL_CURSOR] = 0; }
     const int slot = (int)(p.slot0 + i);
     const int ray = slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0);
     p.list[0][i] = ray < 0 ? -1 : slot;
@@ -510,6 +510,11 @@ __device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int slot, War
     const bool have = lane < cnt;
     const float min_depth = s.bounce == 0 ? (in.start_from_first ? 0.2f : 0.0f) : 0.06f;       // forward.cu:353
     const int gidx = (int)((unsigned int)key >> 1);
+    if (have && in.colors_precomp == nullptr) {       // the colour row is on its way while the hit is evaluated
+        const float* row = in.shs + 3 * (size_t)gidx * in.sh_coeffs;
+        asm volatile("prefetch.global.L1 [%0];" :: "l"(row));
+        if (in.sh_coeffs > 8) asm volatile("prefetch.global.L1 [%0];" :: "l"(row + 32));
+    }
     SlotEval e;
     e.dpt = 0.f; e.alpha = 0.f;
     const bool ok = have && eval_slot(key, s.offset, s.sox, s.soy, s.soz, s.sdx, s.sdy, s.sdz, min_depth, p.cache, gidx, e);
@@ -627,11 +632,15 @@ __global__ void __launch_bounds__(WTAIL_THREADS, DST_WTAIL_BLOCKS) k_fwd_tail_wa
     const int n = p.counts[round];
     const int* list = p.list[round & 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int warps = gridDim.x * (WTAIL_THREADS / 32);
     const float absmax = __ldg(p.bvh.header + 6);
     WarpShade& ws = shade_mem[w];
     TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
-    for (int i = blockIdx.x * (WTAIL_THREADS / 32) + w; i < n; i += warps) {
+    for (;;) {
+        // (taken from a cursor: rays differ by a factor of ten in what they cost)
+        int i = 0;
+        if (lane == 0) i = atomicAdd(p.counts + DST_TAIL_CURSOR, 1);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= n) break;
         const int slot = list[i];
         if (slot < 0) continue;
         if (lane < (int)(sizeof(FwdState) / 16))
@@ -971,9 +980,12 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
         if (h->bound_off_calls > 0) h->bound_off_calls--;
         else if (h->bound_stats) { p.bound_stats = h->bound_stats; p.bound_factor = DST_BOUND_FACTOR; DST_CUDA_TRY(h, cudaMemsetAsync(h->bound_stats, 0, 8, st)); }
     }
-    DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_counts, 0, 4 * (size_t)DST_COUNTS_STRIDE * DST_MAX_SLICES, st));
-    rc = dst_live_lists(h, slots, &p.lv, st);
-    if (rc != DST_OK) return rc;
+    memset(&p.lv, 0, sizeof(p.lv));
+    if (wave) {       // (a call without rounds uses two of the counters, which k_fwd_init sets)
+        DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_counts, 0, 4 * (size_t)DST_COUNTS_STRIDE * DST_MAX_SLICES, st));
+        rc = dst_live_lists(h, slots, &p.lv, st);
+        if (rc != DST_OK) return rc;
+    }
     dst_prof_mark(h, 1, 0, st);
     // the slices: ranges of whole list blocks, each with its own view of the lists and counters
     FwdParams ps[DST_MAX_SLICES];
@@ -1146,7 +1158,6 @@ extern "C" int dst_forward_static(dst_handle* h, const dst_fwd_args* a, void* st
     p.log_keys = nullptr; p.log_next = nullptr; p.log_count = nullptr; p.log_head = p.log_num = nullptr; p.log_ok = nullptr;
     p.log_cap = 0; p.log_slots = 0;
     // the array keeps the previous call's contents: the round counters must start at zero, everything else is rewritten
-    DST_CUDA_TRY(h, cudaMemsetAsync(p.counts, 0, 4 * DST_COUNTS_STRIDE, st));
     if (a->training && a->a_weights) DST_CUDA_TRY(h, cudaMemsetAsync(a->a_weights, 0, 4 * (size_t)a->in.P, st));
     k_prepare_cache<<<(a->in.P + 255) / 256, 256, 0, st>>>(a->in.P, a->in.means3D, a->in.scales, a->in.rotations, a->in.opacities,
                                                              reinterpret_cast<float4*>(base + ST_OFF_CACHE));

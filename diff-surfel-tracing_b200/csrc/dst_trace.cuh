@@ -306,6 +306,7 @@ constexpr int ENUM_THREADS = 128;
 #define DST_ENUM_MIN_BLOCKS 6         // resident blocks per SM the gather kernel is compiled for
 #endif
 #define DST_WF_ROUNDS 48
+#define DST_TAIL_CURSOR (DST_COUNTS_STRIDE - 1)          // word of a set of round counters no round uses: next list entry of the tail kernel
 #define DST_COUNTS_STRIDE (6 * (DST_WF_ROUNDS + 2))      // ints per set of round counters: list lengths, batch cursors, rays given up by the batches, their cursor
 
 // ---------------------------------------------------------------------------------------------
@@ -406,6 +407,7 @@ struct BeamSlab { float4 in_lo, in_hi, out_lo, out_hi, in_z, out_z; };       // 
 struct WalkMem {
     unsigned long long stack[DST_WALK_STACK];        // subtrees: nearest possible t << 32 | link, nearest on top
     unsigned long long quads[DST_WALK_QUADS];        // quads whose box the hull reaches: nearest possible t << 32 | leaf position
+    unsigned long long place[DST_CHUNK];             // see take_hits()
     BeamSlab slab;
     BeamQ beam;
 };
@@ -605,16 +607,44 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
     if (COUNT && counters) { atomicAdd(counters + 1, tc.enums); atomicAdd(counters + 2, tc.nodes); atomicAdd(counters + 3, tc.quads); }
 }
 
+// Takes the hits found by one quad step (lanes with `hit`, in `key`) into the sorted k-buffer held by lanes 0..15 (`mine`, ~0 where empty). Every
+// hit is handed round once: a lane counts the hits below its own hit and below its buffer entry, and a ballot the entries below
+// each hit. The counts are the new places; nothing waits for the hit before (one insertion after the other was a chain of seven
+// cross-lane operations per hit, a fifth of the latency of a walk). place: DST_CHUNK words of shared memory of the warp.
+__device__ __forceinline__ void take_hits(bool hit, unsigned long long key, unsigned long long& mine, unsigned long long* place) {
+    constexpr unsigned int FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned long long last = __shfl_sync(FULL, mine, DST_CHUNK - 1);
+    unsigned int hits = __ballot_sync(FULL, hit && key < last);      // (nearer than the 16th)
+    if (hits == 0u) return;
+    hit = (hits >> lane) & 1u;
+    const bool held = lane < DST_CHUNK && mine != ~0ull;
+    int at = 0, old_at = lane;
+    while (hits) {
+        const int hl = __ffs(hits) - 1;
+        hits &= hits - 1u;
+        const unsigned long long k = __shfl_sync(FULL, key, hl);
+        const int below = __popc(__ballot_sync(FULL, held && mine < k));
+        at += lane == hl ? below : (k < key ? 1 : 0);
+        old_at += k < mine ? 1 : 0;
+    }
+    const int n = __popc(__ballot_sync(FULL, held)) + __popc(__ballot_sync(FULL, hit));
+    __syncwarp();
+    if (held && old_at < DST_CHUNK) place[old_at] = mine;
+    if (hit && at < DST_CHUNK) place[at] = key;
+    __syncwarp();
+    mine = lane < n && lane < DST_CHUNK ? place[lane] : ~0ull;
+}
+
 // The 16 nearest hits of ONE ray, found by a whole warp (same result as knearest()): the walk of a hull that is a single
-// ray, its quads tested exactly, one per lane. The k-buffer lives in registers, one key per lane (lanes 0..15, ascending);
-// an insertion is a ballot and a shuffle. All arguments are warp-uniform.
+// ray, its quads tested exactly, one per lane. The k-buffer lives in registers, one key per lane (lanes 0..15, ascending).
+// All arguments are warp-uniform.
 template <bool COUNT>
 __device__ __forceinline__ int knearest_warp(const BvhView& bvh, float ox, float oy, float oz, float dx, float dy, float dz, float kmax0, float absmax,
                                              WalkMem& m, unsigned long long& mykey, unsigned int* status, TraceCounters& tc) {
     constexpr unsigned int FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     mykey = ~0ull;
-    int n = 0;
     if (bvh.P <= 0) return 0;
     if (!(fabsf(ox) < INFINITY && fabsf(oy) < INFINITY && fabsf(oz) < INFINITY && fabsf(dx) < INFINITY && fabsf(dy) < INFINITY && fabsf(dz) < INFINITY)) return 0;
     make_beam(m, true, ox, oy, oz, dx, dy, dz, absmax);
@@ -631,24 +661,13 @@ __device__ __forceinline__ int knearest_warp(const BvhView& bvh, float ox, float
                 hit = true;
             }
         }
-        unsigned int hits = __ballot_sync(FULL, hit);
-        unsigned long long last = __shfl_sync(FULL, mykey, DST_CHUNK - 1);
-        while (hits) {
-            const int hl = 31 - __clz(hits);
-            hits &= ~(1u << hl);
-            const unsigned long long k = __shfl_sync(FULL, key, hl);
-            if (k >= last) continue;                                        // not among the 16 nearest
-            const int at = __popc(__ballot_sync(FULL, lane < DST_CHUNK && mykey < k));
-            const unsigned long long up = __shfl_up_sync(FULL, mykey, 1);
-            if (lane < DST_CHUNK) mykey = lane < at ? mykey : (lane == at ? k : up);
-            last = __shfl_sync(FULL, mykey, DST_CHUNK - 1);
-            if (n < DST_CHUNK) n++;
-        }
-        if (n == DST_CHUNK) krun = hitkey_t(last);
+        take_hits(hit, key, mykey, m.place);
+        const unsigned long long last = __shfl_sync(FULL, mykey, DST_CHUNK - 1);
+        if (last != ~0ull) krun = hitkey_t(last);
         return true;
     });
     if (!done && lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW);
-    return n;
+    return __popc(__ballot_sync(FULL, lane < DST_CHUNK && mykey != ~0ull));
 }
 
 // Second step of a gather: the batches k_enum gave up, in groups of DST_GROUP rays, one warp per group. The walk is again
@@ -694,22 +713,12 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
                 const float4 ra = srays[w][r][0], rb = srays[w][r][1];
                 float t; int tri;
                 const bool hit = valid && ray_quad(q.a, q.b, q.c, ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, t, tri);
-                unsigned int hits = __ballot_sync(FULL, hit);
                 float kr = rb.z;
-                if (hits) {
+                if (__any_sync(FULL, hit)) {
                     const unsigned long long key = make_key(t, 2u * q.gid + (unsigned int)tri);
-                    unsigned long long mine = skeys[w][r][lane & (DST_CHUNK - 1)];
-                    unsigned long long last = __shfl_sync(FULL, mine, DST_CHUNK - 1);
-                    while (hits) {
-                        const int hl = 31 - __clz(hits);
-                        hits &= ~(1u << hl);
-                        const unsigned long long k = __shfl_sync(FULL, key, hl);
-                        if (k >= last) continue;
-                        const int at = __popc(__ballot_sync(FULL, lane < DST_CHUNK && mine < k));
-                        const unsigned long long up = __shfl_up_sync(FULL, mine, 1);
-                        if (lane < DST_CHUNK) mine = lane < at ? mine : (lane == at ? k : up);
-                        last = __shfl_sync(FULL, mine, DST_CHUNK - 1);
-                    }
+                    unsigned long long mine = lane < DST_CHUNK ? skeys[w][r][lane] : ~0ull;
+                    take_hits(hit, key, mine, m.place);
+                    const unsigned long long last = __shfl_sync(FULL, mine, DST_CHUNK - 1);
                     if (lane < DST_CHUNK) skeys[w][r][lane] = mine;
                     if (last != ~0ull) { kr = hitkey_t(last); if (lane == 0) srays[w][r][1].z = kr; }
                 }
