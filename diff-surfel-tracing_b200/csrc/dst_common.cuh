@@ -146,7 +146,7 @@ int dst_knearest_impl(dst_handle* h, const float* ro, const float* rd, int64_t n
 int dst_prepare_cache(dst_handle* h, const dst_trace_inputs* in, cudaStream_t st);
 int dst_export_frames_impl(dst_handle* h, float* out, cudaStream_t st);
 int dst_ensure_wavefront(dst_handle* h, long long slots, size_t state_bytes);
-int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int grid_w, int tiled, long long slots, dst_handle::Log** log, cudaStream_t st);
+int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int grid_w, int tiled, long long slots, dst_handle::Log** log, int* append);
 void dst_drop_logs(dst_handle* h);
 int dst_wavefront_grid(const dst_handle* h, long long slots, int threads, int per_sm);
 

@@ -59,7 +59,6 @@ struct FwdParams {
     const float4* cache;
     unsigned int* status;
     int tiled, grid_h, grid_w;      // ray order: 8x4 tiles over a grid_h x grid_w pixel grid, or linear
-    long long slot0;                // first ray slot of the slice these lists belong to (see forward_common)
     int* bound_stats;               // {bounded searches issued, of them failed} in this call, or null: no predicted bounds
     float bound_factor;
     // wavefront scratch
@@ -95,11 +94,8 @@ static_assert(DST_MAX_CHUNKS < 65536, "chunk counter of the ray state");
 // Per-surfel shading record: tangent-frame rows from the quaternion exactly as
 // quat_to_rotmat_transpose does on an IEEE host (optix_tracer/auxiliary.h:403-429, with rsqrtf
 // taken as 1/sqrt), the frame origin T = R p (forward.cu:76), opacity and scales.
-__global__ void __launch_bounds__(256) k_prepare_cache(int P, const float* __restrict__ means, const float* __restrict__ scales,
-                                                       const float* __restrict__ rots, const float* __restrict__ opac,
-                                                       float4* __restrict__ cache) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= P) return;
+__device__ __forceinline__ void surfel_record(int g, const float* __restrict__ means, const float* __restrict__ scales,
+                                              const float* __restrict__ rots, const float* __restrict__ opac, float4* __restrict__ cache) {
     const float q0 = rots[4 * (size_t)g], q1 = rots[4 * (size_t)g + 1], q2 = rots[4 * (size_t)g + 2], q3 = rots[4 * (size_t)g + 3];
     const float s = xdiv(1.0f, xsqrt(xadd(xadd(xadd(xmul(q3, q3), xmul(q0, q0)), xmul(q1, q1)), xmul(q2, q2))));
     const float w = xmul(q0, s), x = xmul(q1, s), y = xmul(q2, s), z = xmul(q3, s);
@@ -120,6 +116,12 @@ __global__ void __launch_bounds__(256) k_prepare_cache(int P, const float* __res
     o[2] = make_float4(r2x, r2y, r2z, opac[g]);
     const float sx = scales[2 * (size_t)g], sy = scales[2 * (size_t)g + 1];
     o[3] = make_float4(sx, sy, xdiv(1.0f, sx), xdiv(1.0f, sy));
+}
+__global__ void __launch_bounds__(256) k_prepare_cache(int P, const float* __restrict__ means, const float* __restrict__ scales,
+                                                       const float* __restrict__ rots, const float* __restrict__ opac,
+                                                       float4* __restrict__ cache) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < P) surfel_record(g, means, scales, rots, opac, cache);
 }
 
 // a_weights[gidx] += w (optix_tracer/forward.cu:295), aggregated over the warp: neighbouring pixels composite the same surfels
@@ -382,12 +384,32 @@ __device__ __forceinline__ void flush_counters(unsigned long long* counters, con
     if (tc.contribs) atomicAdd(counters + 5, tc.contribs);
 }
 
-// round 0: list of all rays in tile order, initial state and first enumeration request
-__global__ void __launch_bounds__(256) k_fwd_init(const __grid_constant__ FwdParams p, long long slots) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= slots) return;
-    if (i == 0) { p.counts[0] = (int)slots; p.counts[DST_TAIL_CURSOR] = 0; }
-    const int slot = (int)(p.slot0 + i);
+// First kernel of a forward, everything that needs nothing before it: the surfel records and zeroed weights (the first `record_blocks` blocks), the
+// list of all rays in tile order with their initial states and requests, and the counters. As kernels and memsets of their own
+// these were five launches, as long as the rest of a small call.
+struct FwdBegin {
+    float4* cache; int record_blocks;
+    long long slots; int slices; long long slice_end[DST_MAX_SLICES];
+    int* log_count; int log_append;
+};
+__global__ void __launch_bounds__(256) k_fwd_begin(const __grid_constant__ FwdParams p, const __grid_constant__ FwdBegin f) {
+    const dst_trace_inputs& in = p.a.in;
+    if ((int)blockIdx.x < f.record_blocks) {
+        const int g = blockIdx.x * 256 + threadIdx.x;
+        if (g == 0 && f.log_count) { const int used = f.log_append ? f.log_count[0] : 0; f.log_count[0] = used; f.log_count[1] = used; }
+        if (g >= in.P) return;
+        surfel_record(g, in.means3D, in.scales, in.rotations, in.opacities, f.cache);
+        if (p.a.training && p.a.a_weights) p.a.a_weights[g] = 0.0f;
+        return;
+    }
+    const long long i = (long long)(blockIdx.x - f.record_blocks) * 256 + threadIdx.x;
+    if (i < f.slices) {
+        int* counts = p.counts + i * DST_COUNTS_STRIDE;
+        counts[0] = (int)(f.slice_end[i] - (i > 0 ? f.slice_end[i - 1] : 0));
+        counts[DST_TAIL_CURSOR] = 0;
+    }
+    if (i >= f.slots) return;
+    const int slot = (int)i;
     const int ray = slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0);
     p.list[0][i] = ray < 0 ? -1 : slot;
     if (ray < 0) return;
@@ -702,17 +724,22 @@ int dst_check_inputs(dst_handle* h, const dst_trace_inputs* in) {
     return DST_OK;
 }
 
-int dst_prepare_cache(dst_handle* h, const dst_trace_inputs* in, cudaStream_t st) {
+static int ensure_cache(dst_handle* h, const dst_trace_inputs* in) {
     if (in->P > h->cache_cap) {
         cudaFree(h->cache); h->cache = nullptr; h->cache_cap = 0;
         const int64_t cap = in->P + in->P / 8 + 1024;
         if (cudaMalloc(&h->cache, 64 * cap) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "surfel cache allocation failed"); }
         h->cache_cap = cap;
     }
-    k_prepare_cache<<<(in->P + 255) / 256, 256, 0, st>>>(in->P, in->means3D, in->scales, in->rotations, in->opacities, h->cache);
-    h->launches += 1;
     h->cache_serial = 0;
     h->cache_src[0] = in->means3D; h->cache_src[1] = in->scales; h->cache_src[2] = in->rotations; h->cache_src[3] = in->opacities; h->cache_P = in->P;
+    return DST_OK;
+}
+int dst_prepare_cache(dst_handle* h, const dst_trace_inputs* in, cudaStream_t st) {
+    const int rc = ensure_cache(h, in);
+    if (rc != DST_OK) return rc;
+    k_prepare_cache<<<(in->P + 255) / 256, 256, 0, st>>>(in->P, in->means3D, in->scales, in->rotations, in->opacities, h->cache);
+    h->launches += 1;
     DST_CUDA_TRY(h, cudaGetLastError());
     return DST_OK;
 }
@@ -777,7 +804,7 @@ void dst_drop_logs(dst_handle* h) {
 //
 // The log of the forward before is overwritten, unless its backward has not come yet and the caller wants logs kept: then this
 // one is appended, if the records both are expected to need fit.
-int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int grid_w, int tiled, long long slots, dst_handle::Log** log, cudaStream_t st) {
+int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int grid_w, int tiled, long long slots, dst_handle::Log** log, int* append) {
     const long long rays = (long long)in->H * in->W, sig = dst_call_signature(in);
     const int segs = in->max_trace_depth + 1;
     if (h->log_needed_host && h->log_needed_event && cudaEventQuery(h->log_needed_event) == cudaSuccess) {
@@ -805,8 +832,8 @@ int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int gri
             h->log_cap = want;
         }
         if (!h->log_count && cudaMalloc(&h->log_count, 8) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed"); }
-        DST_CUDA_TRY(h, cudaMemsetAsync(h->log_count, 0, 8, st));
-    } else DST_CUDA_TRY(h, cudaMemcpyAsync(h->log_count + 1, h->log_count, 4, cudaMemcpyDeviceToDevice, st));
+        *append = 0;
+    } else *append = 1;
     dst_handle::Log& l = h->logs[h->logs_used];
     if (slots * segs > l.index_cap) {
         cudaFree(l.head); cudaFree(l.num); cudaFree(l.ok); l.head = l.num = nullptr; l.ok = nullptr; l.index_cap = 0;
@@ -890,7 +917,6 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     FwdParams p;
     p.a = *a; p.bvh = dst_bvh_view(h); p.cache = h->cache; p.status = h->status;
     p.cam_on = cam != nullptr;
-    p.slot0 = 0;
     p.dist_on = h->distortion;
     if (cam) camera_constants(cam, &p.cam); else memset(&p.cam, 0, sizeof(p.cam));
     dst_slot_grid(h, &a->in, &p.grid_h, &p.grid_w);
@@ -898,10 +924,12 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     const long long slots = slots_of_grid(p.grid_h, p.grid_w, p.tiled != 0);
     rc = dst_ensure_wavefront(h, slots, sizeof(FwdState));
     if (rc != DST_OK) return rc;
-    rc = dst_prepare_cache(h, &a->in, st);
+    rc = ensure_cache(h, &a->in);
     if (rc != DST_OK) return rc;
     p.cache = h->cache;
-    if (a->training && a->a_weights) DST_CUDA_TRY(h, cudaMemsetAsync(a->a_weights, 0, 4 * (size_t)a->in.P, st));
+    FwdBegin begin;
+    begin.cache = h->cache; begin.record_blocks = (a->in.P + 255) / 256;
+    begin.slots = slots; begin.log_count = nullptr; begin.log_append = 0;
     p.state = static_cast<float4*>(h->wf_state); p.req = static_cast<float4*>(h->wf_req); p.kbuf = h->wf_kbuf; p.kcnt = h->wf_kcnt;
     p.list[0] = h->wf_list[0]; p.list[1] = h->wf_list[1]; p.counts = h->wf_counts;
     // contribution log for the backward (training calls only)
@@ -910,8 +938,9 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     h->log_serial = 0;
     if (a->training && h->log_enabled) {
         dst_handle::Log* log = nullptr;
-        rc = dst_begin_log(h, &a->in, p.grid_h, p.grid_w, p.tiled, slots, &log, st);
+        rc = dst_begin_log(h, &a->in, p.grid_h, p.grid_w, p.tiled, slots, &log, &begin.log_append);
         if (rc != DST_OK) return rc;
+        begin.log_count = h->log_count;
         p.log_keys = h->log_keys; p.log_next = h->log_next; p.log_count = h->log_count; p.log_head = log->head; p.log_num = log->num;
         p.log_ok = log->ok; p.log_cap = (int)h->log_cap;
         h->cache_serial = log->serial;
@@ -981,7 +1010,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
         else if (h->bound_stats) { p.bound_stats = h->bound_stats; p.bound_factor = DST_BOUND_FACTOR; DST_CUDA_TRY(h, cudaMemsetAsync(h->bound_stats, 0, 8, st)); }
     }
     memset(&p.lv, 0, sizeof(p.lv));
-    if (wave) {       // (a call without rounds uses two of the counters, which k_fwd_init sets)
+    if (wave) {       // (a call without rounds uses two of the counters, which k_fwd_begin sets)
         DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_counts, 0, 4 * (size_t)DST_COUNTS_STRIDE * DST_MAX_SLICES, st));
         rc = dst_live_lists(h, slots, &p.lv, st);
         if (rc != DST_OK) return rc;
@@ -998,7 +1027,6 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
             const long long s0 = b0 * DST_LIVE_BLOCK, s1 = g == nsl - 1 ? slots : b1 * DST_LIVE_BLOCK;
             FwdParams& q = ps[g];
             q = p;
-            q.slot0 = s0;
             q.list[0] = p.list[0] + s0; q.list[1] = p.list[1] + s0;
             q.counts = p.counts + (size_t)g * DST_COUNTS_STRIDE;
             q.lv.tmp = p.lv.tmp + s0; q.lv.wcnt = p.lv.wcnt + s0 / 32;
@@ -1007,11 +1035,13 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
             sst[g] = g == 0 ? st : h->slice_stream[g - 1];
         }
     }
+    begin.slices = nsl;
+    for (int g = 0; g < nsl; g++) begin.slice_end[g] = (g > 0 ? begin.slice_end[g - 1] : 0) + sslots[g];
+    k_fwd_begin<<<(unsigned int)(begin.record_blocks + (slots + 255) / 256), 256, 0, st>>>(p, begin);
     if (nsl > 1) {
         DST_CUDA_TRY(h, cudaEventRecord(h->slice_fork, st));
         for (int g = 1; g < nsl; g++) DST_CUDA_TRY(h, cudaStreamWaitEvent(sst[g], h->slice_fork, 0));
     }
-    for (int g = 0; g < nsl; g++) k_fwd_init<<<(unsigned int)((sslots[g] + 255) / 256), 256, 0, sst[g]>>>(ps[g], sslots[g]);
     for (int r = 0; r < p.rounds; r++) {
         for (int g = 0; g < nsl; g++) {
             const FwdParams& q = ps[g];
@@ -1046,7 +1076,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     }
     dst_prof_mark(h, 1, 1, st);
     DST_CUDA_TRY(h, cudaGetLastError());
-    h->launches += (long long)nsl * (2 + (p.lv.stable ? 5 : 4) * p.rounds);       // per slice: ray init, the rounds (three gather steps, composite, hand-over), tail
+    h->launches += 1 + (long long)nsl * (1 + (p.lv.stable ? 5 : 4) * p.rounds);       // per slice: the rounds (three gather steps, composite, hand-over), tail
     if (wave) {
         if (!h->rounds_host) {
             if (cudaMallocHost(&h->rounds_host, 4 * (size_t)DST_COUNTS_STRIDE * DST_MAX_SLICES) != cudaSuccess) { cudaGetLastError(); h->rounds_host = nullptr; }
@@ -1065,7 +1095,8 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
         cudaEventRecord(h->bound_event, st);
         h->bound_pending = true;
     }
-    if (p.log_keys) {
+    const bool log_known = h->log_known_needed > 0 && h->log_known_sig == dst_call_signature(&a->in);
+    if (p.log_keys && (!log_known || (h->serial_counter & 7) == 0)) {
         // how many records this call wanted, for sizing the log of the next one (no synchronisation here)
         if (!h->log_needed_host) {
             if (cudaMallocHost(&h->log_needed_host, 8) != cudaSuccess) { cudaGetLastError(); h->log_needed_host = nullptr; }
@@ -1146,7 +1177,7 @@ extern "C" int dst_forward_static(dst_handle* h, const dst_fwd_args* a, void* st
     FwdParams p;
     p.a = *a; p.bvh = dst_bvh_view(h); p.status = h->status; p.tiled = tiled; p.grid_h = a->in.H; p.grid_w = a->in.W;
     p.cam_on = 0; memset(&p.cam, 0, sizeof(p.cam));
-    p.slot0 = 0; p.bound_stats = nullptr; p.bound_factor = 0.0f;
+    p.bound_stats = nullptr; p.bound_factor = 0.0f;
     p.dist_on = h->distortion;
     p.cache = reinterpret_cast<const float4*>(base + ST_OFF_CACHE);
     p.state = reinterpret_cast<float4*>(base + ST_OFF_STATE);
@@ -1157,11 +1188,10 @@ extern "C" int dst_forward_static(dst_handle* h, const dst_fwd_args* a, void* st
     memset(&p.lv, 0, sizeof(p.lv));                              // no rounds, no list hand-over
     p.log_keys = nullptr; p.log_next = nullptr; p.log_count = nullptr; p.log_head = p.log_num = nullptr; p.log_ok = nullptr;
     p.log_cap = 0; p.log_slots = 0;
-    // the array keeps the previous call's contents: the round counters must start at zero, everything else is rewritten
-    if (a->training && a->a_weights) DST_CUDA_TRY(h, cudaMemsetAsync(a->a_weights, 0, 4 * (size_t)a->in.P, st));
-    k_prepare_cache<<<(a->in.P + 255) / 256, 256, 0, st>>>(a->in.P, a->in.means3D, a->in.scales, a->in.rotations, a->in.opacities,
-                                                             reinterpret_cast<float4*>(base + ST_OFF_CACHE));
-    k_fwd_init<<<(unsigned int)((slots + 255) / 256), 256, 0, st>>>(p, slots);
+    FwdBegin begin;
+    begin.cache = reinterpret_cast<float4*>(base + ST_OFF_CACHE); begin.record_blocks = (a->in.P + 255) / 256;
+    begin.slots = slots; begin.slices = 1; begin.slice_end[0] = slots; begin.log_count = nullptr; begin.log_append = 0;
+    k_fwd_begin<<<(unsigned int)(begin.record_blocks + (slots + 255) / 256), 256, 0, st>>>(p, begin);
     const bool diag = a->hit_log || a->hit_cnt || a->counters;
     if (slots <= DST_WARP_TAIL_MAX_RAYS) {
         const int g_wtail = dst_wavefront_grid(h, slots * 32, WTAIL_THREADS, 16);
@@ -1173,6 +1203,6 @@ extern "C" int dst_forward_static(dst_handle* h, const dst_fwd_args* a, void* st
         else k_fwd_tail<false, false><<<g_tail, TAIL_THREADS, 0, st>>>(p);
     }
     DST_CUDA_TRY(h, cudaGetLastError());
-    h->launches += 3;
+    h->launches += 2;
     return DST_OK;
 }

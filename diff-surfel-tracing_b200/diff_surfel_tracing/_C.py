@@ -111,6 +111,8 @@ def _on_device(state, t, name):
 
 def _cuda_f32(t, name, state=None):
     """Contiguous float32 CUDA storage of `t`, 16-byte aligned (the kernels use vector loads)."""
+    if state is not None and t.dtype is torch.float32 and t.is_contiguous() and t.get_device() == state.device and not t.data_ptr() & 15:
+        return t
     _on_device(state, t, name)
     if t.dtype != torch.float32:
         raise RuntimeError(f"{name} must be float32")
@@ -140,6 +142,8 @@ class OptiXStateWrapper:
         if rc != 0:
             raise RuntimeError(lib().dst_last_error(None).decode())
         self.handle = h
+        self._image_width = 0
+        self.next_camera = None
         self._keep = None
         self.last_forward_serial = 0
         self._logged_mid = None
@@ -172,7 +176,9 @@ class OptiXStateWrapper:
 
     def set_image_width(self, width):
         """Hint for (B, h*w, 3) ray batches of whole images: the image width (0: unknown). Scheduling only."""
-        _check(self, lib().dst_set_option(self.handle, 6, int(width)))
+        if width != self._image_width:
+            _check(self, lib().dst_set_option(self.handle, 6, int(width)))
+            self._image_width = width
 
     def set_single_kernel_refit(self, on):
         """build_from_surfels(rebuild=0): expand the quads inside the refit kernel (one launch) instead of before it."""
@@ -277,44 +283,46 @@ def build_acceleration_structure(state, vertices, triangles, rebuild):
 def _check_element_counts(P, t):
     """Element counts the kernels rely on (a wrong-sized tensor would be read out of bounds on the device).
     t: name -> tensor; empty tensors stand for absent optional inputs."""
-    want = dict(vertices=12 * P, background=3, opacities=P, scales=2 * P, rotations=4 * P)
-    if t["colors_precomp"].numel() != 0:
-        want["colors_precomp"] = 3 * P
-    if t["others_precomp"].numel() != 0:
-        want["others_precomp"] = 2 * P
-    for n, cnt in want.items():
-        if t[n].numel() != cnt:
-            raise RuntimeError(f"{n} has {t[n].numel()} elements, expected {cnt} for {P} surfels")
-    if t["shs"].numel() != 0 and (t["shs"].dim() != 3 or t["shs"].size(0) != P or t["shs"].size(2) != 3):
+    for n, cnt in (("vertices", 12 * P), ("background", 3), ("opacities", P), ("scales", 2 * P), ("rotations", 4 * P),
+                   ("colors_precomp", 3 * P), ("others_precomp", 2 * P)):
+        have = t[n].numel()
+        if have != cnt and (have != 0 or not n.endswith("_precomp")):
+            raise RuntimeError(f"{n} has {have} elements, expected {cnt} for {P} surfels")
+    shs = t["shs"]
+    if shs.numel() != 0 and (shs.dim() != 3 or shs.size(0) != P or shs.size(2) != 3):
         raise RuntimeError(f"shs must have dimensions ({P}, coefficients, 3)")
 
 
-def _inputs(state, start_from_first, ray_o, ray_d, vertices, background, means3D, shs, degree, colors_precomp,
+_NAMES = ("ray_o", "ray_d", "vertices", "background", "means3D", "shs", "colors_precomp", "others_precomp", "opacities", "scales", "rotations")
+
+
+def _inputs(state, i, start_from_first, ray_o, ray_d, vertices, background, means3D, shs, degree, colors_precomp,
             others_precomp, opacities, scales, scale_modifier, rotations, max_trace_depth, specular_threshold):
+    """Checks the tensors of a call and fills the argument block `i`; returns the tensors the kernels read, in the order of
+    _NAMES."""
     if means3D.dim() != 2 or means3D.size(1) != 3:
         raise RuntimeError("means3D must have dimensions (num_points, 3)")
     if ray_o.dim() != 3 or ray_o.size(2) != 3 or ray_o.shape != ray_d.shape:
         raise RuntimeError("ray_o and ray_d must have dimensions (H, W, 3)")
-    keep = {n: _cuda_f32(t, n, state) for n, t in (
-        ("ray_o", ray_o), ("ray_d", ray_d), ("vertices", vertices), ("background", background), ("means3D", means3D), ("shs", shs),
-        ("colors_precomp", colors_precomp), ("others_precomp", others_precomp), ("opacities", opacities), ("scales", scales),
-        ("rotations", rotations))}
-    if keep["scales"].numel() == 0 or keep["rotations"].numel() == 0:
+    keep = [_cuda_f32(t, n, state) for n, t in zip(_NAMES, (ray_o, ray_d, vertices, background, means3D, shs, colors_precomp, others_precomp,
+                                                           opacities, scales, rotations))]
+    H, W, _ = ray_o.shape
+    P = means3D.size(0)
+    if keep[9].numel() == 0 or keep[10].numel() == 0:
         raise RuntimeError("scales and rotations are required (a precomputed covariance is never read by the tracer)")
-    _check_element_counts(means3D.size(0), keep)
-    i = _TraceInputs()
-    i.H, i.W, i.P = ray_o.size(0), ray_o.size(1), means3D.size(0)
+    _check_element_counts(P, dict(zip(_NAMES, keep)))
+    i.H, i.W, i.P = H, W, P
     i.sh_degree = int(degree)
-    i.sh_coeffs = keep["shs"].size(1) if keep["shs"].numel() != 0 else 0
-    i.max_trace_depth = int(max_trace_depth)
-    i.mid_stride = MID_CHANNELS * max(2, int(max_trace_depth) + 1)
+    i.sh_coeffs = keep[5].size(1) if keep[5].numel() != 0 else 0
+    depth = int(max_trace_depth)
+    i.max_trace_depth = depth
+    i.mid_stride = MID_CHANNELS * max(2, depth + 1)
     i.start_from_first = int(bool(start_from_first))
     i.specular_threshold = float(specular_threshold)
     i.scale_modifier = float(scale_modifier)
-    for n in ("ray_o", "ray_d", "vertices", "background", "means3D", "shs", "colors_precomp", "others_precomp",
-              "opacities", "scales", "rotations"):
-        setattr(i, n, _ptr(keep[n]))
-    return i, keep
+    (i.ray_o, i.ray_d, i.vertices, i.background, i.means3D, i.shs, i.colors_precomp, i.others_precomp, i.opacities, i.scales,
+     i.rotations) = [t.data_ptr() or None for t in keep]
+    return keep
 
 
 def trace_surfels(state, training, start_from_first, ray_o, ray_d, vertices, background, means3D, shs, degree,
@@ -326,21 +334,22 @@ def trace_surfels(state, training, start_from_first, ray_o, ray_d, vertices, bac
     `mid_val` has 16 * max(2, max_trace_depth + 1) channels (the reference is compiled for one bounce
     and always returns 32). `_diag`, if a dict, receives per-ray hit logs and traversal counters.
     """
-    i, keep = _inputs(state, start_from_first, ray_o, ray_d, vertices, background, means3D, shs, degree, colors_precomp,
-                      others_precomp, opacities, scales, scale_modifier, rotations, max_trace_depth, specular_threshold)
+    a = _FwdArgs()
+    i = a.inp
+    keep = _inputs(state, i, start_from_first, ray_o, ray_d, vertices, background, means3D, shs, degree, colors_precomp,
+                   others_precomp, opacities, scales, scale_modifier, rotations, max_trace_depth, specular_threshold)
     H, W, P = i.H, i.W, i.P
     dev = means3D.device
     f32 = dict(dtype=torch.float32, device=dev)
-    out_rgb = torch.empty((H, W, NUM_CHANNELS), **f32)
-    out_dpt = torch.empty((H, W, 1), **f32)
-    out_acc = torch.empty((H, W, 1), **f32)
-    out_norm = torch.empty((H, W, 3), **f32)
-    out_dist = torch.empty((H, W, 3), **f32)
-    out_aux = torch.empty((H, W, AUX_CHANNELS), **f32)
-    mid_val = torch.empty((H, W, i.mid_stride), **f32)
-    a_weights = torch.empty((P, 1), **f32) if training else None
-    a = _FwdArgs()
-    a.inp = i
+    empty = torch.empty
+    out_rgb = empty((H, W, NUM_CHANNELS), **f32)
+    out_dpt = empty((H, W, 1), **f32)
+    out_acc = empty((H, W, 1), **f32)
+    out_norm = empty((H, W, 3), **f32)
+    out_dist = empty((H, W, 3), **f32)
+    out_aux = empty((H, W, AUX_CHANNELS), **f32)
+    mid_val = empty((H, W, i.mid_stride), **f32)
+    a_weights = empty((P, 1), **f32) if training else None
     a.training = int(bool(training))
     a.out_rgb, a.out_dpt, a.out_acc, a.out_norm = out_rgb.data_ptr(), out_dpt.data_ptr(), out_acc.data_ptr(), out_norm.data_ptr()
     a.out_dist, a.out_aux, a.mid_val = out_dist.data_ptr(), out_aux.data_ptr(), mid_val.data_ptr()
@@ -353,10 +362,10 @@ def trace_surfels(state, training, start_from_first, ray_o, ray_d, vertices, bac
             a.hit_cap, a.hit_log, a.hit_cnt = cap, _diag["hit_log"].data_ptr(), _diag["hit_cnt"].data_ptr()
         _diag["counters"] = torch.zeros((8,), dtype=torch.int64, device=dev)
         a.counters = _diag["counters"].data_ptr()
-    cam = getattr(state, "next_camera", None)
+    cam = state.next_camera
     state.next_camera = None
     if cam is not None:       # the rays are generated by the first kernel of the call, into ray_o / ray_d
-        if keep["ray_o"].data_ptr() != ray_o.data_ptr() or keep["ray_d"].data_ptr() != ray_d.data_ptr():
+        if keep[0] is not ray_o or keep[1] is not ray_d:
             raise RuntimeError("with a camera, ray_o and ray_d must be contiguous 16-byte aligned buffers")
         _check(state, lib().dst_forward_camera(state.handle, C.byref(a), C.byref(cam), _stream(state)))
     else:
@@ -389,8 +398,10 @@ def trace_surfels_backward(state, start_from_first, ray_o, ray_d, vertices, back
     if _forward_serial is None:
         key = (mid_val.data_ptr(), tuple(mid_val.shape))
         _forward_serial = state.last_forward_serial if getattr(state, "_logged_mid", None) == key else 0
-    i, keep = _inputs(state, start_from_first, ray_o, ray_d, vertices, background, means3D, shs, degree, colors_precomp,
-                      others_precomp, opacities, scales, scale_modifier, rotations, max_trace_depth, specular_threshold)
+    a = _BwdArgs()
+    i = a.inp
+    keep = _inputs(state, i, start_from_first, ray_o, ray_d, vertices, background, means3D, shs, degree, colors_precomp,
+                   others_precomp, opacities, scales, scale_modifier, rotations, max_trace_depth, specular_threshold)
     H, W, P, M = i.H, i.W, i.P, i.sh_coeffs
     if mid_val.size(-1) != i.mid_stride:
         raise RuntimeError(f"mid_val must have {i.mid_stride} channels for max_trace_depth={max_trace_depth}")
@@ -411,7 +422,7 @@ def trace_surfels_backward(state, start_from_first, ray_o, ray_d, vertices, back
     # The per-surfel gradients a caller can use live in ONE flat buffer (16-byte aligned views), so that a multi-GPU
     # run sums them with a single all-reduce. Gradients nobody receives (of the colour or auxiliary tensor that was
     # not given) are computed as the reference computes them, but kept out of that buffer.
-    has_colors, has_others = keep["colors_precomp"].numel() != 0, keep["others_precomp"].numel() != 0
+    has_colors, has_others = keep[6].numel() != 0, keep[7].numel() != 0
     sizes = [("rot", P * 4, True), ("means", P * 3, True), ("g3d", P * 3, True), ("shs", P * M * 3, True),
              ("colors", P * NUM_CHANNELS, has_colors), ("others", P * AUX_CHANNELS, has_others), ("opac", P, True), ("scales", P * 2, True)]
     offs, total, side_total = {}, 0, 0
@@ -425,23 +436,22 @@ def trace_surfels_backward(state, start_from_first, ray_o, ray_d, vertices, back
     bucket = torch.empty((total,), **f32)
     side = torch.empty((side_total,), **f32)
 
-    def view(name, n, shape):
+    def view(name, *shape):
         shared, off = offs[name]
-        return (bucket if shared else side)[off:off + n].view(shape)
+        stride = (shape[1], 1) if len(shape) == 2 else (shape[1] * shape[2], shape[2], 1)
+        return torch.as_strided(bucket if shared else side, shape, stride, off)
 
-    g_rot = view("rot", P * 4, (P, 4))
-    g_means = view("means", P * 3, (P, 3))
-    g_g3d = view("g3d", P * 3, (P, 3))
-    g_shs = view("shs", P * M * 3, (P, M, 3))
-    g_colors = view("colors", P * NUM_CHANNELS, (P, NUM_CHANNELS))
-    g_others = view("others", P * AUX_CHANNELS, (P, AUX_CHANNELS))
-    g_opac = view("opac", P, (P, 1))
-    g_scales = view("scales", P * 2, (P, 2))
+    g_rot = view("rot", P, 4)
+    g_means = view("means", P, 3)
+    g_g3d = view("g3d", P, 3)
+    g_shs = view("shs", P, M, 3)
+    g_colors = view("colors", P, NUM_CHANNELS)
+    g_others = view("others", P, AUX_CHANNELS)
+    g_opac = view("opac", P, 1)
+    g_scales = view("scales", P, 2)
     g_g3d_abs = torch.zeros((P, 3), **f32) if _zeros else None
     state.grad_bucket = bucket
     g_trans = torch.zeros((P, 9), **f32) if _zeros else None
-    a = _BwdArgs()
-    a.inp = i
     (a.out_rgb, a.out_dpt, a.out_acc, a.out_norm, a.out_dist, a.out_aux, a.mid_val) = [t.data_ptr() for t in sv]
     (a.dL_drgb, a.dL_ddpt, a.dL_dacc, a.dL_dnorm, a.dL_ddist, a.dL_daux) = [_ptr(t) for t in ug]
     a.dL_dray_o, a.dL_dray_d, a.dL_dmeans3D, a.dL_dgrads3D = g_ray_o.data_ptr(), g_ray_d.data_ptr(), g_means.data_ptr(), g_g3d.data_ptr()
@@ -497,14 +507,14 @@ def trace_surfels_static(state, training, start_from_first, ray_o, ray_d, vertic
     that cannot take an allocation's synchronisation; the output tensors here are still allocated
     by torch before the call.
     Concurrent calls on one device share the array and must be serialised."""
-    i, keep = _inputs(state, start_from_first, ray_o, ray_d, vertices, background, means3D, shs, degree, colors_precomp,
-                      others_precomp, opacities, scales, scale_modifier, rotations, max_trace_depth, specular_threshold)
+    a = _FwdArgs()
+    i = a.inp
+    keep = _inputs(state, i, start_from_first, ray_o, ray_d, vertices, background, means3D, shs, degree, colors_precomp,
+                   others_precomp, opacities, scales, scale_modifier, rotations, max_trace_depth, specular_threshold)
     H, W, P = i.H, i.W, i.P
     f32 = dict(dtype=torch.float32, device=means3D.device)
     outs = [torch.empty((H, W, c), **f32) for c in (NUM_CHANNELS, 1, 1, 3, 3, AUX_CHANNELS, i.mid_stride)]
     a_weights = torch.empty((P, 1), **f32) if training else None
-    a = _FwdArgs()
-    a.inp = i
     a.training = int(bool(training))
     (a.out_rgb, a.out_dpt, a.out_acc, a.out_norm, a.out_dist, a.out_aux, a.mid_val) = [t.data_ptr() for t in outs]
     a.a_weights = _ptr(a_weights)
@@ -558,6 +568,8 @@ def build_from_surfels(state, means3D, scales, rotations, rebuild, vertices=None
 def make_camera(K, R, T, correct_pix=True, z_depth=False):
     """dst_camera from 3x3 K, 3x3 R and 3 (or 3x1) T given as tensors, arrays or nested lists."""
     def flat(x, n):
+        if isinstance(x, torch.Tensor) and x.dtype is torch.float32 and not x.is_cuda and x.numel() == n:
+            return x.reshape(-1).tolist()
         if isinstance(x, torch.Tensor):
             x = x.detach().cpu()
         t = torch.as_tensor(x, dtype=torch.float32).reshape(-1)

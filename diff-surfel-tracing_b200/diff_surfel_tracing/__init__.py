@@ -25,34 +25,45 @@ def cpu_deep_copy_tuple(input_tuple):
 
 def trace_surfels(optix_context, training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D, shs,
                   colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings):
-    return _TraceSurfels.apply(optix_context, training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D, shs,
-                               colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings)
+    args = (optix_context, training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D, shs,
+            colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings)
+    if not torch.is_grad_enabled():       # rendering: nothing to record
+        return _forward(*args)[0]
+    return _TraceSurfels.apply(*args)
+
+
+def _forward(optix_context, training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D, shs,
+             colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, s):
+    """The forward call: what the tracer returns, and the tensors its backward needs."""
+    # image_width / image_height are unused by the reference's tracer; here they tell the kernels that a
+    # (B, h*w, 3) ray batch consists of whole images, so that they can be walked in pixel tiles (scheduling only)
+    iw, ih = int(s.image_width or 0), int(s.image_height or 0)
+    optix_context.set_image_width(iw if (iw > 0 and ih > 0 and ray_o.dim() == 3 and ray_o.shape[1] == iw * ih) else 0)
+    args = (optix_context, training, start_from_first, ray_o, ray_d, vertices, s.bg, means3D, shs, s.sh_degree,
+            colors_precomp, others_precomp, opacities, scales, s.scale_modifier, rotations, cov3Ds_precomp,
+            s.viewmatrix, s.projmatrix, s.campos, s.prefiltered, s.debug, s.max_trace_depth, s.specular_threshold)
+    if s.debug:
+        cpu_args = cpu_deep_copy_tuple(args[1:])
+        try:
+            out = _C.trace_surfels(*args)
+        except Exception as ex:
+            torch.save(cpu_args, "snapshot_fw.dump")
+            print("\nAn error occured in forward. Please forward snapshot_fw.dump for debugging.")
+            raise ex
+    else:
+        out = _C.trace_surfels(*args)
+    out_rgb, out_dpt, out_acc, out_norm, out_dist, out_aux, mid_val, a_weights = out
+    acc_wet = a_weights if a_weights is not None else means3D.new_zeros(means3D.shape[0])
+    return (out_rgb, out_dpt, out_acc, out_norm, out_dist[..., :1].clone(), out_aux, mid_val, acc_wet), out_dist
 
 
 class _TraceSurfels(torch.autograd.Function):
     @staticmethod
     def forward(ctx, optix_context, training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D, shs,
                 colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings):
-        s = tracer_settings
-        # image_width / image_height are unused by the reference's tracer; here they tell the kernels that a
-        # (B, h*w, 3) ray batch consists of whole images, so that they can be walked in pixel tiles (scheduling only)
-        iw, ih = int(s.image_width or 0), int(s.image_height or 0)
-        optix_context.set_image_width(iw if (iw > 0 and ih > 0 and ray_o.dim() == 3 and ray_o.shape[1] == iw * ih) else 0)
-        args = (optix_context, training, start_from_first, ray_o, ray_d, vertices, s.bg, means3D, shs, s.sh_degree,
-                colors_precomp, others_precomp, opacities, scales, s.scale_modifier, rotations, cov3Ds_precomp,
-                s.viewmatrix, s.projmatrix, s.campos, s.prefiltered, s.debug, s.max_trace_depth, s.specular_threshold)
-        if s.debug:
-            cpu_args = cpu_deep_copy_tuple(args[1:])
-            try:
-                out = _C.trace_surfels(*args)
-            except Exception as ex:
-                torch.save(cpu_args, "snapshot_fw.dump")
-                print("\nAn error occured in forward. Please forward snapshot_fw.dump for debugging.")
-                raise ex
-        else:
-            out = _C.trace_surfels(*args)
-        out_rgb, out_dpt, out_acc, out_norm, out_dist, out_aux, mid_val, a_weights = out
-
+        result, out_dist = _forward(optix_context, training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D, shs,
+                                    colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings)
+        out_rgb, out_dpt, out_acc, out_norm, _, out_aux, mid_val, _ = result
         ctx.set_materialize_grads(False)       # outputs the loss does not use: None instead of a tensor of zeros
         ctx.tracer_settings = tracer_settings
         ctx.optix_context = optix_context
@@ -60,8 +71,7 @@ class _TraceSurfels(torch.autograd.Function):
         ctx.forward_serial = getattr(optix_context, "last_forward_serial", 0)
         ctx.save_for_backward(ray_o, ray_d, vertices, means3D, shs, colors_precomp, others_precomp, opacities, scales,
                               rotations, cov3Ds_precomp, out_rgb, out_dpt, out_acc, out_norm, out_dist, out_aux, mid_val)
-        acc_wet = a_weights if a_weights is not None else torch.zeros_like(means3D[:, 0])
-        return out_rgb, out_dpt, out_acc, out_norm, out_dist[..., :1].clone(), out_aux, mid_val, acc_wet
+        return result
 
     @staticmethod
     def backward(ctx, grad_out_rgb, grad_out_dpt, grad_out_acc, grad_out_norm, grad_out_dist, grad_out_aux, grad_mid_val,
@@ -116,6 +126,7 @@ class SurfelTracer(nn.Module):
     def __init__(self) -> None:
         super().__init__()
         self.pkg_dir = _C._PKG
+        self._empty = None
         # name kept from the reference; the object owns the hierarchy and scratch memory of this GPU
         self.optix_context = _C.OptiXStateWrapper(self.pkg_dir)
         self.optix_context.set_kept_logs(4)       # several views traced before one backward: autograd names the forward it belongs to
@@ -146,15 +157,16 @@ class SurfelTracer(nn.Module):
                 ((scales is not None or rotations is not None) and cov3D_precomp is not None):
             raise Exception('Please provide exactly one of either scale/rotation pair or precomputed 3D covariance!')
 
-        dev = means3D.device
-        empty = lambda: torch.empty((0,), dtype=torch.float32, device=dev)
-        if shs is None: shs = empty()
-        if colors_precomp is None: colors_precomp = empty()
-        if others_precomp is None: others_precomp = empty()
-        if scales is None: scales = empty()
-        if rotations is None: rotations = empty()
-        if cov3D_precomp is None: cov3D_precomp = empty()
-        if vertices is None: vertices = empty()
+        empty = self._empty       # stands for every input that is not given
+        if empty is None or empty.device != means3D.device:
+            empty = self._empty = torch.empty((0,), dtype=torch.float32, device=means3D.device)
+        if shs is None: shs = empty
+        if colors_precomp is None: colors_precomp = empty
+        if others_precomp is None: others_precomp = empty
+        if scales is None: scales = empty
+        if rotations is None: rotations = empty
+        if cov3D_precomp is None: cov3D_precomp = empty
+        if vertices is None: vertices = empty
 
         return trace_surfels(self.optix_context, self.training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D,
                              shs, colors_precomp, others_precomp, opacities, scales, rotations, cov3D_precomp, tracer_settings)
