@@ -338,7 +338,7 @@ __device__ __forceinline__ bool bwd_init_state(const BwdParams& p, int ray, BwdS
 }
 
 // what the hits of one ray segment have in common
-struct BwdSegment { bool use_sh, has_aux, sh_aligned, dist_on; int ncoef; float tot_acc, t_dist, dist_mu, dist_V; };
+struct BwdSegment { bool use_sh, has_aux, sh_aligned, sh_wide, dist_on; int ncoef; float tot_acc, t_dist, dist_mu, dist_V; };
 
 // Called by the lanes with `in` at the start of a chunk / segment; writes the lane's SH basis.
 template <bool DIST>
@@ -349,6 +349,7 @@ __device__ __forceinline__ BwdSegment bwd_segment(const BwdParams& p, bool in_se
     x.has_aux = in.others_precomp != nullptr;
     x.ncoef = (in.sh_degree + 1) * (in.sh_degree + 1);
     x.sh_aligned = (in.sh_coeffs & 3) == 0 && ((reinterpret_cast<uintptr_t>(in.shs) & 15) == 0);
+    x.sh_wide = x.ncoef == 16 && in.sh_coeffs == 16 && ((reinterpret_cast<uintptr_t>(in.shs) & 31) == 0);
     x.dist_on = false; x.tot_acc = x.t_dist = x.dist_mu = x.dist_V = 0.f;
     if (x.use_sh && in_seg) {
         float sb[16];
@@ -402,25 +403,44 @@ __device__ __forceinline__ void bwd_hit(const BwdParams& p, BwdState& s, const B
     if (x.use_sh) {
         float c0 = 0.5f, c1 = 0.5f, c2 = 0.5f;
         const float* sh = in.shs + 3 * (size_t)gidx * in.sh_coeffs;
+        if (x.sh_wide) {       // degree 3, the usual layout: six 256-bit loads
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            if (4 * q < x.ncoef) {
-                float c[12];
-                if (x.sh_aligned) {
+            for (int i = 0; i < 2; i++) {
+                float c[24];
 #pragma unroll
-                    for (int l = 0; l < 3; l++) {
-                        const float4 v = __ldg(reinterpret_cast<const float4*>(sh) + 3 * q + l);
-                        c[4 * l] = v.x; c[4 * l + 1] = v.y; c[4 * l + 2] = v.z; c[4 * l + 3] = v.w;
-                    }
-                } else {
-#pragma unroll
-                    for (int l = 0; l < 12; l++) c[l] = 12 * q + l < 3 * x.ncoef ? __ldg(sh + 12 * q + l) : 0.0f;
+                for (int l = 0; l < 3; l++) {
+                    float4 q, r;
+                    ldg256(reinterpret_cast<const float4*>(sh) + 6 * i + 2 * l, q, r);
+                    c[8 * l] = q.x; c[8 * l + 1] = q.y; c[8 * l + 2] = q.z; c[8 * l + 3] = q.w;
+                    c[8 * l + 4] = r.x; c[8 * l + 5] = r.y; c[8 * l + 6] = r.z; c[8 * l + 7] = r.w;
                 }
 #pragma unroll
-                for (int l = 0; l < 4; l++) {
-                    if (4 * q + l < x.ncoef) {
-                        const float b = ws.basis[4 * q + l][lane];
-                        c0 = fmaf(b, c[3 * l], c0); c1 = fmaf(b, c[3 * l + 1], c1); c2 = fmaf(b, c[3 * l + 2], c2);
+                for (int l = 0; l < 8; l++) {
+                    const float b = ws.basis[8 * i + l][lane];
+                    c0 = fmaf(b, c[3 * l], c0); c1 = fmaf(b, c[3 * l + 1], c1); c2 = fmaf(b, c[3 * l + 2], c2);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (4 * q < x.ncoef) {
+                    float c[12];
+                    if (x.sh_aligned) {
+#pragma unroll
+                        for (int l = 0; l < 3; l++) {
+                            const float4 v = __ldg(reinterpret_cast<const float4*>(sh) + 3 * q + l);
+                            c[4 * l] = v.x; c[4 * l + 1] = v.y; c[4 * l + 2] = v.z; c[4 * l + 3] = v.w;
+                        }
+                    } else {
+#pragma unroll
+                        for (int l = 0; l < 12; l++) c[l] = 12 * q + l < 3 * x.ncoef ? __ldg(sh + 12 * q + l) : 0.0f;
+                    }
+#pragma unroll
+                    for (int l = 0; l < 4; l++) {
+                        if (4 * q + l < x.ncoef) {
+                            const float b = ws.basis[4 * q + l][lane];
+                            c0 = fmaf(b, c[3 * l], c0); c1 = fmaf(b, c[3 * l + 1], c1); c2 = fmaf(b, c[3 * l + 2], c2);
+                        }
                     }
                 }
             }
@@ -439,7 +459,7 @@ __device__ __forceinline__ void bwd_hit(const BwdParams& p, BwdState& s, const B
         const float2 ax = __ldg(reinterpret_cast<const float2*>(in.others_precomp) + gidx);
         F += s.t_aux0 * ax.x + s.t_aux1 * ax.y;
     }
-    const float inv = 1.0f / (1.0f - alpha);
+    const float inv = __frcp_rn(1.0f - alpha);
     s.rem = fmaf(-w, F, s.rem);
     float dL_dalpha = T_prev * (F + s.t_acc) - s.rem * inv;
     float dist_dd = 0.f;       // gradient of the distortion with respect to this hit's depth
@@ -471,7 +491,7 @@ __device__ __forceinline__ void bwd_hit(const BwdParams& p, BwdState& s, const B
     const V3 e1 = pa - pb, e2 = pa - pc;
     const V3 nn = cross(e1, e2);
     const V3 cvec = (t0 ? pa : v1) - v3(s.sox, s.soy, s.soz);
-    const float iq = 1.0f / dot(nn, rd), depth = dot(nn, cvec) * iq;
+    const float iq = __frcp_rn(dot(nn, rd)), depth = dot(nn, cvec) * iq;
     const V3 h = cvec - depth * rd;
     const float E = dL_dd * iq;
     const V3 En = E * nn;
@@ -685,8 +705,8 @@ __global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_tail(const 
 // A warp composites its rays' contributions in step, entry by entry, and only the lanes whose ray is in the latest segment still
 // open in the warp (the backward visits a ray's segments last to first): neighbouring pixels then composite the same surfels in
 // the same pass, which is what send_rows() feeds on.
-template <bool DIAG, bool DIST>
-__global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_logged(const __grid_constant__ BwdParams p, long long slots, int per) {
+template <bool DIAG, bool DIST, int BLOCKS>
+__global__ void __launch_bounds__(BWD_THREADS, BLOCKS) k_bwd_logged(const __grid_constant__ BwdParams p, long long slots, int per) {
     constexpr unsigned int FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const long long i = ((long long)blockIdx.x * (BWD_THREADS / 32) + (threadIdx.x >> 5)) * per + lane;
@@ -778,13 +798,21 @@ static int backward_kernel_setup(dst_handle* h) {
     static bool done[64] = { false };
     if (h->device >= 0 && h->device < 64 && done[h->device]) return DST_OK;
     cudaError_t e = cudaSuccess;
-#define DST_SETUP(K) if (e == cudaSuccess) e = allow_stage_smem(K<false, false>); if (e == cudaSuccess) e = allow_stage_smem(K<false, true>); \
-                     if (e == cudaSuccess) e = allow_stage_smem(K<true, false>); if (e == cudaSuccess) e = allow_stage_smem(K<true, true>);
-    DST_SETUP(k_bwd_shade) DST_SETUP(k_bwd_tail) DST_SETUP(k_bwd_logged)
+#define DST_SETUP(...) if (e == cudaSuccess) e = allow_stage_smem(__VA_ARGS__);
+    DST_SETUP(k_bwd_shade<false, false>) DST_SETUP(k_bwd_shade<false, true>) DST_SETUP(k_bwd_shade<true, false>) DST_SETUP(k_bwd_shade<true, true>)
+    DST_SETUP(k_bwd_tail<false, false>) DST_SETUP(k_bwd_tail<false, true>) DST_SETUP(k_bwd_tail<true, false>) DST_SETUP(k_bwd_tail<true, true>)
+    DST_SETUP(k_bwd_logged<false, false, 4>) DST_SETUP(k_bwd_logged<false, true, 4>) DST_SETUP(k_bwd_logged<true, false, 4>) DST_SETUP(k_bwd_logged<true, true, 4>)
+    DST_SETUP(k_bwd_logged<false, false, 5>) DST_SETUP(k_bwd_logged<false, true, 5>) DST_SETUP(k_bwd_logged<true, false, 5>) DST_SETUP(k_bwd_logged<true, true, 5>)
 #undef DST_SETUP
     if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_CUDA, "raising the shared-memory limit of the backward kernels failed: %s", cudaGetErrorString(e)); }
     if (h->device >= 0 && h->device < 64) done[h->device] = true;
     return DST_OK;
+}
+
+template <int BLOCKS>
+static void launch_logged(bool diag, bool dist, unsigned int blocks, cudaStream_t st, const BwdParams& p, long long slots, int per) {
+    if (dist) { if (diag) k_bwd_logged<true, true, BLOCKS><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); else k_bwd_logged<false, true, BLOCKS><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); }
+    else { if (diag) k_bwd_logged<true, false, BLOCKS><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); else k_bwd_logged<false, false, BLOCKS><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); }
 }
 
 int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
@@ -863,8 +891,9 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
         while (per > 8 && slots / per * 2 <= (long long)h->sm_count * DST_BWD_BLOCKS * (BWD_THREADS / 32)) per >>= 1;
         const long long per_block = per * (BWD_THREADS / 32);
         const unsigned int blocks = (unsigned int)((slots + per_block - 1) / per_block);
-        if (dist) { if (diag) k_bwd_logged<true, true><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); else k_bwd_logged<false, true><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); }
-        else { if (diag) k_bwd_logged<true, false><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); else k_bwd_logged<false, false><<<blocks, BWD_THREADS, BWD_STAGE_BYTES, st>>>(p, slots, per); }
+        // 20 warps an SM at 96 registers where there is twice the work to fill them (a tenth faster there), 16 at 128 registers otherwise
+        if (slots / 32 >= 2ll * h->sm_count * 5 * (BWD_THREADS / 32)) launch_logged<5>(diag, dist, blocks, st, p, slots, per);
+        else launch_logged<4>(diag, dist, blocks, st, p, slots, per);
     } else {
         k_bwd_init<<<(unsigned int)((slots + 255) / 256), 256, 0, st>>>(p, slots);
     }
