@@ -413,6 +413,23 @@ __global__ void __launch_bounds__(REFIT_THREADS) k_refit(const float* __restrict
     }
 }
 
+// Four children per node for the warps' walk: the grandchildren, one thread each.
+__global__ void __launch_bounds__(256) k_widen(int n, const BvhNode* __restrict__ nodes, BvhChild* __restrict__ wide) {
+    const int i = (int)(((long long)blockIdx.x * 256 + threadIdx.x) >> 2), s = threadIdx.x & 3;
+    if (i >= n) return;
+    const float4* src = reinterpret_cast<const float4*>(nodes[i].child + (s >> 1));
+    float4 a = __ldg(src), b = __ldg(src + 1);
+    const int c = __float_as_int(b.z);
+    if (c >= 0) {
+        const float4* g = reinterpret_cast<const float4*>(nodes[c].child + (s & 1));
+        a = __ldg(g); b = __ldg(g + 1);
+    } else if (s & 1) {       // no second grandchild: an empty box
+        a = make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY); b = make_float4(INFINITY, -INFINITY, __int_as_float(~0), 0.0f);
+    }
+    float4* dst = reinterpret_cast<float4*>(wide + 4 * (size_t)i + s);
+    dst[0] = a; dst[1] = b;
+}
+
 // plane frames back in surfel order, for tests
 __global__ void __launch_bounds__(256) k_export_frames(int P, const float4* __restrict__ quads, float* __restrict__ out) {
     const int pos = blockIdx.x * blockDim.x + threadIdx.x;
@@ -426,16 +443,17 @@ __global__ void __launch_bounds__(256) k_export_frames(int P, const float4* __re
 int ensure_capacity(dst_handle* h, int64_t P) {
     if (P <= h->cap) return DST_OK;
     // grow-only arena; the old buffers are released first (a rebuild does not need them)
-    cudaFree(h->nodes); cudaFree(h->quads); cudaFree(h->leaf_parent); cudaFree(h->arrive);
+    cudaFree(h->nodes); cudaFree(h->wide); cudaFree(h->quads); cudaFree(h->leaf_parent); cudaFree(h->arrive);
     cudaFree(h->node_parent); h->node_parent = nullptr;
     cudaFree(h->keys); cudaFree(h->keys_alt); cudaFree(h->vals); cudaFree(h->vals_alt); cudaFree(h->block_hist);
-    h->nodes = nullptr; h->quads = nullptr; h->leaf_parent = nullptr; h->arrive = nullptr;
+    h->nodes = nullptr; h->wide = nullptr; h->quads = nullptr; h->leaf_parent = nullptr; h->arrive = nullptr;
     h->keys = h->keys_alt = nullptr; h->vals = h->vals_alt = nullptr; h->block_hist = nullptr;
     h->cap = 0; h->built = false;
     const int64_t cap = P + P / 8 + 1024;
     const int64_t nblocks = (cap + SORT_TILE - 1) / SORT_TILE;
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = cudaMalloc(&h->nodes, sizeof(BvhNode) * cap);
+    if (e == cudaSuccess) e = cudaMalloc(&h->wide, 4 * sizeof(BvhChild) * cap);
     if (e == cudaSuccess) e = cudaMalloc(&h->quads, 64 * cap);
     if (e == cudaSuccess) e = cudaMalloc(&h->leaf_parent, 4 * cap);
     if (e == cudaSuccess) e = cudaMalloc(&h->arrive, 4 * cap);
@@ -525,9 +543,11 @@ int dst_bvh_build_impl(dst_handle* h, const float* v, int64_t P, int rebuild, cu
         k_refit<true><<<grid, tpb, 0, st>>>(v, src, n, h->vals, h->nodes, h->leaf_parent, h->node_parent, h->arrive, h->quads, h->header);
     else
         k_refit<false><<<grid, tpb, 0, st>>>(v, src, n, h->vals, h->nodes, h->leaf_parent, h->node_parent, h->arrive, h->quads, h->header);
+    const int inner = n > 1 ? n - 1 : 1;
+    k_widen<<<(unsigned int)((4ll * inner + 255) / 256), 256, 0, st>>>(inner, h->nodes, h->wide);
     dst_prof_mark(h, 0, 1, st);
     DST_CUDA_TRY(h, cudaGetLastError());
-    h->launches += (rebuild ? 27 + (n > 1 ? 1 : 0) : 0) + (from_surfels && (rebuild || !h->single_kernel_refit) ? 1 : 0) + (n == 1 ? 1 : 0) + 1;
+    h->launches += 1 + (rebuild ? 27 + (n > 1 ? 1 : 0) : 0) + (from_surfels && (rebuild || !h->single_kernel_refit) ? 1 : 0) + (n == 1 ? 1 : 0) + 1;
     h->built = true;
     return DST_OK;
 }

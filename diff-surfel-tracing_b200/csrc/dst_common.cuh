@@ -9,6 +9,7 @@
 // Hierarchy layout in HBM
 //   nodes      (P-1) x 64 B : 32 bytes per child: box and link, one 256-bit load
 //                             per child box (the walk tests one child box per lane)
+//   wide       (P-1) x 128 B: per node its four grandchildren (a leaf child stands for itself), what the warps' walk reads
 //   quads      P x 64 B     : plane frame of each quad and its surfel id in LEAF ORDER (two 256-bit loads per test)
 // ---------------------------------------------------------------------------------------------
 struct __align__(32) BvhChild {
@@ -25,6 +26,7 @@ static_assert(sizeof(BvhNode) == 64, "node must be one 64-byte record");
 
 struct BvhView {
     const BvhNode* nodes;
+    const BvhChild* wide;   // 4 per node
     const float4* quads;    // 4 per quad: p0 n.x | n.yz wu.xy | wu.z wv | surfel id
     const float* header;
     int P;          // surfels = leaves
@@ -50,6 +52,7 @@ struct dst_handle {
     int64_t P;            // surfels of the current hierarchy
     int64_t cap;          // surfels the build buffers can hold
     BvhNode* nodes;
+    BvhChild* wide;
     float4* quads;
     int* leaf_parent;
     int* node_parent;             // -1 for the root

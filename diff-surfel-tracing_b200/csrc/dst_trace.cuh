@@ -21,9 +21,9 @@ __device__ __forceinline__ float hitkey_t(unsigned long long k) { return __uint_
 __device__ __forceinline__ void ldg256(const void* p, float4& lo, float4& hi) {
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w), "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w) : "l"(p));
 }
-__device__ __forceinline__ BvhChild load_child(const BvhView& bvh, int node, int k) {
+__device__ __forceinline__ BvhChild load_child(const BvhChild* p) {
     float4 a, b;
-    ldg256(bvh.nodes[node].child + k, a, b);
+    ldg256(p, a, b);
     BvhChild c;
     c.lox = a.x; c.loy = a.y; c.hix = a.z; c.hiy = a.w; c.loz = b.x; c.hiz = b.y; c.c = __float_as_int(b.z); c.pad = 0;
     return c;
@@ -108,7 +108,7 @@ __device__ __forceinline__ int knearest(const BvhView& bvh, float ox, float oy, 
     for (;;) {
         // "while-while": lanes walk internal nodes until each holds a leaf (or is done), then test leaves together
         while ((unsigned int)cur < (unsigned int)DONE) {
-            const BvhChild k0 = load_child(bvh, cur, 0), k1 = load_child(bvh, cur, 1);
+            const BvhChild k0 = load_child(bvh.nodes[cur].child), k1 = load_child(bvh.nodes[cur].child + 1);
             if (COUNT) tc.nodes++;
             const float n0x = px ? k0.lox : k0.hix, f0x = px ? k0.hix : k0.lox;
             const float n0y = py ? k0.loy : k0.hiy, f0y = py ? k0.hiy : k0.loy;
@@ -341,7 +341,9 @@ constexpr int ENUM_THREADS = 128;
 #define DST_GROUP_STEPS 192
 #endif
 #define DST_GROUP_MIN_BLOCKS 8
-#define DST_WALK_STACK 320                 // one step adds at most 16 entries; see the width rule in beam_walk()
+#ifndef DST_WALK_STACK
+#define DST_WALK_STACK 352                 // one step adds at most 24 entries; see the width rule in beam_walk()
+#endif
 #define DST_WALK_QUADS 64
 #define DST_WALK_STEP_LIMIT (1 << 20)      // bound on the steps of a walk that cannot be given up (status flag instead of a hang)
 // Hull of a set of rays, component by component: origins oc +- orad, directions dc +- drad.
@@ -351,8 +353,8 @@ struct BeamQ { float oc[3], orad[3], dc[3], drad[3], dsum, dmax; };      // dsum
 // farther than kmaxb? The steps are those of ray_quad(): t = n.(p0 - o) / n.d, h = t d - (p0 - o), u = wu.h, v = wv.h,
 // accepted iff 0 <= t <= kmax and u, v in [0, 1]. Every interval is widened by margins orders of magnitude above the
 // rounding of either computation, so a quad some ray hits is never rejected. For neighbouring rays (close origins, directions a
-// degree apart) the intervals are narrow, and nearly every quad that no ray hits is rejected here by ONE lane.
-__device__ __forceinline__ bool hull_quad(const BeamQ& bm, const float4 qa, const float4 qb, const float4 qc, float kmaxb) {
+// degree apart) the intervals are narrow, and nearly every quad that no ray hits is rejected here by ONE lane. tl: nearest possible hit.
+__device__ __forceinline__ bool hull_quad(const BeamQ& bm, const float4 qa, const float4 qb, const float4 qc, float kmaxb, float& tl) {
     const float p0[3] = { qa.x, qa.y, qa.z }, nn[3] = { qa.w, qb.x, qb.y }, wu[3] = { qb.z, qb.w, qc.x }, wv[3] = { qc.y, qc.z, qc.w };
     float rc[3], bc = 0.f, br = 0.f, ac = 0.f, ar = 0.f, scale = 0.f;
 #pragma unroll
@@ -365,10 +367,12 @@ __device__ __forceinline__ bool hull_quad(const BeamQ& bm, const float4 qa, cons
     const float nmag = fabsf(nn[0]) + fabsf(nn[1]) + fabsf(nn[2]);
     br = fmaf(4e-6f * nmag, bm.dsum, br); ar = fmaf(12e-6f * nmag, scale, ar);
     const float bs = fabsf(bc), as = bc < 0.f ? -ac : ac;
+    tl = 0.f;
     if (!(bs - br > 1e-30f)) return true;        // some direction of the hull is (all but) parallel to the plane: no bound
     // quotients by approximate reciprocals (two units in the last place; the interval is widened by 1e-5 relative below)
     const float al = as - ar, ah = as + ar;
-    float tl = __fdividef(al, al >= 0.f ? bs + br : bs - br), th = __fdividef(ah, ah >= 0.f ? bs - br : bs + br);
+    tl = __fdividef(al, al >= 0.f ? bs + br : bs - br);
+    float th = __fdividef(ah, ah >= 0.f ? bs - br : bs + br);
     tl -= 1e-5f * fabsf(tl) + 1e-30f; th += 1e-5f * fabsf(th) + 1e-30f;
     if (!(th >= 0.f && tl <= kmaxb)) return false;
     tl = fmaxf(tl, 0.f); th = fminf(th, kmaxb);
@@ -412,7 +416,7 @@ struct WalkMem {
     BeamQ beam;
 };
 
-// Walks the hierarchy for the hull in m.beam / m.slab: a step takes up to 16 nodes from the top of the stack and tests their 32
+// Walks the hierarchy for the hull in m.beam / m.slab: a step takes up to 8 nodes from the top of the stack and tests their 32
 // child boxes, one per lane. Single quads whose box passes go to a queue; whenever it holds 32 of them (or no node is
 // left) leaf_step(valid, position) gets one quad per lane. krun (uniform) is the largest distance any ray still searches;
 // leaf_step lowers it, and returns false to give the walk up. Returns false when given up or after max_steps steps.
@@ -420,7 +424,7 @@ template <bool COUNT, class LeafStep>
 __device__ __forceinline__ bool beam_walk(const BvhView& bvh, WalkMem& m, float& krun, int max_steps, unsigned int* status, TraceCounters& tc, LeafStep leaf_step) {
     constexpr unsigned int FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const unsigned int below = (1u << lane) - 1u, pair_below = (1u << (lane & 30)) - 1u;
+    const unsigned int below = (1u << lane) - 1u, quad_below = (1u << (lane & 28)) - 1u;
     int sp = 1, nq = 0;
     if (lane == 0) m.stack[0] = 0ull;
     __syncwarp();
@@ -434,35 +438,35 @@ __device__ __forceinline__ bool beam_walk(const BvhView& bvh, WalkMem& m, float&
             if (!leaf_step(lane < take && __uint_as_float((unsigned int)(e >> 32)) <= krun, (int)(unsigned int)e)) return false;
             continue;
         }
-        // lanes 30/31 take the top entry, lanes 28/29 the next, ...: lane order is then the order in which surviving children
+        // lanes 28..31 take the top entry, lanes 24..27 the next, ...: lane order is then the order in which surviving children
         // go back onto the stack (farthest first). A nearly full stack is walked one node at a time (it then grows by at most
-        // one entry per level of the tree).
-        int width = 16;
-        if (sp > DST_WALK_STACK - 112) {
+        // three entries per two levels of the tree).
+        int width = 8;
+        if (sp > DST_WALK_STACK - 176) {
             width = 1;
-            if (sp > DST_WALK_STACK - 2) { if (lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW); return true; }
+            if (sp > DST_WALK_STACK - 4) { if (lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW); return true; }
         }
         const int take = sp < width ? sp : width;
-        const bool valid = 15 - (lane >> 1) < take;
-        const unsigned long long e = valid ? m.stack[sp - 16 + (lane >> 1)] : 0ull;
+        const bool valid = 7 - (lane >> 2) < take;
+        const unsigned long long e = valid ? m.stack[sp - 8 + (lane >> 2)] : 0ull;
         sp -= take;
         __syncwarp();
-        const BvhChild b = load_child(bvh, (int)(unsigned int)e, lane & 1);          // (lanes without an entry read the root)
-        if (COUNT && valid && (lane & 1) == 0) tc.nodes++;
+        const BvhChild b = load_child(bvh.wide + 4 * (size_t)(unsigned int)e + (lane & 3));          // (lanes without an entry read the root)
+        if (COUNT && valid && (lane & 3) == 0) tc.nodes++;
         const float2 il = fma2(b.lox, b.loy, m.slab.in_lo), ih = fma2(b.hix, b.hiy, m.slab.in_hi), iz = fma2(b.loz, b.hiz, m.slab.in_z);
         const float2 ol = fma2(b.lox, b.loy, m.slab.out_lo), oh = fma2(b.hix, b.hiy, m.slab.out_hi), oz = fma2(b.loz, b.hiz, m.slab.out_z);
         const float tn = max3(max3(il.x, il.y, ih.x), max3(ih.y, iz.x, iz.y), 0.0f);
         const float tf = min3(min3(ol.x, ol.y, oh.x), oh.y, fminf(oz.x, oz.y));
         const bool h = valid && __uint_as_float((unsigned int)(e >> 32)) <= krun && tn <= fminf(tf, krun);
-        // Of a pair the nearer child goes on top: entered first, on a tie (the rays start inside both boxes) left first.
-        const float ptn = __shfl_xor_sync(FULL, tn, 1), ptf = __shfl_xor_sync(FULL, tf, 1);
-        const bool on_top = tn < ptn || (tn == ptn && (tf < ptf || (tf == ptf && !(lane & 1))));
-        const unsigned int inner = __ballot_sync(FULL, h && b.c >= 0), leaves = __ballot_sync(FULL, h && b.c < 0);
+        const bool inside = h && b.c >= 0;
+        const unsigned int inner = __ballot_sync(FULL, inside), leaves = __ballot_sync(FULL, h && b.c < 0);
+        // Of the four children the nearest goes on top: entered first, or left first among those the rays start inside of. The key orders
+        // them so (its two low bits are the lane's, so that no two are equal; 0: does not go on the stack).
+        const unsigned int key = inside ? (((tn > 0.0f ? 0x80000000u | __float_as_uint(tn) : __float_as_uint(fmaxf(tf, 0.0f))) & ~3u) | (lane & 3)) : 0u;
+        const int farther = (__shfl_xor_sync(FULL, key, 1) > key) + (__shfl_xor_sync(FULL, key, 2) > key) + (__shfl_xor_sync(FULL, key, 3) > key);
         const unsigned long long entry = ((unsigned long long)__float_as_uint(tn) << 32) | (unsigned int)(b.c ^ (b.c >> 31));      // (~c for a quad)
-        if (h) {
-            if (b.c >= 0) m.stack[sp + __popc(inner & pair_below) + (on_top ? (int)((inner >> (lane ^ 1)) & 1u) : 0)] = entry;
-            else m.quads[nq + __popc(leaves & below)] = entry;
-        }
+        if (inside) m.stack[sp + __popc(inner & quad_below) + farther] = entry;
+        else if (h) m.quads[nq + __popc(leaves & below)] = entry;
         sp += __popc(inner);
         nq += __popc(leaves);
         __syncwarp();
@@ -558,17 +562,23 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
             float krun = redux_max(kmax);
             int cands = 0;
             done = beam_walk<COUNT>(bvh, m, krun, DST_BEAM_STEPS, status, tc, [&](bool valid, int pos) {
+                // the quads that pass, nearest first: hits then come almost in order, and nothing is left to do at the first quad
+                // that begins beyond every ray's 16th hit
+                float tl = 0.0f;
                 bool pass = false;
-                if (valid) { const Quad q = load_quad(bvh, pos); pass = hull_quad(m.beam, q.a, q.b, q.c, krun); }
-                unsigned int maybe = __ballot_sync(FULL, pass);
-                cands += __popc(maybe);
+                if (valid) { const Quad q = load_quad(bvh, pos); pass = hull_quad(m.beam, q.a, q.b, q.c, krun, tl); }
+                cands += __popc(__ballot_sync(FULL, pass));
                 if (cands > DST_BEAM_CANDS) return false;
+                unsigned int order = pass ? (__float_as_uint(tl) & ~31u) | lane : ~0u;
+                unsigned int first = __reduce_min_sync(FULL, order);
                 Quad next;       // (the next quad is on its way while this one is tested)
-                if (maybe) next = load_quad(bvh, __shfl_sync(FULL, pos, 31 - __clz(maybe)));
-                while (maybe) {
+                if (first != ~0u) next = load_quad(bvh, __shfl_sync(FULL, pos, first & 31));
+                while (first != ~0u) {
                     const Quad q = next;
-                    maybe &= ~(1u << (31 - __clz(maybe)));
-                    if (maybe) next = load_quad(bvh, __shfl_sync(FULL, pos, 31 - __clz(maybe)));
+                    if (!__any_sync(FULL, __uint_as_float(first & ~31u) <= kmax)) break;
+                    if (lane == (first & 31)) order = ~0u;
+                    first = __reduce_min_sync(FULL, order);
+                    if (first != ~0u) next = load_quad(bvh, __shfl_sync(FULL, pos, first & 31));
                     if (COUNT && lane == 0) tc.quads++;
                     float t; int tri;
                     if (!ray_quad(q.a, q.b, q.c, ox, oy, oz, dx, dy, dz, kmax, t, tri)) continue;
@@ -677,13 +687,13 @@ template <bool COUNT>
 __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_group(BvhView bvh, float4* req, const int* __restrict__ list,
                                                        const int* __restrict__ count_ptr, int* cursor,
                                                        unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
-                                                       unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count) {
+                                                       unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count, int direct_max) {
     constexpr unsigned int FULL = 0xffffffffu;
     __shared__ WalkMem walk_mem[ENUM_THREADS / 32];
     __shared__ unsigned long long skeys[ENUM_THREADS / 32][DST_GROUP][DST_CHUNK];
     __shared__ float4 srays[ENUM_THREADS / 32][DST_GROUP][2];
     const int total = *count_ptr / DST_GROUP;
-    if (total <= 0) return;
+    if (total * DST_GROUP <= direct_max) return;        // none, or few enough for a warp per ray (k_enum_ray takes them)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WalkMem& m = walk_mem[w];
     const float absmax = __ldg(bvh.header + 6);
@@ -750,14 +760,19 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
     if (COUNT && counters) { atomicAdd(counters + 2, tc.nodes); atomicAdd(counters + 3, tc.quads); }
 }
 
-// Last step of a gather: the rays whose batch was given up by k_enum, one warp per ray.
+// Last step of a gather: the rays whose group was given up, one warp per ray. When k_enum gave up no more rays than the GPU has room for
+// warps (direct_max) these are all of its rays: a group's walk tests eight rays one after the other, and a few of them made every
+// round of a small call or of its end half as long again.
 template <bool COUNT>
-__global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray(BvhView bvh, const float4* __restrict__ req, const int* __restrict__ list,
-                                                       const int* __restrict__ count_ptr, int* cursor,
+__global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray(BvhView bvh, const float4* __restrict__ req, const int* __restrict__ heavy,
+                                                       const int* __restrict__ heavy_count, const int* __restrict__ heavy2, const int* __restrict__ heavy2_count,
+                                                       int* cursor, int direct_max,
                                                        unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
                                                        unsigned int* status, unsigned long long* counters) {
     __shared__ WalkMem walk_mem[ENUM_THREADS / 32];
-    const int total = *count_ptr;
+    const int given_up = *heavy_count;
+    const int* list = given_up <= direct_max ? heavy : heavy2;
+    const int total = given_up <= direct_max ? given_up : *heavy2_count;
     if (total <= 0) return;
     const int lane = threadIdx.x & 31;
     WalkMem& m = walk_mem[threadIdx.x >> 5];
@@ -769,6 +784,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray
         i = __shfl_sync(0xffffffffu, i, 0);
         if (i >= total) break;
         const int slot = list[i];
+        if (slot < 0) continue;
         const float4 r0 = req[soa(slot, 0, 2)], r1 = req[soa(slot, 1, 2)];
         unsigned long long key;
         const int n = knearest_warp<COUNT>(bvh, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, absmax, m, key, status, tc);
@@ -781,18 +797,19 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray
 
 // the gather launches of a wavefront round (diag: with traversal counters). cnt: the round's entry in the set of round counters;
 // heavy, heavy2: lists of as many rays as the round has slots
-static inline void launch_gather(bool diag, int grid, cudaStream_t st, const BvhView& bvh, float4* req, const int* list,
+static inline void launch_gather(bool diag, int grid, int sm_count, cudaStream_t st, const BvhView& bvh, float4* req, const int* list,
                                  const int* count_ptr, int* cnt, int min_count, unsigned long long* kbuf, int* kcnt, unsigned int* status,
                                  unsigned long long* counters, int* heavy, int* heavy2) {
     constexpr int R = DST_WF_ROUNDS + 2;
+    const int direct_max = sm_count * DST_GROUP_MIN_BLOCKS * (ENUM_THREADS / 32), ray_grid = sm_count * DST_GROUP_MIN_BLOCKS;
     if (diag) {
         k_enum<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, counters, heavy, cnt + 2 * R);
-        k_enum_group<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, counters, heavy2, cnt + 4 * R);
-        k_enum_ray<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy2, cnt + 4 * R, cnt + 5 * R, kbuf, kcnt, status, counters);
+        k_enum_group<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, counters, heavy2, cnt + 4 * R, direct_max);
+        k_enum_ray<true><<<ray_grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, heavy2, cnt + 4 * R, cnt + 5 * R, direct_max, kbuf, kcnt, status, counters);
     } else {
         k_enum<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, nullptr, heavy, cnt + 2 * R);
-        k_enum_group<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, nullptr, heavy2, cnt + 4 * R);
-        k_enum_ray<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy2, cnt + 4 * R, cnt + 5 * R, kbuf, kcnt, status, nullptr);
+        k_enum_group<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, nullptr, heavy2, cnt + 4 * R, direct_max);
+        k_enum_ray<false><<<ray_grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, heavy2, cnt + 4 * R, cnt + 5 * R, direct_max, kbuf, kcnt, status, nullptr);
     }
 }
 
