@@ -1048,7 +1048,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
             const int g_enum = dst_wavefront_grid(h, sslots[g], ENUM_THREADS, DST_ENUM_GRID_PER_SM), g_shade = dst_wavefront_grid(h, sslots[g], SHADE_THREADS, DST_SHADE_GRID_PER_SM);
             const int g_compact = (int)((sslots[g] + DST_LIVE_BLOCK - 1) / DST_LIVE_BLOCK);
             dst_prof_mark(h, 3, 0, sst[g]);
-            launch_gather(diag, g_enum, h->sm_count, sst[g], q.bvh, q.req, q.list[r & 1], q.counts + r, q.counts + r, q.min_count, q.kbuf, q.kcnt,
+            launch_gather(diag, g_enum, h->sm_count, nsl, sst[g], q.bvh, q.req, q.list[r & 1], q.counts + r, q.counts + r, q.min_count, q.kbuf, q.kcnt,
                           q.status, a->counters, q.lv.tmp, q.list[(r + 1) & 1]);
             dst_prof_mark(h, 3, 1, sst[g]);
             if (diag) k_fwd_shade<true><<<g_shade, SHADE_THREADS, 0, sst[g]>>>(q, r);

@@ -303,7 +303,7 @@ __device__ __forceinline__ float& req_bound(float4* req, int slot) { return req[
 
 constexpr int ENUM_THREADS = 128;
 #ifndef DST_ENUM_MIN_BLOCKS
-#define DST_ENUM_MIN_BLOCKS 6         // resident blocks per SM the gather kernel is compiled for
+#define DST_ENUM_MIN_BLOCKS 8         // resident blocks per SM the gather kernel is compiled for
 #endif
 #define DST_WF_ROUNDS 48
 #define DST_TAIL_CURSOR (DST_COUNTS_STRIDE - 1)          // word of a set of round counters no round uses: next list entry of the tail kernel
@@ -323,27 +323,30 @@ constexpr int ENUM_THREADS = 128;
 //                 steps or DST_BEAM_CANDS such quads.
 //   k_enum_group  8 rays per warp (a 4x2 patch of the tile); every lane holds one quad and tests the 8 rays in turn. Given up past DST_GROUP_STEPS.
 //   k_enum_ray    one ray per warp (the hull is the ray), one quad per lane.
-// Gather time of one forward, one launch after another (3M-surfel 1080p one-bounce scene / 6M-surfel two-bounce scene at 4 x 540 x 960), against
-// a walk in which every lane tested its own ray against each node's two boxes: 40 -> 16 ms and 250 -> 106 ms; a primary round of
-// 2.07M rays 4.0 -> 1.2 ms. Limits: half of DST_BEAM_* costs the two-bounce scene 20 ms, twice as much costs the
-// scenes with silhouettes 5-10 % (the slowest batch of a round gets longer). Groups of 4 or 16: 10-15 % slower on the two-bounce scene.
-// Runs of 2 or 4 quads as leaves of the walk: 2-9 % slower than single quads.
+// Forward (3M-surfel 1080p one-bounce scene / 6M-surfel two-bounce scene at 4 x 540 x 960) against a walk in which every lane tested its own
+// ray against each node's two boxes: 43 -> 18.4 ms and 230 -> 88.7 ms (composite included). Groups of 4 or 16: 10-15 % slower on the two-bounce
+// scene. Runs of 2 or 4 quads as leaves of the walk: 2-9 % slower than single quads.
 // Blocks are persistent and take batches from a cursor; no block waits for another.
 // ---------------------------------------------------------------------------------------------
-#ifndef DST_BEAM_STEPS
+// What a walk may take before it is given up: steps, and quads that pass the hull test. A launch with a few times more work than it has
+// warps (all slices of a call counted) takes the larger limits, because giving up costs work; with less, the time is that of its longest walk,
+// and the smaller ones are the faster. Measured, one set of limits (160 / 300 / 192) against two: two-bounce scene 93.3 -> 88.7 ms, 400 x 400
+// object views 4.40 -> 3.63 ms, four LiDAR sweeps 2.44 -> 2.26 ms.
+#define DST_LOADED_BEAMS 2                 // times as many batches as warps of the launch
+#define DST_LOADED_GROUPS 3
 #define DST_BEAM_STEPS 160
-#endif
-#ifndef DST_BEAM_CANDS
-#define DST_BEAM_CANDS 300
-#endif
+#define DST_BEAM_STEPS_LOADED 240
+#define DST_BEAM_CANDS 200
+#define DST_BEAM_CANDS_LOADED 400
+#define DST_GROUP_STEPS 150
+#define DST_GROUP_STEPS_LOADED 260
 #define DST_GROUP 8
-#ifndef DST_GROUP_STEPS
-#define DST_GROUP_STEPS 192
-#endif
-#define DST_GROUP_MIN_BLOCKS 8
-#ifndef DST_WALK_STACK
-#define DST_WALK_STACK 352                 // one step adds at most 24 entries; see the width rule in beam_walk()
-#endif
+#define DST_GROUP_MIN_BLOCKS 10
+// Stack entries: one step adds at most 24. The stacks are most of a warp's shared memory, and what the walks wait for is memory latency, so they are
+// as small as they can be: 32 instead of 24 warps an SM in k_enum and 40 in the other steps take 8 % off the two-bounce scene. A walk that may be
+// given up is when its stack is full; one that has to end needs room for a depth-first descent.
+#define DST_BEAM_STACK 192
+#define DST_WALK_STACK 288
 #define DST_WALK_QUADS 64
 #define DST_WALK_STEP_LIMIT (1 << 20)      // bound on the steps of a walk that cannot be given up (status flag instead of a hang)
 // Hull of a set of rays, component by component: origins oc +- orad, directions dc +- drad.
@@ -408,65 +411,75 @@ __device__ __forceinline__ float2 fma2(float ax, float ay, float4 fo) {      // 
 // Each is one multiply-add of a box coordinate, taken two at a time (factors x, y and offsets z, w); an impossible direction has a huge factor.
 struct BeamSlab { float4 in_lo, in_hi, out_lo, out_hi, in_z, out_z; };       // x and y of lo, x and y of hi, z of lo and hi
 #define DST_KCNT_WIDE 0x100                // flag in a ray's hit count: answered by a later step than k_enum
-struct WalkMem {
-    unsigned long long stack[DST_WALK_STACK];        // subtrees: nearest possible t << 32 | link, nearest on top
-    unsigned long long quads[DST_WALK_QUADS];        // quads whose box the hull reaches: nearest possible t << 32 | leaf position
+struct WalkMemBase {
     unsigned long long place[DST_CHUNK];             // see take_hits()
     BeamSlab slab;
     BeamQ beam;
+    int quads[DST_WALK_QUADS];                       // leaf positions of quads whose box the hull reaches
 };
+template <int STACK>
+struct WalkStack : WalkMemBase {
+    int stack[STACK];                                // subtrees, nearest on top
+    unsigned short stack_t[STACK];                   // their nearest possible t, upper half (rounded towards 0: still a lower bound)
+};
+typedef WalkStack<DST_WALK_STACK> WalkMem;           // walks of one ray, which have to end
+typedef WalkStack<DST_BEAM_STACK> BeamMem;           // walks of a hull, which may be given up
 
 // Walks the hierarchy for the hull in m.beam / m.slab: a step takes up to 8 nodes from the top of the stack and tests their 32
 // child boxes, one per lane. Single quads whose box passes go to a queue; whenever it holds 32 of them (or no node is
 // left) leaf_step(valid, position) gets one quad per lane. krun (uniform) is the largest distance any ray still searches;
 // leaf_step lowers it, and returns false to give the walk up. Returns false when given up or after max_steps steps.
-template <bool COUNT, class LeafStep>
-__device__ __forceinline__ bool beam_walk(const BvhView& bvh, WalkMem& m, float& krun, int max_steps, unsigned int* status, TraceCounters& tc, LeafStep leaf_step) {
+template <bool COUNT, int STACK, class LeafStep>
+__device__ __forceinline__ bool beam_walk(const BvhView& bvh, WalkStack<STACK>& m, float& krun, int max_steps, unsigned int* status, TraceCounters& tc, LeafStep leaf_step) {
     constexpr unsigned int FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned int below = (1u << lane) - 1u, quad_below = (1u << (lane & 28)) - 1u;
     int sp = 1, nq = 0;
-    if (lane == 0) m.stack[0] = 0ull;
+    if (lane == 0) { m.stack[0] = 0; m.stack_t[0] = 0; }
     __syncwarp();
     for (int step = 0; step < max_steps; step++) {
         if (nq >= 32 || sp == 0) {
             if (nq == 0) return true;
             const int take = nq < 32 ? nq : 32;
             nq -= take;
-            const unsigned long long e = lane < take ? m.quads[nq + lane] : 0ull;
+            const int pos = lane < take ? m.quads[nq + lane] : 0;
             __syncwarp();
-            if (!leaf_step(lane < take && __uint_as_float((unsigned int)(e >> 32)) <= krun, (int)(unsigned int)e)) return false;
+            if (!leaf_step(lane < take, pos)) return false;
             continue;
         }
         // lanes 28..31 take the top entry, lanes 24..27 the next, ...: lane order is then the order in which surviving children
-        // go back onto the stack (farthest first). A nearly full stack is walked one node at a time (it then grows by at most
-        // three entries per two levels of the tree).
+        // go back onto the stack (farthest first). A walk that may be given up is when its stack is full; a nearly full one of a walk
+        // that has to end is walked one node at a time (it then grows by at most three entries per two levels of the tree).
         int width = 8;
-        if (sp > DST_WALK_STACK - 176) {
+        if (max_steps < DST_WALK_STEP_LIMIT) { if (sp > STACK - 24) return false; }
+        else if (sp > STACK - 176) {
             width = 1;
-            if (sp > DST_WALK_STACK - 4) { if (lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW); return true; }
+            if (sp > STACK - 4) { if (lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW); return true; }
         }
         const int take = sp < width ? sp : width;
         const bool valid = 7 - (lane >> 2) < take;
-        const unsigned long long e = valid ? m.stack[sp - 8 + (lane >> 2)] : 0ull;
+        const int node = valid ? m.stack[sp - 8 + (lane >> 2)] : 0;
+        const float node_t = valid ? __uint_as_float((unsigned int)m.stack_t[sp - 8 + (lane >> 2)] << 16) : INFINITY;
         sp -= take;
         __syncwarp();
-        const BvhChild b = load_child(bvh.wide + 4 * (size_t)(unsigned int)e + (lane & 3));          // (lanes without an entry read the root)
+        const BvhChild b = load_child(bvh.wide + 4 * (size_t)node + (lane & 3));          // (lanes without an entry read the root)
         if (COUNT && valid && (lane & 3) == 0) tc.nodes++;
         const float2 il = fma2(b.lox, b.loy, m.slab.in_lo), ih = fma2(b.hix, b.hiy, m.slab.in_hi), iz = fma2(b.loz, b.hiz, m.slab.in_z);
         const float2 ol = fma2(b.lox, b.loy, m.slab.out_lo), oh = fma2(b.hix, b.hiy, m.slab.out_hi), oz = fma2(b.loz, b.hiz, m.slab.out_z);
         const float tn = max3(max3(il.x, il.y, ih.x), max3(ih.y, iz.x, iz.y), 0.0f);
         const float tf = min3(min3(ol.x, ol.y, oh.x), oh.y, fminf(oz.x, oz.y));
-        const bool h = valid && __uint_as_float((unsigned int)(e >> 32)) <= krun && tn <= fminf(tf, krun);
+        const bool h = node_t <= krun && tn <= fminf(tf, krun);
         const bool inside = h && b.c >= 0;
         const unsigned int inner = __ballot_sync(FULL, inside), leaves = __ballot_sync(FULL, h && b.c < 0);
         // Of the four children the nearest goes on top: entered first, or left first among those the rays start inside of. The key orders
         // them so (its two low bits are the lane's, so that no two are equal; 0: does not go on the stack).
         const unsigned int key = inside ? (((tn > 0.0f ? 0x80000000u | __float_as_uint(tn) : __float_as_uint(fmaxf(tf, 0.0f))) & ~3u) | (lane & 3)) : 0u;
         const int farther = (__shfl_xor_sync(FULL, key, 1) > key) + (__shfl_xor_sync(FULL, key, 2) > key) + (__shfl_xor_sync(FULL, key, 3) > key);
-        const unsigned long long entry = ((unsigned long long)__float_as_uint(tn) << 32) | (unsigned int)(b.c ^ (b.c >> 31));      // (~c for a quad)
-        if (inside) m.stack[sp + __popc(inner & quad_below) + farther] = entry;
-        else if (h) m.quads[nq + __popc(leaves & below)] = entry;
+        if (inside) {
+            const int at = sp + __popc(inner & quad_below) + farther;
+            m.stack[at] = b.c;
+            m.stack_t[at] = (unsigned short)(__float_as_uint(tn) >> 16);
+        } else if (h) m.quads[nq + __popc(leaves & below)] = ~b.c;
         sp += __popc(inner);
         nq += __popc(leaves);
         __syncwarp();
@@ -478,7 +491,7 @@ __device__ __forceinline__ float redux_min(float v) { float r; asm("redux.sync.m
 __device__ __forceinline__ float redux_max(float v) { float r; asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v)); return r; }
 
 // hull of the rays of the lanes with `active` (at least one), into m.beam and m.slab
-__device__ __forceinline__ void make_beam(WalkMem& m, bool active, float ox, float oy, float oz, float dx, float dy, float dz, float absmax) {
+__device__ __forceinline__ void make_beam(WalkMemBase& m, bool active, float ox, float oy, float oz, float dx, float dy, float dz, float absmax) {
     const int lane = threadIdx.x & 31;
     const float o3[3] = { ox, oy, oz }, d3[3] = { dx, dy, dz };
     float olo[3], ohi[3], dlo[3], dhi[3], om = 0.0f;
@@ -522,17 +535,19 @@ template <bool COUNT>
 __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhView bvh, float4* req, const int* __restrict__ list,
                                                        const int* __restrict__ count_ptr, int* cursor, int min_count,
                                                        unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
-                                                       unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count) {
+                                                       unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count, int slices) {
     __shared__ unsigned long long kshared[DST_CHUNK * ENUM_THREADS];
-    __shared__ WalkMem walk_mem[ENUM_THREADS / 32];
+    __shared__ BeamMem walk_mem[ENUM_THREADS / 32];
     const int total = *count_ptr;
     if (total < min_count || bvh.P <= 0) return;
     constexpr int KS = ENUM_THREADS;
     constexpr unsigned int FULL = 0xffffffffu;
     unsigned long long* kb = kshared + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    WalkMem& m = walk_mem[threadIdx.x >> 5];
+    BeamMem& m = walk_mem[threadIdx.x >> 5];
     const float absmax = __ldg(bvh.header + 6);
+    const bool loaded = (long long)total * slices > DST_LOADED_BEAMS * (long long)(gridDim.x * ENUM_THREADS);
+    const int max_steps = loaded ? DST_BEAM_STEPS_LOADED : DST_BEAM_STEPS, max_cands = loaded ? DST_BEAM_CANDS_LOADED : DST_BEAM_CANDS;
     TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
     for (;;) {
         int base = 0;
@@ -561,14 +576,14 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
             make_beam(m, active, ox, oy, oz, dx, dy, dz, absmax);
             float krun = redux_max(kmax);
             int cands = 0;
-            done = beam_walk<COUNT>(bvh, m, krun, DST_BEAM_STEPS, status, tc, [&](bool valid, int pos) {
+            done = beam_walk<COUNT>(bvh, m, krun, max_steps, status, tc, [&](bool valid, int pos) {
                 // the quads that pass, nearest first: hits then come almost in order, and nothing is left to do at the first quad
                 // that begins beyond every ray's 16th hit
                 float tl = 0.0f;
                 bool pass = false;
                 if (valid) { const Quad q = load_quad(bvh, pos); pass = hull_quad(m.beam, q.a, q.b, q.c, krun, tl); }
                 cands += __popc(__ballot_sync(FULL, pass));
-                if (cands > DST_BEAM_CANDS) return false;
+                if (cands > max_cands) return false;
                 unsigned int order = pass ? (__float_as_uint(tl) & ~31u) | lane : ~0u;
                 unsigned int first = __reduce_min_sync(FULL, order);
                 Quad next;       // (the next quad is on its way while this one is tested)
@@ -687,15 +702,16 @@ template <bool COUNT>
 __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_group(BvhView bvh, float4* req, const int* __restrict__ list,
                                                        const int* __restrict__ count_ptr, int* cursor,
                                                        unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
-                                                       unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count, int direct_max) {
+                                                       unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count, int direct_max, int slices) {
     constexpr unsigned int FULL = 0xffffffffu;
-    __shared__ WalkMem walk_mem[ENUM_THREADS / 32];
+    __shared__ BeamMem walk_mem[ENUM_THREADS / 32];
     __shared__ unsigned long long skeys[ENUM_THREADS / 32][DST_GROUP][DST_CHUNK];
     __shared__ float4 srays[ENUM_THREADS / 32][DST_GROUP][2];
     const int total = *count_ptr / DST_GROUP;
     if (total * DST_GROUP <= direct_max) return;        // none, or few enough for a warp per ray (k_enum_ray takes them)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    WalkMem& m = walk_mem[w];
+    BeamMem& m = walk_mem[w];
+    const int max_steps = (long long)total * slices > DST_LOADED_GROUPS * (long long)(gridDim.x * (ENUM_THREADS / 32)) ? DST_GROUP_STEPS_LOADED : DST_GROUP_STEPS;
     const float absmax = __ldg(bvh.header + 6);
     TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
     for (;;) {
@@ -713,7 +729,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
         for (int k = lane; k < DST_GROUP * DST_CHUNK; k += 32) (&skeys[w][0][0])[k] = ~0ull;
         make_beam(m, slot >= 0, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, absmax);
         float krun = redux_max(bound0);
-        const bool done = beam_walk<COUNT>(bvh, m, krun, DST_GROUP_STEPS, status, tc, [&](bool valid, int pos) {
+        const bool done = beam_walk<COUNT>(bvh, m, krun, max_steps, status, tc, [&](bool valid, int pos) {
             Quad q;
             q.a = q.b = q.c = make_float4(0.f, 0.f, 0.f, 0.f); q.gid = 0u;
             if (valid) { q = load_quad(bvh, pos); if (COUNT) tc.quads++; }
@@ -796,19 +812,19 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray
 }
 
 // the gather launches of a wavefront round (diag: with traversal counters). cnt: the round's entry in the set of round counters;
-// heavy, heavy2: lists of as many rays as the round has slots
-static inline void launch_gather(bool diag, int grid, int sm_count, cudaStream_t st, const BvhView& bvh, float4* req, const int* list,
+// heavy, heavy2: lists of as many rays as the round has slots; slices: launches of other slices this one shares the GPU with, itself included
+static inline void launch_gather(bool diag, int grid, int sm_count, int slices, cudaStream_t st, const BvhView& bvh, float4* req, const int* list,
                                  const int* count_ptr, int* cnt, int min_count, unsigned long long* kbuf, int* kcnt, unsigned int* status,
                                  unsigned long long* counters, int* heavy, int* heavy2) {
     constexpr int R = DST_WF_ROUNDS + 2;
     const int direct_max = sm_count * DST_GROUP_MIN_BLOCKS * (ENUM_THREADS / 32), ray_grid = sm_count * DST_GROUP_MIN_BLOCKS;
     if (diag) {
-        k_enum<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, counters, heavy, cnt + 2 * R);
-        k_enum_group<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, counters, heavy2, cnt + 4 * R, direct_max);
+        k_enum<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, counters, heavy, cnt + 2 * R, slices);
+        k_enum_group<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, counters, heavy2, cnt + 4 * R, direct_max, slices);
         k_enum_ray<true><<<ray_grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, heavy2, cnt + 4 * R, cnt + 5 * R, direct_max, kbuf, kcnt, status, counters);
     } else {
-        k_enum<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, nullptr, heavy, cnt + 2 * R);
-        k_enum_group<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, nullptr, heavy2, cnt + 4 * R, direct_max);
+        k_enum<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, nullptr, heavy, cnt + 2 * R, slices);
+        k_enum_group<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, nullptr, heavy2, cnt + 4 * R, direct_max, slices);
         k_enum_ray<false><<<ray_grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, heavy2, cnt + 4 * R, cnt + 5 * R, direct_max, kbuf, kcnt, status, nullptr);
     }
 }
