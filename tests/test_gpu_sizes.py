@@ -1,0 +1,113 @@
+"""Sizes at which the kernels change their split of the work: tiles of the sort, blocks of the bottom-up pass, rays per warp of the
+logged backward, the number of forwards whose logs are kept, upstream gradients that are not given."""
+import numpy as np
+import pytest
+import torch
+
+import helpers as hp
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def C():
+    from diff_surfel_tracing import _C
+    assert torch.cuda.is_available()
+    _C.lib()
+    return _C
+
+
+def _state(C, wc, wave=None):
+    st = C.OptiXStateWrapper("")
+    if wave is not None:
+        st.set_wavefront_min_rays(0 if wave else 1 << 40)
+    C.build_acceleration_structure(st, wc["v"], wc["f"], 1)
+    return st
+
+
+@pytest.mark.parametrize("P", [1, 2, 3, 5, 255, 256, 257, 4095, 4096, 4097, 8193])
+def test_forward_at_block_and_tile_edges_of_the_build(C, oracle_mod, P):
+    """Build and refit, rounds and per-ray kernel, against the oracle bit for bit; a ragged grid."""
+    w = hp.workloads.make_workload(1, P=P, H=37, W=45)
+    w["scales"] = w["scales"] * 3.0
+    w["v"], w["f"] = hp.workloads.get_triangles(w["means3D"], w["scales"], w["rotations"])
+    wc = hp.to_cuda(w)
+    want = oracle_mod.Oracle(oracle_mod.Scene(w["v"]), impl="restatement", portable_exp=True).forward(w, training=True)
+    for wave in (False, True):
+        st = _state(C, wc, wave)
+        for rebuild in (1, 0):
+            C.build_acceleration_structure(st, wc["v"], wc["f"], rebuild)
+            got = hp.cuda_forward(C, st, wc)
+            torch.cuda.synchronize()
+            assert st.status() == 0
+            for k in ("rgb", "dpt", "acc", "norm", "mid"):
+                assert np.array_equal(got[k].cpu().numpy().reshape(want[k].shape).view(np.uint32), want[k].view(np.uint32)), (wave, rebuild, k)
+
+
+@pytest.mark.parametrize("H,W", [(17, 9), (64, 64), (129, 130), (190, 200), (460, 470)])
+def test_logged_backward_at_every_split(C, H, W):
+    """8, 16 and 32 rays per warp and the build for large calls: the gradients of the re-tracing backward."""
+    w = hp.workloads.make_workload(3, P=30_000, H=H, W=W)
+    wc = hp.to_cuda(w)
+    st = _state(C, wc)
+    f = hp.cuda_forward(C, st, wc)
+    up = {k: torch.randn(f[k].shape, device="cuda") for k in ("rgb", "dpt", "norm", "aux")}
+    logged = hp.cuda_backward(C, st, wc, f, up, serial=st.last_forward_serial)
+    traced = hp.cuda_backward(C, st, wc, f, up, serial=0)
+    torch.cuda.synchronize()
+    assert st.status() == 0
+    for k in hp.GRAD_KEYS:
+        a, b = logged[k].cpu().numpy(), traced[k].cpu().numpy()
+        m = np.isfinite(b)
+        assert hp.rel_l2(a[m], b[m]) < 1e-4, k
+
+
+@pytest.mark.parametrize("views", [2, 4, 5])
+def test_logs_of_several_forwards(C, views):
+    """Views traced one after the other, then their backwards: over the kept logs from the second step on, the first of more views than
+    logs are kept by re-tracing; the gradients of a state that keeps one log."""
+    w = hp.workloads.make_workload(3, P=20_000, H=48, W=64)
+    wc = hp.to_cuda(w)
+    ref, st = _state(C, wc), _state(C, wc)
+    st.set_kept_logs(4)
+    rays = [hp.workloads.pinhole_rays(48, 64, 50.0, (np.sin(a) * 4, -np.cos(a) * 4, 0.0)) for a in range(views)]
+    cs = [dict(wc, ray_o=o.cuda(), ray_d=d.cuda()) for o, d in rays]
+    for step in range(3):
+        fs = []
+        for c in cs:
+            f = hp.cuda_forward(C, st, c)
+            torch.cuda.synchronize()
+            fs.append((f, st.last_forward_serial))
+        walked = []
+        for c, (f, serial) in zip(cs, fs):
+            dg, up = {}, dict(rgb=torch.ones_like(f["rgb"]))
+            g = hp.cuda_backward(C, st, c, f, up, diag=dg, serial=serial)
+            r = hp.cuda_backward(C, ref, c, f, up, serial=0)
+            torch.cuda.synchronize()
+            walked.append(int(dg["counters"][2]) > 0)
+            for k in ("means3D", "shs", "opacities", "scales", "rotations", "ray_o"):
+                assert hp.rel_l2(g[k].cpu().numpy(), r[k].cpu().numpy()) < 1e-4, (step, k)
+        assert st.status() == 0
+    assert sum(walked) == (0 if views <= 4 else 4)        # a fifth forward finds the logs full and starts anew
+
+
+def test_missing_upstream_gradients_are_zeros_and_the_arena_stays_clean(C):
+    """None for an upstream gradient equals a tensor of zeros; a call's rows do not leak into the next one's, also across surfel counts."""
+    st = C.OptiXStateWrapper("")
+    e = torch.empty((0,), device="cuda")
+    for P in (9_000, 4_000, 9_000):
+        wc = hp.to_cuda(hp.workloads.make_workload(3, P=P, H=40, W=56))
+        C.build_acceleration_structure(st, wc["v"], wc["f"], 1)
+        f = hp.cuda_forward(C, st, wc)
+        full = hp.cuda_backward(C, st, wc, f, dict(dpt=torch.ones_like(f["dpt"])), serial=st.last_forward_serial)
+        part = C.trace_surfels_backward(st, True, wc["ray_o"], wc["ray_d"], wc["v"], wc["bg"], wc["means3D"], wc["shs"], wc["sh_degree"], e,
+                                        wc["others_precomp"], wc["opacities"], wc["scales"], 1.0, wc["rotations"], e, e, e, e, False, False,
+                                        wc["max_trace_depth"], wc["specular_threshold"], *(f[k] for k in ("rgb", "dpt", "acc", "norm", "dist", "aux", "mid")),
+                                        None, torch.ones_like(f["dpt"]), None, None, None, None, _forward_serial=st.last_forward_serial)
+        torch.cuda.synchronize()
+        assert st.status() == 0
+        for k, i in (("ray_o", 0), ("means3D", 2), ("shs", 5), ("opacities", 8), ("scales", 9), ("rotations", 10)):
+            a, b = part[i].cpu().numpy(), full[k].cpu().numpy()
+            assert np.array_equal(np.isfinite(a), np.isfinite(b)), k
+            m = np.isfinite(b)
+            assert hp.rel_l2(a[m], b[m]) < 1e-5, (P, k)
