@@ -386,7 +386,7 @@ __device__ __forceinline__ RowTarget row_target(const BwdParams& p) {
 // The reference differentiates each composited quantity on its own. All of them are sums of w f over the hits, so the gradient of a hit's alpha
 // needs only F = (upstream gradients) . (what the hit contributes) and the one running value s.rem = (upstream gradients) . (totals of the
 // segment, background and opacity included) - sum of w F so far: dL/dalpha = T (F + t_acc) - rem / (1 - alpha). The vertex terms are
-// written in the edges e1, e2 of the triangle at one corner: the gradients of the three corners add up to E n, and their
+// written in two edges of the triangle: the gradients of the three corners add up to E n, and their
 // moments with the corner signs (the gradients of the scaled tangents) to 6 E e x h -+ 3 E n. Both are the reference's
 // sums in exact arithmetic with a fraction of the operations.
 template <bool DIST>
@@ -486,17 +486,19 @@ __device__ __forceinline__ void bwd_hit(const BwdParams& p, BwdState& s, const B
     const float4* vq = reinterpret_cast<const float4*>(in.vertices + 12 * (size_t)gidx);
     const float4 va = __ldg(vq), vb = __ldg(vq + 1), vc = __ldg(vq + 2);
     const bool t0 = (pidx & 1) == 0;
+    // corners p1, p2, p3 of the triangle, its normal as the reference forms it (at a grazing angle the quotients by n . d magnify the rounding of n)
     const V3 v1 = v3(va.w, vb.x, vb.y), v2 = v3(vb.z, vb.w, vc.x);
-    const V3 pa = t0 ? v3(va.x, va.y, va.z) : v3(vc.y, vc.z, vc.w), pb = t0 ? v1 : v2, pc = t0 ? v2 : v1;
-    const V3 e1 = pa - pb, e2 = pa - pc;
-    const V3 nn = cross(e1, e2);
-    const V3 cvec = (t0 ? pa : v1) - v3(s.sox, s.soy, s.soz);
+    const V3 p1 = t0 ? v3(va.x, va.y, va.z) : v1, p2 = t0 ? v1 : v2, p3 = t0 ? v2 : v3(vc.y, vc.z, vc.w);
+    const V3 f1 = p2 - p1, f2 = p3 - p1;
+    const V3 nn = cross(f1, f2);
+    const V3 cvec = p1 - v3(s.sox, s.soy, s.soz);
     const float iq = __frcp_rn(dot(nn, rd)), depth = dot(nn, cvec) * iq;
     const V3 h = cvec - depth * rd;
     const float E = dL_dd * iq;
     const V3 En = E * nn;
-    const float E6 = t0 ? 6.0f * E : -6.0f * E, En3 = t0 ? 3.0f : -3.0f;
-    const V3 shx = E6 * cross(e1, h) - 3.0f * En, shy = E6 * cross(e2, h) + En3 * En;
+    const float E6 = 6.0f * E, E6s = t0 ? -E6 : E6, En3 = t0 ? 3.0f : -3.0f;
+    const V3 ex = t0 ? f1 : p3 - p2;
+    const V3 shx = E6s * cross(ex, h) - 3.0f * En, shy = E6s * cross(f2, h) + En3 * En;
     const V3 dmean = En - dxyz;
     s.dro_x -= dmean.x; s.dro_y -= dmean.y; s.dro_z -= dmean.z;
     if (!x.use_sh) {   // with SH the value is replaced below
