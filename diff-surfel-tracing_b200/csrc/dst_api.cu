@@ -104,7 +104,7 @@ int dst_destroy(dst_handle* h) {
     cudaFree(h->nodes); cudaFree(h->wide); cudaFree(h->quads); cudaFree(h->leaf_parent); cudaFree(h->arrive);
     cudaFree(h->node_parent);
     cudaFree(h->keys); cudaFree(h->keys_alt); cudaFree(h->vals); cudaFree(h->vals_alt); cudaFree(h->block_hist);
-    cudaFree(h->header); cudaFree(h->status); cudaFree(h->cache); cudaFree(h->arena); cudaFree(h->cam_dev);
+    cudaFree(h->header); cudaFree(h->status); cudaFree(h->cache); cudaFree(h->arena); cudaFree(h->wsum); cudaFree(h->cam_dev);
     if (h->log_needed_host) cudaFreeHost(h->log_needed_host);
     if (h->log_needed_event) cudaEventDestroy(h->log_needed_event);
     if (h->rounds_host) cudaFreeHost(h->rounds_host);

@@ -65,6 +65,7 @@ struct dst_handle {
     unsigned int* status;         // device status word
     float4* cache; int64_t cache_cap;
     unsigned long long cache_serial; const float* cache_src[4]; int64_t cache_P;      // training forward (serial) and tensors the records were built from
+    unsigned long long* wsum; int64_t wsum_cap; bool wsum_clean;      // fixed-point weight sums; clean: all zeros once the work enqueued so far has run
     float* arena;  int64_t arena_cap; bool arena_clean;       // clean: all zeros once the work enqueued so far has run
     void* cam_dev;      // camera constants of the last ray-generation call
     long long image_width;     // hint: rays given as (B, h*w, 3) are whole images of this width (0: unknown)

@@ -61,6 +61,7 @@ struct FwdParams {
     int tiled, grid_h, grid_w;      // ray order: 8x4 tiles over a grid_h x grid_w pixel grid, or linear
     int* bound_stats;               // {bounded searches issued, of them failed} in this call, or null: no predicted bounds
     float bound_factor;
+    unsigned long long* wsum; float wscale;      // weight sums in fixed point and their scale (see add_weight), or null: added to a_weights
     // wavefront scratch
     float4* state;
     float4* req;        // null: no gather kernels run
@@ -130,7 +131,14 @@ __global__ void __launch_bounds__(256) k_prepare_cache(int P, const float* __res
 // the same surfel takes or hands over the sum, which leaves one lane per patch of the tile (35 instructions; grouping all lanes with
 // the same surfel by match_any and a shuffle loop leaves a few atomics less and took 4 ms more on the 3M-surfel 1080p workload).
 // Called by all 32 lanes.
-__device__ __forceinline__ void add_weight(float* __restrict__ a_weights, int gidx, float w) {
+//
+// In large calls the sums are fixed-point (p.wsum, brought to a_weights by k_weights): hundreds of thousands of rays add to one surfel,
+// and a float sum of that size takes small weights only in part or not at all (1e-4 of the sums of 2M rays with two reflections).
+__device__ __forceinline__ void store_weight(const FwdParams& p, int gidx, float w) {
+    if (p.wsum) atomicAdd(p.wsum + gidx, (unsigned long long)__float2ull_rn(w * p.wscale));
+    else atomicAdd(p.a.a_weights + gidx, w);
+}
+__device__ __forceinline__ void add_weight(const FwdParams& p, int gidx, float w) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int step = 1; step < 32; step <<= 1) {
@@ -138,7 +146,7 @@ __device__ __forceinline__ void add_weight(float* __restrict__ a_weights, int gi
         const float pw = __shfl_xor_sync(0xffffffffu, w, step);
         if (pg == gidx) { w += pw; if (lane & step) gidx = -1; }
     }
-    if (gidx >= 0) atomicAdd(a_weights + gidx, w);
+    if (gidx >= 0) store_weight(p, gidx, w);
 }
 
 __device__ __forceinline__ void fwd_begin_segment(FwdState& s) {
@@ -357,7 +365,7 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, bool in_chunk, int
             s.hit_count++;
         }
         } while (false);
-        if (weights) add_weight(p.a.a_weights, wg, w);          // forward.cu:295
+        if (weights) add_weight(p, wg, w);          // forward.cu:295
     }
     if (!in_chunk) return false;
     return fwd_end_chunk(p, slot, s, stop || T_next < T_threshold, cnt, DIAG);
@@ -399,7 +407,7 @@ __global__ void __launch_bounds__(256) k_fwd_begin(const __grid_constant__ FwdPa
         if (g == 0 && f.log_count) { const int used = f.log_append ? f.log_count[0] : 0; f.log_count[0] = used; f.log_count[1] = used; }
         if (g >= in.P) return;
         surfel_record(g, in.means3D, in.scales, in.rotations, in.opacities, f.cache);
-        if (p.a.training && p.a.a_weights) p.a.a_weights[g] = 0.0f;
+        if (p.a.training && p.a.a_weights && !p.wsum) p.a.a_weights[g] = 0.0f;
         return;
     }
     const long long i = (long long)(blockIdx.x - f.record_blocks) * 256 + threadIdx.x;
@@ -425,6 +433,15 @@ __global__ void __launch_bounds__(256) k_fwd_begin(const __grid_constant__ FwdPa
         fwd_request(s, q);
         store_req(p.req, slot, q);
     }
+}
+
+// fixed-point weight sums -> the caller's tensor; clears them for the next call
+__global__ void __launch_bounds__(256) k_weights(int P, unsigned long long* __restrict__ wsum, double unit, float* __restrict__ a_weights) {
+    const int g = blockIdx.x * 256 + threadIdx.x;
+    if (g >= P) return;
+    const unsigned long long v = wsum[g];
+    a_weights[g] = (float)((double)v * unit);
+    if (v) wsum[g] = 0ull;
 }
 
 template <bool DIAG>
@@ -600,7 +617,7 @@ __device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int slot, War
         float2 ax = make_float2(0.f, 0.f);
         if (in.others_precomp) ax = __ldg(reinterpret_cast<const float2*>(in.others_precomp) + gidx);
         t[7] = xmul(w, ax.x); t[8] = xmul(w, ax.y);
-        if (p.a.training && p.a.a_weights) atomicAdd(p.a.a_weights + gidx, w);          // forward.cu:295
+        if (p.a.training && p.a.a_weights) store_weight(p, gidx, w);          // forward.cu:295
         if (DIAG && p.a.hit_log) {
             const int at = s.hit_count + __popc(contrib & ((1u << lane) - 1u));
             if (at < p.a.hit_cap) p.a.hit_log[(size_t)slot_ray(slot, p.grid_h, p.grid_w, p.tiled != 0) * p.a.hit_cap + at] = (int)(unsigned int)key;
@@ -1009,6 +1026,22 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
         if (h->bound_off_calls > 0) h->bound_off_calls--;
         else if (h->bound_stats) { p.bound_stats = h->bound_stats; p.bound_factor = DST_BOUND_FACTOR; DST_CUDA_TRY(h, cudaMemsetAsync(h->bound_stats, 0, 8, st)); }
     }
+    p.wsum = nullptr; p.wscale = 0.0f;
+    double wunit = 0.0;
+    if (wave && a->training && a->a_weights) {
+        if (a->in.P > h->wsum_cap) {
+            cudaFree(h->wsum); h->wsum = nullptr; h->wsum_cap = 0;
+            const int64_t cap = a->in.P + a->in.P / 8 + 1024;
+            if (cudaMalloc(&h->wsum, 8 * cap) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "weight sum allocation failed"); }
+            h->wsum_cap = cap; h->wsum_clean = false;
+        }
+        if (!h->wsum_clean) DST_CUDA_TRY(h, cudaMemsetAsync(h->wsum, 0, 8 * (size_t)h->wsum_cap, st));
+        h->wsum_clean = false;      // until k_weights has been enqueued
+        int bits = 62;              // the weights of a ray segment add up to less than 1
+        for (long long n = (long long)a->in.H * a->in.W * (a->in.max_trace_depth + 1); n > 0; n >>= 1) bits--;
+        if (bits > 40) bits = 40;
+        p.wsum = h->wsum; p.wscale = (float)(1ll << bits); wunit = 1.0 / (double)(1ll << bits);
+    }
     memset(&p.lv, 0, sizeof(p.lv));
     if (wave) {       // (a call without rounds uses two of the counters, which k_fwd_begin sets)
         DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_counts, 0, 4 * (size_t)DST_COUNTS_STRIDE * DST_MAX_SLICES, st));
@@ -1073,6 +1106,10 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     for (int g = 1; g < nsl; g++) {
         DST_CUDA_TRY(h, cudaEventRecord(h->slice_join[g - 1], sst[g]));
         DST_CUDA_TRY(h, cudaStreamWaitEvent(st, h->slice_join[g - 1], 0));
+    }
+    if (p.wsum) {
+        k_weights<<<(a->in.P + 255) / 256, 256, 0, st>>>(a->in.P, p.wsum, wunit, a->a_weights);
+        h->wsum_clean = true; h->launches += 1;
     }
     dst_prof_mark(h, 1, 1, st);
     DST_CUDA_TRY(h, cudaGetLastError());
@@ -1177,6 +1214,7 @@ extern "C" int dst_forward_static(dst_handle* h, const dst_fwd_args* a, void* st
     FwdParams p;
     p.a = *a; p.bvh = dst_bvh_view(h); p.status = h->status; p.tiled = tiled; p.grid_h = a->in.H; p.grid_w = a->in.W;
     p.cam_on = 0; memset(&p.cam, 0, sizeof(p.cam));
+    p.wsum = nullptr; p.wscale = 0.0f;
     p.bound_stats = nullptr; p.bound_factor = 0.0f;
     p.dist_on = h->distortion;
     p.cache = reinterpret_cast<const float4*>(base + ST_OFF_CACHE);
