@@ -29,9 +29,6 @@
 #ifndef DST_BOUND_FACTOR
 #define DST_BOUND_FACTOR 3.0f         // search bound of a continuing segment in units of the previous chunk's span (0: none)
 #endif
-#ifndef DST_BOUND_FAIL
-#define DST_BOUND_FAIL 2               // predicted bounds are dropped when one in this many fails
-#endif
 #define DST_BOUND_OFF_CALLS 64        // calls without predicted bounds after a call in which they failed too often
 #ifndef DST_SHADE_GRID_PER_SM
 #define DST_SHADE_GRID_PER_SM 4        // what fits an SM at once at 128 registers (measured: 8 is 2.5 % slower on the headline workload)
@@ -455,16 +452,16 @@ __global__ void __launch_bounds__(SHADE_THREADS, DST_SHADE_GRID_PER_SM) k_fwd_sh
     int* next_list = p.list[(round + 1) & 1];
     TraceCounters tc = { 0, 0, 0, 0, 0, 0 };
     const int n_pad = (n + 31) & ~31;
-    // Predicted bounds stay on while enough of them hold: a bounded search that comes back short (a segment that runs out of hits) is
-    // repeated without a bound in the later steps of the same gather.
+    // Predicted bounds stay on while they hold: where rays run out of hits (a sparse scene, the rim of an object) a bounded
+    // search that comes back short has to be repeated, and past one failure in twelve the repeats cost more than the bounds save.
     bool bound_on = false;
     if (p.bound_stats && p.bound_factor > 0.0f) {
         const int issued = __ldcg(p.bound_stats), fails = __ldcg(p.bound_stats + 1);
-        bound_on = issued < 4096 || (long long)fails * DST_BOUND_FAIL < issued;
+        bound_on = issued < 4096 || fails * 12 < issued;
     }
     for (int i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < n_pad; i += gridDim.x * SHADE_THREADS) {
         const int slot = i < n ? list[i] : -1;
-        bool alive = false, bounded = false, wide = false;
+        bool alive = false, bounded = false, failed = false, wide = false;
         int cls = 0, cnt = 0;
         FwdState s;
         const unsigned long long* kb = p.kbuf + soa(slot >= 0 ? slot : 0, 0, DST_CHUNK);
@@ -473,9 +470,17 @@ __global__ void __launch_bounds__(SHADE_THREADS, DST_SHADE_GRID_PER_SM) k_fwd_sh
             wide = (cnt & DST_KCNT_WIDE) != 0;
             cnt &= DST_KCNT_WIDE - 1;
             load_state(p.state, slot, s);
+            // Fewer than 16 hits within a predicted distance (below) say nothing about what lies beyond. Nothing is composited; the
+            // same request goes out again without a bound.
+            failed = cnt < DST_CHUNK && req_bound(p.req, slot) < DST_T_MAX;
         }
-        alive = fwd_shade<DIAG, 32>(p, slot >= 0, slot, s, kb, cnt, tc);
-        if (alive) {
+        alive = fwd_shade<DIAG, 32>(p, slot >= 0 && !failed, slot, s, kb, cnt, tc);
+        if (failed) {
+            req_bound(p.req, slot) = DST_T_MAX;
+            alive = true;
+            cls = s.bounce > 0;
+            if (DIAG && p.a.counters) atomicAdd(p.a.counters + 1, ~0ull);        // (the counter reports completed enumerations)
+        } else if (alive) {
             store_state(p.state, slot, s);
             EnumReq q;
             fwd_request(s, q);
@@ -492,8 +497,8 @@ __global__ void __launch_bounds__(SHADE_THREADS, DST_SHADE_GRID_PER_SM) k_fwd_sh
             cls = s.bounce > 0;
         }
         if (p.bound_stats) {
-            const unsigned int mb = __ballot_sync(0xffffffffu, bounded);
-            if (mb && (threadIdx.x & 31) == 0) atomicAdd(p.bound_stats, __popc(mb));
+            const unsigned int mb = __ballot_sync(0xffffffffu, bounded), mf = __ballot_sync(0xffffffffu, failed);
+            if ((threadIdx.x & 31) == 0) { if (mb) atomicAdd(p.bound_stats, __popc(mb)); if (mf) atomicAdd(p.bound_stats + 1, __popc(mf)); }
         }
         if (p.lv.stable) live_out(p.lv, round, i, alive, slot, cls);
         else append_alive(alive, slot, next_list, p.counts + round + 1);
@@ -1016,7 +1021,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
         }
         if (h->bound_pending && h->bound_event && cudaEventQuery(h->bound_event) == cudaSuccess) {
             h->bound_pending = false;
-            if (h->bound_host[0] >= 4096 && (long long)h->bound_host[1] * DST_BOUND_FAIL >= h->bound_host[0]) h->bound_off_calls = DST_BOUND_OFF_CALLS;
+            if (h->bound_host[0] >= 4096 && (long long)h->bound_host[1] * 12 >= h->bound_host[0]) h->bound_off_calls = DST_BOUND_OFF_CALLS;
         } else cudaGetLastError();
         if (h->bound_off_calls > 0) h->bound_off_calls--;
         else if (h->bound_stats) { p.bound_stats = h->bound_stats; p.bound_factor = DST_BOUND_FACTOR; DST_CUDA_TRY(h, cudaMemsetAsync(h->bound_stats, 0, 8, st)); }
@@ -1077,7 +1082,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
             const int g_compact = (int)((sslots[g] + DST_LIVE_BLOCK - 1) / DST_LIVE_BLOCK);
             dst_prof_mark(h, 3, 0, sst[g]);
             launch_gather(diag, g_enum, h->sm_count, nsl, sst[g], q.bvh, q.req, q.list[r & 1], q.counts + r, q.counts + r, q.min_count, q.kbuf, q.kcnt,
-                          q.status, a->counters, q.lv.tmp, q.list[(r + 1) & 1], p.bound_stats);
+                          q.status, a->counters, q.lv.tmp, q.list[(r + 1) & 1]);
             dst_prof_mark(h, 3, 1, sst[g]);
             if (diag) k_fwd_shade<true><<<g_shade, SHADE_THREADS, 0, sst[g]>>>(q, r);
             else k_fwd_shade<false><<<g_shade, SHADE_THREADS, 0, sst[g]>>>(q, r);

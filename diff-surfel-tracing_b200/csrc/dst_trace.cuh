@@ -535,7 +535,7 @@ template <bool COUNT>
 __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhView bvh, float4* req, const int* __restrict__ list,
                                                        const int* __restrict__ count_ptr, int* cursor, int min_count,
                                                        unsigned long long* __restrict__ kbuf, int* __restrict__ kcnt,
-                                                       unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count, int slices, int* bound_stats) {
+                                                       unsigned int* status, unsigned long long* counters, int* heavy, int* heavy_count, int slices) {
     __shared__ unsigned long long kshared[DST_CHUNK * ENUM_THREADS];
     __shared__ BeamMem walk_mem[ENUM_THREADS / 32];
     const int total = *count_ptr;
@@ -558,14 +558,14 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
         // the slow ones, so they start first and the cheap batches of primary rays fill the end of the round.
         const int idx = (((total + 31) >> 5) - 1 - (base >> 5)) * 32 + lane;
         const int slot = idx < total ? list[idx] : -1;
-        bool active = false, wide = false, bounded = false;
+        bool active = false, wide = false;
         int n = 0;
         float kmax = -1.0f, ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f;
         if (slot >= 0) {
             const EnumReq q = load_req(req, slot);
             ox = q.ox; oy = q.oy; oz = q.oz; dx = q.dx; dy = q.dy; dz = q.dz;
             active = fabsf(ox) < INFINITY && fabsf(oy) < INFINITY && fabsf(oz) < INFINITY && fabsf(dx) < INFINITY && fabsf(dy) < INFINITY && fabsf(dz) < INFINITY;
-            if (active) { kmax = q.kmax0; wide = q.step > 0.0f; bounded = kmax < DST_T_MAX; }
+            if (active) { kmax = q.kmax0; wide = q.step > 0.0f; }
             if (COUNT) tc.enums++;
         }
         const unsigned int am = __ballot_sync(FULL, active);
@@ -621,19 +621,6 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
                 heavy[__shfl_sync(FULL, at, 0) + lane] = active ? slot : -1;
                 if (active) { req_bound(req, slot) = kmax; continue; }
                 n = 0;
-            } else {
-                // Fewer than 16 hits within a predicted distance say nothing about what lies beyond: those rays search again, without a
-                // bound, in the steps that follow.
-                const bool again = bounded && n < DST_CHUNK;
-                const unsigned int m_again = __ballot_sync(FULL, again);
-                if (m_again) {
-                    const int count = __popc(m_again), padded = (count + DST_GROUP - 1) / DST_GROUP * DST_GROUP;      // whole groups
-                    int at = 0;
-                    if (lane == 0) { at = atomicAdd(heavy_count, padded); if (bound_stats) atomicAdd(bound_stats + 1, count); }
-                    at = __shfl_sync(FULL, at, 0);
-                    if (lane >= count && lane < padded) heavy[at + lane] = -1;
-                    if (again) { heavy[at + __popc(m_again & ((1u << lane) - 1u))] = slot; req_bound(req, slot) = DST_T_MAX; continue; }
-                }
             }
         }
         if (slot >= 0) {
@@ -768,8 +755,6 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
             return true;
         });
         __syncwarp();
-        // to the last step: all rays of a group that is given up, or those whose predicted bound held fewer than 16 hits
-        unsigned int left = done ? 0u : members;
         if (done) {
 #pragma unroll 1
             for (int r = 0; r < DST_GROUP; r++) {
@@ -777,16 +762,14 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
                 const int to = __shfl_sync(FULL, slot, r);
                 const unsigned long long mine = skeys[w][r][lane & (DST_CHUNK - 1)];
                 const int n = __popc(__ballot_sync(FULL, lane < DST_CHUNK && mine != ~0ull));
-                if (n < DST_CHUNK && __shfl_sync(FULL, bound0, r) < DST_T_MAX) { left |= 1u << r; continue; }
                 if (lane < n) kbuf[soa(to, lane, DST_CHUNK)] = mine;
                 if (lane == 0) kcnt[to] = n | DST_KCNT_WIDE;
             }
-        }
-        if (left) {
+        } else {
             int at = 0;
-            if (lane == 0) at = atomicAdd(heavy_count, __popc(left));
-            at = __shfl_sync(FULL, at, 0) + __popc(left & ((1u << lane) - 1u));
-            if ((left >> lane) & 1u) { heavy[at] = slot; req_bound(req, slot) = done ? DST_T_MAX : srays[w][lane][1].z; }
+            if (lane == 0) at = atomicAdd(heavy_count, __popc(members));
+            at = __shfl_sync(FULL, at, 0) + __popc(members & ((1u << lane) - 1u));
+            if (slot >= 0) { heavy[at] = slot; req_bound(req, slot) = srays[w][lane][1].z; }
         }
         __syncwarp();
     }
@@ -820,8 +803,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray
         if (slot < 0) continue;
         const float4 r0 = req[soa(slot, 0, 2)], r1 = req[soa(slot, 1, 2)];
         unsigned long long key;
-        int n = knearest_warp<COUNT>(bvh, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, absmax, m, key, status, tc);
-        if (n < DST_CHUNK && r1.z < DST_T_MAX) n = knearest_warp<COUNT>(bvh, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, DST_T_MAX, absmax, m, key, status, tc);
+        const int n = knearest_warp<COUNT>(bvh, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, absmax, m, key, status, tc);
         if (lane < n) kbuf[soa(slot, lane, DST_CHUNK)] = key;
         if (lane == 0) kcnt[slot] = n | DST_KCNT_WIDE;
         __syncwarp();
@@ -833,15 +815,15 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray
 // heavy, heavy2: lists of as many rays as the round has slots; slices: launches of other slices this one shares the GPU with, itself included
 static inline void launch_gather(bool diag, int grid, int sm_count, int slices, cudaStream_t st, const BvhView& bvh, float4* req, const int* list,
                                  const int* count_ptr, int* cnt, int min_count, unsigned long long* kbuf, int* kcnt, unsigned int* status,
-                                 unsigned long long* counters, int* heavy, int* heavy2, int* bound_stats) {
+                                 unsigned long long* counters, int* heavy, int* heavy2) {
     constexpr int R = DST_WF_ROUNDS + 2;
     const int direct_max = sm_count * DST_GROUP_MIN_BLOCKS * (ENUM_THREADS / 32), ray_grid = sm_count * DST_GROUP_MIN_BLOCKS;
     if (diag) {
-        k_enum<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, counters, heavy, cnt + 2 * R, slices, bound_stats);
+        k_enum<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, counters, heavy, cnt + 2 * R, slices);
         k_enum_group<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, counters, heavy2, cnt + 4 * R, direct_max, slices);
         k_enum_ray<true><<<ray_grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, heavy2, cnt + 4 * R, cnt + 5 * R, direct_max, kbuf, kcnt, status, counters);
     } else {
-        k_enum<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, nullptr, heavy, cnt + 2 * R, slices, bound_stats);
+        k_enum<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, nullptr, heavy, cnt + 2 * R, slices);
         k_enum_group<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, nullptr, heavy2, cnt + 4 * R, direct_max, slices);
         k_enum_ray<false><<<ray_grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, heavy2, cnt + 4 * R, cnt + 5 * R, direct_max, kbuf, kcnt, status, nullptr);
     }
