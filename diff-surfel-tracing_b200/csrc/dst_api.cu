@@ -101,18 +101,15 @@ int dst_create(int device, dst_handle** out) {
 int dst_destroy(dst_handle* h) {
     if (!h) return DST_OK;
     DeviceGuard g(h->device);
-    cudaFree(h->nodes); cudaFree(h->wide); cudaFree(h->quads); cudaFree(h->leaf_parent); cudaFree(h->arrive);
-    cudaFree(h->node_parent);
-    cudaFree(h->keys); cudaFree(h->keys_alt); cudaFree(h->vals); cudaFree(h->vals_alt); cudaFree(h->block_hist);
+    cudaFree(h->build_block);
     cudaFree(h->header); cudaFree(h->status); cudaFree(h->cache); cudaFree(h->arena); cudaFree(h->wsum); cudaFree(h->cam_dev);
     if (h->log_needed_host) cudaFreeHost(h->log_needed_host);
     if (h->log_needed_event) cudaEventDestroy(h->log_needed_event);
     if (h->rounds_host) cudaFreeHost(h->rounds_host);
     if (h->rounds_event) cudaEventDestroy(h->rounds_event);
-    cudaFree(h->log_keys); cudaFree(h->log_next); cudaFree(h->log_count);
-    for (int k = 0; k < DST_MAX_LOGS; k++) { cudaFree(h->logs[k].head); cudaFree(h->logs[k].num); cudaFree(h->logs[k].ok); }
-    cudaFree(h->wf_state); cudaFree(h->wf_req); cudaFree(h->wf_kbuf); cudaFree(h->wf_kcnt); cudaFree(h->wf_list[0]); cudaFree(h->wf_list[1]); cudaFree(h->wf_counts);
-    cudaFree(h->wf_tmp); cudaFree(h->wf_wcnt); cudaFree(h->wf_bcnt);
+    cudaFree(h->log_block); cudaFree(h->log_count);
+    for (int k = 0; k < DST_MAX_LOGS; k++) cudaFree(h->logs[k].index_block);
+    cudaFree(h->wf_block);
     cudaFree(h->bound_stats);
     if (h->bound_host) cudaFreeHost(h->bound_host);
     if (h->bound_event) cudaEventDestroy(h->bound_event);

@@ -443,26 +443,15 @@ __global__ void __launch_bounds__(256) k_export_frames(int P, const float4* __re
 int ensure_capacity(dst_handle* h, int64_t P) {
     if (P <= h->cap) return DST_OK;
     // grow-only arena; the old buffers are released first (a rebuild does not need them)
-    cudaFree(h->nodes); cudaFree(h->wide); cudaFree(h->quads); cudaFree(h->leaf_parent); cudaFree(h->arrive);
-    cudaFree(h->node_parent); h->node_parent = nullptr;
-    cudaFree(h->keys); cudaFree(h->keys_alt); cudaFree(h->vals); cudaFree(h->vals_alt); cudaFree(h->block_hist);
-    h->nodes = nullptr; h->wide = nullptr; h->quads = nullptr; h->leaf_parent = nullptr; h->arrive = nullptr;
-    h->keys = h->keys_alt = nullptr; h->vals = h->vals_alt = nullptr; h->block_hist = nullptr;
     h->cap = 0; h->built = false;
     const int64_t cap = P + P / 8 + 1024;
     const int64_t nblocks = (cap + SORT_TILE - 1) / SORT_TILE;
-    cudaError_t e = cudaSuccess;
-    if (e == cudaSuccess) e = cudaMalloc(&h->nodes, sizeof(BvhNode) * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->wide, 4 * sizeof(BvhChild) * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->quads, 64 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->leaf_parent, 4 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->arrive, 4 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->node_parent, 4 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->keys, 8 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->keys_alt, 8 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->vals, 4 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->vals_alt, 4 * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->block_hist, 4 * 256 * (nblocks + 1));       // + the 256 digit totals
+    const DstPart parts[] = {
+        {(void**)&h->nodes, sizeof(BvhNode) * cap}, {(void**)&h->wide, 4 * sizeof(BvhChild) * cap}, {(void**)&h->quads, 64 * (size_t)cap},
+        {(void**)&h->leaf_parent, 4 * (size_t)cap}, {(void**)&h->arrive, 4 * (size_t)cap}, {(void**)&h->node_parent, 4 * (size_t)cap},
+        {(void**)&h->keys, 8 * (size_t)cap}, {(void**)&h->keys_alt, 8 * (size_t)cap}, {(void**)&h->vals, 4 * (size_t)cap}, {(void**)&h->vals_alt, 4 * (size_t)cap},
+        {(void**)&h->block_hist, 4 * 256 * (size_t)(nblocks + 1)}};       // + the 256 digit totals
+    const cudaError_t e = dst_alloc_parts(&h->build_block, parts, sizeof(parts) / sizeof(parts[0]));
     if (e != cudaSuccess) {
         cudaGetLastError();
         return dst_set_error(h, DST_E_NOMEM, "device allocation for %lld surfels failed: %s", (long long)P, cudaGetErrorString(e));

@@ -51,6 +51,7 @@ struct dst_handle {
     bool built;
     int64_t P;            // surfels of the current hierarchy
     int64_t cap;          // surfels the build buffers can hold
+    void* build_block;            // one allocation for the buffers from here to block_hist
     BvhNode* nodes;
     BvhChild* wide;
     float4* quads;
@@ -71,7 +72,8 @@ struct dst_handle {
     long long image_width;     // hint: rays given as (B, h*w, 3) are whole images of this width (0: unknown)
     int single_kernel_refit;   // dst_build_from_surfels(rebuild = 0): expand the quads inside the refit kernel
     int sm_count;
-    // ray scratch of the wavefront trace (grow-only): state records, enumeration requests, hit buffers, live lists
+    // ray scratch of the wavefront trace (grow-only, in one allocation): state records, enumeration requests, hit buffers, live lists
+    void* wf_block;
     void* wf_state; size_t wf_state_bytes; void* wf_req; unsigned long long* wf_kbuf; int* wf_kcnt; int* wf_list[2]; int* wf_counts;
     int* wf_tmp; int* wf_wcnt; int* wf_bcnt;      // order-preserving list hand-over (LiveLists in dst_trace.cuh); wf_bcnt holds both counter sets
     long long wf_cap;
@@ -91,7 +93,7 @@ struct dst_handle {
     int* bound_stats; int* bound_host; cudaEvent_t bound_event; bool bound_pending; int bound_off_calls;
     // contribution log of training forwards (dst_begin_log), so that the backward re-composites it without walking the
     // hierarchy again
-    unsigned long long* log_keys; int* log_next; int* log_count;      // records of all logs; log_count: {records in use, of them before the last forward}
+    void* log_block; unsigned long long* log_keys; int* log_next; int* log_count;      // records (log_block) of all logs; log_count: {records in use, of them before the last forward}
     long long log_cap;            // records
     unsigned long long log_serial;      // serial of the last forward call if it left a log (0 = none)
     unsigned long long serial_counter;
@@ -102,7 +104,7 @@ struct dst_handle {
         bool consumed;                  // a backward has used it: the next forward may overwrite it
         int H, W, depth, grid_h, grid_w, tiled;
         long long slots;
-        int* head; int* num; unsigned char* ok; long long index_cap;       // per slot and segment: first record, entries; per slot: complete
+        void* index_block; int* head; int* num; unsigned char* ok; long long index_cap;       // per slot and segment: first record, entries; per slot: complete
     } logs[DST_MAX_LOGS];
     int logs_used, logs_keep, logs_wanted; long long log_use;       // logs_wanted: logs a backward has asked for at the same time
     int log_enabled;
@@ -122,6 +124,22 @@ struct dst_handle {
 #define DST_PROF_SLOTS 1024
 // records the start (which_end = 0) or stop (1) event of the current launch of `kind`; no-op unless profiling
 void dst_prof_mark(dst_handle* h, int kind, int which_end, cudaStream_t st);
+
+// Replaces *block by one allocation that holds n buffers, each on a 256-byte boundary, and sets their pointers (all null if it
+// fails). A new handle's first calls are host work, and that is mostly allocations: each takes as long as a small trace, so the
+// buffers that grow together share one (a new handle's first 64 x 64 render: 10 allocations fewer).
+struct DstPart { void** p; size_t bytes; };
+static inline cudaError_t dst_alloc_parts(void** block, const DstPart* parts, int n) {
+    cudaFree(*block);
+    *block = nullptr;
+    size_t total = 0;
+    for (int k = 0; k < n; k++) { *parts[k].p = nullptr; total += (parts[k].bytes + 255) / 256 * 256; }
+    const cudaError_t e = cudaMalloc(block, total);
+    if (e != cudaSuccess) { *block = nullptr; return e; }
+    char* at = (char*)*block;
+    for (int k = 0; k < n; k++) { *parts[k].p = at; at += (parts[k].bytes + 255) / 256 * 256; }
+    return cudaSuccess;
+}
 
 #define DST_CUDA_TRY(h, expr)                                                                    \
     do {                                                                                         \

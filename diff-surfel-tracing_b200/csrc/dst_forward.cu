@@ -767,21 +767,12 @@ int dst_ensure_wavefront(dst_handle* h, long long slots, size_t state_bytes) {
     if (slots <= h->wf_cap && state_bytes <= h->wf_state_bytes) return DST_OK;
     const long long cap = slots > h->wf_cap ? (slots + slots / 16 + 1024 + 31) / 32 * 32 : h->wf_cap;
     const size_t sb = state_bytes > h->wf_state_bytes ? state_bytes : h->wf_state_bytes;
-    cudaFree(h->wf_state); cudaFree(h->wf_req); cudaFree(h->wf_kbuf); cudaFree(h->wf_kcnt); cudaFree(h->wf_list[0]); cudaFree(h->wf_list[1]);
-    cudaFree(h->wf_counts); cudaFree(h->wf_tmp); cudaFree(h->wf_wcnt); cudaFree(h->wf_bcnt);
-    h->wf_state = nullptr; h->wf_req = nullptr; h->wf_kbuf = nullptr; h->wf_kcnt = nullptr; h->wf_list[0] = h->wf_list[1] = nullptr; h->wf_counts = nullptr;
-    h->wf_tmp = nullptr; h->wf_wcnt = nullptr; h->wf_bcnt = nullptr;
     h->wf_cap = 0; h->wf_state_bytes = 0;
-    cudaError_t e = cudaMalloc(&h->wf_state, sb * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->wf_req, 32 * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->wf_kbuf, 8 * DST_CHUNK * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->wf_kcnt, 4 * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->wf_list[0], 4 * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->wf_list[1], 4 * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc(&h->wf_counts, 4 * (size_t)DST_COUNTS_STRIDE * DST_MAX_SLICES);
-    if (e == cudaSuccess) e = cudaMalloc(&h->wf_tmp, 4 * (size_t)(cap + 32));
-    if (e == cudaSuccess) e = cudaMalloc(&h->wf_wcnt, 4 * (size_t)(cap / 32 + 2));
-    if (e == cudaSuccess) e = cudaMalloc(&h->wf_bcnt, 4 * 2 * (size_t)dst_live_blocks(cap));
+    const DstPart parts[] = {
+        {&h->wf_state, sb * (size_t)cap}, {&h->wf_req, 32 * (size_t)cap}, {(void**)&h->wf_kbuf, 8 * DST_CHUNK * (size_t)cap}, {(void**)&h->wf_kcnt, 4 * (size_t)cap},
+        {(void**)&h->wf_list[0], 4 * (size_t)cap}, {(void**)&h->wf_list[1], 4 * (size_t)cap}, {(void**)&h->wf_counts, 4 * (size_t)DST_COUNTS_STRIDE * DST_MAX_SLICES},
+        {(void**)&h->wf_tmp, 4 * (size_t)(cap + 32)}, {(void**)&h->wf_wcnt, 4 * (size_t)(cap / 32 + 2)}, {(void**)&h->wf_bcnt, 4 * 2 * (size_t)dst_live_blocks(cap)}};
+    const cudaError_t e = dst_alloc_parts(&h->wf_block, parts, sizeof(parts) / sizeof(parts[0]));
     if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "ray scratch allocation for %lld rays failed: %s", slots, cudaGetErrorString(e)); }
     h->wf_cap = cap; h->wf_state_bytes = sb;
     return DST_OK;
@@ -842,9 +833,9 @@ int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int gri
         if (h->log_max_records > 0 && want > h->log_max_records) want = h->log_max_records;
         want = (want + 31) / 32 * 32;
         if (want > h->log_cap || (h->log_max_records > 0 && h->log_cap > want)) {
-            cudaFree(h->log_keys); cudaFree(h->log_next); h->log_keys = nullptr; h->log_next = nullptr; h->log_cap = 0;
-            cudaError_t e = cudaMalloc(&h->log_keys, 8 * DST_CHUNK * (size_t)want);
-            if (e == cudaSuccess) e = cudaMalloc(&h->log_next, sizeof(int) * (size_t)want);
+            h->log_cap = 0;
+            const DstPart parts[] = {{(void**)&h->log_keys, 8 * DST_CHUNK * (size_t)want}, {(void**)&h->log_next, sizeof(int) * (size_t)want}};
+            const cudaError_t e = dst_alloc_parts(&h->log_block, parts, 2);
             if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed: %s", cudaGetErrorString(e)); }
             h->log_cap = want;
         }
@@ -853,11 +844,10 @@ int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int gri
     } else *append = 1;
     dst_handle::Log& l = h->logs[h->logs_used];
     if (slots * segs > l.index_cap) {
-        cudaFree(l.head); cudaFree(l.num); cudaFree(l.ok); l.head = l.num = nullptr; l.ok = nullptr; l.index_cap = 0;
+        l.index_cap = 0;
         const long long cap = slots * segs + slots / 16 + 1024;
-        cudaError_t e = cudaMalloc(&l.head, 4 * (size_t)cap);
-        if (e == cudaSuccess) e = cudaMalloc(&l.num, 4 * (size_t)cap);
-        if (e == cudaSuccess) e = cudaMalloc(&l.ok, (size_t)cap);
+        const DstPart parts[] = {{(void**)&l.head, 4 * (size_t)cap}, {(void**)&l.num, 4 * (size_t)cap}, {(void**)&l.ok, (size_t)cap}};
+        const cudaError_t e = dst_alloc_parts(&l.index_block, parts, 3);
         if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed: %s", cudaGetErrorString(e)); }
         l.index_cap = cap;
     }
