@@ -31,7 +31,13 @@
 #endif
 #define DST_BOUND_OFF_CALLS 64        // calls without predicted bounds after a call in which they failed too often
 #ifndef DST_SHADE_GRID_PER_SM
-#define DST_SHADE_GRID_PER_SM 4        // what fits an SM at once at 128 registers (measured: 8 is 2.5 % slower on the headline workload)
+#define DST_SHADE_GRID_PER_SM 4        // blocks an SM holds at once at 128 registers (measured: 8 is 2.5 % slower on the headline workload)
+#endif
+// Rays from which the composite kernel runs 5 blocks an SM at 96 registers (0 spilled) instead of 4 at 128. It waits for loads, so the fifth
+// block pays while its rounds are long: forward of 2M reflective rays 17.6 -> 16.8 ms, of 0.93M 15.8 -> 15.6. Where most rounds hold few rays
+// one warp's chain counts, and with 96 registers an SH row comes in two waits instead of one: 0.64M rays of an object 4.7 -> 4.9 ms.
+#ifndef DST_SHADE_WIDE_SLOTS
+#define DST_SHADE_WIDE_SLOTS (900ll << 10)
 #endif
 #include <string.h>
 
@@ -308,12 +314,17 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, bool in_chunk, int
     bool stop = !in_chunk;
     const bool weights = p.a.training && p.a.a_weights;
     const int n = __reduce_max_sync(0xffffffffu, in_chunk ? cnt : 0);
+    // What this takes is the chain of loads of each hit, its key, its record, its SH row, at 16 to 20 warps an SM. The key of the next hit is
+    // loaded a hit ahead (k_fwd_shade of 2M reflective rays: the whole forward 18.4 -> 17.6 ms; the next record as well needs 16 registers
+    // that are not there, 19.9 ms).
+    unsigned long long next_key = in_chunk && cnt > 0 ? kb[0] : 0;
     for (int i = 0; i < n; i++) {
+        const unsigned long long key = next_key;
+        if (i + 1 < cnt) next_key = kb[(i + 1) * KS];
         int wg = -1;
         float w = 0.f;
         do {
         if (stop || i >= cnt) break;
-        const unsigned long long key = kb[i * KS];
         const int pidx = (int)(unsigned int)key;
         const int gidx = pidx >> 1;
         if (gidx == s.last_gidx) break;                                // forward.cu:207
@@ -332,11 +343,11 @@ __device__ __forceinline__ bool fwd_shade(const FwdParams& p, bool in_chunk, int
         w = xmul(alpha, s.T_prev);
         if (p.log_keys) log_entry(p, slot, s, s.contributor - 1, s.dpt, (unsigned int)pidx);
         if (use_sh) {
-            float c[48];
-            load_sh_row(in.shs + 3 * (size_t)gidx * in.sh_coeffs, 3 * ncoef, sh_aligned, c);
-            s.C0 = xadd(s.C0, xmul(w, fmaxf(sh_channel(ncoef, sb, c, 0), 0.f)));
-            s.C1 = xadd(s.C1, xmul(w, fmaxf(sh_channel(ncoef, sb, c, 1), 0.f)));
-            s.C2 = xadd(s.C2, xmul(w, fmaxf(sh_channel(ncoef, sb, c, 2), 0.f)));
+            float R, G, B;
+            sh_rgb(in.shs + 3 * (size_t)gidx * in.sh_coeffs, ncoef, sh_aligned, sb, R, G, B);
+            s.C0 = xadd(s.C0, xmul(w, fmaxf(R, 0.f)));
+            s.C1 = xadd(s.C1, xmul(w, fmaxf(G, 0.f)));
+            s.C2 = xadd(s.C2, xmul(w, fmaxf(B, 0.f)));
         } else {
             const float* cp = in.colors_precomp + 3 * (size_t)gidx;
             s.C0 = xadd(s.C0, xmul(w, __ldg(cp))); s.C1 = xadd(s.C1, xmul(w, __ldg(cp + 1))); s.C2 = xadd(s.C2, xmul(w, __ldg(cp + 2)));
@@ -444,8 +455,9 @@ __global__ void __launch_bounds__(256) k_weights(int P, unsigned long long* __re
     if (v) wsum[g] = 0ull;
 }
 
-template <bool DIAG>
-__global__ void __launch_bounds__(SHADE_THREADS, DST_SHADE_GRID_PER_SM) k_fwd_shade(const __grid_constant__ FwdParams p, int round) {
+// BLOCKS per SM: 4 at 128 registers, 5 at 96 (DST_SHADE_WIDE_SLOTS)
+template <bool DIAG, int BLOCKS>
+__global__ void __launch_bounds__(SHADE_THREADS, BLOCKS) k_fwd_shade(const __grid_constant__ FwdParams p, int round) {
     const int n = p.counts[round];
     if (n < p.min_count) return;
     const int* list = p.list[round & 1];
@@ -1065,17 +1077,19 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
         DST_CUDA_TRY(h, cudaEventRecord(h->slice_fork, st));
         for (int g = 1; g < nsl; g++) DST_CUDA_TRY(h, cudaStreamWaitEvent(sst[g], h->slice_fork, 0));
     }
+    const int shade_blocks = !diag && slots >= DST_SHADE_WIDE_SLOTS ? DST_SHADE_GRID_PER_SM + 1 : DST_SHADE_GRID_PER_SM;
     for (int r = 0; r < p.rounds; r++) {
         for (int g = 0; g < nsl; g++) {
             const FwdParams& q = ps[g];
-            const int g_enum = dst_wavefront_grid(h, sslots[g], ENUM_THREADS, DST_ENUM_GRID_PER_SM), g_shade = dst_wavefront_grid(h, sslots[g], SHADE_THREADS, DST_SHADE_GRID_PER_SM);
+            const int g_enum = dst_wavefront_grid(h, sslots[g], ENUM_THREADS, DST_ENUM_GRID_PER_SM), g_shade = dst_wavefront_grid(h, sslots[g], SHADE_THREADS, shade_blocks);
             const int g_compact = (int)((sslots[g] + DST_LIVE_BLOCK - 1) / DST_LIVE_BLOCK);
             dst_prof_mark(h, 3, 0, sst[g]);
             launch_gather(diag, g_enum, h->sm_count, nsl, sst[g], q.bvh, q.req, q.list[r & 1], q.counts + r, q.counts + r, q.min_count, q.kbuf, q.kcnt,
                           q.status, a->counters, q.lv.tmp, q.list[(r + 1) & 1]);
             dst_prof_mark(h, 3, 1, sst[g]);
-            if (diag) k_fwd_shade<true><<<g_shade, SHADE_THREADS, 0, sst[g]>>>(q, r);
-            else k_fwd_shade<false><<<g_shade, SHADE_THREADS, 0, sst[g]>>>(q, r);
+            if (diag) k_fwd_shade<true, DST_SHADE_GRID_PER_SM><<<g_shade, SHADE_THREADS, 0, sst[g]>>>(q, r);
+            else if (shade_blocks == DST_SHADE_GRID_PER_SM) k_fwd_shade<false, DST_SHADE_GRID_PER_SM><<<g_shade, SHADE_THREADS, 0, sst[g]>>>(q, r);
+            else k_fwd_shade<false, DST_SHADE_GRID_PER_SM + 1><<<g_shade, SHADE_THREADS, 0, sst[g]>>>(q, r);
             if (q.lv.stable) k_compact<<<g_compact, 256, 0, sst[g]>>>(q.lv, q.counts + r, q.counts + r + 1, q.min_count, q.list[(r + 1) & 1], r);
         }
     }

@@ -216,6 +216,49 @@ __device__ __forceinline__ float sh_channel(int ncoef, const float* b, const flo
     return xadd(r, 0.5f);
 }
 
+// The three unclamped colour channels of one surfel, summed as its row arrives: the same operations as sh_channel, without the 48
+// registers that hold a row whole (k_fwd_shade fits 96 registers with it; with the row held it spilled 144 bytes there).
+__device__ __forceinline__ void sh_rgb(const float* __restrict__ row, int ncoef, bool aligned, const float* b, float& R, float& G, float& B) {
+    if (ncoef == 16 && aligned && (reinterpret_cast<uintptr_t>(row) & 31) == 0) {
+        float r[3];
+#pragma unroll
+        for (int i = 0; i < 6; i++) {
+            float4 q[2];
+            ldg256(reinterpret_cast<const float4*>(row) + 2 * i, q[0], q[1]);
+            const float* c = reinterpret_cast<const float*>(q);
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int v = 8 * i + k, j = v / 3, ch = v % 3;
+                r[ch] = j == 0 ? xmul(b[0], c[k]) : xadd(r[ch], xmul(b[j], c[k]));
+            }
+        }
+        R = xadd(r[0], 0.5f); G = xadd(r[1], 0.5f); B = xadd(r[2], 0.5f);
+        return;
+    }
+    if (aligned) {
+        float r[3];
+#pragma unroll
+        for (int i = 0; i < 12; i++) {
+            if (4 * i < 3 * ncoef) {       // (an aligned row holds a multiple of four floats)
+                const float4 q = __ldg(reinterpret_cast<const float4*>(row) + i);
+                const float c[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int v = 4 * i + k, j = v / 3, ch = v % 3;
+                    if (j < ncoef) r[ch] = j == 0 ? xmul(b[0], c[k]) : xadd(r[ch], xmul(b[j], c[k]));
+                }
+            }
+        }
+        R = xadd(r[0], 0.5f); G = xadd(r[1], 0.5f); B = xadd(r[2], 0.5f);
+        return;
+    }
+    R = xmul(b[0], __ldg(row)); G = xmul(b[0], __ldg(row + 1)); B = xmul(b[0], __ldg(row + 2));
+#pragma unroll
+    for (int j = 1; j < 16; j++)
+        if (j < ncoef) { R = xadd(R, xmul(b[j], __ldg(row + 3 * j))); G = xadd(G, xmul(b[j], __ldg(row + 3 * j + 1))); B = xadd(B, xmul(b[j], __ldg(row + 3 * j + 2))); }
+    R = xadd(R, 0.5f); G = xadd(G, 0.5f); B = xadd(B, 0.5f);
+}
+
 // exp for x <= 0 as a fixed sequence of rounded operations (Cody-Waite reduction, degree-7 Taylor
 // polynomial, exact power-of-two scaling): reproducible bit for bit on a CPU, about 1 ulp from a
 // correctly rounded exp. The falloff G = exp(-rho/2) decides which hits contribute
