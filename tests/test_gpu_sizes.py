@@ -111,3 +111,20 @@ def test_missing_upstream_gradients_are_zeros_and_the_arena_stays_clean(C):
             assert np.array_equal(np.isfinite(a), np.isfinite(b)), k
             m = np.isfinite(b)
             assert hp.rel_l2(a[m], b[m]) < 1e-5, (P, k)
+
+
+@pytest.mark.parametrize("coeffs,degree", [(16, 3), (16, 1), (9, 2), (4, 1)])
+def test_composite_build_for_large_calls(C, coeffs, degree):
+    """The composite kernel runs another build from 921,600 rays on: each row of rays comes out as in a call below that, for SH rows of
+    every alignment."""
+    w = hp.workloads.make_workload(3, P=20_000, H=960, W=960)
+    wc = hp.to_cuda(w)
+    wc["shs"], wc["sh_degree"] = wc["shs"][:, :coeffs].contiguous(), degree
+    st = _state(C, wc)
+    large = hp.cuda_forward(C, st, wc, training=False)
+    part = dict(wc, ray_o=wc["ray_o"][:952].contiguous(), ray_d=wc["ray_d"][:952].contiguous())
+    small = hp.cuda_forward(C, st, part, training=False)
+    torch.cuda.synchronize()
+    assert st.status() == 0 and float(large["acc"].max()) > 0.5
+    for k in ("rgb", "dpt", "acc", "norm", "mid"):
+        assert torch.equal(large[k][:952], small[k]), k
