@@ -171,7 +171,7 @@ class OptiXStateWrapper:
         _check(self, lib().dst_set_option(self.handle, 1, int(n)))
 
     def set_chunk_log_max_records(self, n):
-        """Upper limit on the chunk-log size in records of 136 bytes (0: built-in limit only)."""
+        """Upper limit on the contribution-log size in records of 132 bytes (0: built-in limit only)."""
         _check(self, lib().dst_set_option(self.handle, 3, int(n)))
 
     def set_image_width(self, width):
@@ -185,7 +185,7 @@ class OptiXStateWrapper:
         _check(self, lib().dst_set_option(self.handle, 4, int(bool(on))))
 
     def set_chunk_log(self, on):
-        """Keep (default) or drop the per-ray chunk log training forwards leave for the backward (about 1.6 KB per ray)."""
+        """Keep (default) or drop the per-ray contribution log training forwards leave for the backward (about 1.6 KB per ray)."""
         _check(self, lib().dst_set_option(self.handle, 2, int(bool(on))))
 
     def kernel_launches(self):
@@ -251,7 +251,7 @@ class OptiXStateWrapper:
         return v.value
 
     def chunk_log(self):
-        """dict(records_wanted, records_held, bytes_per_record) of the chunk log (records_wanted -1: not known yet)."""
+        """dict(records_wanted, records_held, bytes_per_record) of the contribution log (records_wanted -1: not known yet)."""
         a, b, c = C.c_int64(), C.c_int64(), C.c_int64()
         _check(self, lib().dst_debug_chunk_log(self.handle, C.byref(a), C.byref(b), C.byref(c)))
         return dict(records_wanted=a.value, records_held=b.value, bytes_per_record=c.value)
@@ -372,7 +372,7 @@ def trace_surfels(state, training, start_from_first, ray_o, ray_d, vertices, bac
         _check(state, lib().dst_forward(state.handle, C.byref(a), _stream(state)))
     ser = C.c_uint64(0)
     _check(state, lib().dst_forward_serial(state.handle, C.byref(ser)))
-    state.last_forward_serial = ser.value       # names the chunk log this call left in the handle (0: none)
+    state.last_forward_serial = ser.value       # names the contribution log this call left in the handle (0: none)
     # the saved tensor that identifies this call to a backward that is not told the serial (a caller written against
     # the reference's extension module passes exactly the reference's arguments)
     state._logged_mid = (mid_val.data_ptr(), tuple(mid_val.shape)) if ser.value else None
@@ -389,7 +389,7 @@ def trace_surfels_backward(state, start_from_first, ray_o, ray_d, vertices, back
     opacities, scales, rotations, transMat_precomp (zeros).
 
     `_forward_serial`: `state.last_forward_serial` as it was right after the forward call these saved
-    tensors come from; when it still names the handle's chunk log the backward re-composites the logged
+    tensors come from; when it still names the handle's contribution log the backward re-composites the logged
     chunks instead of walking the hierarchy again (same result). When it is not given (None), the call is
     recognised by its `mid_val` tensor: if that is the one the state's last training forward returned, its
     serial is used. Pass 0 to force a re-trace.
@@ -519,7 +519,7 @@ def trace_surfels_static(state, training, start_from_first, ray_o, ray_d, vertic
     (a.out_rgb, a.out_dpt, a.out_acc, a.out_norm, a.out_dist, a.out_aux, a.mid_val) = [t.data_ptr() for t in outs]
     a.a_weights = _ptr(a_weights)
     _check(state, lib().dst_forward_static(state.handle, C.byref(a), _stream(state)))
-    # this entry point keeps no chunk log: a backward of these outputs must re-trace, never reuse the log of an earlier call
+    # this entry point keeps no contribution log: a backward of these outputs must re-trace, never reuse the log of an earlier call
     state.last_forward_serial = 0
     state._logged_mid = None
     return (*outs, a_weights)

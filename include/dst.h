@@ -34,7 +34,7 @@ extern "C" {
 /* bits of the device status word returned by dst_status */
 #define DST_STATUS_STACK_OVERFLOW  1u   /* traversal stack exhausted: some hits may be missing */
 #define DST_STATUS_CHUNK_LIMIT     2u   /* a ray hit the bound on 16-hit enumerations          */
-#define DST_STATUS_LOG_MISMATCH    8u   /* the chunk log ended before the backward of a ray did */
+#define DST_STATUS_LOG_MISMATCH    8u   /* the contribution log ended before the backward of a ray did */
 
 #define DST_MID_CHANNELS 16             /* per-bounce record, optix_tracer/config.h:7-15       */
 #ifndef DST_CHUNK
@@ -117,7 +117,7 @@ typedef struct dst_bwd_args {
     float *dL_drotations;         /* (P, 4)                                                       */
     unsigned long long *counters; /* as in dst_fwd_args, or NULL                                  */
     unsigned long long forward_serial; /* value of dst_forward_serial right after the forward call whose saved state
-                                     this is, or 0. When it still names the chunk log the handle holds, the backward
+                                     this is, or 0. When it still names the contribution log the handle holds, the backward
                                      re-composites the logged chunks instead of walking the hierarchy again
                                      (same result); otherwise it re-traces.                        */
 } dst_bwd_args;
@@ -213,10 +213,10 @@ int dst_bvh_info(const dst_handle* h, int64_t* surfels, int64_t* nodes, int64_t*
  * kernel that takes every ray through its whole path (one warp per ray in the forward, one thread per
  * ray in the backward). Results do not depend on the setting. */
 #define DST_OPT_WAVEFRONT_MIN_RAYS 1
-/* DST_OPT_CHUNK_LOG: 1 (default) keeps the chunk log of training forwards for the backward, 0 disables it. */
+/* DST_OPT_CHUNK_LOG: 1 (default) keeps the contribution log of training forwards for the backward, 0 disables it. */
 #define DST_OPT_CHUNK_LOG 2
-/* DST_OPT_CHUNK_LOG_MAX_RECORDS: upper limit on the records (136 bytes each) the chunk log may hold; 0 = only the
- * built-in limit. Rays whose chunks did not fit are re-traced by the backward, with the same result. */
+/* DST_OPT_CHUNK_LOG_MAX_RECORDS: upper limit on the records (132 bytes each) the contribution log may hold; 0 = only the
+ * built-in limit. Rays whose contributions did not fit are re-traced by the backward, with the same result. */
 #define DST_OPT_CHUNK_LOG_MAX_RECORDS 3
 /* Hint for rays given as (B, h*w, 3) batches of whole images (the reference's "(B, P, 3)" form, __init__.py:246):
  * the image width w. The kernels then walk the rays in 8x4 pixel tiles, as they do for (H, W, 3) rays, so that a
@@ -244,7 +244,7 @@ int dst_bvh_info(const dst_handle* h, int64_t* surfels, int64_t* nodes, int64_t*
 /* Slices of a large forward call (results are not affected): the ray slots are cut into this many contiguous ranges
  * whose wavefront rounds run on streams of their own, ordered after what the caller's stream held at the call and
  * joined into it before the call returns, so that the slow last batches of one slice's round overlap with the other
- * slices' work. 0 (default): 4 for calls of a million rays and more, fewer for smaller ones; 1: no slicing; at most 8. */
+ * slices' work. 0 (default): 4 for calls of 2^20 ray slots and more, up to 6 of at least 98,304 slots each below that; 1: no slicing; at most 8. */
 #define DST_OPT_FORWARD_SLICES 9
 /* Training forwards whose contribution logs the handle keeps until their backward comes (1, the default, to 4). With 1 a
  * forward replaces the log of the one before, whose backward then re-traces. */
@@ -280,7 +280,7 @@ int dst_debug_round_counts(dst_handle* h, int32_t* counts, int32_t cap, void* st
  * `bytes` bytes, `reps` passes, timed with CUDA events on `stream` after a warming pass; allocates and frees
  * the buffer. With a buffer that fits the L2 cache this is the L2 read bandwidth quoted beside the HBM figure. */
 int dst_debug_read_bandwidth(dst_handle* h, int64_t bytes, int reps, float* gb_per_s, void* stream);
-/* Diagnostics: the chunk log of the last training forward whose read-back has completed: records it wanted
+/* Diagnostics: the contribution log of the last training forward whose read-back has completed: records it wanted
  * (-1: not known yet), records the log can hold, bytes per record. Rays whose records did not fit are re-traced
  * by the backward. */
 int dst_debug_chunk_log(const dst_handle* h, int64_t* records_wanted, int64_t* records_held, int64_t* bytes_per_record);
