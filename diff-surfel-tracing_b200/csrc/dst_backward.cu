@@ -306,8 +306,9 @@ __device__ __forceinline__ bool bwd_next_segment(const BwdParams& p, int ray, Bw
         s.sox = m0.x; s.soy = m0.y; s.soz = m0.z; s.sdx = sdx; s.sdy = sdy; s.sdz = sdz;
         s.offset = 0.f; s.dpt = 0.f; s.T_prev = 1.f;
         // everything the segment composited, and the background seen through it (counted a second time, as the reference does, :545-548)
-        s.rem = s.t_rgb0 * tot_c0 + s.t_rgb1 * tot_c1 + s.t_rgb2 * tot_c2 + s.t_aux0 * tot_o0 + s.t_aux1 * m3.x + s.t_dpt * tot_dpt +
-                (t_norm.x * tot_n.x + t_norm.y * tot_n.y + t_norm.z * tot_n.z) + s.t_acc * m1.w +
+        s.rem = s.t_rgb0 * tot_c0 + s.t_rgb1 * tot_c1 + s.t_rgb2 * tot_c2;
+        if (in.others_precomp) s.rem += s.t_aux0 * tot_o0 + s.t_aux1 * m3.x;       // (without auxiliaries tot_o0 is zero and t_aux0 a quotient by it)
+        s.rem += s.t_dpt * tot_dpt + (t_norm.x * tot_n.x + t_norm.y * tot_n.y + t_norm.z * tot_n.z) + s.t_acc * m1.w +
                 (1.0f - m1.w) * (s.t_rgb0 * __ldg(in.background) + s.t_rgb1 * __ldg(in.background + 1) + s.t_rgb2 * __ldg(in.background + 2));
         s.last_gidx = -1; s.contributor = 0; s.chunk = 0; s.seg = i; s.dir_gidx = -1;
         s.dm0 = s.dvs = s.dws = 0.f;

@@ -138,6 +138,33 @@ def test_sh_degrees(C, oracle_mod, degree, coeffs):
     _compare(C, orc, w, wave=(degree == 2))
 
 
+@pytest.mark.parametrize("wave", [False, True], ids=["per-ray", "wavefront"])
+@pytest.mark.parametrize("serial", ["logged", "traced"])
+def test_bounces_without_auxiliaries(C, oracle_mod, wave, serial):
+    """Bounces allowed, no specularity given: no ray is reflected, every quotient by the accumulated specular weight is one by zero, and
+    none of them may reach a gradient (the reference uses them only where auxiliaries are given, optix_tracer/backward.cu)."""
+    w = dict(hp.reduced_workload(3), others_precomp=None, max_trace_depth=1)
+    wc = hp.to_cuda(w)
+    st = _state(C, wc, wave)
+    got = hp.cuda_forward(C, st, wc)
+    H, W = w["ray_o"].shape[:2]
+    gen = torch.Generator().manual_seed(5)
+    up = {k: torch.randn((H, W, c), generator=gen) for k, c in (("rgb", 3), ("dpt", 1), ("acc", 1), ("norm", 3), ("aux", 2))}
+    gb = hp.cuda_backward(C, st, wc, got, {k: v.cuda() for k, v in up.items()}, serial=st.last_forward_serial if serial == "logged" else 0)
+    torch.cuda.synchronize()
+    assert st.status() == 0
+    orc = oracle_mod.Oracle(oracle_mod.Scene(w["v"]), impl="restatement", portable_exp=True)
+    want = orc.forward(w, training=True)
+    ob = orc.backward(w, {k: got[k].cpu().numpy().reshape(want[k].shape) for k in ("rgb", "dpt", "acc", "norm", "dist", "aux", "mid")},
+                      {k: v.numpy() for k, v in up.items()})
+    for k in hp.GRAD_KEYS:
+        g, o = gb[k].cpu().numpy().reshape(ob[k].shape), ob[k]
+        assert np.isfinite(o).all() and np.isfinite(g).all(), k
+        if k in ("means3D", "opacities", "scales", "rotations"):
+            assert float(np.abs(o).max()) > 0, k
+        assert hp.rel_l2(g, o) <= GRAD_RTOL, k
+
+
 def test_inference_mode(C, oracle_mod):
     """training=False: no per-surfel weights, the same per-ray outputs; the module returns zeros of shape (P,)."""
     w = hp.reduced_workload(3)
