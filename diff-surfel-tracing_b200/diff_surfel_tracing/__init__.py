@@ -159,7 +159,8 @@ class SurfelTracer(nn.Module):
 
         empty = self._empty       # stands for every input that is not given
         if empty is None or empty.device != means3D.device:
-            empty = self._empty = torch.empty((0,), dtype=torch.float32, device=means3D.device)
+            with torch.inference_mode(False):       # (a tensor made in inference mode could not be saved for a later call's backward)
+                empty = self._empty = torch.empty((0,), dtype=torch.float32, device=means3D.device)
         if shs is None: shs = empty
         if colors_precomp is None: colors_precomp = empty
         if others_precomp is None: others_precomp = empty

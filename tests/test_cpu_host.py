@@ -354,3 +354,25 @@ def test_two_rank_gradient_exchange_gloo(tmp_path, oracle_mod):
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
     m = re.search(r"RELERR ([0-9.eE+-]+)", r.stdout)
     assert m and float(m.group(1)) < 1e-3
+
+
+def _tracer_without_gpu(monkeypatch, seen):
+    """A SurfelTracer whose calls end where the kernels would start: `seen` gets the arguments."""
+    import diff_surfel_tracing as dst
+    monkeypatch.setattr(dst._C, "OptiXStateWrapper", lambda pkg: type("State", (), dict(set_kept_logs=lambda self, n: None))())
+    monkeypatch.setattr(dst, "trace_surfels", lambda *args: seen.append(args))
+    return dst.SurfelTracer()
+
+
+def test_first_call_in_inference_mode_leaves_training_intact(monkeypatch):
+    """The tensor that stands for absent inputs is kept between calls: it must be one autograd can save, also when the first call is a
+    rendering one in inference mode."""
+    seen = []
+    tracer = _tracer_without_gpu(monkeypatch, seen)
+    x = torch.zeros(2, 3)
+    with torch.inference_mode():
+        tracer(x, x, x, x, x, shs=x, opacities=x, scales=x, rotations=x)
+    tracer(x, x, x, x, x, shs=x, opacities=x, scales=x, rotations=x)
+    for args in seen:
+        absent = [a for a in args if isinstance(a, torch.Tensor) and a.numel() == 0]
+        assert len(absent) == 3 and not any(a.is_inference() for a in absent)       # colours, auxiliaries, covariances
