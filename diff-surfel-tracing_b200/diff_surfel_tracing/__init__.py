@@ -14,6 +14,7 @@ from typing import NamedTuple
 
 import torch
 import torch.nn as nn
+from torch.autograd import forward_ad
 
 from . import _C
 
@@ -27,7 +28,8 @@ def trace_surfels(optix_context, training, start_from_first, ray_o, ray_d, verti
                   colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings):
     args = (optix_context, training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D, shs,
             colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings)
-    if not torch.is_grad_enabled():       # rendering: nothing to record
+    # rendering: nothing to record. Forward-mode derivatives and function transforms go through the autograd function, which refuses them
+    if not torch.is_grad_enabled() and forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active():
         return _forward(*args)[0]
     return _TraceSurfels.apply(*args)
 

@@ -376,3 +376,27 @@ def test_first_call_in_inference_mode_leaves_training_intact(monkeypatch):
     for args in seen:
         absent = [a for a in args if isinstance(a, torch.Tensor) and a.numel() == 0]
         assert len(absent) == 3 and not any(a.is_inference() for a in absent)       # colours, auxiliaries, covariances
+
+
+def test_rendering_without_grad_mode_still_refuses_forward_mode_and_transforms(monkeypatch):
+    """Under no_grad the autograd function is passed by. Tangents of forward-mode differentiation and function transforms must not be
+    dropped on the way: they are refused as with grad mode on."""
+    import diff_surfel_tracing as dst
+    ran = []
+
+    def forward(*args):
+        ran.append(args)
+        out = tuple(torch.zeros(1, 1, c) for c in (3, 1, 1, 3, 1, 2, 32)) + (torch.zeros(2),)
+        return out, torch.zeros(1, 1, 3)
+
+    monkeypatch.setattr(dst, "_forward", forward)
+    state, x, e = type("State", (), {})(), torch.ones(2, 3), torch.empty(0)
+    trace = lambda t: dst.trace_surfels(state, True, True, e, e, e, t, e, e, e, e, e, e, e, e, None)[0]  # noqa: E731
+    with torch.no_grad():
+        assert torch.equal(trace(x), torch.zeros(1, 1, 3)) and len(ran) == 1
+        with torch.autograd.forward_ad.dual_level():
+            with pytest.raises(NotImplementedError, match="jvp"):
+                trace(torch.autograd.forward_ad.make_dual(x, x))
+        for transform in (torch.vmap(trace), torch.func.grad(lambda t: trace(t).sum()), lambda t: torch.func.jvp(trace, (t,), (t,))):
+            with pytest.raises(RuntimeError, match="functorch transforms"):
+                transform(x)
