@@ -747,13 +747,16 @@ __global__ void __launch_bounds__(BWD_THREADS, BLOCKS) k_bwd_logged(const __grid
             if (at < num) {
                 const int pidx = (int)(unsigned int)key;
                 SlotEval e;
-                eval_slot(key, 0.0f, s.sox, s.soy, s.soz, s.sdx, s.sdy, s.sdz, min_depth, p.cache, pidx >> 1, e);      // (accepted, as in the forward)
+                // accepted, as in the forward, unless the caller has changed the surfel since: it then contributes nothing
+                const bool ok = eval_slot(key, 0.0f, s.sox, s.soy, s.soz, s.sdx, s.sdy, s.sdz, min_depth, p.cache, pidx >> 1, e);
                 if (at + 1 < num) {
                     if (((at + 1) & (DST_CHUNK - 1)) == 0) rec = __ldg(p.log_next + rec);
                     key = __ldg(p.log_keys + soa(rec, (at + 1) & (DST_CHUNK - 1), DST_CHUNK));
                 }
-                bwd_hit<DIST>(p, s, x, e, pidx, at == 0, ws);
-                gsent = pidx >> 1;
+                if (ok) {
+                    bwd_hit<DIST>(p, s, x, e, pidx, at == 0, ws);
+                    gsent = pidx >> 1;
+                }
             }
             send_rows(target, ws, gsent, p.tiled != 0);
         }

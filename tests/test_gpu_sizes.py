@@ -128,3 +128,31 @@ def test_composite_build_for_large_calls(C, coeffs, degree):
     assert st.status() == 0 and float(large["acc"].max()) > 0.5
     for k in ("rgb", "dpt", "acc", "norm", "mid"):
         assert torch.equal(large[k][:952], small[k]), k
+
+
+def test_logged_hits_that_no_longer_contribute(C):
+    """Two views traced, then surfels made transparent in place, then the backwards. The first view's records are rebuilt from what the
+    tensors hold by then: its logged hits on those surfels are passed over, as a re-trace passes them over."""
+    wc = hp.to_cuda(hp.workloads.make_workload(3, P=20_000, H=48, W=64))
+    st = _state(C, wc)
+    st.set_kept_logs(4)
+    for step in range(2):       # the second step's logs both fit
+        fs = []
+        for _ in range(2):
+            f = hp.cuda_forward(C, st, wc)
+            torch.cuda.synchronize()
+            fs.append((f, st.last_forward_serial))
+        if step == 0:
+            for f, serial in fs[::-1]:
+                hp.cuda_backward(C, st, wc, f, dict(rgb=torch.ones_like(f["rgb"])), serial=serial)
+    gone = torch.rand(20_000, device="cuda") < 0.5
+    kept = wc["opacities"].clone()
+    wc["opacities"][gone] = 0.0
+    f, serial = fs[0]
+    dg = {}
+    g = hp.cuda_backward(C, st, wc, f, {k: torch.ones_like(f[k]) for k in ("rgb", "dpt", "norm")}, diag=dg, serial=serial)
+    torch.cuda.synchronize()
+    wc["opacities"].copy_(kept)
+    assert st.status() == 0 and int(dg["counters"][2]) == 0       # from the log
+    for k in ("means3D", "opacities", "scales", "rotations"):
+        assert float(g[k][gone].abs().max()) == 0.0 and float(g[k][~gone].abs().max()) > 0.0, k
