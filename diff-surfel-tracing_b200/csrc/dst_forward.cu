@@ -557,6 +557,10 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_fwd_tail(const __grid_constant
 // side instead of one dependent load after another. What has an order keeps it: the transmittance is a chain of uniform
 // products, and the nine running sums (C, D, N, O: neighbours in FwdState) are added up hit by hit, one sum per lane, so every bit is
 // that of the serial loop. s and terms are shared memory of the warp; key: lane i's hit.
+// Floats of a colour row that a degree reads: what lies beyond may not belong to the caller's tensor (the last row of 9 coefficients is 27
+// floats), so nothing beyond is prefetched either. Degree 3 is the one with floats in a second 128-byte line.
+__host__ __device__ constexpr int sh_row_floats(int degree) { return 3 * (degree + 1) * (degree + 1); }
+static_assert(sh_row_floats(2) <= 32 && sh_row_floats(3) > 32, "the second prefetch of fwd_shade_warp is degree 3's alone");
 struct WarpShade { FwdState s; float terms[DST_CHUNK][9]; };
 template <bool DIAG>
 __device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int slot, WarpShade& ws, unsigned long long key, int cnt, TraceCounters& tc) {
@@ -570,7 +574,7 @@ __device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int slot, War
     if (have && in.colors_precomp == nullptr) {       // the colour row is on its way while the hit is evaluated
         const float* row = in.shs + 3 * (size_t)gidx * in.sh_coeffs;
         asm volatile("prefetch.global.L1 [%0];" :: "l"(row));
-        if (in.sh_coeffs > 8) asm volatile("prefetch.global.L1 [%0];" :: "l"(row + 32));
+        if (sh_row_floats(in.sh_degree) > 32) asm volatile("prefetch.global.L1 [%0];" :: "l"(row + 32));
     }
     SlotEval e;
     e.dpt = 0.f; e.alpha = 0.f;

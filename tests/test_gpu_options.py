@@ -138,6 +138,17 @@ def test_sh_degrees(C, oracle_mod, degree, coeffs):
     _compare(C, orc, w, wave=(degree == 2))
 
 
+@pytest.mark.parametrize("degree,coeffs", [(2, 9), (2, 10), (1, 10), (2, 11)])
+def test_sh_rows_that_end_short_of_a_second_line(C, oracle_mod, degree, coeffs):
+    """The per-ray kernel's rows of 9 to 11 coefficients (27 to 33 floats), the last one at the end of its allocation."""
+    w = hp.reduced_workload(1)
+    gen = torch.Generator().manual_seed(2)
+    shs = 0.1 * torch.randn((w["means3D"].shape[0], coeffs, 3), generator=gen)
+    w = dict(w, shs=shs, sh_degree=degree)
+    orc = oracle_mod.Oracle(oracle_mod.Scene(w["v"]), impl="restatement", hit_cap=320, portable_exp=True)
+    _compare(C, orc, w, wave=False)
+
+
 @pytest.mark.parametrize("wave", [False, True], ids=["per-ray", "wavefront"])
 @pytest.mark.parametrize("serial", ["logged", "traced"])
 def test_bounces_without_auxiliaries(C, oracle_mod, wave, serial):
