@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(256) k_unpack(int P, float* __restrict__ arena
 BvhView dst_bvh_view(const dst_handle* h);
 int dst_check_inputs(dst_handle* h, const dst_trace_inputs* in);
 long long dst_call_signature(const dst_trace_inputs* in);
-void dst_slot_grid(const dst_handle* h, const dst_trace_inputs* in, int* gh, int* gw);
+long long dst_slot_grid(const dst_handle* h, const dst_trace_inputs* in, int* gh, int* gw, int* tiled);
 
 // the staging rows need more dynamic shared memory than a kernel gets by default: raise the limit of every instantiation once per device
 template <typename K>
@@ -861,10 +861,8 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
         const unsigned long long since = h->serial_counter - a->forward_serial + 1;
         if (!log && h->logs_keep > 1 && since > 1) h->logs_wanted = since < (unsigned long long)h->logs_keep ? (int)since : h->logs_keep;
     }
-    dst_slot_grid(h, &a->in, &p.grid_h, &p.grid_w);
-    p.tiled = p.grid_h >= 16;
-    if (log) { p.grid_h = log->grid_h; p.grid_w = log->grid_w; p.tiled = log->tiled; log->consumed = true; }       // the log is indexed by its forward's slots
-    const long long slots = slots_of_grid(p.grid_h, p.grid_w, p.tiled != 0);
+    long long slots = dst_slot_grid(h, &a->in, &p.grid_h, &p.grid_w, &p.tiled);
+    if (log) { p.grid_h = log->grid_h; p.grid_w = log->grid_w; p.tiled = log->tiled; slots = log->slots; log->consumed = true; }       // the log is indexed by its forward's slots
     rc = dst_ensure_wavefront(h, slots, sizeof(BwdState));
     if (rc != DST_OK) return rc;
     p.state = static_cast<float4*>(h->wf_state); p.req = static_cast<float4*>(h->wf_req); p.kbuf = h->wf_kbuf; p.kcnt = h->wf_kcnt;

@@ -810,12 +810,16 @@ int dst_live_lists(dst_handle* h, long long slots, LiveLists* lv, cudaStream_t s
     return DST_OK;
 }
 
-// Pixel grid the rays are walked over in 8x4 tiles. Rays given as (B, h*w, 3) batches of whole images are
-// contiguous image rows, so with the image width known they form one (B*h) x w grid; otherwise the (H, W) of the call.
-void dst_slot_grid(const dst_handle* h, const dst_trace_inputs* in, int* gh, int* gw) {
+// Ray order of a call: the pixel grid the rays are walked over, in 8x4 tiles or linearly; returns the list slots it takes. Rays given as
+// (B, h*w, 3) batches of whole images are contiguous image rows, so with the image width known they form one (B*h) x w grid; otherwise
+// the (H, W) of the call. Grids of fewer than 16 rows are ray lists, not images: linear. So is a grid whose whole blocks of tiles would take more
+// slots than a list word holds beside its class bit: a column of 2^24 rays, padded to 64x32 pixels, is 2^30 slots.
+long long dst_slot_grid(const dst_handle* h, const dst_trace_inputs* in, int* gh, int* gw, int* tiled) {
     *gh = in->H; *gw = in->W;
     const long long iw = h->image_width;
     if (iw >= 8 && in->W > iw && in->W % iw == 0 && (long long)in->H * (in->W / iw) < 0x7fffffffll) { *gh = (int)(in->H * (in->W / iw)); *gw = (int)iw; }
+    *tiled = *gh >= 16 && slots_of_grid(*gh, *gw, true) < (1ll << DST_LIVE_CLASS_BIT);
+    return slots_of_grid(*gh, *gw, *tiled != 0);
 }
 
 // one number for "the same kind of call": ray grid, surfel count, bounce limit
@@ -948,9 +952,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     p.cam_on = cam != nullptr;
     p.dist_on = h->distortion;
     if (cam) camera_constants(cam, &p.cam); else memset(&p.cam, 0, sizeof(p.cam));
-    dst_slot_grid(h, &a->in, &p.grid_h, &p.grid_w);
-    p.tiled = p.grid_h >= 16;
-    const long long slots = slots_of_grid(p.grid_h, p.grid_w, p.tiled != 0);
+    const long long slots = dst_slot_grid(h, &a->in, &p.grid_h, &p.grid_w, &p.tiled);
     rc = dst_ensure_wavefront(h, slots, sizeof(FwdState));
     if (rc != DST_OK) return rc;
     rc = ensure_cache(h, &a->in);

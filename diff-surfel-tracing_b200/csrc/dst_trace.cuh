@@ -945,9 +945,9 @@ __device__ __forceinline__ void append_alive(bool alive, int ray, int* __restric
 // round r + 1 accumulates into (nothing waits on anything: all of this is ordinary stream order).
 // ---------------------------------------------------------------------------------------------
 #define DST_LIVE_BLOCK 4096
-#define DST_LIVE_CLASS_BIT 30            // ray indices stay below 2^30 (checked on the host)
+#define DST_LIVE_CLASS_BIT 30            // slot numbers stay below 2^30 (dst_slot_grid)
 struct LiveLists {
-    int* tmp;            // per list position of the current round: ray | class << 30, or -1
+    int* tmp;            // per list position of the current round: slot | class << 30, or -1
     int* wcnt;           // per 32 positions: survivors of class 0 | survivors of class 1 << 16
     int* bcnt[2];        // per DST_LIVE_BLOCK positions, same packing; set (round & 1) belongs to the current round
     int stable;          // 0: append_alive() order (atomic per warp)

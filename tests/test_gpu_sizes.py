@@ -156,3 +156,25 @@ def test_logged_hits_that_no_longer_contribute(C):
     assert st.status() == 0 and int(dg["counters"][2]) == 0       # from the log
     for k in ("means3D", "opacities", "scales", "rotations"):
         assert float(g[k][gone].abs().max()) == 0.0 and float(g[k][~gone].abs().max()) > 0.0, k
+
+
+def test_column_of_rays_whose_padded_tiles_exceed_a_list_word(C):
+    """2^24 rays as one column: padded to whole blocks of tiles they would be 2^30 list slots, so they are walked linearly. The outputs and
+    gradients of the same rays as 64 rows."""
+    wc = hp.to_cuda(hp.workloads.make_workload(1, P=2_000, H=128, W=128))
+    n = 1 << 24
+    o, d = (wc[k].reshape(-1, 3).repeat(n // 128**2, 1) for k in ("ray_o", "ray_d"))
+    got = []
+    for shape in ((n, 1, 3), (64, n // 64, 3)):
+        st = _state(C, wc)
+        c = dict(wc, ray_o=o.view(shape), ray_d=d.view(shape))
+        f = hp.cuda_forward(C, st, c, training=False)
+        g = hp.cuda_backward(C, st, c, f, dict(rgb=torch.ones_like(f["rgb"])))
+        torch.cuda.synchronize()
+        assert st.status() == 0 and float(f["acc"].max()) > 0.5
+        got.append((f["rgb"].view(n, 3), f["dpt"].view(n), f["mid"].view(n, -1)[:, :16].clone(), g["ray_o"].view(n, 3), g["opacities"]))
+        del st, f, g, c
+    for a, b in zip(got[0][:3], got[1][:3]):
+        assert torch.equal(a, b)
+    for a, b in zip(got[0][3:], got[1][3:]):       # (sums of 32-bit terms in another order)
+        assert float((a - b).double().norm() / b.double().norm()) < 1e-4
