@@ -329,6 +329,12 @@ int dst_debug_read_bandwidth(dst_handle* h, int64_t bytes, int reps, float* gb_p
     return rc;
 }
 
+int dst_debug_log_alloc_limit(dst_handle* h, int64_t bytes) {
+    if (!h) return DST_E_ARG;
+    h->log_alloc_limit = bytes > 0 ? (size_t)bytes : 0;
+    return DST_OK;
+}
+
 int dst_debug_chunk_log(const dst_handle* h, int64_t* records_wanted, int64_t* records_held, int64_t* bytes_per_record) {
     if (!h) return DST_E_ARG;
     if (records_wanted) *records_wanted = (h->log_needed_host && h->log_needed_event && cudaEventQuery(h->log_needed_event) == cudaSuccess) ? h->log_needed_host[0] - h->log_needed_host[1] : -1;

@@ -859,7 +859,7 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
         }
         // a log that was overwritten before its backward came: room for the forwards since then next time
         const unsigned long long since = h->serial_counter - a->forward_serial + 1;
-        if (!log && h->logs_keep > 1 && since > 1) h->logs_wanted = since < (unsigned long long)h->logs_keep ? (int)since : h->logs_keep;
+        if (!log && h->logs_keep > 1 && since > 1) { h->logs_wanted = since < (unsigned long long)h->logs_keep ? (int)since : h->logs_keep; h->logs_missed = true; }
     }
     long long slots = dst_slot_grid(h, &a->in, &p.grid_h, &p.grid_w, &p.tiled);
     if (log) { p.grid_h = log->grid_h; p.grid_w = log->grid_w; p.tiled = log->tiled; slots = log->slots; log->consumed = true; }       // the log is indexed by its forward's slots

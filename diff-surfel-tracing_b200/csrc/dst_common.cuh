@@ -106,7 +106,11 @@ struct dst_handle {
         long long slots;
         void* index_block; int* head; int* num; unsigned char* ok; long long index_cap;       // per slot and segment: first record, entries; per slot: complete
     } logs[DST_MAX_LOGS];
-    int logs_used, logs_keep, logs_wanted; long long log_use;       // logs_wanted: logs a backward has asked for at the same time
+    int logs_used, logs_keep; long long log_use;
+    // logs to make room for: what a backward that found its log overwritten asks for (logs_missed: since the last forward that found none
+    // pending), lowered again to the forwards that then were pending at the same time (logs_begun)
+    int logs_wanted, logs_begun; bool logs_missed;
+    size_t log_alloc_limit;       // test hook (dst_debug_log_alloc_limit)
     int log_enabled;
     long long log_max_records;    // user limit on the log size (0: only the built-in limit)
     int* log_needed_host; cudaEvent_t log_needed_event;     // pinned read-back of log_count after the last forward

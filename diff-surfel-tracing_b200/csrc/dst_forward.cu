@@ -832,15 +832,29 @@ void dst_drop_logs(dst_handle* h) {
     h->logs_used = 0; h->log_use = 0; h->log_serial = 0;
 }
 
+// Log buffers: false where the device has no room for them (or a test says so).
+static bool alloc_log_parts(const dst_handle* h, void** block, const DstPart* parts, int n) {
+    size_t total = 0;
+    for (int k = 0; k < n; k++) total += parts[k].bytes;
+    const bool full = h->log_alloc_limit && total > h->log_alloc_limit;
+    if (full) { cudaFree(*block); *block = nullptr; }
+    if (!full && dst_alloc_parts(block, parts, n) == cudaSuccess) return true;
+    cudaGetLastError();
+    for (int k = 0; k < n; k++) *parts[k].p = nullptr;
+    return false;
+}
+
 // Starts the contribution log of a training forward. The forward logs every contribution (depth along the segment, primitive) so that
 // the backward can composite them again without walking the hierarchy: records of 16 entries, chained per segment, 32 records
 // interleaved (soa()); per segment and slot the first record and the number of entries. Buffers are grow-only.
 //
 // The log of the forward before is overwritten, unless its backward has not come yet and the caller wants logs kept: then this
-// one is appended, if the records both are expected to need fit.
+// one is appended, if the records both are expected to need fit. Room for several is asked for only when a backward has missed its log, and
+// a log is never worth an error: without the memory for several there is room for one, without that (*log null) the backward re-traces.
 int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int grid_w, int tiled, long long slots, dst_handle::Log** log, int* append) {
     const long long rays = (long long)in->H * in->W, sig = dst_call_signature(in);
     const int segs = in->max_trace_depth + 1;
+    *log = nullptr; *append = 0;
     if (h->log_needed_host && h->log_needed_event && cudaEventQuery(h->log_needed_event) == cudaSuccess) {
         const long long seen = (long long)h->log_needed_host[0] - h->log_needed_host[1];
         if (seen > 0) { h->log_known_needed = seen; h->log_known_sig = h->log_pending_sig; }
@@ -851,30 +865,35 @@ int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int gri
     const long long need = h->log_known_needed > 0 && h->log_known_sig == sig ? h->log_known_needed + h->log_known_needed / 8 + 1024 : guess;
     bool pending = false;
     for (int k = 0; k < h->logs_used; k++) pending |= h->logs[k].serial != 0 && !h->logs[k].consumed;
-    if (!(pending && h->logs_used < h->logs_keep && h->log_use + need <= h->log_cap)) {
+    if (!pending) {
+        if (!h->logs_missed && h->logs_begun < h->logs_wanted) h->logs_wanted = h->logs_begun;
+        h->logs_missed = false; h->logs_begun = 0;
+    }
+    h->logs_begun++;
+    if (pending && h->logs_used < h->logs_keep && h->log_use + need <= h->log_cap) *append = 1;
+    else {
         dst_drop_logs(h);
-        long long want = need > guess ? need : guess;
-        if (h->logs_wanted > 1 && need * h->logs_wanted > want) want = need * h->logs_wanted;
-        if (want > DST_LOG_MAX_RECORDS) want = DST_LOG_MAX_RECORDS;
-        if (h->log_max_records > 0 && want > h->log_max_records) want = h->log_max_records;
-        want = (want + 31) / 32 * 32;
-        if (want > h->log_cap || (h->log_max_records > 0 && h->log_cap > want)) {
+        for (;;) {
+            long long want = need > guess ? need : guess;
+            if (h->logs_wanted > 1 && need * h->logs_wanted > want) want = need * h->logs_wanted;
+            if (want > DST_LOG_MAX_RECORDS) want = DST_LOG_MAX_RECORDS;
+            if (h->log_max_records > 0 && want > h->log_max_records) want = h->log_max_records;
+            want = (want + 31) / 32 * 32;
+            if (want <= h->log_cap && (h->log_max_records <= 0 || h->log_cap <= want)) break;
             h->log_cap = 0;
             const DstPart parts[] = {{(void**)&h->log_keys, 8 * DST_CHUNK * (size_t)want}, {(void**)&h->log_next, sizeof(int) * (size_t)want}};
-            const cudaError_t e = dst_alloc_parts(&h->log_block, parts, 2);
-            if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed: %s", cudaGetErrorString(e)); }
-            h->log_cap = want;
+            if (alloc_log_parts(h, &h->log_block, parts, 2)) { h->log_cap = want; break; }
+            if (h->logs_wanted <= 1) return DST_OK;
+            h->logs_wanted = 1;
         }
-        if (!h->log_count && cudaMalloc(&h->log_count, 8) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed"); }
-        *append = 0;
-    } else *append = 1;
+        if (!h->log_count && cudaMalloc(&h->log_count, 8) != cudaSuccess) { cudaGetLastError(); h->log_count = nullptr; return DST_OK; }
+    }
     dst_handle::Log& l = h->logs[h->logs_used];
     if (slots * segs > l.index_cap) {
         l.index_cap = 0;
         const long long cap = slots * segs + slots / 16 + 1024;
         const DstPart parts[] = {{(void**)&l.head, 4 * (size_t)cap}, {(void**)&l.num, 4 * (size_t)cap}, {(void**)&l.ok, (size_t)cap}};
-        const cudaError_t e = dst_alloc_parts(&l.index_block, parts, 3);
-        if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "contribution log allocation failed: %s", cudaGetErrorString(e)); }
+        if (!alloc_log_parts(h, &l.index_block, parts, 3)) return DST_OK;
         l.index_cap = cap;
     }
     h->logs_used++;
@@ -971,10 +990,12 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
         dst_handle::Log* log = nullptr;
         rc = dst_begin_log(h, &a->in, p.grid_h, p.grid_w, p.tiled, slots, &log, &begin.log_append);
         if (rc != DST_OK) return rc;
-        begin.log_count = h->log_count;
-        p.log_keys = h->log_keys; p.log_next = h->log_next; p.log_count = h->log_count; p.log_head = log->head; p.log_num = log->num;
-        p.log_ok = log->ok; p.log_cap = (int)h->log_cap;
-        h->cache_serial = log->serial;
+        if (log) {
+            begin.log_count = h->log_count;
+            p.log_keys = h->log_keys; p.log_next = h->log_next; p.log_count = h->log_count; p.log_head = log->head; p.log_num = log->num;
+            p.log_ok = log->ok; p.log_cap = (int)h->log_cap;
+            h->cache_serial = log->serial;
+        }
     }
     // small launches go straight to the per-ray kernel; large ones run wavefront rounds until few rays are left
     const bool wave = slots >= h->wf_min_rays;

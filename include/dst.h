@@ -284,6 +284,9 @@ int dst_debug_read_bandwidth(dst_handle* h, int64_t bytes, int reps, float* gb_p
  * (-1: not known yet), records the log can hold, bytes per record. Rays whose records did not fit are re-traced
  * by the backward. */
 int dst_debug_chunk_log(const dst_handle* h, int64_t* records_wanted, int64_t* records_held, int64_t* bytes_per_record);
+/* Test hook: allocations of the contribution log above `bytes` fail as on a full device (0: none do). A training forward then makes
+ * do with a smaller log, or with none: the backward re-traces. */
+int dst_debug_log_alloc_limit(dst_handle* h, int64_t bytes);
 /* Diagnostics: copies the per-quad plane frames (12 floats each, surfel order) to `out`. */
 int dst_debug_quad_frames(dst_handle* h, float* out, void* stream);
 

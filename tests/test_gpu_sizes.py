@@ -178,3 +178,71 @@ def test_column_of_rays_whose_padded_tiles_exceed_a_list_word(C):
         assert torch.equal(a, b)
     for a, b in zip(got[0][3:], got[1][3:]):       # (sums of 32-bit terms in another order)
         assert float((a - b).double().norm() / b.double().norm()) < 1e-4
+
+
+def _dense(H, W):
+    """Rays with 256 contributions each: 16 records, more than the 12 a log is first sized for."""
+    w = hp.workloads.make_workload(3, P=20_000, H=H, W=W)
+    w["scales"], w["opacities"], w["max_trace_depth"] = 10.0 * w["scales"], torch.full_like(w["opacities"], 0.05), 0
+    w["v"], w["f"] = hp.workloads.get_triangles(w["means3D"], w["scales"], w["rotations"])
+    return hp.to_cuda(w)
+
+
+def test_no_memory_for_the_log_is_no_error(C):
+    """Where several views' logs do not fit the device there is one view's, where that does not either there is none: the backward
+    re-traces, with the gradients of a state that has its log."""
+    wc = _dense(48, 64)
+    ref = _state(C, wc)
+    keys = ("means3D", "shs", "opacities", "scales", "rotations", "ray_o")
+
+    def step(st, views):
+        fs = []
+        for _ in range(views):
+            f = hp.cuda_forward(C, st, wc)
+            torch.cuda.synchronize()
+            fs.append((f, st.last_forward_serial))
+        for f, serial in fs:
+            g = hp.cuda_backward(C, st, wc, f, dict(rgb=torch.ones_like(f["rgb"])), serial=serial)
+            r = hp.cuda_backward(C, ref, wc, f, dict(rgb=torch.ones_like(f["rgb"])), serial=0)
+            torch.cuda.synchronize()
+            for k in keys:
+                assert hp.rel_l2(g[k].cpu().numpy(), r[k].cpu().numpy()) < 1e-4, k
+        assert st.status() == 0
+        return [serial for _, serial in fs], st.chunk_log()["records_held"]
+
+    st = _state(C, wc)
+    st.set_kept_logs(4)
+    for _ in range(10):       # (what a forward wants is read back now and then)
+        _, one = step(st, 1)
+    st.set_log_alloc_limit(one * 132)
+    for _ in range(3):       # from the second step on room for four is asked for
+        serials, held = step(st, 4)
+        assert all(serials) and held <= one
+    st.set_log_alloc_limit(0)
+    for _ in range(2):
+        _, held = step(st, 4)
+    assert held > one
+    for limit in (1, 48 * 64 * 12 * 8):       # no records; records, but no room for their index or the other way round
+        st = _state(C, wc)
+        st.set_log_alloc_limit(limit)
+        serials, held = step(st, 1)
+        assert serials == [0] and held == 0
+        st.set_log_alloc_limit(0)
+        serials, held = step(st, 1)
+        assert serials[0] > 0 and held > 0
+
+
+def test_room_for_several_logs_is_asked_for_only_while_they_are_used(C):
+    """Four views per step grow the log to four; after steps of one view a larger call's log is sized for one."""
+    wc, big = _dense(48, 64), _dense(96, 128)
+    held = {}
+    for views in (1, 4):
+        st = _state(C, wc)
+        st.set_kept_logs(4)
+        for c, n in (*[(wc, 1)] * 10, *[(wc, views)] * 3, (wc, 1), (wc, 1), (big, 1)):
+            fs = [(hp.cuda_forward(C, st, c), st.last_forward_serial) for _ in range(n)]
+            for f, serial in fs:
+                hp.cuda_backward(C, st, c, f, dict(rgb=torch.ones_like(f["rgb"])), serial=serial)
+            torch.cuda.synchronize()
+            held.setdefault(views, []).append(st.chunk_log()["records_held"])
+    assert held[4][-2] > held[1][-2] and held[4][-1] == max(held[4][-2], held[1][-1]) and held[1][-1] > held[1][-2]
