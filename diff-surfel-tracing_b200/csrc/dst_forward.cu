@@ -878,10 +878,10 @@ int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int gri
             if (h->logs_wanted > 1 && need * h->logs_wanted > want) want = need * h->logs_wanted;
             if (want > DST_LOG_MAX_RECORDS) want = DST_LOG_MAX_RECORDS;
             if (h->log_max_records > 0 && want > h->log_max_records) want = h->log_max_records;
-            want = (want + 31) / 32 * 32;
             if (want <= h->log_cap && (h->log_max_records <= 0 || h->log_cap <= want)) break;
             h->log_cap = 0;
-            const DstPart parts[] = {{(void**)&h->log_keys, 8 * DST_CHUNK * (size_t)want}, {(void**)&h->log_next, sizeof(int) * (size_t)want}};
+            const size_t whole = (size_t)((want + 31) / 32 * 32);       // (32 records are interleaved; the limit is the number in use)
+            const DstPart parts[] = {{(void**)&h->log_keys, 8 * DST_CHUNK * whole}, {(void**)&h->log_next, sizeof(int) * whole}};
             if (alloc_log_parts(h, &h->log_block, parts, 2)) { h->log_cap = want; break; }
             if (h->logs_wanted <= 1) return DST_OK;
             h->logs_wanted = 1;

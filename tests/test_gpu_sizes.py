@@ -246,3 +246,19 @@ def test_room_for_several_logs_is_asked_for_only_while_they_are_used(C):
             torch.cuda.synchronize()
             held.setdefault(views, []).append(st.chunk_log()["records_held"])
     assert held[4][-2] > held[1][-2] and held[4][-1] == max(held[4][-2], held[1][-1]) and held[1][-1] > held[1][-2]
+
+
+@pytest.mark.parametrize("limit", [1, 31, 33, 1000])
+def test_log_holds_no_more_records_than_its_limit(C, limit):
+    """Limits that are no multiple of the 32 records that are interleaved: the rays that fit are taken from the log, the others re-traced."""
+    wc = hp.to_cuda(hp.workloads.make_workload(3, P=20_000, H=48, W=64))
+    st = _state(C, wc)
+    st.set_chunk_log_max_records(limit)
+    f = hp.cuda_forward(C, st, wc)
+    up, dg = dict(rgb=torch.ones_like(f["rgb"])), {}
+    logged = hp.cuda_backward(C, st, wc, f, up, diag=dg, serial=st.last_forward_serial)
+    traced = hp.cuda_backward(C, st, wc, f, up, serial=0)
+    torch.cuda.synchronize()
+    assert st.status() == 0 and st.chunk_log()["records_held"] == limit and int(dg["counters"][2]) > 0
+    for k in ("means3D", "shs", "opacities", "scales", "rotations", "ray_o"):
+        assert hp.rel_l2(logged[k].cpu().numpy(), traced[k].cpu().numpy()) < 1e-4, k
