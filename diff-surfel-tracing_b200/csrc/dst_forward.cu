@@ -986,7 +986,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     p.log_keys = nullptr; p.log_next = nullptr; p.log_count = nullptr; p.log_head = p.log_num = nullptr; p.log_ok = nullptr;
     p.log_cap = 0; p.log_slots = slots;
     h->log_serial = 0;
-    if (a->training && h->log_enabled) {
+    if (a->training && a->training != DST_TRAINING_NO_BACKWARD && h->log_enabled) {
         dst_handle::Log* log = nullptr;
         rc = dst_begin_log(h, &a->in, p.grid_h, p.grid_w, p.tiled, slots, &log, &begin.log_append);
         if (rc != DST_OK) return rc;

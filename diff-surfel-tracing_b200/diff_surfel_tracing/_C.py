@@ -17,6 +17,7 @@ _LIB_PATH = os.path.join(os.path.dirname(_PKG), "libdst_b200.so")
 
 NUM_CHANNELS = 3
 AUX_CHANNELS = 2
+TRAINING_NO_BACKWARD = 2      # DST_TRAINING_NO_BACKWARD, include/dst.h
 MID_CHANNELS = 16
 
 
@@ -333,11 +334,12 @@ def _inputs(state, i, start_from_first, ray_o, ray_d, vertices, background, mean
 def trace_surfels(state, training, start_from_first, ray_o, ray_d, vertices, background, means3D, shs, degree,
                   colors_precomp, others_precomp, opacities, scales, scale_modifier, rotations, transMat_precomp,
                   viewmatrix, projmatrix, campos, prefiltered, debug, max_trace_depth, specular_threshold,
-                  _diag=None):
+                  _diag=None, _log=True):
     """trace_surfels.cpp:162-304. Returns out_rgb, out_dpt, out_acc, out_norm, out_dist, out_aux, mid_val, a_weights.
 
     `mid_val` has 16 * max(2, max_trace_depth + 1) channels (the reference is compiled for one bounce
     and always returns 32). `_diag`, if a dict, receives per-ray hit logs and traversal counters.
+    `_log`: False when no backward will follow, so that none of the kept contribution logs makes way for this call's.
     """
     a = _FwdArgs()
     i = a.inp
@@ -355,7 +357,7 @@ def trace_surfels(state, training, start_from_first, ray_o, ray_d, vertices, bac
     out_aux = empty((H, W, AUX_CHANNELS), **f32)
     mid_val = empty((H, W, i.mid_stride), **f32)
     a_weights = empty((P, 1), **f32) if training else None
-    a.training = int(bool(training))
+    a.training = (1 if _log else TRAINING_NO_BACKWARD) if training else 0
     a.out_rgb, a.out_dpt, a.out_acc, a.out_norm = out_rgb.data_ptr(), out_dpt.data_ptr(), out_acc.data_ptr(), out_norm.data_ptr()
     a.out_dist, a.out_aux, a.mid_val = out_dist.data_ptr(), out_aux.data_ptr(), mid_val.data_ptr()
     a.a_weights = _ptr(a_weights)

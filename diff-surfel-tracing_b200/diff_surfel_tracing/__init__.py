@@ -30,13 +30,13 @@ def trace_surfels(optix_context, training, start_from_first, ray_o, ray_d, verti
             colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings)
     # rendering: nothing to record. Forward-mode derivatives and function transforms go through the autograd function, which refuses them
     if not torch.is_grad_enabled() and forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active():
-        return _forward(*args)[0]
+        return _forward(*args, log=False)[0]
     return _TraceSurfels.apply(*args)
 
 
 def _forward(optix_context, training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D, shs,
-             colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, s):
-    """The forward call: what the tracer returns, and the tensors its backward needs."""
+             colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, s, log):
+    """The forward call: what the tracer returns, and the tensors its backward needs. log: a backward may follow."""
     # image_width / image_height are unused by the reference's tracer; here they tell the kernels that a
     # (B, h*w, 3) ray batch consists of whole images, so that they can be walked in pixel tiles (scheduling only)
     iw, ih = int(s.image_width or 0), int(s.image_height or 0)
@@ -47,13 +47,13 @@ def _forward(optix_context, training, start_from_first, ray_o, ray_d, vertices, 
     if s.debug:
         cpu_args = cpu_deep_copy_tuple(args[1:])
         try:
-            out = _C.trace_surfels(*args)
+            out = _C.trace_surfels(*args, _log=log)
         except Exception as ex:
             torch.save(cpu_args, "snapshot_fw.dump")
             print("\nAn error occured in forward. Please forward snapshot_fw.dump for debugging.")
             raise ex
     else:
-        out = _C.trace_surfels(*args)
+        out = _C.trace_surfels(*args, _log=log)
     out_rgb, out_dpt, out_acc, out_norm, out_dist, out_aux, mid_val, a_weights = out
     acc_wet = a_weights if a_weights is not None else means3D.new_zeros(means3D.shape[0])
     return (out_rgb, out_dpt, out_acc, out_norm, out_dist[..., :1].clone(), out_aux, mid_val, acc_wet), out_dist
@@ -64,7 +64,8 @@ class _TraceSurfels(torch.autograd.Function):
     def forward(ctx, optix_context, training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D, shs,
                 colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings):
         result, out_dist = _forward(optix_context, training, start_from_first, ray_o, ray_d, vertices, means3D, grads3D, shs,
-                                    colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings)
+                                    colors_precomp, others_precomp, opacities, scales, rotations, cov3Ds_precomp, tracer_settings,
+                                    log=any(ctx.needs_input_grad))
         out_rgb, out_dpt, out_acc, out_norm, _, out_aux, mid_val, _ = result
         ctx.set_materialize_grads(False)       # outputs the loss does not use: None instead of a tensor of zeros
         ctx.tracer_settings = tracer_settings

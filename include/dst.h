@@ -79,9 +79,11 @@ typedef struct dst_trace_inputs {
     const float *rotations;       /* (P, 4) as (w, x, y, z)                                       */
 } dst_trace_inputs;
 
+#define DST_TRAINING_NO_BACKWARD 2      /* dst_fwd_args.training: no backward will follow, so no log is kept (and none displaced) */
 typedef struct dst_fwd_args {
     dst_trace_inputs in;
-    int32_t training;             /* accumulate per-surfel weights into a_weights                 */
+    int32_t training;             /* accumulate per-surfel weights into a_weights, and keep a contribution log for the
+                                     backward; DST_TRAINING_NO_BACKWARD: the weights only         */
     int32_t hit_cap;              /* slots per ray of hit_log                                     */
     /* outputs, all written for every ray (no pre-zeroing needed)                                 */
     float *out_rgb;               /* (H, W, 3)  */

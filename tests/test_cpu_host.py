@@ -384,8 +384,9 @@ def test_rendering_without_grad_mode_still_refuses_forward_mode_and_transforms(m
     import diff_surfel_tracing as dst
     ran = []
 
-    def forward(*args):
+    def forward(*args, log):
         ran.append(args)
+        assert not log
         out = tuple(torch.zeros(1, 1, c) for c in (3, 1, 1, 3, 1, 2, 32)) + (torch.zeros(2),)
         return out, torch.zeros(1, 1, 3)
 

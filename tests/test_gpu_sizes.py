@@ -262,3 +262,37 @@ def test_log_holds_no_more_records_than_its_limit(C, limit):
     assert st.status() == 0 and st.chunk_log()["records_held"] == limit and int(dg["counters"][2]) > 0
     for k in ("means3D", "shs", "opacities", "scales", "rotations", "ray_o"):
         assert hp.rel_l2(logged[k].cpu().numpy(), traced[k].cpu().numpy()) < 1e-4, k
+
+
+def test_training_forwards_without_a_backward_keep_no_log(C):
+    """Weights gathered under no_grad, or with nothing that takes a gradient: such calls leave no log behind, and the log of the forward
+    whose backward is still to come stays."""
+    from diff_surfel_tracing import SurfelTracer, SurfelTracingSettings
+    w = hp.workloads.make_workload(3, P=20_000, H=48, W=64)
+    wc = hp.to_cuda(w)
+    tracer = SurfelTracer()
+    tracer.build_acceleration_structure(wc["v"], wc["f"], rebuild=True)
+    e = torch.zeros(1, device="cuda")
+    settings = SurfelTracingSettings(48, 64, 1.0, 1.0, wc["bg"], 1.0, e, e, w["sh_degree"], e, False, False, w["max_trace_depth"], w["specular_threshold"])
+    names = ("shs", "others_precomp", "opacities", "scales", "rotations")
+
+    def trace(leaf):
+        p = {k: wc[k].clone().requires_grad_(leaf) for k in names}
+        return tracer(wc["ray_o"], wc["ray_d"], wc["v"], wc["means3D"], torch.zeros_like(wc["means3D"]), tracer_settings=settings, **p)
+
+    first = trace(True)
+    serial = tracer.optix_context.last_forward_serial
+    assert serial > 0
+    for k in range(6):
+        if k % 2:
+            out = trace(False)
+        else:
+            with torch.no_grad():
+                out = trace(True)
+        assert tracer.optix_context.last_forward_serial == 0
+        assert torch.equal(out[0], first[0]) and torch.allclose(out[7], first[7], rtol=1e-5)
+    diag = {}
+    hp.cuda_backward(C, tracer.optix_context, wc, dict(zip(hp.FWD_KEYS, (t.detach() for t in first))), dict(rgb=torch.ones_like(first[0])),
+                     diag=diag, serial=serial)
+    torch.cuda.synchronize()
+    assert tracer.optix_context.status() == 0 and int(diag["counters"][2]) == 0       # nothing was walked again
