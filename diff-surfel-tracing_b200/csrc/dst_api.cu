@@ -233,6 +233,7 @@ int dst_set_option(dst_handle* h, int option, int64_t value) {
         case DST_OPT_STABLE_LISTS: h->stable_lists = value != 0; return DST_OK;
         case DST_OPT_FORWARD_SLICES: h->fwd_slices = value < 0 ? 0 : (value > DST_MAX_SLICES ? DST_MAX_SLICES : (int)value); return DST_OK;
         case DST_OPT_CHUNK_LOG: h->log_enabled = value != 0; if (!h->log_enabled) dst_drop_logs(h); return DST_OK;
+        case DST_OPT_ABSENT_GRADIENTS: h->absent_gradients = value != 0; return DST_OK;
         case DST_OPT_KEPT_LOGS: h->logs_keep = value < 1 ? 1 : (value > DST_MAX_LOGS ? DST_MAX_LOGS : (int)value); return DST_OK;
         default: return dst_set_error(h, DST_E_ARG, "unknown option %d", option);
     }

@@ -827,6 +827,8 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     rc = backward_kernel_setup(h);
     if (rc != DST_OK) return rc;
     if (!a->out_rgb || !a->mid_val) return dst_set_error(h, DST_E_ARG, "a saved forward output pointer is null");
+    if (!h->absent_gradients && (!a->dL_drgb || !a->dL_ddpt || !a->dL_dacc || !a->dL_dnorm || !a->dL_daux))
+        return dst_set_error(h, DST_E_ARG, "an upstream gradient pointer is null");
     if (!a->dL_dray_o || !a->dL_dray_d || !a->dL_dmeans3D || !a->dL_dgrads3D || !a->dL_dcolors || !a->dL_dothers ||
         !a->dL_dopacities || !a->dL_dscales || !a->dL_drotations || (a->in.shs && !a->dL_dshs))
         return dst_set_error(h, DST_E_ARG, "a gradient output pointer is null");

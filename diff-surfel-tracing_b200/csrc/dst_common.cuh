@@ -112,6 +112,7 @@ struct dst_handle {
     int logs_wanted, logs_begun; bool logs_missed;
     size_t log_alloc_limit;       // test hook (dst_debug_log_alloc_limit)
     int log_enabled;
+    int absent_gradients;         // null upstream gradients are zeros (DST_OPT_ABSENT_GRADIENTS)
     long long log_max_records;    // user limit on the log size (0: only the built-in limit)
     int* log_needed_host; cudaEvent_t log_needed_event;     // pinned read-back of log_count after the last forward
     long long log_known_sig, log_known_needed;              // last completed read-back: call shape and records wanted (0: none yet)

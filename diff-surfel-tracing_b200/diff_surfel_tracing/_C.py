@@ -152,6 +152,7 @@ class OptiXStateWrapper:
         self.reduce_gradients = False   # sum the per-surfel gradients over `process_group` inside every backward call
         self.process_group = None
         self.grad_bucket = None     # flat buffer holding the per-surfel gradients of the last backward call
+        self.set_absent_gradients(True)
 
     def __del__(self):
         try:
@@ -215,6 +216,10 @@ class OptiXStateWrapper:
         """Training forwards whose contribution logs are kept until their backward comes (default 1: a forward replaces the log of
         the one before, whose backward then re-traces)."""
         _check(self, lib().dst_set_option(self.handle, 10, int(n)))
+
+    def set_absent_gradients(self, on):
+        """Upstream gradients given as None: zeros (what this module sets) or an error (the library's default)."""
+        _check(self, lib().dst_set_option(self.handle, 11, int(bool(on))))
 
     def profile(self, on=True):
         """Records CUDA events around the build, forward and backward kernels of later calls; on=2 also around

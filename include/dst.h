@@ -105,7 +105,8 @@ typedef struct dst_bwd_args {
     dst_trace_inputs in;
     /* state saved by the forward call */
     const float *out_rgb, *out_dpt, *out_acc, *out_norm, *out_dist, *out_aux, *mid_val;
-    /* upstream gradients, shapes of the forward outputs; dL_ddist is (H, W, 1), read only with DST_OPT_DISTORTION */
+    /* upstream gradients, shapes of the forward outputs; dL_ddist is (H, W, 1), read only with DST_OPT_DISTORTION, and may be
+       NULL; the others only with DST_OPT_ABSENT_GRADIENTS */
     const float *dL_drgb, *dL_ddpt, *dL_dacc, *dL_dnorm, *dL_ddist, *dL_daux;
     /* gradient outputs, fully written by the call (no pre-zeroing needed)                        */
     float *dL_dray_o, *dL_dray_d; /* (H, W, 3)                                                    */
@@ -251,6 +252,9 @@ int dst_bvh_info(const dst_handle* h, int64_t* surfels, int64_t* nodes, int64_t*
 /* Training forwards whose contribution logs the handle keeps until their backward comes (1, the default, to 4). With 1 a
  * forward replaces the log of the one before, whose backward then re-traces. */
 #define DST_OPT_KEPT_LOGS 10
+/* Upstream gradients of a backward that are null: 0 (default) is an error for all but dL_ddist, 1 takes them for zeros (the
+ * Python module sets it: outputs a loss does not use then need no tensor of zeros). */
+#define DST_OPT_ABSENT_GRADIENTS 11
 int dst_set_option(dst_handle* h, int option, int64_t value);
 
 /* Timing of the main kernels with CUDA events on the launching stream. While enabled, every

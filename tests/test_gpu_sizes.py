@@ -113,6 +113,24 @@ def test_missing_upstream_gradients_are_zeros_and_the_arena_stays_clean(C):
             assert hp.rel_l2(a[m], b[m]) < 1e-5, (P, k)
 
 
+@pytest.mark.parametrize("missing", ["rgb", "dpt", "acc", "norm", "aux"])
+def test_absent_upstream_gradients_are_an_error_unless_asked_for(C, missing):
+    """A library caller that forgets a pointer is told; the module switches the meaning to zeros for its own calls."""
+    wc = hp.to_cuda(hp.workloads.make_workload(1, P=2_000, H=32, W=32))
+    st = _state(C, wc)
+    f = hp.cuda_forward(C, st, wc)
+    up = {k: torch.ones((*f["rgb"].shape[:2], 2 if k == "aux" else f[k].shape[-1]), device="cuda") for k in ("rgb", "dpt", "acc", "norm", "aux")}
+    up[missing] = None
+    hp.cuda_backward(C, st, wc, f, up)
+    st.set_absent_gradients(False)
+    with pytest.raises(RuntimeError, match="upstream gradient pointer is null"):
+        hp.cuda_backward(C, st, wc, f, up)
+    up[missing] = torch.ones((*f["rgb"].shape[:2], 2 if missing == "aux" else f[missing].shape[-1]), device="cuda")
+    hp.cuda_backward(C, st, wc, f, dict(up, dist=None))
+    torch.cuda.synchronize()
+    assert st.status() == 0
+
+
 @pytest.mark.parametrize("coeffs,degree", [(16, 3), (16, 1), (9, 2), (4, 1)])
 def test_composite_build_for_large_calls(C, coeffs, degree):
     """The composite kernel runs another build from 921,600 rays on: each row of rays comes out as in a call below that, for SH rows of
