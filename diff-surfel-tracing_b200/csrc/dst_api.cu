@@ -292,14 +292,15 @@ int dst_debug_round_counts(dst_handle* h, int32_t* counts, int32_t cap, void* st
     if (!h || !counts || cap < 0) return DST_E_ARG;
     if (!h->wf_counts) return dst_set_error(h, DST_E_STATE, "no trace call has run on this handle");
     DeviceGuard g(h->device);
-    const int n = cap < 300 ? cap : 300;      // DST_WF_ROUNDS + 2 list lengths
+    constexpr int rounds = DST_WF_ROUNDS + 2, stride = DST_COUNTS_STRIDE;      // list lengths come first in a set of counters; the cursors behind them are not reported
+    const int n = cap < rounds ? cap : rounds;
     // one set of counters per slice of the last forward call (one set for every other call): the lengths add up
-    int32_t all[DST_MAX_SLICES * 300];
+    int32_t all[DST_MAX_SLICES * stride];
     const int sets = h->slices_used > 1 ? h->slices_used : 1;
-    DST_CUDA_TRY(h, cudaMemcpyAsync(all, h->wf_counts, sizeof(int32_t) * 300 * (size_t)sets, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    DST_CUDA_TRY(h, cudaMemcpyAsync(all, h->wf_counts, sizeof(int32_t) * stride * (size_t)sets, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     DST_CUDA_TRY(h, cudaStreamSynchronize((cudaStream_t)stream));
     for (int i = 0; i < cap; i++) counts[i] = 0;
-    for (int g = 0; g < sets; g++) for (int i = 0; i < n; i++) counts[i] += all[g * 300 + i];
+    for (int g = 0; g < sets; g++) for (int i = 0; i < n; i++) counts[i] += all[g * stride + i];
     return DST_OK;
 }
 

@@ -43,6 +43,8 @@ struct SurfelCacheView { const float4* rec; };
 #define DST_ARENA_FLOATS 20
 #define DST_LOG_MAX_RECORDS (320ll << 20)     // 132 B each: at most 44.3 GB of contribution log
 
+#define DST_WF_ROUNDS 48              // most wavefront rounds of a call
+#define DST_COUNTS_STRIDE (6 * (DST_WF_ROUNDS + 2))      // ints per set of round counters: list lengths, batch cursors, rays given up by the batches, their cursor
 #define DST_MAX_SLICES 8
 #define DST_MAX_LOGS 4                 // forwards whose contribution logs a handle can keep at once
 struct dst_handle {

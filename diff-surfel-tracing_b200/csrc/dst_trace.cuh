@@ -348,9 +348,7 @@ constexpr int ENUM_THREADS = 128;
 #ifndef DST_ENUM_MIN_BLOCKS
 #define DST_ENUM_MIN_BLOCKS 8         // resident blocks per SM the gather kernel is compiled for
 #endif
-#define DST_WF_ROUNDS 48
 #define DST_TAIL_CURSOR (DST_COUNTS_STRIDE - 1)          // word of a set of round counters no round uses: next list entry of the tail kernel
-#define DST_COUNTS_STRIDE (6 * (DST_WF_ROUNDS + 2))      // ints per set of round counters: list lengths, batch cursors, rays given up by the batches, their cursor
 
 // ---------------------------------------------------------------------------------------------
 // Gather: per live ray, the 16 nearest hits from the requested origin (same result as knearest()).

@@ -314,3 +314,16 @@ def test_training_forwards_without_a_backward_keep_no_log(C):
                      diag=diag, serial=serial)
     torch.cuda.synchronize()
     assert tracer.optix_context.status() == 0 and int(diag["counters"][2]) == 0       # nothing was walked again
+
+
+def test_round_counts_hold_list_lengths_only(C):
+    """A caller's array longer than the list lengths is filled up with zeros, not with the counters that lie behind them."""
+    import ctypes
+    wc = hp.to_cuda(hp.workloads.make_workload(3, P=20_000, H=96, W=128))
+    st = _state(C, wc, wave=True)
+    hp.cuda_forward(C, st, wc)
+    buf = (ctypes.c_int32 * 300)(*[-1] * 300)
+    assert C.lib().dst_debug_round_counts(st.handle, buf, 300, None) == 0
+    short = st.round_counts()
+    assert len(short) > 1 and short == sorted(short, reverse=True)
+    assert list(buf) == short + [0] * (300 - len(short))
