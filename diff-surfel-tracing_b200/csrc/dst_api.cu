@@ -101,16 +101,15 @@ int dst_create(int device, dst_handle** out) {
 int dst_destroy(dst_handle* h) {
     if (!h) return DST_OK;
     DeviceGuard g(h->device);
-    cudaFree(h->build_block);
-    cudaFree(h->header); cudaFree(h->status); cudaFree(h->cache); cudaFree(h->arena); cudaFree(h->wsum); cudaFree(h->cam_dev);
+    cudaFree(h->header); cudaFree(h->status);
+    for (void* p : {(void*)h->build_block, (void*)h->cache, (void*)h->arena, (void*)h->wsum, h->cam_dev, (void*)h->log_block, (void*)h->log_count, h->wf_block, (void*)h->bound_stats})
+        dst_mem_free(h, p);
+    for (int k = 0; k < DST_MAX_LOGS; k++) dst_mem_free(h, h->logs[k].index_block);
+    cudaFree(h->slab);
     if (h->log_needed_host) cudaFreeHost(h->log_needed_host);
     if (h->log_needed_event) cudaEventDestroy(h->log_needed_event);
     if (h->rounds_host) cudaFreeHost(h->rounds_host);
     if (h->rounds_event) cudaEventDestroy(h->rounds_event);
-    cudaFree(h->log_block); cudaFree(h->log_count);
-    for (int k = 0; k < DST_MAX_LOGS; k++) cudaFree(h->logs[k].index_block);
-    cudaFree(h->wf_block);
-    cudaFree(h->bound_stats);
     if (h->bound_host) cudaFreeHost(h->bound_host);
     if (h->bound_event) cudaEventDestroy(h->bound_event);
     if (h->slice_streams_ready) {
@@ -329,6 +328,12 @@ int dst_debug_read_bandwidth(dst_handle* h, int64_t bytes, int reps, float* gb_p
     if (e1) cudaEventDestroy(e1);
     cudaFree(buf); cudaFree(sink);
     return rc;
+}
+
+int dst_debug_device_allocations(const dst_handle* h, int64_t* allocations) {
+    if (!h || !allocations) return DST_E_ARG;
+    *allocations = h->mapped;
+    return DST_OK;
 }
 
 int dst_debug_log_alloc_limit(dst_handle* h, int64_t bytes) {

@@ -838,9 +838,9 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
         return dst_set_error(h, DST_E_ARG, "mid_val, vertices, rotations and dL_drotations must be 16-byte aligned");
     const int64_t P = a->in.P;
     if (P > h->arena_cap) {
-        cudaFree(h->arena); h->arena = nullptr; h->arena_cap = 0;
+        dst_mem_free(h, h->arena); h->arena = nullptr; h->arena_cap = 0;
         const int64_t cap = P + P / 8 + 1024;
-        if (cudaMalloc(&h->arena, 4 * DST_ARENA_FLOATS * cap) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "gradient arena allocation failed"); }
+        if (dst_mem_alloc(h, (void**)&h->arena, 4 * DST_ARENA_FLOATS * cap) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "gradient arena allocation failed"); }
         h->arena_cap = cap; h->arena_clean = false;
     }
     if (!h->arena_clean) DST_CUDA_TRY(h, cudaMemsetAsync(h->arena, 0, 4 * DST_ARENA_FLOATS * (size_t)h->arena_cap, st));

@@ -451,7 +451,10 @@ int ensure_capacity(dst_handle* h, int64_t P) {
         {(void**)&h->leaf_parent, 4 * (size_t)cap}, {(void**)&h->arrive, 4 * (size_t)cap}, {(void**)&h->node_parent, 4 * (size_t)cap},
         {(void**)&h->keys, 8 * (size_t)cap}, {(void**)&h->keys_alt, 8 * (size_t)cap}, {(void**)&h->vals, 4 * (size_t)cap}, {(void**)&h->vals_alt, 4 * (size_t)cap},
         {(void**)&h->block_hist, 4 * 256 * (size_t)(nblocks + 1)}};       // + the 256 digit totals
-    const cudaError_t e = dst_alloc_parts(&h->build_block, parts, sizeof(parts) / sizeof(parts[0]));
+    size_t total = 0;
+    for (const DstPart& part : parts) total += part.bytes;
+    if (total <= DST_SLAB_BUILD) dst_open_slab(h);
+    const cudaError_t e = dst_alloc_parts(h, &h->build_block, parts, sizeof(parts) / sizeof(parts[0]));
     if (e != cudaSuccess) {
         cudaGetLastError();
         return dst_set_error(h, DST_E_NOMEM, "device allocation for %lld surfels failed: %s", (long long)P, cudaGetErrorString(e));

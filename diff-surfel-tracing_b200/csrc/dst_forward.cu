@@ -765,9 +765,9 @@ int dst_check_inputs(dst_handle* h, const dst_trace_inputs* in) {
 
 static int ensure_cache(dst_handle* h, const dst_trace_inputs* in) {
     if (in->P > h->cache_cap) {
-        cudaFree(h->cache); h->cache = nullptr; h->cache_cap = 0;
+        dst_mem_free(h, h->cache); h->cache = nullptr; h->cache_cap = 0;
         const int64_t cap = in->P + in->P / 8 + 1024;
-        if (cudaMalloc(&h->cache, 64 * cap) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "surfel cache allocation failed"); }
+        if (dst_mem_alloc(h, (void**)&h->cache, 64 * cap) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "surfel cache allocation failed"); }
         h->cache_cap = cap;
     }
     h->cache_serial = 0;
@@ -794,7 +794,7 @@ int dst_ensure_wavefront(dst_handle* h, long long slots, size_t state_bytes) {
         {&h->wf_state, sb * (size_t)cap}, {&h->wf_req, 32 * (size_t)cap}, {(void**)&h->wf_kbuf, 8 * DST_CHUNK * (size_t)cap}, {(void**)&h->wf_kcnt, 4 * (size_t)cap},
         {(void**)&h->wf_list[0], 4 * (size_t)cap}, {(void**)&h->wf_list[1], 4 * (size_t)cap}, {(void**)&h->wf_counts, 4 * (size_t)DST_COUNTS_STRIDE * DST_MAX_SLICES},
         {(void**)&h->wf_tmp, 4 * (size_t)(cap + 32)}, {(void**)&h->wf_wcnt, 4 * (size_t)(cap / 32 + 2)}, {(void**)&h->wf_bcnt, 4 * 2 * (size_t)dst_live_blocks(cap)}};
-    const cudaError_t e = dst_alloc_parts(&h->wf_block, parts, sizeof(parts) / sizeof(parts[0]));
+    const cudaError_t e = dst_alloc_parts(h, &h->wf_block, parts, sizeof(parts) / sizeof(parts[0]));
     if (e != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "ray scratch allocation for %lld rays failed: %s", slots, cudaGetErrorString(e)); }
     h->wf_cap = cap; h->wf_state_bytes = sb;
     return DST_OK;
@@ -833,12 +833,12 @@ void dst_drop_logs(dst_handle* h) {
 }
 
 // Log buffers: false where the device has no room for them (or a test says so).
-static bool alloc_log_parts(const dst_handle* h, void** block, const DstPart* parts, int n) {
+static bool alloc_log_parts(dst_handle* h, void** block, const DstPart* parts, int n) {
     size_t total = 0;
     for (int k = 0; k < n; k++) total += parts[k].bytes;
     const bool full = h->log_alloc_limit && total > h->log_alloc_limit;
-    if (full) { cudaFree(*block); *block = nullptr; }
-    if (!full && dst_alloc_parts(block, parts, n) == cudaSuccess) return true;
+    if (full) { dst_mem_free(h, *block); *block = nullptr; }
+    if (!full && dst_alloc_parts(h, block, parts, n) == cudaSuccess) return true;
     cudaGetLastError();
     for (int k = 0; k < n; k++) *parts[k].p = nullptr;
     return false;
@@ -886,7 +886,7 @@ int dst_begin_log(dst_handle* h, const dst_trace_inputs* in, int grid_h, int gri
             if (h->logs_wanted <= 1) return DST_OK;
             h->logs_wanted = 1;
         }
-        if (!h->log_count && cudaMalloc(&h->log_count, 8) != cudaSuccess) { cudaGetLastError(); h->log_count = nullptr; return DST_OK; }
+        if (!h->log_count && dst_mem_alloc(h, (void**)&h->log_count, 8) != cudaSuccess) { cudaGetLastError(); h->log_count = nullptr; return DST_OK; }
     }
     dst_handle::Log& l = h->logs[h->logs_used];
     if (slots * segs > l.index_cap) {
@@ -944,7 +944,7 @@ int dst_pinhole_rays_impl(dst_handle* h, const dst_camera* cams, int n_cameras, 
     const long long total = (long long)n_cameras * H * W;
     if (total > 0x3fffffffll) return dst_set_error(h, DST_E_ARG, "too many rays");
     if (!h->cam_dev) {
-        if (cudaMalloc(&h->cam_dev, sizeof(CamConst) * DST_MAX_CAMERAS) != cudaSuccess) { cudaGetLastError(); h->cam_dev = nullptr; return dst_set_error(h, DST_E_NOMEM, "camera buffer allocation failed"); }
+        if (dst_mem_alloc(h, &h->cam_dev, sizeof(CamConst) * DST_MAX_CAMERAS) != cudaSuccess) { cudaGetLastError(); h->cam_dev = nullptr; return dst_set_error(h, DST_E_NOMEM, "camera buffer allocation failed"); }
     }
     // a copy from pageable host memory has left the source buffer when the call returns, so a local array will do
     CamConst stage[DST_MAX_CAMERAS];
@@ -1050,7 +1050,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     p.bound_stats = nullptr; p.bound_factor = 0.0f;
     if (wave && DST_BOUND_FACTOR > 0.0f) {
         if (!h->bound_stats) {
-            if (cudaMalloc(&h->bound_stats, 8) != cudaSuccess) { cudaGetLastError(); h->bound_stats = nullptr; }
+            if (dst_mem_alloc(h, (void**)&h->bound_stats, 8) != cudaSuccess) { cudaGetLastError(); h->bound_stats = nullptr; }
             if (h->bound_stats && cudaMallocHost(&h->bound_host, 8) != cudaSuccess) { cudaGetLastError(); h->bound_host = nullptr; }
             if (h->bound_host && cudaEventCreateWithFlags(&h->bound_event, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); h->bound_event = nullptr; }
         }
@@ -1065,9 +1065,9 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     double wunit = 0.0;
     if (wave && a->training && a->a_weights) {
         if (a->in.P > h->wsum_cap) {
-            cudaFree(h->wsum); h->wsum = nullptr; h->wsum_cap = 0;
+            dst_mem_free(h, h->wsum); h->wsum = nullptr; h->wsum_cap = 0;
             const int64_t cap = a->in.P + a->in.P / 8 + 1024;
-            if (cudaMalloc(&h->wsum, 8 * cap) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "weight sum allocation failed"); }
+            if (dst_mem_alloc(h, (void**)&h->wsum, 8 * cap) != cudaSuccess) { cudaGetLastError(); return dst_set_error(h, DST_E_NOMEM, "weight sum allocation failed"); }
             h->wsum_cap = cap; h->wsum_clean = false;
         }
         if (!h->wsum_clean) DST_CUDA_TRY(h, cudaMemsetAsync(h->wsum, 0, 8 * (size_t)h->wsum_cap, st));

@@ -68,6 +68,7 @@ def lib():
         l.dst_build.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_int, C.c_void_p]
         l.dst_forward.argtypes = [C.c_void_p, C.POINTER(_FwdArgs), C.c_void_p]
         l.dst_backward.argtypes = [C.c_void_p, C.POINTER(_BwdArgs), C.c_void_p]
+        l.dst_debug_device_allocations.argtypes = [C.c_void_p, C.POINTER(C.c_int64)]
         l.dst_debug_log_alloc_limit.argtypes = [C.c_void_p, C.c_int64]
         l.dst_forward_static.argtypes = [C.c_void_p, C.POINTER(_FwdArgs), C.c_void_p]
         l.dst_surfel_quads.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
@@ -262,6 +263,12 @@ class OptiXStateWrapper:
         a, b, c = C.c_int64(), C.c_int64(), C.c_int64()
         _check(self, lib().dst_debug_chunk_log(self.handle, C.byref(a), C.byref(b), C.byref(c)))
         return dict(records_wanted=a.value, records_held=b.value, bytes_per_record=c.value)
+
+    def device_allocations(self):
+        """Device allocations this state has made since it was created."""
+        n = C.c_int64(0)
+        _check(self, lib().dst_debug_device_allocations(self.handle, C.byref(n)))
+        return n.value
 
     def set_log_alloc_limit(self, nbytes):
         """Test hook: allocations of the contribution log above `nbytes` fail as on a full device (0: none do)."""

@@ -290,6 +290,9 @@ int dst_debug_read_bandwidth(dst_handle* h, int64_t bytes, int reps, float* gb_p
  * (-1: not known yet), records the log can hold, bytes per record. Rays whose records did not fit are re-traced
  * by the backward. */
 int dst_debug_chunk_log(const dst_handle* h, int64_t* records_wanted, int64_t* records_held, int64_t* bytes_per_record);
+/* Diagnostics: device allocations the handle has made since its creation. A handle whose first build is small makes one and takes the
+ * buffers of its calls from it while it lasts. */
+int dst_debug_device_allocations(const dst_handle* h, int64_t* allocations);
 /* Test hook: allocations of the contribution log above `bytes` fail as on a full device (0: none do). A training forward then makes
  * do with a smaller log, or with none: the backward re-traces. */
 int dst_debug_log_alloc_limit(dst_handle* h, int64_t bytes);

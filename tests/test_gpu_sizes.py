@@ -327,3 +327,32 @@ def test_round_counts_hold_list_lengths_only(C):
     short = st.round_counts()
     assert len(short) > 1 and short == sorted(short, reverse=True)
     assert list(buf) == short + [0] * (300 - len(short))
+
+
+def test_first_steps_of_a_small_state_map_memory_once(C):
+    """Build, forward and backward of a new state with 10,000 surfels and 128 x 128 rays: one device allocation. Buffers that grow from call to
+    call move to other places of it and then out of it; the results are a fresh state's."""
+    w = hp.workloads.make_workload(1)
+    wc = hp.to_cuda(w)
+    st = _state(C, wc)
+    f = hp.cuda_forward(C, st, wc)
+    hp.cuda_backward(C, st, wc, f, dict(rgb=torch.ones_like(f["rgb"])), serial=st.last_forward_serial)
+    assert st.device_allocations() == 1
+    torch.cuda.synchronize()
+    st = C.OptiXStateWrapper("")
+    for P, side in ((500, 32), (2_000, 48), (5_000, 130), (20_000, 260), (45_000, 300), (120_000, 64), (1_000, 40)):
+        wc = hp.to_cuda(hp.workloads.make_workload(3, P=P, H=side, W=side))
+        C.build_acceleration_structure(st, wc["v"], wc["f"], 1)
+        fresh = _state(C, wc)
+        got = []
+        for s in (st, fresh):
+            f = hp.cuda_forward(C, s, wc)
+            g = hp.cuda_backward(C, s, wc, f, dict(rgb=torch.ones_like(f["rgb"])), serial=s.last_forward_serial)
+            got.append((f, g))
+        torch.cuda.synchronize()
+        assert st.status() == 0
+        for k in ("rgb", "dpt", "acc", "norm", "mid"):
+            assert torch.equal(got[0][0][k], got[1][0][k]), (P, k)
+        for k in ("means3D", "shs", "opacities", "scales", "rotations", "ray_o"):
+            assert hp.rel_l2(got[0][1][k].cpu().numpy(), got[1][1][k].cpu().numpy()) < 1e-5, (P, k)
+    assert st.device_allocations() > 1
