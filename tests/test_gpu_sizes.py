@@ -131,21 +131,45 @@ def test_absent_upstream_gradients_are_an_error_unless_asked_for(C, missing):
     assert st.status() == 0
 
 
+def _slots(H, W):
+    """List slots of an image: whole blocks of 64 x 32 pixels."""
+    return -(-W // 64) * -(-H // 32) * 2048
+
+
 @pytest.mark.parametrize("coeffs,degree", [(16, 3), (16, 1), (9, 2), (4, 1)])
 def test_composite_build_for_large_calls(C, coeffs, degree):
-    """The composite kernel runs another build from 921,600 rays on: each row of rays comes out as in a call below that, for SH rows of
+    """The composite kernel runs another build from 921,600 list slots on: each row of rays comes out as in a call below that, for SH rows of
     every alignment."""
     w = hp.workloads.make_workload(3, P=20_000, H=960, W=960)
+    assert _slots(960, 960) >= 900 << 10 > _slots(928, 960)
     wc = hp.to_cuda(w)
     wc["shs"], wc["sh_degree"] = wc["shs"][:, :coeffs].contiguous(), degree
     st = _state(C, wc)
     large = hp.cuda_forward(C, st, wc, training=False)
-    part = dict(wc, ray_o=wc["ray_o"][:952].contiguous(), ray_d=wc["ray_d"][:952].contiguous())
+    part = dict(wc, ray_o=wc["ray_o"][:928].contiguous(), ray_d=wc["ray_d"][:928].contiguous())
     small = hp.cuda_forward(C, st, part, training=False)
     torch.cuda.synchronize()
     assert st.status() == 0 and float(large["acc"].max()) > 0.5
     for k in ("rgb", "dpt", "acc", "norm", "mid"):
-        assert torch.equal(large[k][:952], small[k]), k
+        assert torch.equal(large[k][:928], small[k]), k
+
+
+def test_weight_sums_of_large_calls_against_64_bits(C):
+    """The per-surfel weights of a call in fixed point against sums in 64 bits of what calls of four rows each give. Bounds: a contribution is
+    at least 1e-4 / 255 and rounded to 2^-41 (1.2e-6 of it), the result and the parts to 2^-24; sums of 216,200 rays in float are off by
+    9e-7 in the 2-norm here."""
+    wc = hp.to_cuda(hp.workloads.make_workload(3, P=30_000, H=460, W=470))
+    st = _state(C, wc)
+    wet = hp.cuda_forward(C, st, wc)["wet"].double()
+    parts = _state(C, wc, wave=False)
+    want = torch.zeros_like(wet)
+    for r in range(0, 460, 4):
+        part = dict(wc, ray_o=wc["ray_o"][r:r + 4].contiguous(), ray_d=wc["ray_d"][r:r + 4].contiguous())
+        want += hp.cuda_forward(C, parts, part)["wet"].double()
+    torch.cuda.synchronize()
+    assert st.status() == 0 and int((want > 0).sum()) > 10_000
+    assert float((wet - want).norm() / want.norm()) < 3e-7
+    assert float(((wet - want).abs() - 2e-6 * want).max()) <= 0.0
 
 
 def test_logged_hits_that_no_longer_contribute(C):
