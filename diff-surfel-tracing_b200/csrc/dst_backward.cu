@@ -877,7 +877,7 @@ int dst_backward_impl(dst_handle* h, const dst_bwd_args* a, cudaStream_t st) {
     DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_counts, 0, 4 * DST_COUNTS_STRIDE, st));
     h->slices_used = 1;
     const bool wave = slots >= h->wf_min_rays;
-    rc = dst_live_lists(h, slots, &p.lv, st);
+    rc = dst_live_lists(h, &p.lv, st);
     if (rc != DST_OK) return rc;
     const int g_compact = (int)((slots + DST_LIVE_BLOCK - 1) / DST_LIVE_BLOCK);
     p.rounds = wave ? DST_WF_ROUNDS : 0;

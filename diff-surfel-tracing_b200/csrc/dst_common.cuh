@@ -36,7 +36,6 @@ struct BvhView {
 // training step): rows of the tangent frame, the frame origin, opacity and scales, 64 B so that
 // one evaluated hit costs two 32-byte sectors instead of four scattered gathers.
 //   f4[0] = (R0.xyz, T.x)  f4[1] = (R1.xyz, T.y)  f4[2] = (R2.xyz, opacity)  f4[3] = (sx, sy, 1/sx, 1/sy)
-struct SurfelCacheView { const float4* rec; };
 
 // packed per-surfel gradient rows (16-byte aligned so that 4-float vector reductions apply):
 //   [0..3] rotation  [4..6] mean  [7] opacity  [8..10] grads3D  [11] -  [12..13] scale  [14..15] others  [16..18] colour  [19] -

@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(SHADE_THREADS, BLOCKS) k_fwd_shade(const __gri
 }
 
 // runs every ray of the first list the wavefront left alone to completion, one thread per ray
-template <bool BRUTE, bool DIAG>
+template <bool DIAG>
 __global__ void __launch_bounds__(TAIL_THREADS) k_fwd_tail(const __grid_constant__ FwdParams p) {
     __shared__ unsigned long long kshared[DST_CHUNK * TAIL_THREADS];
     const int round = first_skipped_round(p.counts, p.rounds, p.min_count);
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_fwd_tail(const __grid_constant
             if (alive) {
                 EnumReq q;
                 fwd_request(s, q);
-                cnt = knearest<BRUTE, DIAG, TAIL_THREADS>(p.bvh, q.ox, q.oy, q.oz, q.dx, q.dy, q.dz, kb, p.status, tc, q.kmax0);
+                cnt = knearest<false, DIAG, TAIL_THREADS>(p.bvh, q.ox, q.oy, q.oz, q.dx, q.dy, q.dz, kb, p.status, tc, q.kmax0);
                 if (DIAG) tc.enums++;
             }
             __syncwarp();
@@ -801,12 +801,11 @@ int dst_ensure_wavefront(dst_handle* h, long long slots, size_t state_bytes) {
 }
 
 // the list hand-over buffers of the handle as the kernels see them; clears both sets of block counters
-int dst_live_lists(dst_handle* h, long long slots, LiveLists* lv, cudaStream_t st) {
+int dst_live_lists(dst_handle* h, LiveLists* lv, cudaStream_t st) {
     lv->tmp = h->wf_tmp; lv->wcnt = h->wf_wcnt;
     lv->bcnt[0] = h->wf_bcnt; lv->bcnt[1] = h->wf_bcnt + dst_live_blocks(h->wf_cap);
     lv->stable = h->stable_lists;
     if (lv->stable) DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_bcnt, 0, 4 * 2 * (size_t)dst_live_blocks(h->wf_cap), st));
-    (void)slots;
     return DST_OK;
 }
 
@@ -1080,7 +1079,7 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
     memset(&p.lv, 0, sizeof(p.lv));
     if (wave) {       // (a call without rounds uses two of the counters, which k_fwd_begin sets)
         DST_CUDA_TRY(h, cudaMemsetAsync(h->wf_counts, 0, 4 * (size_t)DST_COUNTS_STRIDE * DST_MAX_SLICES, st));
-        rc = dst_live_lists(h, slots, &p.lv, st);
+        rc = dst_live_lists(h, &p.lv, st);
         if (rc != DST_OK) return rc;
     }
     dst_prof_mark(h, 1, 0, st);
@@ -1136,8 +1135,8 @@ static int forward_common(dst_handle* h, const dst_fwd_args* a, const dst_camera
             else k_fwd_tail_warp<false><<<g_wtail, WTAIL_THREADS, 0, sst[g]>>>(q);
         } else {
             const int g_tail = dst_wavefront_grid(h, tail_rays, TAIL_THREADS, 8);
-            if (diag) k_fwd_tail<false, true><<<g_tail, TAIL_THREADS, 0, sst[g]>>>(q);
-            else k_fwd_tail<false, false><<<g_tail, TAIL_THREADS, 0, sst[g]>>>(q);
+            if (diag) k_fwd_tail<true><<<g_tail, TAIL_THREADS, 0, sst[g]>>>(q);
+            else k_fwd_tail<false><<<g_tail, TAIL_THREADS, 0, sst[g]>>>(q);
         }
     }
     for (int g = 1; g < nsl; g++) {
@@ -1274,8 +1273,8 @@ extern "C" int dst_forward_static(dst_handle* h, const dst_fwd_args* a, void* st
         else k_fwd_tail_warp<false><<<g_wtail, WTAIL_THREADS, 0, st>>>(p);
     } else {
         const int g_tail = dst_wavefront_grid(h, slots, TAIL_THREADS, 8);
-        if (diag) k_fwd_tail<false, true><<<g_tail, TAIL_THREADS, 0, st>>>(p);
-        else k_fwd_tail<false, false><<<g_tail, TAIL_THREADS, 0, st>>>(p);
+        if (diag) k_fwd_tail<true><<<g_tail, TAIL_THREADS, 0, st>>>(p);
+        else k_fwd_tail<false><<<g_tail, TAIL_THREADS, 0, st>>>(p);
     }
     DST_CUDA_TRY(h, cudaGetLastError());
     h->launches += 2;

@@ -951,7 +951,7 @@ struct LiveLists {
     int stable;          // 0: append_alive() order (atomic per warp)
 };
 static inline long long dst_live_blocks(long long slots) { return slots / DST_LIVE_BLOCK + 2; }
-int dst_live_lists(dst_handle* h, long long slots, LiveLists* lv, cudaStream_t st);
+int dst_live_lists(dst_handle* h, LiveLists* lv, cudaStream_t st);
 
 // called by all 32 lanes of a warp for 32 consecutive list positions (i of lane 0 is a multiple of 32)
 __device__ __forceinline__ void live_out(const LiveLists& lv, int round, int i, bool alive, int ray, int cls) {
