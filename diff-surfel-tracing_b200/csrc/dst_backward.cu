@@ -2,12 +2,11 @@
 // traceRay 332-655 and its helpers) and the host launcher TraceSurfelsBackwardCUDA
 // (trace_surfels.cpp:307-464).
 //
-// Bounces are visited last to first; each segment is re-traced front to back with the forward
-// kernel's exact decision code (eval_slot), and every contributing hit adds its gradients. As in
-// the forward trace the per-ray loop is a state machine run as wavefront rounds (k_enum gathers,
-// k_bwd_shade composites and differentiates) with a one-thread-per-ray tail. Per-surfel gradients go to a packed arena of 16-byte aligned rows with 4-float
-// vector reductions (5 per contribution instead of 18 scalar atomics; SH rows 12 instead of 48),
-// and are unpacked into the caller's tensors by a streaming kernel afterwards.
+// Bounces are visited last to first, each segment front to back with the forward kernel's exact evaluation (eval_slot), and every
+// contributing hit adds its gradients. Where the forward left a contribution log, k_bwd_logged composites it again; rays without one are
+// traced again as wavefront rounds (the gather kernels, k_bwd_shade) with a tail of one warp per few rays. Per-surfel gradients go to
+// a packed arena of 16-byte aligned rows: rows are staged in shared memory, those of lanes with the same surfel added up there, and
+// leave as one bulk reduction each (see send_rows); a streaming kernel unpacks the arena into the caller's tensors afterwards.
 #include "dst_trace.cuh"
 
 namespace {

@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(256) k_sort_scan(unsigned int* __restrict__ bl
 
 // Stable scatter: warp w of a block owns 512 consecutive keys and ranks them 32 at a time. The block's keys are put in digit order in
 // shared memory first, so that what a digit gets from this block (16 keys on average) is written as one run: written straight from the
-// registers every key was a memory sector of its own (51 -> 27 us per pass at 3M keys).
+// registers every key was a memory sector of its own (3M keys, mean of the eight passes: 63 -> 42 us under ncu).
 struct SortTile { unsigned long long key[SORT_TILE]; unsigned int val[SORT_TILE]; unsigned short wc[SORT_WARPS][256]; unsigned int start[256], base[256], sum[SORT_WARPS]; };
 __device__ __forceinline__ unsigned int scan256(unsigned int x, unsigned int* warp_sum) {       // exclusive, over the 256 threads of the block
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256) k_surfel_quads(SurfelSource src, int P, i
 // written to the caller's vertex buffer on the way (the refit then never reads the vertices).
 //
 // Nodes whose leaves all lie in one block (all but one in a hundred) are merged through shared memory; only the rest exchange boxes and
-// arrivals through the L2, where a level costs a fence and an atomic, about a microsecond (406 -> 250 us at 3M surfels).
+// arrivals through the L2, where a level costs a fence and an atomic, about a microsecond (3M surfels, under ncu: 495 -> 319 us).
 template <bool FROM_SURFELS>
 __global__ void __launch_bounds__(REFIT_THREADS) k_refit(const float* __restrict__ verts, SurfelSource src, int P, const unsigned int* __restrict__ vals,
                                                BvhNode* nodes, const int* __restrict__ leaf_parent, const int* __restrict__ node_parent,
@@ -526,7 +526,7 @@ int dst_bvh_build_impl(dst_handle* h, const float* v, int64_t P, int rebuild, cu
         h->P = P;
     } else if (from_surfels && !h->single_kernel_refit) {
         // measured at 3M surfels: the coalesced expansion pass (0.07 ms) plus the refit's gathered re-read of the
-        // vertices is faster than one kernel that scatters 48-byte vertex writes in Morton order (0.57 vs 0.64 ms)
+        // vertices is faster than one kernel that scatters 48-byte vertex writes in Morton order (0.47 vs 0.59 ms)
         k_surfel_quads<<<grid, tpb, 0, st>>>(src, n, nullptr);
     }
     DST_CUDA_TRY(h, cudaMemsetAsync(h->arrive, 0, 4 * (size_t)(n > 1 ? n - 1 : 1), st));

@@ -21,9 +21,10 @@
 #define DST_WARP_TAIL_MAX_RAYS 32768   // up to this many rays the tail kernel runs one warp per ray
 #endif
 // Slices of a forward call (see forward_common): up to 4 from DST_SLICE_LARGE_SLOTS ray slots on, up to 6 below, none under DST_SLICE_MIN_SLOTS
-// slots. Below a million rays a round is short and mostly its slowest batch, which more slices cover: 0.64M rays of an object in 2 slices
-// 4.7 ms, 4 4.35, 5 4.2, 6 4.15, 8 4.1; 0.93M reflective rays in 3 15.5, 6 15.05. 2M reflective rays in 3 17.1, 4 16.9, 6 17.1; with two
-// bounces 85.6, 86.1, 87.0. Slices of 40,000 cost more launches than they cover (0.16M rays in one slice 3.6 ms, in 4 4.8).
+// slots. Below a million rays a round is short and mostly its slowest batch, which more slices cover. Forward of an object (0.5M surfels) | of
+// a reflective scene (1M, one bounce), ms in 4 and 6 slices: 0.67M slots 4.46, 4.27 | 10.64, 10.53; 0.92M 5.08, 4.95 | 12.64, 12.80; 1.25M 6.17, 6.10 |
+// 15.54, 15.67; 2.12M 8.15, 8.15 | 21.76, 21.96. 0.64M rays of an object in 2 4.7, 8 4.1; two bounces, 2M rays in 3 85.6, 4 86.1, 6 87.0.
+// Slices of 40,000 cost more launches than they cover (0.16M rays in one slice 3.6 ms, in 4 4.8).
 #ifndef DST_FWD_SLICES
 #define DST_FWD_SLICES 4
 #define DST_FWD_SLICES_SMALL 6
@@ -39,9 +40,11 @@
 #ifndef DST_SHADE_GRID_PER_SM
 #define DST_SHADE_GRID_PER_SM 4        // blocks an SM holds at once at 128 registers (measured: 8 is 2.5 % slower on the headline workload)
 #endif
-// Rays from which the composite kernel runs 5 blocks an SM at 96 registers (0 spilled) instead of 4 at 128. It waits for loads, so the fifth
-// block pays while its rounds are long: forward of 2M reflective rays 17.6 -> 16.8 ms, of 0.93M 15.8 -> 15.6. Where most rounds hold few rays
-// one warp's chain counts, and with 96 registers an SH row comes in two waits instead of one: 0.64M rays of an object 4.7 -> 4.9 ms.
+// List slots from which the composite kernel runs 5 blocks an SM at 96 registers (0 spilled) instead of 4 at 128. It waits for loads, so the
+// fifth block pays while its rounds are long; where most rounds hold few rays one warp's chain counts, and with 96 registers an SH row
+// comes in two waits instead of one. Forward of an object (0.5M surfels) | of a reflective scene (1M, one bounce), ms with 4 -> 5 blocks:
+// 0.41M slots 3.75 -> 3.77 | 8.56 -> 8.52, 0.67M 4.31 -> 4.28 | 10.54 -> 10.46, 0.92M 5.04 -> 4.96 | 13.02 -> 12.83, 1.25M 6.30 -> 6.22 | 15.90 -> 15.69,
+// 2.12M 8.03 -> 7.89 | 22.21 -> 21.72: the line lies where the gain leaves the noise, on both scenes.
 #ifndef DST_SHADE_WIDE_SLOTS
 #define DST_SHADE_WIDE_SLOTS (900ll << 10)
 #endif
@@ -681,6 +684,7 @@ __device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int slot, War
 
 // Few rays (what the wavefront leaves over, or a small call): one WARP per ray to completion. The warp gathers the chunk together
 // (knearest_warp) and composites it together (fwd_shade_warp): what such a call takes is the serial work of its longest rays.
+// 10 blocks an SM: 40 warps at 48 registers, with spills (784 B of stores, 556 of loads a thread).
 constexpr int WTAIL_THREADS = 128;
 #ifndef DST_WTAIL_BLOCKS
 #define DST_WTAIL_BLOCKS 10

@@ -317,13 +317,13 @@ __device__ __forceinline__ bool eval_slot(unsigned long long key, float offset, 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Wavefront plumbing. A trace call runs as rounds of two kernels over the list of rays that are
-// still alive: k_enum gathers the 16 nearest hits of each ray's current enumeration (small
-// register footprint, every lane busy), a shade kernel composites them and decides what the ray
-// does next. Ray state, hit buffers and the lists live in scratch memory owned by the handle.
+// Wavefront plumbing. A trace call runs as rounds of kernels over the list of rays that are
+// still alive: the gather (k_enum, k_enum_group, k_enum_ray) finds the 16 nearest hits of each ray's
+// current enumeration, a shade kernel composites them and decides what the ray does next. Ray state, hit buffers and the lists live in scratch memory owned by the handle.
 // counts[r] is the length of list[r & 1] in round r; a round whose list is shorter than
-// `min_count` is skipped by both kernels and left to the tail kernel, which runs the remaining
-// rays to completion one thread per ray.
+// `min_count` is skipped by all of them and left to the tail kernel, which runs the remaining rays to
+// completion: a warp per ray, in the backward a warp per few rays, and a thread per ray where a forward
+// leaves more than 32,768.
 // ---------------------------------------------------------------------------------------------
 struct __align__(16) EnumReq { float ox, oy, oz, dx, dy, dz, kmax0, step; };      // step: gather step that answered the ray's last request (0: k_enum)
 

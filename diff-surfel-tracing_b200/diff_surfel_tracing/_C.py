@@ -171,7 +171,7 @@ class OptiXStateWrapper:
 
     def set_wavefront_min_rays(self, n):
         """Trace calls with at least `n` rays run as rounds of gather / composite kernels over the
-        live rays; smaller calls use one thread per ray for the whole path (same results)."""
+        live rays; smaller calls run one kernel that takes every ray through its whole path (same results)."""
         _check(self, lib().dst_set_option(self.handle, 1, int(n)))
 
     def set_chunk_log_max_records(self, n):

@@ -34,7 +34,7 @@ extern "C" {
 /* bits of the device status word returned by dst_status */
 #define DST_STATUS_STACK_OVERFLOW  1u   /* traversal stack exhausted: some hits may be missing */
 #define DST_STATUS_CHUNK_LIMIT     2u   /* a ray hit the bound on 16-hit enumerations          */
-#define DST_STATUS_LOG_MISMATCH    8u   /* the contribution log ended before the backward of a ray did */
+#define DST_STATUS_LOG_MISMATCH    8u   /* not raised: a contribution log holds what its forward composited, and nothing else is read from it */
 
 #define DST_MID_CHANNELS 16             /* per-bounce record, optix_tracer/config.h:7-15       */
 #ifndef DST_CHUNK
@@ -213,8 +213,8 @@ int dst_bvh_info(const dst_handle* h, int64_t* surfels, int64_t* nodes, int64_t*
 
 /* Tunables. DST_OPT_WAVEFRONT_MIN_RAYS: trace calls with at least this many rays run as rounds of
  * separate gather / composite kernels over the live rays (default 32768); smaller calls run one
- * kernel that takes every ray through its whole path (one warp per ray in the forward, one thread per
- * ray in the backward). Results do not depend on the setting. */
+ * kernel that takes every ray through its whole path (one warp per ray in the forward, one warp per few
+ * rays in a re-tracing backward). Results do not depend on the setting. */
 #define DST_OPT_WAVEFRONT_MIN_RAYS 1
 /* DST_OPT_CHUNK_LOG: 1 (default) keeps the contribution log of training forwards for the backward, 0 disables it. */
 #define DST_OPT_CHUNK_LOG 2
