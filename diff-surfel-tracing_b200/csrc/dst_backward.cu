@@ -244,9 +244,7 @@ __device__ __forceinline__ void bwd_store_state(float4* base, int slot, const Bw
 }
 
 __device__ __forceinline__ void bwd_request(const BwdState& s, EnumReq& q) {
-    if (s.chunk == 0) { q.ox = s.sox; q.oy = s.soy; q.oz = s.soz; }
-    else { q.ox = xadd(s.sox, xmul(s.offset, s.sdx)); q.oy = xadd(s.soy, xmul(s.offset, s.sdy)); q.oz = xadd(s.soz, xmul(s.offset, s.sdz)); }
-    q.dx = s.sdx; q.dy = s.sdy; q.dz = s.sdz; q.kmax0 = DST_T_MAX; q.step = 0.0f;
+    q.ox = s.sox; q.oy = s.soy; q.oz = s.soz; q.dx = s.sdx; q.dy = s.sdy; q.dz = s.sdz; q.kmax0 = DST_T_MAX; q.off = s.chunk == 0 ? 0.0f : s.offset;
 }
 
 // Finds the next segment to differentiate, from segment `start` downwards (backward.cu:706-802):
@@ -643,7 +641,7 @@ __global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_shade(const
             bwd_store_state(p.state, slot, s);
             EnumReq q;
             bwd_request(s, q);
-            q.step = wide && s.chunk > 0 ? 1.0f : 0.0f;
+            if (wide) q.off = -q.off;
             store_req(p.req, slot, q);
             cls = s.seg > 0;
         }
@@ -680,7 +678,7 @@ __global__ void __launch_bounds__(BWD_THREADS, DST_BWD_BLOCKS) k_bwd_tail(const 
             const unsigned int todo = __ballot_sync(FULL, alive);
             if (todo == 0u) break;
             EnumReq q = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
-            if (alive) { bwd_request(s, q); if (DIAG) tc.enums++; }
+            if (alive) { EnumReq r; bwd_request(s, r); q = r; r.start(q.ox, q.oy, q.oz); if (DIAG) tc.enums++; }
             int cnt = 0;
             for (unsigned int m = todo; m; m &= m - 1u) {
                 const int r = __ffs(m) - 1;

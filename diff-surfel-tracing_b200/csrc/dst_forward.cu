@@ -220,11 +220,9 @@ __device__ __forceinline__ void fwd_init_state(const FwdParams& p, int ray, FwdS
     fwd_begin_segment(s);
 }
 
-// origin of the next enumeration: the segment origin, moved along the ray past the last evaluated hit (forward.cu:303-306)
+// next enumeration of the segment
 __device__ __forceinline__ void fwd_request(const FwdState& s, EnumReq& q) {
-    if (s.chunk == 0) { q.ox = s.sox; q.oy = s.soy; q.oz = s.soz; }
-    else { q.ox = xadd(s.sox, xmul(s.offset, s.sdx)); q.oy = xadd(s.soy, xmul(s.offset, s.sdy)); q.oz = xadd(s.soz, xmul(s.offset, s.sdz)); }
-    q.dx = s.sdx; q.dy = s.sdy; q.dz = s.sdz; q.kmax0 = DST_T_MAX; q.step = 0.0f;
+    q.ox = s.sox; q.oy = s.soy; q.oz = s.soz; q.dx = s.sdx; q.dy = s.sdy; q.dz = s.sdz; q.kmax0 = DST_T_MAX; q.off = s.chunk == 0 ? 0.0f : s.offset;
 }
 
 // After the hits of a chunk: the segment goes on (returns true), or it is finished (forward.cu:309-314, tracePath 378-422) and
@@ -505,7 +503,7 @@ __global__ void __launch_bounds__(SHADE_THREADS, BLOCKS) k_fwd_shade(const __gri
             store_state(p.state, slot, s);
             EnumReq q;
             fwd_request(s, q);
-            q.step = wide && s.chunk > 0 ? 1.0f : 0.0f;
+            if (wide) q.off = -q.off;
             // A segment that goes on: its next 16 hits are searched within bound_factor times the distance the last 16
             // spanned (first to last). A walk that knows its bound from the start opens a fifth fewer nodes than one that
             // learns it from its 16th hit; the spans of consecutive chunks differ by less than that factor for all but
@@ -546,7 +544,9 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_fwd_tail(const __grid_constant
             if (alive) {
                 EnumReq q;
                 fwd_request(s, q);
-                cnt = knearest<false, DIAG, TAIL_THREADS>(p.bvh, q.ox, q.oy, q.oz, q.dx, q.dy, q.dz, kb, p.status, tc, q.kmax0);
+                float x, y, z;
+                q.start(x, y, z);
+                cnt = knearest<false, DIAG, TAIL_THREADS>(p.bvh, x, y, z, q.dx, q.dy, q.dz, kb, p.status, tc, q.kmax0);
                 if (DIAG) tc.enums++;
             }
             __syncwarp();
@@ -715,8 +715,10 @@ __global__ void __launch_bounds__(WTAIL_THREADS, DST_WTAIL_BLOCKS) k_fwd_tail_wa
         while (alive) {
             EnumReq q;
             fwd_request(ws.s, q);
+            float x, y, z;
+            q.start(x, y, z);
             unsigned long long key;
-            const int cnt = knearest_warp<DIAG>(p.bvh, q.ox, q.oy, q.oz, q.dx, q.dy, q.dz, q.kmax0, absmax, walk_mem[w], key, p.status, tc);
+            const int cnt = knearest_warp<DIAG>(p.bvh, x, y, z, q.dx, q.dy, q.dz, q.kmax0, absmax, walk_mem[w], key, p.status, tc);
             alive = fwd_shade_warp<DIAG>(p, slot, ws, key, cnt, tc);
             __syncwarp();
         }

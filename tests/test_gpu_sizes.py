@@ -131,6 +131,31 @@ def test_absent_upstream_gradients_are_an_error_unless_asked_for(C, missing):
     assert st.status() == 0
 
 
+@pytest.mark.parametrize("shift", [0.0, 300.0, 2e4])
+@pytest.mark.parametrize("config", [1, 3])
+def test_hulls_of_later_enumerations(C, config, shift):
+    """The rounds walk for hulls of whole segments, the per-ray kernel for one ray from its moved origin: the same bits, also where moving the
+    origin rounds coarsely (a scene far from the world's origin)."""
+    w = hp.workloads.make_workload(config, P=40_000, H=128, W=160)
+    w["scales"] = w["scales"] * 2.0
+    t = torch.tensor([shift, -0.5 * shift, shift])
+    w["means3D"], w["ray_o"] = w["means3D"] + t, w["ray_o"] + t
+    w["v"], w["f"] = hp.workloads.get_triangles(w["means3D"], w["scales"], w["rotations"])
+    wc = hp.to_cuda(w)
+    got, chunks = [], 0
+    for wave in (True, False):
+        st = _state(C, wc, wave)
+        dg = {}
+        f = hp.cuda_forward(C, st, wc, diag=dg)
+        torch.cuda.synchronize()
+        assert st.status() == 0
+        got.append(f)
+        chunks = int(dg["counters"][1])
+    assert chunks > 2 * 128 * 160
+    for k in ("rgb", "dpt", "acc", "norm", "aux", "mid"):
+        assert np.array_equal(got[0][k].cpu().numpy().view(np.uint32), got[1][k].cpu().numpy().view(np.uint32)), k
+
+
 def _slots(H, W):
     """List slots of an image: whole blocks of 64 x 32 pixels."""
     return -(-W // 64) * -(-H // 32) * 2048
