@@ -666,19 +666,9 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
                 if (cands > max_cands) return false;
                 unsigned int order = pass ? (__float_as_uint(tl) & ~31u) | lane : ~0u;
                 unsigned int first = __reduce_min_sync(FULL, order);
-                Quad next;       // (the next quad is on its way while this one is tested)
-                if (first != ~0u) next = load_quad(bvh, __shfl_sync(FULL, pos, first & 31));
-                while (first != ~0u) {
-                    const Quad q = next;
-                    if (!__any_sync(FULL, __uint_as_float(first & ~31u) <= from_hull(rel, kmax))) break;
-                    if (lane == (first & 31)) order = ~0u;
-                    first = __reduce_min_sync(FULL, order);
-                    if (first != ~0u) next = load_quad(bvh, __shfl_sync(FULL, pos, first & 31));
-                    if (COUNT && lane == 0) tc.quads++;
-                    float t; int tri;
-                    if (!ray_quad(q.a, q.b, q.c, ox, oy, oz, dx, dy, dz, kmax, t, tri)) continue;
+                auto take = [&](const Quad& q, float t, int tri) {
                     const unsigned long long key = make_key(t, 2u * q.gid + (unsigned int)tri);
-                    if (n == DST_CHUNK && key >= kb[(DST_CHUNK - 1) * KS]) continue;
+                    if (n == DST_CHUNK && key >= kb[(DST_CHUNK - 1) * KS]) return;
                     int j = n < DST_CHUNK ? n : DST_CHUNK - 1;
                     while (j > 0) {
                         const unsigned long long prev = kb[(j - 1) * KS];
@@ -689,6 +679,24 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
                     kb[j * KS] = key;
                     if (n < DST_CHUNK) n++;
                     if (n == DST_CHUNK) kmax = hitkey_t(kb[(DST_CHUNK - 1) * KS]);
+                };
+                // Two at a time, whose loads and tests do not wait for each other: a launch is as long as its slowest walks, and those are chains of such
+                // tests. k_enum of 2M reflective rays 9.66 -> 9.21 ms, of an 800 x 800 object view 1.13 -> 1.04 (one quad ahead, loaded and not yet
+                // tested, before); whole passes 1 to 3 %.
+                while (first != ~0u) {
+                    if (!__any_sync(FULL, __uint_as_float(first & ~31u) <= from_hull(rel, kmax))) break;
+                    const Quad qa = load_quad(bvh, __shfl_sync(FULL, pos, first & 31));
+                    if (lane == (first & 31)) order = ~0u;
+                    const unsigned int second = __reduce_min_sync(FULL, order);
+                    const Quad qb = load_quad(bvh, __shfl_sync(FULL, pos, second & 31));
+                    if (lane == (second & 31)) order = ~0u;
+                    first = __reduce_min_sync(FULL, order);
+                    if (COUNT && lane == 0) tc.quads += second != ~0u ? 2 : 1;
+                    float ta, tb; int tria, trib;
+                    const bool ha = ray_quad(qa.a, qa.b, qa.c, ox, oy, oz, dx, dy, dz, kmax, ta, tria);
+                    const bool hb = second != ~0u && ray_quad(qb.a, qb.b, qb.c, ox, oy, oz, dx, dy, dz, kmax, tb, trib);
+                    if (ha) take(qa, ta, tria);
+                    if (hb) take(qb, tb, trib);
                 }
                 krun = redux_max(from_hull(rel, kmax));
                 return true;
