@@ -382,14 +382,16 @@ constexpr int ENUM_THREADS = 128;
 // What a walk may take before it is given up: steps, and quads that pass the hull test. A launch with a few times more work than it has
 // warps (all slices of a call counted) takes the larger limits, because giving up costs work; with less, the time is that of its longest walk,
 // and the smaller ones are the faster. Measured, one set of limits (160 / 300 / 192) against two: two-bounce scene 93.3 -> 88.7 ms, 400 x 400
-// object views 4.40 -> 3.63 ms, four LiDAR sweeps 2.44 -> 2.26 ms.
+// object views 4.40 -> 3.63 ms, four LiDAR sweeps 2.44 -> 2.26 ms. The smaller limits with the present kernels, 70 quads and 100 steps of a group against
+// 200 and 150: object views 4.11 -> 3.45 ms, LiDAR sweeps 2.41 -> 2.21, an 800 x 800 object view 3.87 -> 3.79 (45 quads: 3.40, 2.18, 3.76, but 2M reflective
+// rays 29.7 -> 30.1); 300 quads in a loaded launch cost two bounces 1 %, 400 or 600 steps of a group there 1-2 % and the object view 9-23 %.
 #define DST_LOADED_BEAMS 2                 // times as many batches as warps of the launch
 #define DST_LOADED_GROUPS 3
 #define DST_BEAM_STEPS 160
 #define DST_BEAM_STEPS_LOADED 240
-#define DST_BEAM_CANDS 200
+#define DST_BEAM_CANDS 70
 #define DST_BEAM_CANDS_LOADED 400
-#define DST_GROUP_STEPS 150
+#define DST_GROUP_STEPS 100
 #define DST_GROUP_STEPS_LOADED 260
 #define DST_GROUP 8
 #define DST_GROUP_MIN_BLOCKS 10
