@@ -382,14 +382,17 @@ constexpr int ENUM_THREADS = 128;
 // What a walk may take before it is given up: steps, and quads that pass the hull test. A launch with a few times more work than it has
 // warps (all slices of a call counted) takes the larger limits, because giving up costs work; with less, the time is that of its longest walk,
 // and the smaller ones are the faster. Measured, one set of limits (160 / 300 / 192) against two: two-bounce scene 93.3 -> 88.7 ms, 400 x 400
-// object views 4.40 -> 3.63 ms, four LiDAR sweeps 2.44 -> 2.26 ms. The smaller limits with the present kernels, 70 quads and 100 steps of a group against
-// 200 and 150: object views 4.11 -> 3.45 ms, LiDAR sweeps 2.41 -> 2.21, an 800 x 800 object view 3.87 -> 3.79 (45 quads: 3.40, 2.18, 3.76, but 2M reflective
-// rays 29.7 -> 30.1); 300 quads in a loaded launch cost two bounces 1 %, 400 or 600 steps of a group there 1-2 % and the object view 9-23 %.
+// object views 4.40 -> 3.63 ms, four LiDAR sweeps 2.44 -> 2.26 ms.
+// Steps of a group in a launch without a load: 150 -> 100 object views 4.13 -> 3.99 ms, LiDAR sweeps 2.46 -> 2.36. A load of groups counts at most four slices (the
+// others are at other stages by then): an 800 x 800 object view in six slices 3.78 -> 3.61 ms. 200 instead of 260 steps in all loaded launches cost two
+// bounces 1 %, 400 or 600 the object view 9-23 %. Fewer quads without a load (70) suit scenes where a quad is hit by few of a batch's rays (object views 3.43 ms
+// instead of 3.92), but a 200 x 200 patch of a dense scene takes 4.15 ms instead of 3.52, and with the rays' hits as the criterion a 170 x 150 view
+// of a ball 200 us instead of 180.
 #define DST_LOADED_BEAMS 2                 // times as many batches as warps of the launch
 #define DST_LOADED_GROUPS 3
 #define DST_BEAM_STEPS 160
 #define DST_BEAM_STEPS_LOADED 240
-#define DST_BEAM_CANDS 70
+#define DST_BEAM_CANDS 200
 #define DST_BEAM_CANDS_LOADED 400
 #define DST_GROUP_STEPS 100
 #define DST_GROUP_STEPS_LOADED 260
@@ -753,10 +756,8 @@ __device__ __forceinline__ void take_hits(bool hit, unsigned long long key, unsi
 
 // The 16 nearest hits of ONE ray, found by a whole warp (same result as knearest()): the walk of a hull that is a single
 // ray, its quads tested exactly, one per lane. The k-buffer lives in registers, one key per lane (lanes 0..15, ascending).
-// All arguments are warp-uniform. FINISH: kmax0 is a guess. Where there are fewer than 16 hits up to it, a second walk, of the ray from there on, adds those
-// beyond it, so that nothing is searched twice. With it k_fwd_tail_warp searches within predicted bounds as the rounds do: 30,000 loose rays in a scene
-// of 0.5M surfels 3.23 -> 3.11 ms a training step, a 200 x 200 patch of one of 3M 3.59 -> 3.54; rays that end in their first chunk are no slower.
-template <bool COUNT, bool FINISH = false>
+// All arguments are warp-uniform.
+template <bool COUNT>
 __device__ __forceinline__ int knearest_warp(const BvhView& bvh, float ox, float oy, float oz, float dx, float dy, float dz, float kmax0, float absmax,
                                              WalkMem& m, unsigned long long& mykey, unsigned int* status, TraceCounters& tc) {
     constexpr unsigned int FULL = 0xffffffffu;
@@ -764,34 +765,27 @@ __device__ __forceinline__ int knearest_warp(const BvhView& bvh, float ox, float
     mykey = ~0ull;
     if (bvh.P <= 0) return 0;
     if (!(fabsf(ox) < INFINITY && fabsf(oy) < INFINITY && fabsf(oz) < INFINITY && fabsf(dx) < INFINITY && fabsf(dy) < INFINITY && fabsf(dz) < INFINITY)) return 0;
-    float from = 0.0f, cut = kmax0;      // hits up to `from` have been found; those beyond `cut` are of no interest
-    for (;;) {
-        if (FINISH) make_beam<true>(m, true, fmaf(from, dx, ox), fmaf(from, dy, oy), fmaf(from, dz, oz), dx, dy, dz, from, absmax);
-        else make_beam<true>(m, true, ox, oy, oz, dx, dy, dz, 0.0f, absmax);
-        const float rel = (1e-6f - 1.0f) * from;
-        float krun = FINISH ? from_hull(rel, cut) : cut;
-        const bool done = beam_walk<COUNT>(bvh, m, krun, DST_WALK_STEP_LIMIT, status, tc, [&](bool valid, int pos) {
-            bool hit = false;
-            unsigned long long key = 0ull;
-            if (valid) {
-                const Quad q = load_quad(bvh, pos);
-                float t; int tri;
-                if (COUNT) tc.quads++;
-                if (ray_quad(q.a, q.b, q.c, ox, oy, oz, dx, dy, dz, cut, t, tri) && (!FINISH || t > from || from == 0.0f)) {
-                    key = make_key(t, 2u * q.gid + (unsigned int)tri);
-                    hit = true;
-                }
+    make_beam<true>(m, true, ox, oy, oz, dx, dy, dz, 0.0f, absmax);
+    float krun = kmax0;
+    const bool done = beam_walk<COUNT>(bvh, m, krun, DST_WALK_STEP_LIMIT, status, tc, [&](bool valid, int pos) {
+        bool hit = false;
+        unsigned long long key = 0ull;
+        if (valid) {
+            const Quad q = load_quad(bvh, pos);
+            float t; int tri;
+            if (COUNT) tc.quads++;
+            if (ray_quad(q.a, q.b, q.c, ox, oy, oz, dx, dy, dz, krun, t, tri)) {
+                key = make_key(t, 2u * q.gid + (unsigned int)tri);
+                hit = true;
             }
-            take_hits(hit, key, mykey, m.place);
-            const unsigned long long last = __shfl_sync(FULL, mykey, DST_CHUNK - 1);
-            if (last != ~0ull) { cut = hitkey_t(last); krun = FINISH ? from_hull(rel, cut) : cut; }
-            return true;
-        });
-        if (!done && lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW);
-        const int n = __popc(__ballot_sync(FULL, lane < DST_CHUNK && mykey != ~0ull));
-        if (!FINISH || n == DST_CHUNK || cut >= DST_T_MAX) return n;
-        from = cut; cut = DST_T_MAX;
-    }
+        }
+        take_hits(hit, key, mykey, m.place);
+        const unsigned long long last = __shfl_sync(FULL, mykey, DST_CHUNK - 1);
+        if (last != ~0ull) krun = hitkey_t(last);
+        return true;
+    });
+    if (!done && lane == 0) atomicOr(status, DST_STATUS_STACK_OVERFLOW);
+    return __popc(__ballot_sync(FULL, lane < DST_CHUNK && mykey != ~0ull));
 }
 
 // Second step of a gather: the batches k_enum gave up, in groups of DST_GROUP rays, one warp per group. The walk is again
@@ -925,11 +919,11 @@ static inline void launch_gather(bool diag, int grid, int sm_count, int slices, 
     const int direct_max = sm_count * DST_GROUP_MIN_BLOCKS * (ENUM_THREADS / 32), ray_grid = sm_count * DST_GROUP_MIN_BLOCKS;
     if (diag) {
         k_enum<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, counters, heavy, cnt + 2 * R, slices);
-        k_enum_group<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, counters, heavy2, cnt + 4 * R, direct_max, slices);
+        k_enum_group<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, counters, heavy2, cnt + 4 * R, direct_max, slices < 4 ? slices : 4);
         k_enum_ray<true><<<ray_grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, heavy2, cnt + 4 * R, cnt + 5 * R, direct_max, kbuf, kcnt, status, counters);
     } else {
         k_enum<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, nullptr, heavy, cnt + 2 * R, slices);
-        k_enum_group<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, nullptr, heavy2, cnt + 4 * R, direct_max, slices);
+        k_enum_group<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, nullptr, heavy2, cnt + 4 * R, direct_max, slices < 4 ? slices : 4);
         k_enum_ray<false><<<ray_grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, heavy2, cnt + 4 * R, cnt + 5 * R, direct_max, kbuf, kcnt, status, nullptr);
     }
 }
