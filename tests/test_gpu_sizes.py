@@ -156,35 +156,6 @@ def test_hulls_of_later_enumerations(C, config, shift):
         assert np.array_equal(got[0][k].cpu().numpy().view(np.uint32), got[1][k].cpu().numpy().view(np.uint32)), k
 
 
-@pytest.mark.parametrize("layers", [(20, 5, 30), (16, 1, 15), (17, 40), (32, 16), (3,)])
-def test_predicted_bounds_of_the_per_ray_kernel(C, oracle_mod, layers):
-    """Quads in groups far apart: a search within a multiple of the last hits' span ends in a gap, and the hits beyond it belong to the same
-    enumeration. Against the oracle bit for bit."""
-    P = sum(layers)
-    w = hp.workloads.make_workload(1, P=P, H=32, W=48)
-    g = torch.Generator().manual_seed(7)
-    z = torch.cat([4.0 ** k * (1.0 + 0.004 * torch.arange(n)) for k, n in enumerate(layers)])
-    w["means3D"] = torch.cat([0.02 * z[:, None] * torch.randn((P, 2), generator=g), z[:, None]], dim=-1).contiguous()
-    w["scales"] = (z[:, None] * (0.1 + 0.4 * torch.rand((P, 2), generator=g))).contiguous()
-    rot = torch.cat([torch.ones((P, 1)), 0.03 * torch.randn((P, 3), generator=g)], dim=-1)
-    w["rotations"] = (rot / rot.norm(dim=-1, keepdim=True)).contiguous()
-    w["opacities"] = torch.full((P, 1), 0.05)
-    d = torch.stack(torch.meshgrid(torch.linspace(-0.3, 0.3, 32), torch.linspace(-0.4, 0.4, 48), indexing="ij") + (torch.ones(32, 48),), dim=-1)
-    w["ray_d"] = (d / d.norm(dim=-1, keepdim=True)).contiguous()
-    w["ray_o"] = torch.zeros_like(w["ray_d"])
-    w["v"], w["f"] = hp.workloads.get_triangles(w["means3D"], w["scales"], w["rotations"])
-    wc = hp.to_cuda(w)
-    want = oracle_mod.Oracle(oracle_mod.Scene(w["v"]), impl="restatement", portable_exp=True).forward(w, training=True)
-    st = _state(C, wc, False)
-    dg = dict(hit_cap=0)
-    got = hp.cuda_forward(C, st, wc, diag=dg)
-    torch.cuda.synchronize()
-    assert st.status() == 0
-    assert P < 17 or int(dg["counters"][1]) > 32 * 48
-    for k in ("rgb", "dpt", "acc", "norm", "mid"):
-        assert np.array_equal(got[k].cpu().numpy().reshape(want[k].shape).view(np.uint32), want[k].view(np.uint32)), k
-
-
 def _slots(H, W):
     """List slots of an image: whole blocks of 64 x 32 pixels."""
     return -(-W // 64) * -(-H // 32) * 2048
