@@ -549,20 +549,52 @@ __device__ __forceinline__ bool beam_walk(const BvhView& bvh, WalkStack<STACK>& 
 __device__ __forceinline__ float redux_min(float v) { float r; asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v)); return r; }
 __device__ __forceinline__ float redux_max(float v) { float r; asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v)); return r; }
 
-// hull of the rays of the lanes with `active` (at least one), into m.beam and m.slab. moved: largest distance the origins have been moved along their rays
-// (they, and those the exact tests use, are off the rays by the rounding of that). ONE: a single ray, the same in all lanes, whose quads no hull test sees.
+// Where a hull of rays starts. The rays of a batch are at different distances along their segments, and where they come from one place a hull of the points
+// they have reached is that much longer than it is wide, in a box with sides along the axes wide too. So such rays are taken back to the distance the least
+// advanced of them has reached, and each searches `rel` further than from where its enumeration starts (rounded up). Where the box of the points reached
+// is the narrower one (rays that started at distances of their own towards the same surface, directions of different length) the hull starts at those.
+// Hulls of the points reached -> of the lines: 0.93M rays of a reflective scene 15.1 -> 10.7 ms (k_enum_group 8.2 -> 3.7: rays k_enum and k_enum_group
+// gave up before), four LiDAR sweeps 2.91 -> 2.46, two 400 x 400 object views 4.50 -> 4.13; 2M rays with one or two bounces, whose hulls are as wide as
+// their directions fan out either way, 30.8 -> 30.5 and 114.4 -> 114.5. Hulls of whole segments (back to distance 0) lose 2 % there.
+// 560 x 900 views of 0.3M surfels on an object, lines for all | the narrower: starts jittered along the rays 12.0 | 8.2 ms, directions of 0.8 to 1 units
+// 7.7 | 5.6 (of 0.6M surfels and a reflection 17.4 | 12.5); views from one place with directions of one length as they were (within 0.3 %).
+// Asking for 0.7 or 0.4 of the lines' extent gains nothing anywhere and costs a reflective scene with such directions 2 and 12 %.
+struct HullStart { float lo[3], hi[3], rel, moved; };      // box of the origins; moved: largest distance an origin has been moved along its ray
+__device__ __forceinline__ HullStart hull_start(bool active, const EnumReq& q) {
+    const float off = fabsf(q.off), first = redux_min(active ? off : INFINITY);
+    HullStart s;
+    auto box = [&](float x, float y, float z, float* lo, float* hi) {
+        lo[0] = redux_min(active ? x : INFINITY); lo[1] = redux_min(active ? y : INFINITY); lo[2] = redux_min(active ? z : INFINITY);
+        hi[0] = redux_max(active ? x : -INFINITY); hi[1] = redux_max(active ? y : -INFINITY); hi[2] = redux_max(active ? z : -INFINITY);
+        return (hi[0] - lo[0]) + (hi[1] - lo[1]) + (hi[2] - lo[2]);
+    };
+    const float extent = box(fmaf(first, q.dx, q.ox), fmaf(first, q.dy, q.oy), fmaf(first, q.dz, q.oz), s.lo, s.hi);
+    s.moved = redux_max(active ? off : 0.0f);
+    s.rel = (off - first) + 1e-6f * off;
+    if (s.moved > first) {
+        float x, y, z, lo[3], hi[3];
+        q.start(x, y, z);
+        if (box(x, y, z, lo, hi) < extent) {
+#pragma unroll
+            for (int a = 0; a < 3; a++) { s.lo[a] = lo[a]; s.hi[a] = hi[a]; }
+            s.rel = s.moved = 0.0f;
+        }
+    }
+    return s;
+}
+
+// Hull of the rays of the lanes with `active` (at least one), whose origins lie in the box [olo, ohi], into m.beam and m.slab. moved: largest distance the origins
+// have been moved along their rays (they, and those the exact tests use, are off the rays by the rounding of that). ONE: a single ray, the same in all
+// lanes, whose quads no hull test sees.
 template <bool ONE = false>
-__device__ __forceinline__ void make_beam(WalkMemBase& m, bool active, float ox, float oy, float oz, float dx, float dy, float dz, float moved, float absmax) {
+__device__ __forceinline__ void make_beam(WalkMemBase& m, bool active, const float* olo, const float* ohi, float dx, float dy, float dz, float moved, float absmax) {
     const int lane = threadIdx.x & 31;
-    const float o3[3] = { ox, oy, oz }, d3[3] = { dx, dy, dz };
-    float olo[3], ohi[3], dlo[3], dhi[3], om = 0.0f;
+    const float d3[3] = { dx, dy, dz };
+    float dlo[3], dhi[3], om = 0.0f;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        if (ONE) { olo[a] = ohi[a] = o3[a]; dlo[a] = dhi[a] = d3[a]; }
-        else {
-            olo[a] = redux_min(active ? o3[a] : INFINITY); ohi[a] = redux_max(active ? o3[a] : -INFINITY);
-            dlo[a] = redux_min(active ? d3[a] : INFINITY); dhi[a] = redux_max(active ? d3[a] : -INFINITY);
-        }
+        if (ONE) { dlo[a] = dhi[a] = d3[a]; }
+        else { dlo[a] = redux_min(active ? d3[a] : INFINITY); dhi[a] = redux_max(active ? d3[a] : -INFINITY); }
         om = fmaxf(om, fmaf(moved, fmaxf(fabsf(dlo[a]), fabsf(dhi[a])), fmaxf(fabsf(olo[a]), fabsf(ohi[a]))));
     }
     if (lane < 3) {
@@ -595,21 +627,6 @@ __device__ __forceinline__ void make_beam(WalkMemBase& m, bool active, float ox,
     __syncwarp();
 }
 
-// Where a hull of rays starts. The rays of a batch are at different distances along their segments, and a hull of the points they have reached is that much
-// longer than it is wide, in a box with sides along the axes wide too. So the rays are taken back to the distance the least advanced of them has
-// reached, and each searches `rel` further than from where its enumeration starts (rounded up). moved, all of it: see make_beam().
-// Passes with hulls of the points reached -> these: 0.93M rays of a reflective scene 15.1 -> 10.7 ms (k_enum_group 8.2 -> 3.7: rays k_enum and k_enum_group
-// gave up before), four LiDAR sweeps 2.91 -> 2.46, two 400 x 400 object views 4.50 -> 4.13; 2M rays with one or two bounces, whose hulls are as wide as
-// their directions fan out either way, 30.8 -> 30.5 and 114.4 -> 114.5. Hulls of whole segments (back to distance 0) lose 2 % there.
-struct HullStart { float x, y, z, rel, moved; };
-__device__ __forceinline__ HullStart hull_start(bool active, const EnumReq& q) {
-    const float off = fabsf(q.off), first = redux_min(active ? off : INFINITY);
-    HullStart s;
-    s.moved = redux_max(active ? off : 0.0f);
-    s.x = fmaf(first, q.dx, q.ox); s.y = fmaf(first, q.dy, q.oy); s.z = fmaf(first, q.dz, q.oz);
-    s.rel = (off - first) + 1e-6f * off;
-    return s;
-}
 // First step of a gather: 32 consecutive entries of the live list per warp. A batch that is given up goes to `heavy` with its 32 slots, each ray
 // with the search bound it has found.
 template <bool COUNT>
@@ -657,7 +674,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
             bool done = 2 * __popc(__ballot_sync(FULL, wide)) <= __popc(am);
             if (done) {
             const HullStart hs = hull_start(active, q);
-            make_beam(m, active, hs.x, hs.y, hs.z, dx, dy, dz, hs.moved, absmax);
+            make_beam(m, active, hs.lo, hs.hi, dx, dy, dz, hs.moved, absmax);
             const float rel = hs.rel;
             float krun = redux_max(from_hull(rel, kmax));
             int cands = 0;
@@ -765,7 +782,8 @@ __device__ __forceinline__ int knearest_warp(const BvhView& bvh, float ox, float
     mykey = ~0ull;
     if (bvh.P <= 0) return 0;
     if (!(fabsf(ox) < INFINITY && fabsf(oy) < INFINITY && fabsf(oz) < INFINITY && fabsf(dx) < INFINITY && fabsf(dy) < INFINITY && fabsf(dz) < INFINITY)) return 0;
-    make_beam<true>(m, true, ox, oy, oz, dx, dy, dz, 0.0f, absmax);
+    const float o3[3] = { ox, oy, oz };
+    make_beam<true>(m, true, o3, o3, dx, dy, dz, 0.0f, absmax);
     float krun = kmax0;
     const bool done = beam_walk<COUNT>(bvh, m, krun, DST_WALK_STEP_LIMIT, status, tc, [&](bool valid, int pos) {
         bool hit = false;
@@ -824,7 +842,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
             srays[w][lane][0] = make_float4(x, y, z, q.dx); srays[w][lane][1] = make_float4(q.dy, q.dz, q.kmax0, hs.rel);
         }
         for (int k = lane; k < DST_GROUP * DST_CHUNK; k += 32) (&skeys[w][0][0])[k] = ~0ull;
-        make_beam(m, slot >= 0, hs.x, hs.y, hs.z, q.dx, q.dy, q.dz, hs.moved, absmax);
+        make_beam(m, slot >= 0, hs.lo, hs.hi, q.dx, q.dy, q.dz, hs.moved, absmax);
         float krun = redux_max(from_hull(hs.rel, q.kmax0));
         const bool done = beam_walk<COUNT>(bvh, m, krun, max_steps, status, tc, [&](bool valid, int pos) {
             Quad q;

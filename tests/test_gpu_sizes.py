@@ -156,6 +156,31 @@ def test_hulls_of_later_enumerations(C, config, shift):
         assert np.array_equal(got[0][k].cpu().numpy().view(np.uint32), got[1][k].cpu().numpy().view(np.uint32)), k
 
 
+@pytest.mark.parametrize("rays,limit", [("starts", 4.9), ("lengths", 3.4)])
+def test_hulls_of_rays_that_start_or_step_differently(C, rays, limit):
+    """Rays that start at distances of their own towards one surface, or whose directions differ in length, are walked from the points they have
+    reached, whose box is narrower than that of their lines: nodes per walk against those of the plain view (lines only: 6.1 to 7 and 4.2
+    times as many, the narrower of both: 3.9 and 2.8; the limits lie between), and the bits of the per-ray kernel."""
+    w = hp.workloads.make_workload(2, P=300_000, H=300, W=400)
+    r = torch.rand((300, 400, 1), generator=torch.Generator().manual_seed(1))
+    nodes = []
+    for o, d in ((w["ray_o"], w["ray_d"]), (w["ray_o"] + 2.5 * r * w["ray_d"], w["ray_d"]) if rays == "starts" else (w["ray_o"], w["ray_d"] * (0.8 + 0.2 * r))):
+        wc = hp.to_cuda(dict(w, ray_o=o.contiguous(), ray_d=d.contiguous()))
+        got = []
+        for wave in (True, False):
+            st, dg = _state(C, wc, wave), {}
+            f = hp.cuda_forward(C, st, wc)
+            hp.cuda_forward(C, st, wc, diag=dg)
+            torch.cuda.synchronize()
+            assert st.status() == 0
+            got.append(f)
+            if wave:
+                nodes.append(int(dg["counters"][2]) / int(dg["counters"][1]))
+    for k in ("rgb", "dpt", "acc", "norm", "mid"):
+        assert np.array_equal(got[0][k].cpu().numpy().view(np.uint32), got[1][k].cpu().numpy().view(np.uint32)), k
+    assert nodes[1] < limit * nodes[0], nodes
+
+
 def _slots(H, W):
     """List slots of an image: whole blocks of 64 x 32 pixels."""
     return -(-W // 64) * -(-H // 32) * 2048
