@@ -132,28 +132,47 @@ def test_absent_upstream_gradients_are_an_error_unless_asked_for(C, missing):
 
 
 @pytest.mark.parametrize("shift", [0.0, 300.0, 2e4])
-@pytest.mark.parametrize("config", [1, 3])
-def test_hulls_of_later_enumerations(C, config, shift):
-    """The rounds walk for hulls of whole segments, the per-ray kernel for one ray from its moved origin: the same bits, also where moving the
-    origin rounds coarsely (a scene far from the world's origin)."""
-    w = hp.workloads.make_workload(config, P=40_000, H=128, W=160)
-    w["scales"] = w["scales"] * 2.0
+@pytest.mark.parametrize("config,size", [(1, 4.0), (3, 2.0)])
+def test_hulls_of_later_enumerations(C, config, size, shift):
+    """The rounds walk for hulls of the rays from the least advanced one's distance on (or of the points they have reached), the per-ray kernel for one
+    ray from its moved origin: the same bits, also where moving the origin rounds coarsely (a scene far from the world's origin), from the
+    kernels with and without counters; the re-tracing backward composites the hits the forward logged."""
+    w = hp.workloads.make_workload(config, P=150_000, H=256, W=320)
+    w["scales"] = w["scales"] * size
     t = torch.tensor([shift, -0.5 * shift, shift])
     w["means3D"], w["ray_o"] = w["means3D"] + t, w["ray_o"] + t
     w["v"], w["f"] = hp.workloads.get_triangles(w["means3D"], w["scales"], w["rotations"])
     wc = hp.to_cuda(w)
-    got, chunks = [], 0
-    for wave in (True, False):
-        st = _state(C, wc, wave)
-        dg = {}
-        f = hp.cuda_forward(C, st, wc, diag=dg)
+    st, ray = _state(C, wc, True), _state(C, wc, False)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        f = hp.cuda_forward(C, st, wc)
+        serial = st.last_forward_serial
         torch.cuda.synchronize()
-        assert st.status() == 0
-        got.append(f)
-        chunks = int(dg["counters"][1])
-    assert chunks > 2 * 128 * 160
+    # what this is about did run: later enumerations of most rays in the rounds, and batches walked in groups (an idle launch takes 2 us)
+    assert st.round_counts()[3] > 256 * 320 // 2
+    assert sum("k_enum_group" in e.name and e.device_time > 30 for e in prof.events()) > 3
+    up = dict(rgb=torch.randn(f["rgb"].shape, device="cuda"))
+    logged, traced = {}, {}
+    g = hp.cuda_backward(C, st, wc, f, up, diag=logged, serial=serial)
+    counted = hp.cuda_forward(C, st, wc, diag={})
+    r = hp.cuda_backward(C, st, wc, f, up, diag=traced, serial=0)
+    rounds = st.round_counts()
+    plain = hp.cuda_backward(C, st, wc, f, up, serial=0)
+    want = hp.cuda_forward(C, ray, wc)
+    torch.cuda.synchronize()
+    assert st.status() == 0 and ray.status() == 0
     for k in ("rgb", "dpt", "acc", "norm", "aux", "mid"):
-        assert np.array_equal(got[0][k].cpu().numpy().view(np.uint32), got[1][k].cpu().numpy().view(np.uint32)), k
+        bits = want[k].cpu().numpy().view(np.uint32)
+        assert np.array_equal(f[k].cpu().numpy().view(np.uint32), bits), k
+        assert np.array_equal(counted[k].cpu().numpy().view(np.uint32), bits), k
+    assert rounds[2] > 256 * 320 // 2 and int(traced["counters"][2]) > 0 and int(logged["counters"][2]) == 0
+    assert int(traced["counters"][5]) == int(logged["counters"][5])
+    for k in hp.GRAD_KEYS:
+        for got in (r, plain):
+            a, b = got[k].cpu().numpy(), g[k].cpu().numpy()
+            assert np.array_equal(np.isfinite(a), np.isfinite(b)), k
+            m = np.isfinite(b)
+            assert hp.rel_l2(a[m], b[m]) < 1e-4, k
 
 
 @pytest.mark.parametrize("rays,limit", [("starts", 4.9), ("lengths", 3.4)])
