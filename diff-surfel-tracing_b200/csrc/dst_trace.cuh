@@ -380,16 +380,19 @@ constexpr int ENUM_THREADS = 128;
 // Blocks are persistent and take batches from a cursor; no block waits for another.
 // ---------------------------------------------------------------------------------------------
 // What a walk may take before it is given up: steps, and quads that pass the hull test. A launch with a few times more work than it has
-// warps (all slices of a call counted) takes the larger limits, because giving up costs work; with less, the time is that of its longest walk,
+// warps (with what the call's other slices launch) takes the larger limits, because giving up costs work; with less, the time is that of its longest walk,
 // and the smaller ones are the faster. Measured, one set of limits (160 / 300 / 192) against two: two-bounce scene 93.3 -> 88.7 ms, 400 x 400
 // object views 4.40 -> 3.63 ms, four LiDAR sweeps 2.44 -> 2.26 ms.
-// Steps of a group in a launch without a load: 150 -> 100 object views 4.13 -> 3.99 ms, LiDAR sweeps 2.46 -> 2.36. A load of groups counts at most four slices (the
-// others are at other stages by then): an 800 x 800 object view in six slices 3.78 -> 3.61 ms. 200 instead of 260 steps in all loaded launches cost two
+// Steps of a group in a launch without a load: 150 -> 100 object views 4.13 -> 3.99 ms, LiDAR sweeps 2.46 -> 2.36. 200 instead of 260 steps in all loaded launches cost two
 // bounces 1 %, 400 or 600 the object view 9-23 %. Fewer quads without a load (70) suit scenes where a quad is hit by few of a batch's rays (object views 3.43 ms
 // instead of 3.92), but a 200 x 200 patch of a dense scene takes 4.15 ms instead of 3.52, and with the rays' hits as the criterion a 170 x 150 view
 // of a ball 200 us instead of 180.
 #define DST_LOADED_BEAMS 2                 // times as many batches as warps of the launch
 #define DST_LOADED_GROUPS 3
+// A group launch counts the work of at most this many slices, itself included: with more, the others are at other stages when it runs. All slices
+// counted | four, forwards in five and six slices: 560 x 900 and 720 x 1280 views of an object (0.3M surfels) 3.08 | 2.86 and 3.51 | 3.55 ms, secondary rays from its
+// surface 3.20 | 3.01 and 4.70 | 4.41, views of a scene (0.6M) with a reflection 8.41 | 8.34 and 11.12 | 11.04, with two 36.9 | 36.8 and 60.1 | 60.2.
+#define DST_GROUP_LOAD_SLICES 4
 #define DST_BEAM_STEPS 160
 #define DST_BEAM_STEPS_LOADED 240
 #define DST_BEAM_CANDS 200
@@ -929,19 +932,20 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_ray
 }
 
 // the gather launches of a wavefront round (diag: with traversal counters). cnt: the round's entry in the set of round counters;
-// heavy, heavy2: lists of as many rays as the round has slots; slices: launches of other slices this one shares the GPU with, itself included
+// heavy, heavy2: lists of as many rays as the round has slots; slices: slices of the call, this one included
 static inline void launch_gather(bool diag, int grid, int sm_count, int slices, cudaStream_t st, const BvhView& bvh, float4* req, const int* list,
                                  const int* count_ptr, int* cnt, int min_count, unsigned long long* kbuf, int* kcnt, unsigned int* status,
                                  unsigned long long* counters, int* heavy, int* heavy2) {
     constexpr int R = DST_WF_ROUNDS + 2;
     const int direct_max = sm_count * DST_GROUP_MIN_BLOCKS * (ENUM_THREADS / 32), ray_grid = sm_count * DST_GROUP_MIN_BLOCKS;
+    const int group_slices = slices < DST_GROUP_LOAD_SLICES ? slices : DST_GROUP_LOAD_SLICES;
     if (diag) {
         k_enum<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, counters, heavy, cnt + 2 * R, slices);
-        k_enum_group<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, counters, heavy2, cnt + 4 * R, direct_max, slices < 4 ? slices : 4);
+        k_enum_group<true><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, counters, heavy2, cnt + 4 * R, direct_max, group_slices);
         k_enum_ray<true><<<ray_grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, heavy2, cnt + 4 * R, cnt + 5 * R, direct_max, kbuf, kcnt, status, counters);
     } else {
         k_enum<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, list, count_ptr, cnt + R, min_count, kbuf, kcnt, status, nullptr, heavy, cnt + 2 * R, slices);
-        k_enum_group<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, nullptr, heavy2, cnt + 4 * R, direct_max, slices < 4 ? slices : 4);
+        k_enum_group<false><<<grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, cnt + 3 * R, kbuf, kcnt, status, nullptr, heavy2, cnt + 4 * R, direct_max, group_slices);
         k_enum_ray<false><<<ray_grid, ENUM_THREADS, 0, st>>>(bvh, req, heavy, cnt + 2 * R, heavy2, cnt + 4 * R, cnt + 5 * R, direct_max, kbuf, kcnt, status, nullptr);
     }
 }
