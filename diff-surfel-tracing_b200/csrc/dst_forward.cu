@@ -684,7 +684,7 @@ __device__ __forceinline__ bool fwd_shade_warp(const FwdParams& p, int slot, War
 
 // Few rays (what the wavefront leaves over, or a small call): one WARP per ray to completion. The warp gathers the chunk together
 // (knearest_warp) and composites it together (fwd_shade_warp): what such a call takes is the serial work of its longest rays.
-// 10 blocks an SM: 40 warps at 48 registers, with spills (784 B of stores, 556 of loads a thread); 8 blocks at 64: a LiDAR sweep rendered 3 % slower, loose
+// 10 blocks an SM: 40 warps at 48 registers, with spills (788 B of stores, 560 of loads a thread); 8 blocks at 64: a LiDAR sweep rendered 3 % slower, loose
 // rays 4 %.
 constexpr int WTAIL_THREADS = 128;
 #ifndef DST_WTAIL_BLOCKS

@@ -413,8 +413,9 @@ struct BeamQ { float oc[3], orad[3], dc[3], drad[3], dsum, dmax; };      // dsum
 
 // Conservative test of one quad against the hull, in interval arithmetic (centre and radius): can ANY ray of the set pass ray_quad() with a hit no
 // farther than kmaxb? The steps are those of ray_quad(): t = n.(p0 - o) / n.d, h = t d - (p0 - o), u = wu.h, v = wv.h,
-// accepted iff 0 <= t <= kmax and u, v in [0, 1]. Every interval is widened by margins orders of magnitude above the
-// rounding of either computation, so a quad some ray hits is never rejected. For neighbouring rays (close origins, directions a
+// accepted iff 0 <= t <= kmax and u, v in [0, 1]. Every interval is widened by more than the rounding of either computation, so a quad some ray hits is
+// never rejected: by an order of magnitude more in what grows with the quad's distance from the hull's origin, the distance to the hit and the
+// direction, by 1.6 times as much in what grows with how far the rays have been moved (in orad, see make_beam()). For neighbouring rays (close origins, directions a
 // degree apart) the intervals are narrow, and nearly every quad that no ray hits is rejected here by ONE lane. tl: nearest possible hit.
 __device__ __forceinline__ bool hull_quad(const BeamQ& bm, const float4 qa, const float4 qb, const float4 qc, float kmaxb, float& tl) {
     const float p0[3] = { qa.x, qa.y, qa.z }, nn[3] = { qa.w, qb.x, qb.y }, wu[3] = { qb.z, qb.w, qc.x }, wv[3] = { qc.y, qc.z, qc.w };
@@ -483,9 +484,6 @@ struct WalkStack : WalkMemBase {
 };
 typedef WalkStack<DST_WALK_STACK> WalkMem;           // walks of one ray, which have to end
 typedef WalkStack<DST_BEAM_STACK> BeamMem;           // walks of a hull, which may be given up
-
-// distance k from the start of a ray's enumeration, from the start of the hull (k < 0: none)
-__device__ __forceinline__ float from_hull(float rel, float k) { return k < 0.0f ? k : (1.0f + 1e-6f) * (rel + k); }
 
 // Walks the hierarchy for the hull in m.beam / m.slab: a step takes up to 8 nodes from the top of the stack and tests their 32
 // child boxes, one per lane. Single quads whose box passes go to a queue; whenever it holds 32 of them (or no node is
@@ -586,44 +584,58 @@ __device__ __forceinline__ HullStart hull_start(bool active, const EnumReq& q) {
     return s;
 }
 
-// Hull of the rays of the lanes with `active` (at least one), whose origins lie in the box [olo, ohi], into m.beam and m.slab. moved: largest distance the origins
-// have been moved along their rays (they, and those the exact tests use, are off the rays by the rounding of that). ONE: a single ray, the same in all
-// lanes, whose quads no hull test sees.
-template <bool ONE = false>
-__device__ __forceinline__ void make_beam(WalkMemBase& m, bool active, const float* olo, const float* ohi, float dx, float dy, float dz, float moved, float absmax) {
+// distance k from the start of a ray's enumeration, from the start of the hull (k < 0: none)
+__device__ __forceinline__ float from_hull(float rel, float k) { return k < 0.0f ? k : (1.0f + 1e-6f) * (rel + k); }
+
+// Slab constants of one axis for origins in [ol, oh] and directions in [dl, dh]; pad: padding of the boxes.
+__device__ __forceinline__ void make_slab(BeamSlab& slab, int a, float ol, float oh, float dl, float dh, float pad) {
+    const float lo = ol - pad, hi = oh + pad;
+    const float ip = 1.0f / fmaxf(dh, 1e-30f), in = 1.0f / fmaxf(-dl, 1e-30f);
+    const float xp = dl > 1e-20f ? 1.0f / dl : 0.0f, xn = dh < -1e-20f ? 1.0f / dh : 0.0f;
+    const float f_in_lo = ip, o_in_lo = -hi * ip, f_in_hi = -in, o_in_hi = lo * in;
+    const float f_out_lo = xn, o_out_lo = xn != 0.0f ? -hi * xn : 3e38f, f_out_hi = xp, o_out_hi = xp != 0.0f ? -lo * xp : 3e38f;
+    if (a < 2) {
+        (&slab.in_lo.x)[a] = f_in_lo; (&slab.in_lo.z)[a] = o_in_lo; (&slab.in_hi.x)[a] = f_in_hi; (&slab.in_hi.z)[a] = o_in_hi;
+        (&slab.out_lo.x)[a] = f_out_lo; (&slab.out_lo.z)[a] = o_out_lo; (&slab.out_hi.x)[a] = f_out_hi; (&slab.out_hi.z)[a] = o_out_hi;
+    } else {
+        slab.in_z = make_float4(f_in_lo, f_in_hi, o_in_lo, o_in_hi);
+        slab.out_z = make_float4(f_out_lo, f_out_hi, o_out_lo, o_out_hi);
+    }
+}
+
+// The slabs of a single ray, the same in all lanes: its quads are tested exactly, no hull test sees them.
+__device__ __forceinline__ void make_ray(WalkMemBase& m, float ox, float oy, float oz, float dx, float dy, float dz, float absmax) {
+    const int a = threadIdx.x & 31;
+    const float om = fmaxf(fabsf(ox), fmaxf(fabsf(oy), fabsf(oz)));
+    if (a < 3) {
+        const float o = a == 0 ? ox : a == 1 ? oy : oz, d = a == 0 ? dx : a == 1 ? dy : dz;
+        make_slab(m.slab, a, o, o, d, d, DST_PAD_FACTOR * (om + absmax) + 1e-30f);
+    }
+    __syncwarp();
+}
+
+// Hull of the rays of the lanes with `active` (at least one), into m.beam and m.slab.
+// The origins the exact tests use and the box's corners are off the rays by the rounding of moving them along. With u = 2^-24, per axis, D = off |d| and
+// S = |corner| of a ray, D + S <= om: the exact origin is off by u (D + |D + S|) at most, the corner by u S; the steps of ray_quad() see the distance
+// between the two once more, in p0 - o (u D) and in n.(p0 - o) (3 u D). Together 6 u D + 2 u S <= 6 u om = 3.6e-7 om, and the radius takes 6e-7 om.
+__device__ __forceinline__ void make_beam(WalkMemBase& m, bool active, const HullStart& hs, float dx, float dy, float dz, float absmax) {
     const int lane = threadIdx.x & 31;
     const float d3[3] = { dx, dy, dz };
     float dlo[3], dhi[3], om = 0.0f;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        if (ONE) { dlo[a] = dhi[a] = d3[a]; }
-        else { dlo[a] = redux_min(active ? d3[a] : INFINITY); dhi[a] = redux_max(active ? d3[a] : -INFINITY); }
-        om = fmaxf(om, fmaf(moved, fmaxf(fabsf(dlo[a]), fabsf(dhi[a])), fmaxf(fabsf(olo[a]), fabsf(ohi[a]))));
+        dlo[a] = redux_min(active ? d3[a] : INFINITY); dhi[a] = redux_max(active ? d3[a] : -INFINITY);
+        om = fmaxf(om, fmaf(hs.moved, fmaxf(fabsf(dlo[a]), fabsf(dhi[a])), fmaxf(fabsf(hs.lo[a]), fabsf(hs.hi[a]))));
     }
     if (lane < 3) {
         const int a = lane;
-        const float ol = a == 0 ? olo[0] : a == 1 ? olo[1] : olo[2], oh = a == 0 ? ohi[0] : a == 1 ? ohi[1] : ohi[2];
+        const float ol = a == 0 ? hs.lo[0] : a == 1 ? hs.lo[1] : hs.lo[2], oh = a == 0 ? hs.hi[0] : a == 1 ? hs.hi[1] : hs.hi[2];
         const float dl = a == 0 ? dlo[0] : a == 1 ? dlo[1] : dlo[2], dh = a == 0 ? dhi[0] : a == 1 ? dhi[1] : dhi[2];
-        if (!ONE) {
-        m.beam.oc[a] = 0.5f * (ol + oh); m.beam.orad[a] = 0.5f * (oh - ol) + 2e-7f * fmaxf(fabsf(ol), fabsf(oh)) + (moved > 0.0f ? 6e-7f * om : 0.0f);      // (the centre is rounded)
+        m.beam.oc[a] = 0.5f * (ol + oh); m.beam.orad[a] = 0.5f * (oh - ol) + 2e-7f * fmaxf(fabsf(ol), fabsf(oh)) + (hs.moved > 0.0f ? 6e-7f * om : 0.0f);      // (the centre is rounded)
         m.beam.dc[a] = 0.5f * (dl + dh); m.beam.drad[a] = 0.5f * (dh - dl) + 2e-7f * fmaxf(fabsf(dl), fabsf(dh));
-        }
-        // box padding as in knearest(), for the ray with the largest coordinates
-        const float pad = DST_PAD_FACTOR * (om + absmax) + 1e-30f;
-        const float lo = ol - pad, hi = oh + pad;
-        const float ip = 1.0f / fmaxf(dh, 1e-30f), in = 1.0f / fmaxf(-dl, 1e-30f);
-        const float xp = dl > 1e-20f ? 1.0f / dl : 0.0f, xn = dh < -1e-20f ? 1.0f / dh : 0.0f;
-        const float f_in_lo = ip, o_in_lo = -hi * ip, f_in_hi = -in, o_in_hi = lo * in;
-        const float f_out_lo = xn, o_out_lo = xn != 0.0f ? -hi * xn : 3e38f, f_out_hi = xp, o_out_hi = xp != 0.0f ? -lo * xp : 3e38f;
-        if (a < 2) {
-            (&m.slab.in_lo.x)[a] = f_in_lo; (&m.slab.in_lo.z)[a] = o_in_lo; (&m.slab.in_hi.x)[a] = f_in_hi; (&m.slab.in_hi.z)[a] = o_in_hi;
-            (&m.slab.out_lo.x)[a] = f_out_lo; (&m.slab.out_lo.z)[a] = o_out_lo; (&m.slab.out_hi.x)[a] = f_out_hi; (&m.slab.out_hi.z)[a] = o_out_hi;
-        } else {
-            m.slab.in_z = make_float4(f_in_lo, f_in_hi, o_in_lo, o_in_hi);
-            m.slab.out_z = make_float4(f_out_lo, f_out_hi, o_out_lo, o_out_hi);
-        }
+        make_slab(m.slab, a, ol, oh, dl, dh, DST_PAD_FACTOR * (om + absmax) + 1e-30f);      // padding as in knearest(), for the ray with the largest coordinates
     }
-    if (!ONE && lane == 0) {
+    if (lane == 0) {
         const float a0 = fmaxf(fabsf(dlo[0]), fabsf(dhi[0])), a1 = fmaxf(fabsf(dlo[1]), fabsf(dhi[1])), a2 = fmaxf(fabsf(dlo[2]), fabsf(dhi[2]));
         m.beam.dsum = a0 + a1 + a2; m.beam.dmax = fmaxf(a0, fmaxf(a1, a2));
     }
@@ -677,7 +689,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_ENUM_MIN_BLOCKS) k_enum(BvhV
             bool done = 2 * __popc(__ballot_sync(FULL, wide)) <= __popc(am);
             if (done) {
             const HullStart hs = hull_start(active, q);
-            make_beam(m, active, hs.lo, hs.hi, dx, dy, dz, hs.moved, absmax);
+            make_beam(m, active, hs, dx, dy, dz, absmax);
             const float rel = hs.rel;
             float krun = redux_max(from_hull(rel, kmax));
             int cands = 0;
@@ -785,8 +797,7 @@ __device__ __forceinline__ int knearest_warp(const BvhView& bvh, float ox, float
     mykey = ~0ull;
     if (bvh.P <= 0) return 0;
     if (!(fabsf(ox) < INFINITY && fabsf(oy) < INFINITY && fabsf(oz) < INFINITY && fabsf(dx) < INFINITY && fabsf(dy) < INFINITY && fabsf(dz) < INFINITY)) return 0;
-    const float o3[3] = { ox, oy, oz };
-    make_beam<true>(m, true, o3, o3, dx, dy, dz, 0.0f, absmax);
+    make_ray(m, ox, oy, oz, dx, dy, dz, absmax);
     float krun = kmax0;
     const bool done = beam_walk<COUNT>(bvh, m, krun, DST_WALK_STEP_LIMIT, status, tc, [&](bool valid, int pos) {
         bool hit = false;
@@ -845,7 +856,7 @@ __global__ void __launch_bounds__(ENUM_THREADS, DST_GROUP_MIN_BLOCKS) k_enum_gro
             srays[w][lane][0] = make_float4(x, y, z, q.dx); srays[w][lane][1] = make_float4(q.dy, q.dz, q.kmax0, hs.rel);
         }
         for (int k = lane; k < DST_GROUP * DST_CHUNK; k += 32) (&skeys[w][0][0])[k] = ~0ull;
-        make_beam(m, slot >= 0, hs.lo, hs.hi, q.dx, q.dy, q.dz, hs.moved, absmax);
+        make_beam(m, slot >= 0, hs, q.dx, q.dy, q.dz, absmax);
         float krun = redux_max(from_hull(hs.rel, q.kmax0));
         const bool done = beam_walk<COUNT>(bvh, m, krun, max_steps, status, tc, [&](bool valid, int pos) {
             Quad q;
