@@ -554,12 +554,13 @@ __device__ __forceinline__ float redux_max(float v) { float r; asm("redux.sync.m
 // they have reached is that much longer than it is wide, in a box with sides along the axes wide too. So such rays are taken back to the distance the least
 // advanced of them has reached, and each searches `rel` further than from where its enumeration starts (rounded up). Where the box of the points reached
 // is the narrower one (rays that started at distances of their own towards the same surface, directions of different length) the hull starts at those.
-// Hulls of the points reached -> of the lines: 0.93M rays of a reflective scene 15.1 -> 10.7 ms (k_enum_group 8.2 -> 3.7: rays k_enum and k_enum_group
-// gave up before), four LiDAR sweeps 2.91 -> 2.46, two 400 x 400 object views 4.50 -> 4.13; 2M rays with one or two bounces, whose hulls are as wide as
-// their directions fan out either way, 30.8 -> 30.5 and 114.4 -> 114.5. Hulls of whole segments (back to distance 0) lose 2 % there.
+// Hulls of the points reached -> of the lines, by themselves: 0.93M rays of a reflective scene 15.1 -> 10.7 ms (reflective-render of perf/cases.py, seed 5;
+// k_enum_group 8.2 -> 3.7, now 3.2 with the limits above: rays k_enum and k_enum_group gave up before), four LiDAR sweeps 2.91 -> 2.46, two 400 x 400
+// object views 4.50 -> 4.13; 2M rays with one or two bounces, whose hulls are as wide as their directions fan out either way, 30.8 -> 30.5 and 114.4 -> 114.5. Hulls of whole segments (back to distance 0) lose 2 % there.
 // 560 x 900 views of 0.3M surfels on an object, lines for all | the narrower: starts jittered along the rays 12.0 | 8.2 ms, directions of 0.8 to 1 units
 // 7.7 | 5.6 (of 0.6M surfels and a reflection 17.4 | 12.5); views from one place with directions of one length as they were (within 0.3 %).
-// Asking for 0.7 or 0.4 of the lines' extent gains nothing anywhere and costs a reflective scene with such directions 2 and 12 %.
+// Asking for 0.7 or 0.4 of the lines' extent gains nothing anywhere and costs a reflective scene with such directions 2 and 12 %; lines of normalised directions
+// walked by length make them as fast as others and all others 1 to 2 % slower.
 struct HullStart { float lo[3], hi[3], rel, moved; };      // box of the origins; moved: largest distance an origin has been moved along its ray
 __device__ __forceinline__ HullStart hull_start(bool active, const EnumReq& q) {
     const float off = fabsf(q.off), first = redux_min(active ? off : INFINITY);
